@@ -32,6 +32,7 @@ SOURCES = {
     "peak.cu": [],
     "schur_tc.cu": [],
     "dense_root.cu": [],
+    "pose_schur.cu": [],
     "refine.cu": [],
     "problem_device.cu": [],
     "problem_build.cpp": ["-x", "cu"],
@@ -44,7 +45,7 @@ SOURCES = {
     "server.cpp": ["-x", "cu"],
     "kernel_timer.cpp": ["-x", "cu"],
 }
-HEADERS = ["internal.h", "device.cuh", "engine.h", "ldlt.h", "server.h", "host_pool.h", "incremental.h", "schur_tc.h", "kernel_timer.h", "dense_root.h", "front_ops.cuh",
+HEADERS = ["internal.h", "device.cuh", "engine.h", "ldlt.h", "server.h", "host_pool.h", "incremental.h", "schur_tc.h", "kernel_timer.h", "dense_root.h", "pose_schur.h", "front_ops.cuh",
            "trig.cuh"]
 
 

@@ -742,7 +742,7 @@ __global__ void KZeroFronts(DeviceView V, const int32_t* tasks) {
   const SupernodeRec S = V.sn[t[0]];
   const int c = t[1] + static_cast<int>(threadIdx.x >> 5);
   const int lane = static_cast<int>(threadIdx.x & 31);
-  if (c >= S.F) {
+  if (c >= S.fcols) {
     return;
   }
   double* col = V.asm_fronts + S.front_off + static_cast<int64_t>(c) * S.F;

@@ -910,6 +910,8 @@ FactorPlan Engine::Plan() {
   P.dense_tasks = dense_tasks_.get();
   P.dense_sync = dense_sync_.get();
   P.dense_inv = dense_inv_.get();
+  P.pose = PoseSchurArgs{pose_tasks_.get(), static_cast<int64_t>(sym_.pose_tasks.size()), pose_fronts_.get(),
+                         pose_mask_.get(), pose_start_.get(), dvec_.get(), pose_parts_.get(), pose_counters_.get()};
   P.solve_withhold = solve_withhold_;
   P.solve_wait_polls = solve_wait_polls_;
   // only the iteration's own factor and solve phases are timed
@@ -1064,6 +1066,15 @@ void Engine::SetSolveFault(int withhold, uint32_t wait_polls) {
 
 void Engine::UploadSolveTasks(cudaStream_t s) {
   zero_tasks_.Upload(sym_.zero_tasks, s);
+  if (!sym_.pose_tasks.empty()) {
+    pose_tasks_.Upload(sym_.pose_tasks, s);
+    pose_fronts_.Upload(sym_.pose_fronts, s);
+    pose_mask_.Upload(sym_.pose_mask, s);
+    pose_start_.Upload(sym_.pose_start, s);
+    pose_parts_.Alloc(PoseSchurDoubles(sym_.pose_slots));
+    pose_counters_.Alloc(static_cast<size_t>(std::max(sym_.pose_counters, 1)));
+    CudaCheck(cudaMemsetAsync(pose_counters_.get(), 0, pose_counters_.size() * sizeof(int32_t), s), "pose counters");
+  }
   dense_tasks_.Upload(sym_.dense_tasks, s);
   dense_sync_.Alloc(DenseSyncWords(sym_));
   dense_inv_.Alloc(static_cast<size_t>(std::max<int64_t>(1, sym_.dense_inv_doubles)));

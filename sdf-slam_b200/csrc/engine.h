@@ -13,6 +13,7 @@
 
 #include "device.cuh"
 #include "internal.h"
+#include "pose_schur.h"
 #include "schur_tc.h"
 
 namespace sdfgpu {
@@ -179,6 +180,8 @@ struct FactorPlan {
   const int32_t* dense_tasks{nullptr};
   int32_t* dense_sync{nullptr};
   double* dense_inv{nullptr};
+  /// Pose Schur complement (count 0: no pose rows below any front).
+  PoseSchurArgs pose{};
   /// Test hook of the one-launch solve: a supernode whose forward flag is
   /// never published (-1: none) and the polls a wait may take (0: the
   /// default of about a second).
@@ -500,6 +503,10 @@ class Engine {
   DevBuf<int32_t> ea_tasks_, ea_child_, panel_tasks_, update_tasks_, small_tasks_;
   DevBuf<double> fronts_, upd_;
   DevBuf<int32_t> dense_tasks_, dense_sync_;  // tiled dense roots
+  DevBuf<PoseTask> pose_tasks_;               // pose Schur complement
+  DevBuf<int32_t> pose_fronts_, pose_start_, pose_counters_;
+  DevBuf<uint64_t> pose_mask_;
+  DevBuf<double> pose_parts_;
   DevBuf<int32_t> zero_tasks_;                // lower-triangle clearing of the fronts
   DevBuf<double> dense_inv_;
   DevBuf<uint32_t> solve_sync_;  // counter and flags of the one-launch solve

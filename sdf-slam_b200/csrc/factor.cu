@@ -1084,6 +1084,7 @@ __device__ __forceinline__ void SchurEpilogue(const DeviceView& V, const Superno
                                               int c0, const double (&acc)[4][4]) {
   const int k = S.ncols;
   const int F = S.F;
+  const int fc = S.fcols;
   const int tx = threadIdx.x & 15;
   const int ty = threadIdx.x >> 4;
   const bool scatter = S.parent >= 0;
@@ -1099,7 +1100,7 @@ __device__ __forceinline__ void SchurEpilogue(const DeviceView& V, const Superno
 #pragma unroll
     for (int a = 0; a < 4; ++a) {
       const int r = r0 + tx + 16 * a;
-      const bool in = c < F && r < F && r >= c;
+      const bool in = c < fc && r < F && r >= c;
       cur[a] = (kLoadC && in) ? Fs[static_cast<int64_t>(c) * F + r] : 0.0;
       pos[a] = !in ? -1
                    : (scatter ? static_cast<int64_t>(rel[c - k]) * PF + rel[r - k] : static_cast<int64_t>(c) * F + r);
@@ -1126,7 +1127,7 @@ __device__ __forceinline__ void SchurEpilogue(const DeviceView& V, const Superno
 /// a group before its writes; the same roundings as KUpdate's FP32 tiles.
 template <typename TP>
 __device__ __forceinline__ void SchurEpilogueF32(TP* Fp, int64_t PF, const int32_t* rel, const float* Fs, int k,
-                                                 int F, int r0, int c0, const float (&acc)[4][4]) {
+                                                 int F, int fc, int r0, int c0, const float (&acc)[4][4]) {
   const int tx = threadIdx.x & 15;
   const int ty = threadIdx.x >> 4;
   const bool scatter = rel != nullptr;
@@ -1139,7 +1140,7 @@ __device__ __forceinline__ void SchurEpilogueF32(TP* Fp, int64_t PF, const int32
 #pragma unroll
     for (int a = 0; a < 4; ++a) {
       const int r = r0 + tx + 16 * a;
-      const bool in = c < F && r < F && r >= c;
+      const bool in = c < fc && r < F && r >= c;
       cur[a] = (load && in) ? Fs[static_cast<int64_t>(c) * F + r] : 0.0f;
       pos[a] = !in ? -1
                    : (scatter ? static_cast<int64_t>(rel[c - k]) * PF + rel[r - k] : static_cast<int64_t>(c) * F + r);
@@ -1171,6 +1172,7 @@ __device__ __forceinline__ void SchurTile(const DeviceView& V, const SupernodeRe
   auto Bs = reinterpret_cast<T(*)[kSchurK][64]>(sm + 2 * kSchurK * 64);
   const int k = S.ncols;
   const int F = S.F;
+  const int fc = S.fcols;
   const int r0 = k + t[2] * 64;
   const int c0 = k + t[3] * 64;
   T* Fs = WorkFront<T>(V, S);
@@ -1191,7 +1193,7 @@ __device__ __forceinline__ void SchurTile(const DeviceView& V, const SupernodeRe
       } else {
         As[buf][l][rr] = T(0);
       }
-      if (col < k && c0 + rr < F) {
+      if (col < k && c0 + rr < fc) {
         CpAsync(&Bs[buf][l][rr], Fs + base + c0 + rr);
       } else {
         Bs[buf][l][rr] = T(0);
@@ -1266,14 +1268,14 @@ __device__ __forceinline__ void SchurTile(const DeviceView& V, const SupernodeRe
     // a leaf's C is zero (no child adds into it) and is not loaded
     const float* C = S.child_count > 0 ? Fs : nullptr;
     if (S.parent < 0) {
-      SchurEpilogueF32<float>(Fs, F, nullptr, C, k, F, r0, c0, acc);
+      SchurEpilogueF32<float>(Fs, F, nullptr, C, k, F, fc, r0, c0, acc);
     } else {
       const SupernodeRec P = V.sn[S.parent];
       const int32_t* rel = V.sn_rel + S.rows_off;
       if (Fp32Front(V, P)) {
-        SchurEpilogueF32<float>(WorkFront<float>(V, P), P.F, rel, C, k, F, r0, c0, acc);
+        SchurEpilogueF32<float>(WorkFront<float>(V, P), P.F, rel, C, k, F, fc, r0, c0, acc);
       } else {
-        SchurEpilogueF32<double>(WorkFront<double>(V, P), P.F, rel, C, k, F, r0, c0, acc);
+        SchurEpilogueF32<double>(WorkFront<double>(V, P), P.F, rel, C, k, F, fc, r0, c0, acc);
       }
     }
   }
@@ -2578,6 +2580,19 @@ int LaunchFactorLevels(const Symbolic& S, const DeviceView& V, const FactorPlan&
     CudaCheck(cudaMemsetAsync(P.dense_sync, 0, DenseSyncWords(S) * sizeof(int32_t), stream), "dense sync reset");
   }
   for (int l = 0; l < S.num_levels; ++l) {
+    if (l == S.pose_level && P.pose.count > 0) {
+      // every grid front is factored: their pose rows' products into the pose
+      // roots, the last level
+      const TimedLaunch tl(P.timer, KernelTimer::kUpdateSchur, stream, [&] {
+        double w = 0.0;
+        for (const SupernodeRec& r : S.sn) {
+          const double p = r.F - r.fcols;
+          w += static_cast<double>(r.ncols) * p * (p + 1.0);
+        }
+        return w;
+      });
+      launches += LaunchPoseSchur(V, P.pose, P.fp32_fronts, stream);
+    }
     // the extend-add only for update matrices the tensor cores left in place
     const TaskRange ea = S.ea_range[static_cast<size_t>(l)];
     if (ea.count > 0 && P.tc_map != nullptr) {
@@ -2589,8 +2604,10 @@ int LaunchFactorLevels(const Symbolic& S, const DeviceView& V, const FactorPlan&
         return level_sum(l, [&S](const SupernodeRec& r) {
           double b = 0.0;
           for (int ci = 0; ci < r.child_count; ++ci) {
-            const double m = S.sn[static_cast<size_t>(S.child_list[static_cast<size_t>(r.child_begin + ci)])].nrows;
-            b += 24.0 * m * (m + 1.0) / 2.0;
+            const SupernodeRec& c = S.sn[static_cast<size_t>(S.child_list[static_cast<size_t>(r.child_begin + ci)])];
+            const double m = c.nrows;
+            const double p = c.F - c.fcols;
+            b += 24.0 * (m * (m + 1.0) - p * (p + 1.0)) / 2.0;
           }
           return b;
         });
@@ -2704,7 +2721,8 @@ int LaunchFactorLevels(const Symbolic& S, const DeviceView& V, const FactorPlan&
             const double m = r.nrows;
             const double k = r.ncols;
             pack_bytes += 4.0 * m * k + 4.0 * static_cast<double>(TcPackRows(r.ncols, r.nrows)) * kTcChunk;
-            tc_flops += k * m * (m + 1.0);
+            const double p = r.F - r.fcols;
+            tc_flops += k * (m * (m + 1.0) - p * (p + 1.0));
           }
           return 0.0;
         });
@@ -2724,7 +2742,9 @@ int LaunchFactorLevels(const Symbolic& S, const DeviceView& V, const FactorPlan&
       const TimedLaunch tl(P.timer, KernelTimer::kUpdateSchur, stream, [&] {
         return first ? level_sum(l, [tc](const SupernodeRec& r) {
           const double m = r.nrows;
-          return tc && r.tc_pack >= 0 ? 0.0 : static_cast<double>(r.ncols) * m * (m + 1.0);
+          const double p = r.F - r.fcols;
+          return tc && r.tc_pack >= 0 ? 0.0
+                                       : static_cast<double>(r.ncols) * (m * (m + 1.0) - p * (p + 1.0));
         }) : 0.0;
       });
       KSchur<<<static_cast<unsigned>(sr.count), 256, kSchurSmem, stream>>>(V, P.update_tasks + 4 * sr.begin,

@@ -25,6 +25,14 @@ __device__ __forceinline__ double Recip(double d) {
 }
 __device__ __forceinline__ float Recip(float d) { return 1.0f / d; }
 
+/// c += A B for an 8 x 8 block by one warp on the FP64 tensor cores: lane l
+/// holds A(l / 4, l % 4), B(l % 4, l / 4) and C(l / 4, 2 (l % 4) + {0, 1}).
+__device__ __forceinline__ void Dmma884(double (&c)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+               : "+d"(c[0]), "+d"(c[1])
+               : "d"(a), "d"(b));
+}
+
 /// LDL^T of the w x w (w <= 32) diagonal block at B (row r, column c at
 /// B[r * ld + c], lower triangle) by the block's first four warps (threads
 /// 0..127): lane i owns row i, warp q owns columns 8q..8q+7 in registers. At

@@ -178,6 +178,8 @@ struct SupernodeRec {
   int32_t ncols;      // k: pivots
   int32_t nrows;      // m: rows below the pivot block
   int32_t F;          // k + m
+  int32_t fcols;      // columns stored: k and the update columns below them that are not pose
+                      // variables (F for a root and for fronts without pose rows)
   int32_t child_begin;
   int32_t child_count;
   int32_t parent;     // -1 for a root
@@ -245,6 +247,38 @@ constexpr int kBlockRows = 64;
 constexpr int kSolveWideRows = 512;
 constexpr int kSolveRowChunk = 256;
 constexpr int kSolveRootSplit = 256;
+
+/// One task of the pose Schur complement (KPoseSchur): the part of the pose
+/// root's 64 x 64 tile (I, J), I >= J, that the fronts [q0, q1) of its
+/// instance's list contribute. A tile whose fronts are split into several
+/// parts sums them through workspace slots [slot, slot + parts).
+struct PoseTask {
+  int64_t list;     // first entry of the instance's front list
+  int64_t mask;     // first entry of its (block, front) presence masks
+  int32_t len;      // fronts in the list
+  int32_t root;     // the pose root's supernode
+  int32_t I;
+  int32_t J;
+  int32_t q0;
+  int32_t q1;
+  int32_t part;
+  int32_t parts;
+  int32_t slot;     // first workspace tile of the parts (parts > 1)
+  int32_t counter;  // arrival counter of the parts (parts > 1)
+  int64_t cost;     // relative work, the order tasks are launched in
+};
+/// Pose variables from which an instance's pose Schur complement is summed
+/// straight into its pose root; below, its fronts carry their pose columns up
+/// the tree, which costs no extra launch and fewer serial steps. Measured on
+/// B200, LM iteration through the tree against direct: 27 pose variables 524
+/// against 538 us, 225 equal (1.15 ms), 990 2.73 against 2.48 ms, 2727 7.5
+/// against 6.5 ms.
+constexpr int kPoseDirectCols = 256;
+/// Rows and columns of a pose Schur tile, and the parts one tile is split
+/// into at most (the last part to finish sums all of them: 16 tiles of 32 KB
+/// read by one block take about 3 us).
+constexpr int kPoseTile = 64;
+constexpr int kPoseMaxParts = 16;
 
 /// A contiguous block of work items of one kernel launch in the level
 /// schedule.
@@ -328,6 +362,21 @@ struct Symbolic {
   // complement of a mixed solve, which accumulates into them in place.
   std::vector<int32_t> zero_tasks;
   int64_t zero_main{0};
+  // Pose Schur complement: the pose rows of a grid front update pose columns
+  // only of the pose root, so their products are summed straight into the
+  // root's tiles (KPoseSchur, after the last grid level) and the fronts store
+  // no pose columns. pose_fronts: per instance its fronts with pose rows, in
+  // level order; pose_mask: per instance (64-row block of the root, front)
+  // the root rows of the block that the front has (bit r: row r of the
+  // block); pose_start: the front row (from its pivot block) of the first of
+  // them.
+  std::vector<int32_t> pose_fronts;
+  std::vector<uint64_t> pose_mask;
+  std::vector<int32_t> pose_start;
+  std::vector<PoseTask> pose_tasks;
+  int64_t pose_slots{0};
+  int32_t pose_counters{0};
+  int pose_level{-1};                        // level of the pose roots (-1: none)
   std::vector<int32_t> dense_tasks;
   std::vector<TaskRange> dense_range;
   int64_t dense_cnt_words{0};

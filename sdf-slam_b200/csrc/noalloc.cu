@@ -116,6 +116,7 @@ void DenseLdltSolveNoAlloc(int n, const double* a, const double* b, double* x) {
   rec.ncols = n;
   rec.nrows = 0;
   rec.F = n;
+  rec.fcols = n;
   rec.child_begin = 0;
   rec.child_count = 0;
   rec.parent = -1;

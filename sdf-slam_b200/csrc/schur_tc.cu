@@ -323,6 +323,7 @@ __global__ void __launch_bounds__(128, 1) KSchurTc(const __grid_constant__ CUten
   if (ok && *abort == 0) {
     float* Fs = A.fronts32 + S.front_off;
     const int row = ti * kRowsTile + warp * 32 + lane;
+    const int gc = S.fcols - k;  // update columns the front stores
     const uint32_t taddr = tmem + (static_cast<uint32_t>(warp * 32) << 16);
     // 32 columns per batch: the batch's C values are read before any is
     // written (the compiler cannot prove the columns apart), so the reads
@@ -332,7 +333,7 @@ __global__ void __launch_bounds__(128, 1) KSchurTc(const __grid_constant__ CUten
 #pragma unroll
       for (int j = 0; j < 32; ++j) {
         const int col = tj * kRowsTile + j0 + j;
-        cv[j] = (row < m && col <= row) ? Fs[(k + col) * F + k + row] : 0.0f;
+        cv[j] = (row < m && col <= row && col < gc) ? Fs[(k + col) * F + k + row] : 0.0f;
       }
       uint32_t r[32];
       TmemLoad16(taddr + static_cast<uint32_t>(j0), *reinterpret_cast<uint32_t(*)[16]>(r));
@@ -340,7 +341,7 @@ __global__ void __launch_bounds__(128, 1) KSchurTc(const __grid_constant__ CUten
 #pragma unroll
       for (int j = 0; j < 32; ++j) {
         const int col = tj * kRowsTile + j0 + j;
-        if (row < m && col <= row) {
+        if (row < m && col <= row && col < gc) {
           Fs[(k + col) * F + k + row] = cv[j] - __uint_as_float(r[j]);
         }
       }

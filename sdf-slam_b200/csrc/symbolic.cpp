@@ -247,7 +247,12 @@ inline int LocalIndex(const SupernodeRec& s, const int32_t* rows, int r) {
   return s.ncols + static_cast<int>(it - rows);
 }
 
-void AppendInstance(Symbolic& S, const LocalSym& L, int col_off, int instance, std::vector<int>& height) {
+/// pose_begin: first local column of the pose variables (past every column
+/// when there are none). A front of a grid supernode stores its pivot
+/// columns and its update columns before pose_begin: what its pose rows add
+/// to pose columns goes to the pose root directly.
+void AppendInstance(Symbolic& S, const LocalSym& L, int col_off, int instance, int pose_begin,
+                    std::vector<int>& height) {
   const int S0 = static_cast<int>(S.sn.size());
   const int Sn = static_cast<int>(L.rows.size());
   for (int s = 0; s < Sn; ++s) {
@@ -256,10 +261,14 @@ void AppendInstance(Symbolic& S, const LocalSym& L, int col_off, int instance, s
     r.ncols = L.sn_begin[static_cast<size_t>(s) + 1] - L.sn_begin[static_cast<size_t>(s)];
     r.nrows = static_cast<int>(L.rows[static_cast<size_t>(s)].size());
     r.F = r.ncols + r.nrows;
+    const std::vector<int>& R = L.rows[static_cast<size_t>(s)];
+    r.fcols = L.sn_begin[static_cast<size_t>(s)] >= pose_begin
+                  ? r.F
+                  : r.ncols + static_cast<int>(std::lower_bound(R.begin(), R.end(), pose_begin) - R.begin());
     r.parent = L.parent[static_cast<size_t>(s)] >= 0 ? S0 + L.parent[static_cast<size_t>(s)] : -1;
     r.instance = instance;
     r.rows_off = static_cast<int64_t>(S.sn_rows.size());
-    for (const int row : L.rows[static_cast<size_t>(s)]) {
+    for (const int row : R) {
       S.sn_rows.push_back(col_off + row);
     }
     r.child_begin = static_cast<int>(S.child_list.size());
@@ -268,7 +277,7 @@ void AppendInstance(Symbolic& S, const LocalSym& L, int col_off, int instance, s
       S.child_list.push_back(S0 + c);
     }
     r.front_off = S.front_doubles;
-    const int64_t size = static_cast<int64_t>(r.F) * r.F;
+    const int64_t size = static_cast<int64_t>(r.F) * r.fcols;
     S.front_doubles += (size + 31) / 32 * 32;
     r.upd_off = S.update_doubles;
     S.update_doubles += r.nrows;
@@ -318,10 +327,194 @@ void ComputeRel(Symbolic& S) {
   }
 }
 
+/// Tasks of the pose Schur complement (see Symbolic::pose_fronts). A tile's
+/// fronts are split so that an instance alone fills the GPU about four
+/// times over (two blocks per SM); the split depends on the instance only, so that its sums are
+/// the same alone and in a batch. Measured on B200 (910-pose office, 946
+/// tiles; 331-pose room, 136 tiles): see KPoseSchur.
+void PoseTasks(Symbolic& S) {
+  S.pose_fronts.clear();
+  S.pose_mask.clear();
+  S.pose_start.clear();
+  S.pose_tasks.clear();
+  S.pose_slots = 0;
+  S.pose_counters = 0;
+  if (std::none_of(S.sn.begin(), S.sn.end(), [](const SupernodeRec& r) { return r.fcols < r.F; })) {
+    return;
+  }
+  constexpr int kT = kPoseTile;
+  struct Inst {
+    int root{-1};
+    std::vector<int32_t> fronts;
+    std::vector<uint64_t> mask;
+    std::vector<int32_t> start;
+    std::vector<PoseTask> tasks;
+    int64_t slots{0};
+    int32_t counters{0};
+  };
+  int instances = 0;
+  for (const SupernodeRec& r : S.sn) {
+    instances = std::max(instances, r.instance + 1);
+  }
+  std::vector<Inst> inst(static_cast<size_t>(instances));
+  for (const int32_t s : S.level_sn) {
+    const SupernodeRec& r = S.sn[static_cast<size_t>(s)];
+    Inst& in = inst[static_cast<size_t>(r.instance)];
+    if (r.pose_root != 0) {
+      in.root = s;
+    } else if (r.fcols < r.F) {
+      in.fronts.push_back(s);
+    }
+  }
+  PoolRun(instances, [&](int i) {
+    Inst& in = inst[static_cast<size_t>(i)];
+    if (in.root < 0 || in.fronts.empty()) {
+      return;
+    }
+    const SupernodeRec& root = S.sn[static_cast<size_t>(in.root)];
+    const int nb = (root.ncols + kT - 1) / kT;
+    const size_t len = in.fronts.size();
+    in.mask.assign(len * static_cast<size_t>(nb), 0);
+    in.start.assign(len * static_cast<size_t>(nb), 0);
+    // cost of a pair of blocks: pivots (in stages of 16) times the 16 x 8
+    // products of its packed rows, plus the staging (about a quarter of a
+    // full tile's products)
+    auto pair_cost = [](int k, int na, int nb) {
+      return static_cast<int64_t>((k + 15) / 16) * (((na + 15) / 16) * ((nb + 7) / 8) + 8);
+    };
+    std::vector<std::vector<std::pair<int16_t, int8_t>>> present(len);
+    std::vector<int64_t> cost(static_cast<size_t>(nb) * nb, 0);
+    for (size_t q = 0; q < len; ++q) {
+      const SupernodeRec& r = S.sn[static_cast<size_t>(in.fronts[q])];
+      const int32_t* rows = S.sn_rows.data() + r.rows_off;
+      int last = -1;
+      for (int x = r.fcols - r.ncols; x < r.nrows; ++x) {
+        const int pos = rows[x] - root.first_col;
+        const int b = pos / kT;
+        const size_t e = static_cast<size_t>(b) * len + q;
+        if (b != last) {
+          in.start[e] = x;
+          last = b;
+          present[q].emplace_back(static_cast<int16_t>(b), 0);
+        }
+        in.mask[e] |= uint64_t{1} << (pos % kT);
+      }
+      for (auto& p : present[q]) {
+        p.second = static_cast<int8_t>(__builtin_popcountll(in.mask[static_cast<size_t>(p.first) * len + q]));
+      }
+      for (size_t a = 0; a < present[q].size(); ++a) {
+        for (size_t b = 0; b <= a; ++b) {
+          cost[static_cast<size_t>(present[q][a].first) * nb + present[q][b].first] +=
+              pair_cost(r.ncols, present[q][a].second, present[q][b].second);
+        }
+      }
+    }
+    int64_t total = 0;
+    for (const int64_t c : cost) {
+      total += c;
+    }
+    constexpr int64_t kTargetTasks = 8 * 148;
+    constexpr int64_t kMinCost = 8 * 40;  // 128 pivots of full tiles
+    const int64_t target = std::max(total / kTargetTasks, kMinCost);
+    // open task per tile; a part closes once its share of the cost is reached
+    std::vector<PoseTask> open(static_cast<size_t>(nb) * nb);
+    std::vector<int64_t> sum(static_cast<size_t>(nb) * nb, 0);
+    for (int I = 0; I < nb; ++I) {
+      for (int J = 0; J <= I; ++J) {
+        const size_t t = static_cast<size_t>(I) * nb + J;
+        PoseTask& o = open[t];
+        o = PoseTask{};
+        o.len = static_cast<int32_t>(len);
+        o.root = in.root;
+        o.I = I;
+        o.J = J;
+        o.parts = static_cast<int32_t>(std::clamp<int64_t>((cost[t] + target - 1) / target, 1, kPoseMaxParts));
+        if (o.parts > 1) {
+          o.slot = static_cast<int32_t>(in.slots);
+          o.counter = in.counters++;
+          in.slots += o.parts;
+        }
+      }
+    }
+    for (size_t q = 0; q < len; ++q) {
+      const int k = S.sn[static_cast<size_t>(in.fronts[q])].ncols;
+      for (size_t a = 0; a < present[q].size(); ++a) {
+        for (size_t b = 0; b <= a; ++b) {
+          const size_t t = static_cast<size_t>(present[q][a].first) * nb + present[q][b].first;
+          sum[t] += pair_cost(k, present[q][a].second, present[q][b].second);
+          PoseTask& o = open[t];
+          if (o.part + 1 < o.parts && sum[t] * o.parts >= cost[t] * (o.part + 1)) {
+            o.q1 = static_cast<int32_t>(q) + 1;
+            o.cost = cost[t] / o.parts;
+            in.tasks.push_back(o);
+            o.q0 = o.q1;
+            ++o.part;
+          }
+        }
+      }
+    }
+    for (int I = 0; I < nb; ++I) {
+      for (int J = 0; J <= I; ++J) {
+        const size_t t = static_cast<size_t>(I) * nb + J;
+        if (cost[t] == 0) {
+          continue;
+        }
+        // a front that crossed several shares at once leaves empty parts
+        PoseTask& o = open[t];
+        for (; o.part < o.parts; ++o.part) {
+          o.q1 = static_cast<int32_t>(len);
+          o.cost = cost[t] / o.parts;
+          in.tasks.push_back(o);
+          o.q0 = o.q1;
+        }
+      }
+    }
+  });
+  for (Inst& in : inst) {
+    const auto list = static_cast<int64_t>(S.pose_fronts.size());
+    const auto mask = static_cast<int64_t>(S.pose_mask.size());
+    S.pose_fronts.insert(S.pose_fronts.end(), in.fronts.begin(), in.fronts.end());
+    S.pose_mask.insert(S.pose_mask.end(), in.mask.begin(), in.mask.end());
+    S.pose_start.insert(S.pose_start.end(), in.start.begin(), in.start.end());
+    for (PoseTask& t : in.tasks) {
+      t.list = list;
+      t.mask = mask;
+      t.slot += static_cast<int32_t>(S.pose_slots);
+      t.counter += S.pose_counters;
+      S.pose_tasks.push_back(t);
+    }
+    S.pose_slots += in.slots;
+    S.pose_counters += in.counters;
+  }
+  // the largest first, so that the launch ends on small ones
+  std::stable_sort(S.pose_tasks.begin(), S.pose_tasks.end(),
+                   [](const PoseTask& a, const PoseTask& b) { return a.cost > b.cost; });
+}
+
 /// Level lists and task lists once all supernodes exist.
-void Finalize(Symbolic& S, const std::vector<int>& height, int panel_width, int tile) {
+void Finalize(Symbolic& S, std::vector<int> height, int panel_width, int tile) {
   S.panel_width = panel_width;
   S.tile = tile;
+  // the pose roots of all instances share the last level: the pose Schur
+  // complement, which they wait for, is one launch before it
+  S.pose_level = -1;
+  {
+    int grid = -1;
+    bool roots = false;
+    for (size_t s = 0; s < S.sn.size(); ++s) {
+      if (S.sn[s].pose_root != 0) {
+        roots = true;
+      } else {
+        grid = std::max(grid, height[s]);
+      }
+    }
+    for (size_t s = 0; roots && s < S.sn.size(); ++s) {
+      if (S.sn[s].pose_root != 0) {
+        height[s] = grid + 1;
+      }
+    }
+    S.pose_level = roots ? grid + 1 : -1;
+  }
   S.height = height;
   const int Sn = static_cast<int>(S.sn.size());
   int levels = 0;
@@ -465,7 +658,7 @@ void Finalize(Symbolic& S, const std::vector<int>& height, int panel_width, int 
       for (int q = qb; q < qe; ++q) {
         const SupernodeRec& r = S.sn[static_cast<size_t>(S.level_sn[static_cast<size_t>(q)])];
         if (r.child_count > 0) {
-          tasks += (r.F + kEaCols - 1) / kEaCols;
+          tasks += (r.fcols + kEaCols - 1) / kEaCols;
         }
       }
       if (tasks < 2 * kFillBlocks) {
@@ -487,8 +680,8 @@ void Finalize(Symbolic& S, const std::vector<int>& height, int panel_width, int 
       // per child: the range of its update columns that land in [c, chi);
       // the positions ascend, so one cursor per child walks them once
       cursor.assign(static_cast<size_t>(r.child_count), 0);
-      for (int c = 0; c < r.F; c += cols) {
-        const int chi = std::min(r.F, c + cols);
+      for (int c = 0; c < r.fcols; c += cols) {
+        const int chi = std::min(r.fcols, c + cols);
         if (staged) {
           stage = std::max(stage, (chi - c) * (r.F - c));
         }
@@ -501,7 +694,7 @@ void Finalize(Symbolic& S, const std::vector<int>& height, int panel_width, int 
           const int32_t* rel = S.sn_rel.data() + ch.rows_off;
           int32_t& k = cursor[static_cast<size_t>(ci)];
           S.ea_child.push_back(k);
-          while (k < ch.nrows && rel[k] < chi) {
+          while (k < ch.fcols - ch.ncols && rel[k] < chi) {
             ++k;
           }
           S.ea_child.push_back(k);
@@ -599,7 +792,7 @@ void Finalize(Symbolic& S, const std::vector<int>& height, int panel_width, int 
         any = true;
         const SupernodeRec& r = S.sn[static_cast<size_t>(s)];
         const int m = r.nrows;
-        for (int tj = 0; tj * T < m; ++tj) {
+        for (int tj = 0; tj * T < r.fcols - r.ncols; ++tj) {
           for (int ti = tj; ti * T < m; ++ti) {
             S.update_tasks.push_back(s);
             S.update_tasks.push_back(-1);
@@ -705,7 +898,7 @@ void Finalize(Symbolic& S, const std::vector<int>& height, int panel_width, int 
           S.pack_tasks.push_back(c);
         }
       }
-      for (int tj = 0; tj < nT; ++tj) {
+      for (int tj = 0; tj * kTcTile < r.fcols - r.ncols; ++tj) {
         for (int ti = tj; ti < nT; ++ti) {
           S.tc_tasks.push_back(s);
           S.tc_tasks.push_back(ti);
@@ -724,8 +917,8 @@ void Finalize(Symbolic& S, const std::vector<int>& height, int panel_width, int 
   for (int pass = 0; pass < 2; ++pass) {
     for (int s = 0; s < Sn; ++s) {
       const SupernodeRec& r = S.sn[static_cast<size_t>(s)];
-      const int split = r.child_count == 0 ? r.ncols : r.F;
-      for (int c = 0; c < r.F; c += kZeroCols) {
+      const int split = r.child_count == 0 ? r.ncols : r.fcols;
+      for (int c = 0; c < r.fcols; c += kZeroCols) {
         if ((c < split) == (pass == 0)) {
           S.zero_tasks.push_back(s);
           S.zero_tasks.push_back(c);
@@ -736,6 +929,7 @@ void Finalize(Symbolic& S, const std::vector<int>& height, int panel_width, int 
       S.zero_main = static_cast<int64_t>(S.zero_tasks.size() / 2);
     }
   }
+  PoseTasks(S);
   // tiled dense roots: counters, inverse workspace and task lists per level
   S.dense_tasks.clear();
   S.dense_range.assign(static_cast<size_t>(levels), {});
@@ -1225,7 +1419,7 @@ SymPiece AnalyzeInstance(const HostProblem& hp, int margin, int threads, const s
     }
   };
   const LocalSym L = SupernodalSymbolic(np, lower, sn_begin, subtrees);
-  AppendInstance(S, L, col_off, 0, height);
+  AppendInstance(S, L, col_off, 0, np - A >= kPoseDirectCols ? A : np, height);
   // 4. assembly offsets for this instance: 9 stencil slots per node column
   // and one (node, frame) entry per coupled frame (stored node-major in
   // mp_off and frame-major in fmp_off), looked up in a map from the front's
@@ -1490,7 +1684,7 @@ Symbolic Concatenate(const std::vector<SymPiece>& pieces, const std::vector<Inst
 Symbolic ConcatenateOne(SymPiece&& piece, int panel_width, int tile, const Schedule& sched) {
   // a lone piece is already numbered from column, frame and front 0
   Symbolic S = std::move(piece.s);
-  const std::vector<int> height = std::move(piece.height);
+  std::vector<int> height = std::move(piece.height);
   piece = SymPiece{};
   S.small_pivots = sched.small_pivots;
   S.front_rows = sched.front_rows;
@@ -1499,7 +1693,7 @@ Symbolic ConcatenateOne(SymPiece&& piece, int panel_width, int tile, const Sched
   for (SupernodeRec& r : S.sn) {
     r.instance = 0;
   }
-  Finalize(S, height, panel_width, tile);
+  Finalize(S, std::move(height), panel_width, tile);
   return S;
 }
 
@@ -1618,7 +1812,7 @@ Symbolic AnalyzeGeneral(int n, const int32_t* outer, const int32_t* inner, const
   };
   const LocalSym L = SupernodalSymbolic(n, lower, sn_begin);
   std::vector<int> height;
-  AppendInstance(S, L, 0, 0, height);
+  AppendInstance(S, L, 0, 0, n, height);
   ComputeRel(S);
   value_offsets.assign(static_cast<size_t>(outer[n]), -1);
   for (int j = 0; j < n; ++j) {
