@@ -519,319 +519,114 @@ __global__ void __launch_bounds__(kBlockThreads, 1) KPanelBlock(DeviceView V, co
   }
 }
 
-/// Pivot block of a front with at most kSmallPivots columns, factored in
-/// one block: blocked LDL^T of the k x k pivot block in shared memory (warp 0
-/// factors each 32-wide diagonal block, all threads solve the rows below it
-/// inside the pivot block and apply the rank-32 update), then the rows below
-/// the pivot block, `row_begin` onwards, get L(r, :) = A(r, :) L11^-T D^-1,
-/// panel by panel, in registers. Every block of a front repeats the pivot
-/// factorization; the one with row_begin == k writes L11 (the transposed
-/// storage of the diagonal panel blocks) and D. Shared memory holds the pivot
-/// block padded to a multiple of 32 rows and columns (the padding is zero, so
-/// a narrow last panel needs no per-entry tests in the unrolled loops) and
-/// the reciprocals of the pivots.
+/// Fronts with at most kSmallPivots pivots are factored by one kernel: a block
+/// takes the pivot block and a chunk of the rows below it as one trapezoid in
+/// shared memory and factors it right-looking by 8-column panels (BlockLdlt).
+/// Every block of a front repeats the pivot block; the one with
+/// row_begin == k writes L11 and D.
 constexpr int kSmallPivots = 128;
+constexpr int kFrontThreads = 256;
+/// Rows below the pivot block of one task at most.
+constexpr int kFrontMaxRows = 128;
 
-/// Dynamic shared memory of KFactorFront for fronts of at most k pivots: the
-/// padded pivot block, the pivots' reciprocals and W = L D of one panel for
-/// the trailing update (kPanel rows of kpad + 1).
-__host__ __device__ constexpr size_t FactorFrontSmem(int k) {
-  const size_t kpad = static_cast<size_t>((k + kPanel - 1) / kPanel * kPanel);
-  return (kpad * (kpad + 1) + kpad + static_cast<size_t>(kPanel) * (kpad + 1)) * sizeof(double);
+/// Shared memory of a trapezoid of k pivots and `rows` rows below.
+__host__ __device__ constexpr size_t FactorFrontSmem(int k, int rows) {
+  const int kp = (k + 7) / 8 * 8;
+  return LdltSmemDoubles(kp, kp + (rows + 7) / 8 * 8) * sizeof(double);
 }
 
-/// Rows per block up to which the rows below a pivot block are shared by
-/// eight threads each.
-constexpr int kRowsShared = 32;
-
-/// Rows below the pivot block, eight threads per row (row = tid / 8 of a
-/// pass over blockDim / 8 rows, the thread owning columns 4g..4g+3 of every
-/// panel, g = tid % 8): per panel
-/// the earlier panels' L values of the row (kept in shared memory) are
-/// subtracted, then the panel's triangle is solved with the pivot values
-/// passed between the row's threads by shuffles, then scaled by D^-1. Every
-/// entry sees the same operations in the same order as the thread-per-row
-/// path. Y: rows x (kpad + 1) values in shared memory.
-template <typename T>
-__device__ __forceinline__ void RowsBelowShared(T* Fs, int F, int k, int kpad, int ld, int row_begin, int rows,
-                                                const T* D, const T* dinv, T* Y) {
-  const int tid = threadIdx.x;
-  const int lane = tid & 31;
-  const int g = tid & 7;
-  const int base = lane & ~7;
-  const int ldy = kpad + 1;
-  const int np = (k + kPanel - 1) / kPanel;
-  const int64_t F64 = F;
-  const int per_pass = static_cast<int>(blockDim.x) >> 3;
-  for (int rb = 0; rb < rows; rb += per_pass) {
-    const int ri = rb + (tid >> 3);
-    const int r = row_begin + ri;
-    const bool live = ri < rows && r < F;
-    // the row's assembled values in this thread's columns of every panel
-    T a[kSmallPivots / kPanel][4];
-#pragma unroll
-    for (int p = 0; p < kSmallPivots / kPanel; ++p) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int j = p * kPanel + 4 * g + i;
-        a[p][i] = (live && j < k) ? Fs[j * F64 + r] : T(0);
-      }
-    }
-    T* yrow = Y + (live ? ri : 0) * ldy;
-#pragma unroll
-    for (int p = 0; p < kSmallPivots / kPanel; ++p) {
-      if (p >= np) {
-        break;
-      }
-      const int p0 = p * kPanel;
-      T acc[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        acc[i] = a[p][i];
-      }
-      const T* drow = D + (p0 + 4 * g) * ld;
-      // contributions of the earlier panels
-      for (int q = 0; q < p; ++q) {
-        const int q0 = q * kPanel;
-#pragma unroll 8
-        for (int l = 0; l < kPanel; ++l) {
-          const T yl = yrow[q0 + l] * D[(q0 + l) * ld + q0 + l];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            acc[i] -= yl * drow[i * ld + q0 + l];
-          }
-        }
-      }
-      // this panel's triangle: pivot l's final value comes from its owner
-#pragma unroll
-      for (int l = 0; l < kPanel; ++l) {
-        const T yl = __shfl_sync(0xffffffffu, acc[l & 3], base + (l >> 2));
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          if (4 * g + i > l) {
-            acc[i] -= yl * drow[i * ld + p0 + l];
-          }
-        }
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int j = p0 + 4 * g + i;
-        if (j < k && live) {
-          const T v = acc[i] * dinv[j];
-          yrow[j] = v;
-          Fs[j * F64 + r] = v;
-        }
-      }
-      __syncwarp();
-    }
-  }
-}
-
+/// The trapezoid is held in FP64 whatever the front's element type (FP32
+/// fronts are rounded when they are stored). Bound by the panels' pivot chain
+/// where a level has few fronts, by shared-memory traffic where it fills the
+/// GPU. Measured on B200 against 32-column panels factored by four warps with
+/// one barrier per pivot and rows solved one thread each: all levels of the
+/// 10-pose room 108 -> 55 us, of the 76-pose floor plan 248 -> 116, of the
+/// 910-pose office 810 -> 414, of 32 uneven instances 1032 -> 538; a level of
+/// one 100-pivot front with 225 rows 67 -> 28.
 template <typename T>
 __device__ __forceinline__ void FactorFrontBody(const DeviceView& V, const SupernodeRec& S, int row_begin, int rows,
-                                                double* dvec, T* D, T (*lbuf)[kPanel], T (*wbuf)[kPanel]) {
+                                                double* dvec, double* sm) {
   const int k = S.ncols;
-  const int F = S.F;
-  const int kpad = (k + kPanel - 1) / kPanel * kPanel;
-  const int ld = kpad + 1;
-  T* dinv = D + kpad * ld;
-  T* W = dinv + kpad;  // [kPanel][ld]: W(c, l) = L(c, p0 + l) d_l at W[l * ld + c]
+  const int64_t F = S.F;
+  const int kp = (k + 7) & ~7;
+  const int nr = max(0, min(rows, S.F - row_begin));
+  const int R = kp + ((nr + 7) & ~7);
+  const int pm = LdltPitch(R);
   T* Fs = WorkFront<T>(V, S);
   const int tid = threadIdx.x;
-  const int warp = tid >> 5;
-  const int nwarps = static_cast<int>(blockDim.x >> 5);
   const int lane = tid & 31;
-  const int nthreads = static_cast<int>(blockDim.x);
-  // the pivot block's lower triangle, column by column over all threads
-  // (coalesced), eight loads in flight per thread
-  {
-    const int kk = k * k;
-    for (int base = tid; base < kk; base += 8 * nthreads) {
-      T val[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int i = base + u * nthreads;
-        const int c = i / k;
-        const int r = i - c * k;
-        val[u] = (i < kk && r >= c) ? Fs[static_cast<int64_t>(c) * F + r] : T(0);
-      }
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int i = base + u * nthreads;
-        const int c = i / k;
-        const int r = i - c * k;
-        if (i < kk && r >= c) {
-          D[r * ld + c] = val[u];
-        }
+  const int warp = tid >> 5;
+  // column by column, a warp each: the pivot block's lower triangle, then the
+  // chunk's rows; zero elsewhere, the identity on the padding pivots
+  for (int c = warp; c < kp; c += kFrontThreads / 32) {
+    const T* col = Fs + c * F;
+    double* M = sm + c * pm;
+    for (int r = lane; r < R; r += 32) {
+      const int below = r - kp;
+      const bool in = c < k && (r < kp ? r >= c && r < k : below < nr);
+      const T* src = col + (r < kp ? r : row_begin + below);
+      if (in) {
+        LoadElement(M + r, src);
+      } else {
+        M[r] = r == c ? 1.0 : 0.0;
       }
     }
   }
-  for (int idx = k * ld + tid; idx < kpad * ld; idx += blockDim.x) {
-    D[idx] = T(0);
-  }
+  WaitElements();
   __syncthreads();
-  bool zero_pivot = false;
-  for (int p0 = 0; p0 < k; p0 += kPanel) {
-    const int w = min(kPanel, k - p0);
-    if (warp < 4) {
-      zero_pivot = DiagonalBlockLdlt<T>(D + p0 * ld + p0, ld, w, lbuf, wbuf) || zero_pivot;
-      if (tid < w) {
-        dinv[p0 + tid] = Recip(D[(p0 + tid) * ld + p0 + tid]);
-      }
-    }
-    __syncthreads();
-    // rows of the pivot block below this diagonal block (registers; the
-    // panel is full width here because a later row exists)
-    for (int r = p0 + w + tid; r < k; r += blockDim.x) {
-      T* row = D + r * ld + p0;
-      T y[kPanel];
+  const bool first = row_begin == k;
+  // L11 goes transposed into the pivot block's upper triangle: the other
+  // tasks of this front may still be reading its lower triangle (the
+  // assembled A11)
+  const bool zero = BlockLdlt<kFrontThreads>(
+      sm, pm, kp, R,
+      [&](int r, int p0, const double(&l)[8]) {
+        if (r >= kp) {
+          const int below = r - kp;
+          if (below < nr) {
+            T* dst = Fs + p0 * F + row_begin + below;
 #pragma unroll
-      for (int j = 0; j < kPanel; ++j) {
-        y[j] = row[j];
-      }
+            for (int t = 0; t < 8; ++t) {
+              if (p0 + t < k) {
+                dst[t * F] = static_cast<T>(l[t]);
+              }
+            }
+          }
+        } else if (first && r < k) {
+          T* dst = Fs + r * F + p0;
 #pragma unroll
-      for (int j = 1; j < kPanel; ++j) {
-#pragma unroll
-        for (int l = 0; l < j; ++l) {
-          y[j] -= y[l] * D[(p0 + j) * ld + p0 + l];
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < kPanel; ++j) {
-        row[j] = y[j] * dinv[p0 + j];
-      }
-    }
-    __syncthreads();
-    // rank-w update of the trailing pivot block (the panel is full width
-    // here because a trailing column exists): W = L(:, panel) D first, then
-    // one item per (4-row block, column) over all threads, rows read as
-    // broadcasts and W along the columns; even and odd l accumulate
-    // separately, as two chains per entry
-    const int t0 = p0 + w;
-    const int nt = k - t0;
-    if (nt > 0) {
-      for (int idx = tid; idx < kPanel * nt; idx += nthreads) {
-        const int l = idx / nt;
-        const int ci = idx - l * nt;
-        W[l * ld + ci] = D[(t0 + ci) * ld + p0 + l] * D[(p0 + l) * ld + p0 + l];
-      }
-      __syncthreads();
-      const int nrb = (nt + 3) / 4;
-      for (int idx = tid; idx < nrb * nt; idx += nthreads) {
-        const int rb = idx / nt;
-        const int ci = idx - rb * nt;
-        if (4 * rb + 3 < ci) {
-          continue;  // the four rows lie above the diagonal
-        }
-        T a0[4];
-        T a1[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          a0[u] = T(0);
-          a1[u] = T(0);
-        }
-        const T* l0 = D + (t0 + 4 * rb) * ld + p0;
-#pragma unroll
-        for (int l = 0; l < kPanel; l += 2) {
-          const T w0 = W[l * ld + ci];
-          const T w1 = W[(l + 1) * ld + ci];
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            a0[u] = fma(l0[u * ld + l], w0, a0[u]);
-            a1[u] = fma(l0[u * ld + l + 1], w1, a1[u]);
+          for (int t = 0; t < 8; ++t) {
+            dst[t] = static_cast<T>(l[t]);
           }
         }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int r = 4 * rb + u;
-          if (r < nt && r >= ci) {
-            D[(t0 + r) * ld + t0 + ci] -= a0[u] + a1[u];
+      },
+      [&](int p0, const double* diag, int lane_) {
+        const int i = lane_ >> 2;
+        if (first && p0 + i < k) {
+          for (int t = lane_ & 3; t < i; t += 4) {
+            Fs[(p0 + i) * F + p0 + t] = static_cast<T>(diag[8 * i + t]);
+          }
+          if ((lane_ & 3) == 0) {
+            dvec[S.first_col + p0 + i] = diag[72 + i];
           }
         }
-      }
-    }
-    __syncthreads();
-  }
-  if (row_begin == k) {
-    // L11 goes to the pivot block's upper triangle only: the other tasks of
-    // this front may still be reading its lower triangle (the assembled A11)
-    for (int r = warp; r < k; r += nwarps) {
-      T* dst = Fs + static_cast<int64_t>(r) * F;
-      for (int c = lane; c < r; c += 32) {
-        dst[c] = D[r * ld + c];
-      }
-    }
-    for (int j = tid; j < k; j += blockDim.x) {
-      dvec[S.first_col + j] = static_cast<double>(D[j * ld + j]);
-    }
-    if (tid == 0 && zero_pivot) {
-      atomicOr(V.status + S.instance, kStatusZeroPivot);
-    }
-  }
-  if (rows <= kRowsShared && k <= kSmallPivots) {
-    RowsBelowShared<T>(Fs, F, k, kpad, ld, row_begin, rows, D, dinv, W);
-    return;
-  }
-  // rows below the pivot block: thread per row, panel by panel
-  const int r = row_begin + tid;
-  if (r >= F || tid >= rows) {
-    return;
-  }
-  for (int p0 = 0; p0 < k; p0 += kPanel) {
-    const int w = min(kPanel, k - p0);
-    T y[kPanel];
-#pragma unroll
-    for (int j = 0; j < kPanel; ++j) {
-      y[j] = j < w ? Fs[static_cast<int64_t>(p0 + j) * F + r] : T(0);
-    }
-    // contributions of the earlier panels (each panel's 32 values of this
-    // row loaded together, then 32 x 32 multiply-adds)
-    for (int q0 = 0; q0 < p0; q0 += kPanel) {
-      T yq[kPanel];
-#pragma unroll
-      for (int l = 0; l < kPanel; ++l) {
-        yq[l] = Fs[static_cast<int64_t>(q0 + l) * F + r];
-      }
-#pragma unroll
-      for (int l = 0; l < kPanel; ++l) {
-        const T yl = yq[l] * D[(q0 + l) * ld + q0 + l];
-#pragma unroll
-        for (int j = 0; j < kPanel; ++j) {
-          // rows p0 + j >= k (a narrow last panel) are the zero padding
-          y[j] -= yl * D[(p0 + j) * ld + q0 + l];
-        }
-      }
-    }
-    // this panel's triangle (padding rows leave y[j >= w] unchanged)
-#pragma unroll
-    for (int j = 1; j < kPanel; ++j) {
-#pragma unroll
-      for (int l = 0; l < j; ++l) {
-        y[j] -= y[l] * D[(p0 + j) * ld + p0 + l];
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < kPanel; ++j) {
-      if (j < w) {
-        Fs[static_cast<int64_t>(p0 + j) * F + r] = y[j] * dinv[p0 + j];
-      }
-    }
+      });
+  if (first && zero) {
+    atomicOr(V.status + S.instance, kStatusZeroPivot);
   }
 }
 
-__global__ void __launch_bounds__(256) KFactorFront(DeviceView V, const int32_t* tasks, double* dvec) {
-  extern __shared__ double sm[];
+__global__ void __launch_bounds__(kFrontThreads, 2) KFactorFront(DeviceView V, const int32_t* tasks, double* dvec) {
+  extern __shared__ __align__(16) double front_sm[];
   const int32_t* t = tasks + 3 * static_cast<int64_t>(blockIdx.x);
   const SupernodeRec S = V.sn[t[0]];
   if (V.active[S.instance] == 0) {
     return;
   }
-  __shared__ double lw[4][kPanel];
   if (Fp32Front(V, S)) {
-    auto* l = reinterpret_cast<float(*)[kPanel]>(&lw[0][0]);
-    FactorFrontBody<float>(V, S, t[1], t[2], dvec, reinterpret_cast<float*>(sm), l, l + 2);
+    FactorFrontBody<float>(V, S, t[1], t[2], dvec, front_sm);
   } else {
-    FactorFrontBody<double>(V, S, t[1], t[2], dvec, sm, lw, lw + 2);
+    FactorFrontBody<double>(V, S, t[1], t[2], dvec, front_sm);
   }
 }
 
@@ -2506,6 +2301,8 @@ static_assert(kInvBlock == kInvBlockDoubles, "inverted block size");
 /// Dynamic shared memory a block may use on B200.
 constexpr int kMaxSmem = 227 * 1024;
 
+int64_t FrontTaskSmem(int k, int rows) { return static_cast<int64_t>(FactorFrontSmem(k, rows)); }
+
 void ConfigureSolveKernels(int max_front) {
   // The attribute belongs to the kernel, not to an engine: it only grows, so
   // an engine with smaller fronts never lowers another engine's limit.
@@ -2515,8 +2312,7 @@ void ConfigureSolveKernels(int max_front) {
   {
     std::lock_guard<std::mutex> lk(mu);
     if (!front_configured) {
-      const int bytes = static_cast<int>(FactorFrontSmem(kSmallPivots));
-      CudaCheck(cudaFuncSetAttribute(KFactorFront, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes), "smem attr");
+      CudaCheck(cudaFuncSetAttribute(KFactorFront, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem), "smem attr");
       CudaCheck(cudaFuncSetAttribute(KExtendAdd, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      kEaStageDoubles * static_cast<int>(sizeof(double))),
                 "smem attr");
@@ -2618,15 +2414,14 @@ int LaunchFactorLevels(const Symbolic& S, const DeviceView& V, const FactorPlan&
     }
     const TaskRange sm = S.small_range[static_cast<size_t>(l)];
     if (sm.count > 0) {
-      const int kmax = S.small_max_k[static_cast<size_t>(l)];
-      const size_t bytes = FactorFrontSmem(kmax);
+      const size_t bytes = static_cast<size_t>(S.small_smem[static_cast<size_t>(l)]);
       const TimedLaunch tl(P.timer, KernelTimer::kFactorFront, stream, [&] {
         return level_sum(l, [&S](const SupernodeRec& r) {
           const double k = r.ncols;
           return r.ncols <= S.small_pivots ? 2.0 * k * k * k / 3.0 + static_cast<double>(r.nrows) * k * k : 0.0;
         });
       });
-      KFactorFront<<<static_cast<unsigned>(sm.count), S.small_threads[static_cast<size_t>(l)], bytes, stream>>>(
+      KFactorFront<<<static_cast<unsigned>(sm.count), kFrontThreads, bytes, stream>>>(
           V, P.small_tasks + 3 * sm.begin, P.dvec);
       ++launches;
     }

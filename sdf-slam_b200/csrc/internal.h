@@ -399,8 +399,7 @@ struct Symbolic {
   std::vector<int32_t> inv_tasks;
   std::vector<int32_t> small_tasks;
   std::vector<TaskRange> small_range;        // per level
-  std::vector<int32_t> small_max_k;          // per level
-  std::vector<int32_t> small_threads;        // per level: threads per single-kernel block
+  std::vector<int64_t> small_smem;           // per level: shared memory of its largest task
   // Assembly offsets of J^T J entries into the front buffer, indexed by the
   // global natural column of a node.
   std::vector<int64_t> mm_off;               // 9 stencil slots per column (-1: stored elsewhere)
@@ -501,6 +500,10 @@ constexpr int kEaStageDoubles = 12288;
 /// fronts (whose children touch a small part of each column) are added in
 /// place.
 constexpr int kEaStageMaxF = 384;
+
+/// Shared memory of a single-kernel factorization task: k pivots, `rows` rows
+/// below them (factor.cu).
+int64_t FrontTaskSmem(int k, int rows);
 
 /// Schedule parameters of the factorization (see Symbolic).
 struct Schedule {

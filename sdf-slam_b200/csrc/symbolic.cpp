@@ -566,52 +566,42 @@ void Finalize(Symbolic& S, std::vector<int> height, int panel_width, int tile) {
   S.level_panels.assign(static_cast<size_t>(levels), 0);
   S.panel_index_base.assign(static_cast<size_t>(levels) + 1, 0);
   S.small_range.assign(static_cast<size_t>(levels), {});
-  S.small_max_k.assign(static_cast<size_t>(levels), 0);
-  S.small_threads.assign(static_cast<size_t>(levels), S.front_rows);
+  S.small_smem.assign(static_cast<size_t>(levels), 0);
   S.small_tasks.clear();
   for (int l = 0; l < levels; ++l) {
     int maxp = 0;
     S.small_range[static_cast<size_t>(l)].begin = static_cast<int64_t>(S.small_tasks.size() / 3);
-    // Rows per single-kernel task: the schedule's front_rows, or fewer where
-    // the level would not fill the GPU (every task repeats the pivot block,
-    // so small chunks shorten the level when SMs would otherwise idle).
-    int chunk = kFrontRows;
-    int threads = kFrontRows;
-    int fronts = 0;
-    for (int q = S.level_begin[static_cast<size_t>(l)]; q < S.level_begin[static_cast<size_t>(l) + 1]; ++q) {
-      fronts += S.sn[static_cast<size_t>(S.level_sn[static_cast<size_t>(q)])].ncols <= small ? 1 : 0;
-    }
-    // more fronts than SMs: blocks of 128 threads (two per SM by registers)
-    // and chunks of 128 rows keep the level in about one wave
-    const bool many = fronts > kFillBlocks && kFrontRows > 128;
-    for (const int cand : {many ? 128 : kFrontRows, 64, 32}) {
-      chunk = cand;
+    // Rows per single-kernel task: up to 128 (the schedule's front_rows
+    // halved), or fewer where the level would not fill the GPU (every task
+    // repeats the pivot block, so small chunks shorten the level when SMs
+    // would otherwise idle) or the trapezoid would not fit in shared memory.
+    int chunk = kFrontRows / 2;
+    for (const int cand : {kFrontRows / 2, 64, 32}) {
+      chunk = std::min(cand, kFrontRows / 2);
       int64_t blocks = 0;
       for (int q = S.level_begin[static_cast<size_t>(l)]; q < S.level_begin[static_cast<size_t>(l) + 1]; ++q) {
         const SupernodeRec& r = S.sn[static_cast<size_t>(S.level_sn[static_cast<size_t>(q)])];
         if (r.ncols <= small) {
-          blocks += std::max(1, (r.nrows + cand - 1) / cand);
+          blocks += std::max(1, (r.nrows + chunk - 1) / chunk);
         }
       }
       if (blocks >= kFillBlocks) {
         break;
       }
     }
-    if (many) {
-      threads = 128;
-    }
-    S.small_threads[static_cast<size_t>(l)] = threads;
     for (int q = S.level_begin[static_cast<size_t>(l)]; q < S.level_begin[static_cast<size_t>(l) + 1]; ++q) {
       const int sid = S.level_sn[static_cast<size_t>(q)];
       const SupernodeRec& r = S.sn[static_cast<size_t>(sid)];
       if (r.ncols <= small) {
-        const int chunks = std::max(1, (r.nrows + chunk - 1) / chunk);
+        const int rows = r.ncols > 96 ? std::min(chunk, 64) : chunk;
+        const int chunks = std::max(1, (r.nrows + rows - 1) / rows);
         for (int ch = 0; ch < chunks; ++ch) {
           S.small_tasks.push_back(sid);
-          S.small_tasks.push_back(r.ncols + ch * chunk);
-          S.small_tasks.push_back(chunk);
+          S.small_tasks.push_back(r.ncols + ch * rows);
+          S.small_tasks.push_back(rows);
         }
-        S.small_max_k[static_cast<size_t>(l)] = std::max(S.small_max_k[static_cast<size_t>(l)], r.ncols);
+        int64_t& smem = S.small_smem[static_cast<size_t>(l)];
+        smem = std::max<int64_t>(smem, FrontTaskSmem(r.ncols, std::min(rows, r.nrows)));
         continue;
       }
       if (!tiled(r)) {
@@ -1712,8 +1702,7 @@ void Reschedule(Symbolic& S, const Schedule& sched) {
   S.panel_range.clear();
   S.update_range.clear();
   S.small_range.clear();
-  S.small_max_k.clear();
-  S.small_threads.clear();
+  S.small_smem.clear();
   S.level_panels.clear();
   S.panel_index_base.clear();
   const std::vector<int> height = S.height;
