@@ -125,17 +125,29 @@ void Release(int dev, void* p) {
   }
 }
 
-void* Take(int dev, size_t cls) {
+/// Requests from this size on also take a cached block up to half again as
+/// large: two problems of one kind need front buffers a few per cent apart,
+/// which can fall on both sides of a class boundary, and mapping a new block
+/// of this size costs the first solve on a new problem up to 100 ms.
+constexpr size_t kFitFrom = size_t{64} << 20;
+
+/// A cached block of class `*cls` (or, for a large one, the smallest that
+/// fits); *cls becomes its class.
+void* Take(int dev, size_t* cls) {
   Cache& c = TheCache();
   const std::lock_guard<std::mutex> lock(c.mu);
-  auto it = c.free_blocks.find({dev, cls});
-  if (it == c.free_blocks.end() || it->second.empty()) {
-    return nullptr;
+  const size_t most = *cls >= kFitFrom ? *cls + *cls / 2 : *cls;
+  for (auto it = c.free_blocks.lower_bound({dev, *cls});
+       it != c.free_blocks.end() && it->first.first == dev && it->first.second <= most; ++it) {
+    if (!it->second.empty()) {
+      void* p = it->second.back().first;
+      it->second.pop_back();
+      *cls = it->first.second;
+      c.cached_bytes[dev] -= *cls;
+      return p;
+    }
   }
-  void* p = it->second.back().first;
-  it->second.pop_back();
-  c.cached_bytes[dev] -= cls;
-  return p;
+  return nullptr;
 }
 
 /// Caches a released block. Over the limit, the blocks of `dev` released
@@ -213,7 +225,7 @@ void* CachedDeviceAlloc(size_t bytes, size_t* got, int* device) {
   if (device != nullptr) {
     *device = dev;
   }
-  if (void* p = Take(dev, cls)) {
+  if (void* p = Take(dev, got)) {
     return p;
   }
   void* p = nullptr;
@@ -257,7 +269,7 @@ void CachedDeviceFree(void* p, size_t cls, int device) { Keep(device, cls, p, kM
 void* CachedHostAlloc(size_t bytes, size_t* got) {
   const size_t cls = SizeClass(bytes);
   *got = cls;
-  if (void* p = Take(-1, cls)) {
+  if (void* p = Take(-1, got)) {
     return p;
   }
   void* p = nullptr;
