@@ -8,15 +8,19 @@
 // the front is cut into 64 x 64 tiles and factored right-looking as a task
 // graph that every block of one launch works through:
 //
-//   FACTOR(k)      LDL^T of diagonal tile k (two 32-column halves), D into
-//                  dvec, L^-1 of the tile into the inverse workspace; for
-//                  k >= 1 it first does
-//                  SOLVE(k, k - 1) and UPDATE(k, k, k - 1) itself (the
-//                  critical path: no hand-over between those three);
-//   SOLVE(i, k)    L(i, k) = A(i, k) L(k, k)^-T D(k)^-1, as a product with
-//                  the stored inverse (i >= k + 2);
+//   FACTOR(k)      LDL^T of diagonal tile k (BlockLdlt), D into dvec; for
+//                  k >= 1 it first does SOLVE(k, k - 1) and
+//                  UPDATE(k, k, k - 1) itself (the critical path: no hand-over
+//                  between those three). Once the tile is published it also
+//                  forms the tile's L^-1 for the triangular solve;
+//   SOLVE(i, k)    L(i, k) = A(i, k) L(k, k)^-T D(k)^-1 by 8-column block
+//                  substitution, every warp on eight rows of its own
+//                  (i >= k + 2);
 //   UPDATE(i,j,k)  A(i, j) -= L(i, k) D(k) L(j, k)^T, j <= i (lower part;
 //                  not (k + 1, k + 1, k)).
+//
+// The products run on the FP64 tensor cores. Bound by the chain of the FACTOR
+// tasks where the root is small, by the updates where it is large.
 //
 // Each tile (i, j) has a counter: the updates applied to it (k of them before
 // step k), plus one once it is factored (i == j) or solved (i > j); FACTOR(k)
@@ -50,16 +54,21 @@ namespace {
 
 constexpr int kDT = kDenseTileCols;
 constexpr int kDThreads = 256;
-constexpr int kDChunk = 32;
-constexpr int kTLd = kDT + 1;
+constexpr int kWarps = kDThreads / 32;
+constexpr int kDLd = kDT + 4;  // pitch of a staged tile (column major): the four columns a
+                               // tensor-core fragment reads at once fall into different banks
+constexpr int kTLd = kDT + 1;  // pitch of the row-major tile of the inverse
 constexpr int kHLd = 33;
-// FACTOR: the tile, L11^-1, A21 L11^-T, L22^-1 (32 x 33 each), 1 / d, the
-// diagonal-block LDL^T's broadcast buffers and a flag
-constexpr int kFactorDoubles = kDT * kTLd + 3 * 32 * kHLd + kDT + 4 * 32 + 2;
-// SOLVE / UPDATE: two 32 x 64 staging buffers
-constexpr int kGemmDoubles = 2 * kDChunk * kDT;
+constexpr int kTileDoubles = kDT * kDLd;
+// Shared memory: a staged tile, then a region for a second tile or FACTOR's
+// trapezoid, then D, 1 / D and the inverses of eight 8 x 8 diagonal blocks.
+// The inverse of a factored tile reuses both (its rows of L in the first, three
+// 32 x 33 blocks in the second).
+constexpr int kRegion2 = 64 * LdltPitch(64) + 8 * LdltPanelPitch(64) + 2 * kLdltDiag;
+static_assert(kRegion2 >= kTileDoubles && kRegion2 >= 3 * 32 * kHLd && kTileDoubles >= kDT * kTLd);
+constexpr int kDiagInv = kWarps * 64;
 constexpr size_t kDenseSmem =
-    static_cast<size_t>(kFactorDoubles > kGemmDoubles ? kFactorDoubles : kGemmDoubles) * sizeof(double);
+    static_cast<size_t>(kTileDoubles + kRegion2 + 2 * kDT + kDiagInv) * sizeof(double);
 
 __device__ __forceinline__ bool WaitTile(const int32_t* word, int32_t expected, const int32_t* abort,
                                          uint32_t limit) {
@@ -72,7 +81,7 @@ __device__ __forceinline__ bool WaitTile(const int32_t* word, int32_t expected, 
     if (*reinterpret_cast<const volatile int32_t*>(abort) != 0) {
       return false;
     }
-    __nanosleep(64);
+    __nanosleep(20);
   }
   return false;
 }
@@ -87,64 +96,134 @@ __device__ __forceinline__ void PublishTile(int32_t* word, int32_t value) {
   asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(word), "r"(value) : "memory");
 }
 
-/// acc[a][b] += sum over l < kw of X(tx + 16 a, l) s_l Y(ty + 16 b, l) with
-/// X(r, l) = X[l * ldx + r] (r < xr, else 0), Y(c, l) = Y[l * ldy + c]
-/// (c < yr, else 0) and s = xscale (1 when null). K in chunks of 32 staged in
-/// shared memory, the next chunk loaded into registers while the current
-/// one is multiplied. Starts and ends with a block barrier.
-__device__ __forceinline__ void TileProduct(const double* X, int64_t ldx, int xr, const double* Y, int64_t ldy,
-                                            int yr, int kw, const double* xscale, double* sm, double acc[4][4]) {
-  double(*As)[kDT] = reinterpret_cast<double(*)[kDT]>(sm);
-  double(*Bs)[kDT] = reinterpret_cast<double(*)[kDT]>(sm + kDChunk * kDT);
-  const int tid = threadIdx.x;
-  const int tx = tid & 15;
-  const int ty = tid >> 4;
-  double ra[8];
-  double rb[8];
-  auto load = [&](int l0) {
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const int e = tid + kDThreads * q;
-      const int l = l0 + (e >> 6);
-      const int r = e & 63;
-      const bool in = l < kw;
-      const double s = (in && xscale != nullptr) ? xscale[l] : 1.0;
-      ra[q] = (in && r < xr) ? X[static_cast<int64_t>(l) * ldx + r] * s : 0.0;
-      rb[q] = (in && r < yr) ? Y[static_cast<int64_t>(l) * ldy + r] : 0.0;
+/// Stages an h x 64 tile at src (column major, ld) into shared memory, rows
+/// from h on as zeros.
+__device__ __forceinline__ void StageTile(double* dst, const double* src, int64_t ld, int h) {
+  const int r = threadIdx.x & (kDT - 1);
+  for (int c = threadIdx.x >> 6; c < kDT; c += kDThreads / kDT) {
+    if (r < h) {
+      LoadElement(dst + c * kDLd + r, src + c * ld + r);
+    } else {
+      dst[c * kDLd + r] = 0.0;
     }
-  };
-  load(0);
-  for (int l0 = 0; l0 < kw; l0 += kDChunk) {
-    __syncthreads();
+  }
+}
+
+/// acc += X S Y^T for 64 x 64 tiles staged column major, S = diag(s): a warp
+/// owns 16 x 32 entries, C(wr + 8 i + lane / 4, wc + 8 j + 2 (lane % 4) + e) in
+/// acc[i][j][e].
+__device__ __forceinline__ void TileProduct(const double* X, const double* Y, const double* s, int wr, int wc,
+                                            double (&acc)[2][4][2]) {
+  const int q = threadIdx.x & 3;
+  const int g = (threadIdx.x & 31) >> 2;
+#pragma unroll 4
+  for (int l = q; l < kDT; l += 4) {
+    const double d = s[l];
+    const double a0 = X[l * kDLd + wr + g] * d;
+    const double a1 = X[l * kDLd + wr + 8 + g] * d;
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const int e = tid + kDThreads * q;
-      As[e >> 6][e & 63] = ra[q];
-      Bs[e >> 6][e & 63] = rb[q];
+    for (int j = 0; j < 4; ++j) {
+      const double b = Y[l * kDLd + wc + 8 * j + g];
+      Dmma884(acc[0][j], a0, b);
+      Dmma884(acc[1][j], a1, b);
     }
-    __syncthreads();
-    if (l0 + kDChunk < kw) {
-      load(l0 + kDChunk);
+  }
+}
+
+/// Stages the unit lower triangle L of factored diagonal tile k (of full
+/// width), D and 1 / D.
+__device__ __forceinline__ void StageFactor(const SupernodeRec& S, const double* Fs, int k, const DenseArgs& A,
+                                            double* L, double* d) {
+  const int64_t F = S.F;
+  const int c0 = k * kDT;
+  const double* dv = A.dvec + S.first_col + c0;
+  // within the 32 x 32 diagonal blocks L is stored transposed in the upper
+  // triangle: threads along the contiguous index
+  const int x = threadIdx.x & 31;
+  for (int y = threadIdx.x >> 5; y < kDT; y += kWarps) {
+    const int b = y & 32;
+    if (b + x < y) {
+      LoadElement(L + (b + x) * kDLd + y, Fs + (c0 + y) * F + c0 + b + x);  // L(y, b + x)
     }
-#pragma unroll 8
-    for (int l = 0; l < kDChunk; ++l) {
-      double av[4];
-      double bv[4];
+    if (y < 32) {
+      LoadElement(L + y * kDLd + 32 + x, Fs + (c0 + y) * F + c0 + 32 + x);  // L(32 + x, y)
+    }
+  }
+  if (threadIdx.x < kDT) {
+    const double v = __ldcg(dv + threadIdx.x);
+    d[threadIdx.x] = v;
+    d[kDT + threadIdx.x] = Recip(v);
+  }
+}
+
+/// W = A L^-T in place for the 64 x 64 tile A staged at X (column major) and
+/// the staged unit lower triangle L, eight rows per warp with no exchange
+/// between warps: per 8-column block p, A_p - sum_{q < p} W_q L_pq^T, then times
+/// L_pp^-T with the inverses of the 8 x 8 diagonal blocks (warp p forms the
+/// p-th in minv). Starts and ends with a block barrier.
+__device__ __forceinline__ void SubstituteRows(double* X, const double* L, double* minv) {
+  const int lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5;
+  const int q = lane & 3;
+  const int g = lane >> 2;
+  __syncthreads();
+  if (lane < 8) {
+    // column `lane` of the inverse of diagonal block `warp`: (i, lane) at
+    // minv[64 * warp + 8 * lane + i]
+    const double* B = L + 8 * warp * kDLd + 8 * warp;
+    double m[8];
 #pragma unroll
-      for (int a = 0; a < 4; ++a) {
-        av[a] = As[l][tx + 16 * a];
-        bv[a] = Bs[l][ty + 16 * a];
+    for (int i = 0; i < 8; ++i) {
+      m[i] = i == lane ? 1.0 : 0.0;
+    }
+#pragma unroll
+    for (int j = 0; j < 7; ++j) {
+#pragma unroll
+      for (int i = j + 1; i < 8; ++i) {
+        m[i] = fma(-B[j * kDLd + i], m[j], m[i]);
       }
+    }
 #pragma unroll
-      for (int a = 0; a < 4; ++a) {
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-          acc[a][b] = fma(av[a], bv[b], acc[a][b]);
-        }
-      }
+    for (int i = 0; i < 8; ++i) {
+      minv[64 * warp + 8 * lane + i] = m[i];
     }
   }
   __syncthreads();
+  double* W = X + 8 * warp;  // the warp's rows
+#pragma unroll 1
+  for (int p = 0; p < 8; ++p) {
+    double c0[2] = {0.0, 0.0};
+    double c1[2] = {0.0, 0.0};
+    const double* Lp = L + 8 * p + g;
+    for (int l = q; l < 8 * p; l += 8) {
+      Dmma884(c0, W[l * kDLd + g], Lp[l * kDLd]);
+      Dmma884(c1, W[(l + 4) * kDLd + g], Lp[(l + 4) * kDLd]);
+    }
+    double* C = W + (8 * p + 2 * q) * kDLd + g;
+    C[0] -= c0[0] + c1[0];
+    C[kDLd] -= c0[1] + c1[1];
+    __syncwarp();
+    // times L_pp^-T: B(k, n) = L_pp^-1(n, k)
+    const double* Mi = minv + 64 * p;
+    double w[2] = {0.0, 0.0};
+    Dmma884(w, W[(8 * p + q) * kDLd + g], Mi[8 * q + g]);
+    Dmma884(w, W[(8 * p + 4 + q) * kDLd + g], Mi[8 * (q + 4) + g]);
+    __syncwarp();
+    C[0] = w[0];
+    C[kDLd] = w[1];
+    __syncwarp();
+  }
+  __syncthreads();
+}
+
+/// L(i, k) = W D^-1 into the front.
+__device__ __forceinline__ void StoreSolved(double* dst, int64_t ld, int h, const double* W, const double* dinv) {
+  const int r = threadIdx.x & (kDT - 1);
+  if (r < h) {
+    for (int c = threadIdx.x >> 6; c < kDT; c += kDThreads / kDT) {
+      dst[c * ld + r] = W[c * kDLd + r] * dinv[c];
+    }
+  }
 }
 
 /// Columns c of M = L^-1 for the unit lower 32 x 32 triangle at T
@@ -193,302 +272,271 @@ __device__ __forceinline__ void Small32(const double* X, int xld, const double* 
   }
 }
 
-/// FACTOR(k) on the tile already in T (shared, row-major, lower triangle,
-/// the identity beyond w): LDL^T as two 32-column halves (the second
-/// updated by the first's L21 D1 L21^T), D into dvec, L into the front and,
-/// when tiles below exist, L^-1 into the inverse workspace.
-__device__ void FactorLoaded(const DeviceView& V, const SupernodeRec& S, int k, int nt, const DenseArgs& A,
-                             double* sm) {
-  const int64_t F = S.F;
-  const int c0 = k * kDT;
-  const int w = min(kDT, S.ncols - c0);
-  double* Fs = V.fronts + S.front_off;
-  double(*T)[kTLd] = reinterpret_cast<double(*)[kTLd]>(sm);
-  double* M1 = sm + kDT * kTLd;  // L11^-1 (zero above the diagonal)
-  double* Y = M1 + 32 * kHLd;    // A21 L11^-T = L21 D1, then L21 L11^-1
-  double* M2 = Y + 32 * kHLd;    // L22^-1
-  double* dinv = M2 + 32 * kHLd;
-  double(*lbuf)[kPanel] = reinterpret_cast<double(*)[kPanel]>(dinv + kDT);
-  double(*wbuf)[kPanel] = lbuf + 2;
-  int* zflag = reinterpret_cast<int*>(dinv + kDT + 4 * kPanel);
+/// L^-1 = [M1 0; -M2 L21 M1  M2] of a factored tile whose L stands row major
+/// in T (the identity beyond w), column major 64 x 64 into the workspace: the
+/// triangular solve's 64-row panels multiply by it. H: three 32 x 33 blocks.
+__device__ void InvertTile(double (*T)[kTLd], double* H, double* Mo) {
+  double* M1 = H;
+  double* Y = M1 + 32 * kHLd;
+  double* M2 = Y + 32 * kHLd;
   const int tid = threadIdx.x;
-  if (tid < 128) {
-    const bool z = DiagonalBlockLdlt<double>(&T[0][0], kTLd, min(32, w), lbuf, wbuf);
-    if (tid == 0) {
-      *zflag = z ? 1 : 0;
-    }
+  if (tid < 32) {
+    InvertUnitLower32(&T[0][0], M1);
+  } else if (tid >= 64 && tid < 96) {
+    InvertUnitLower32(&T[32][32], M2);
   }
   __syncthreads();
-  if (w > 32) {
-    if (tid < 32) {
-      InvertUnitLower32(&T[0][0], M1);
-    } else if (tid < 64) {
-      dinv[tid - 32] = Recip(T[tid - 32][tid - 32]);
-    }
-    __syncthreads();
-    // Y = A21 M1^T
-    Small32(&T[32][0], kTLd, M1, kHLd, [&](int r, int c, double v) { Y[r * kHLd + c] = v; });
-    __syncthreads();
-    // L21 = Y D1^-1 over A21; A22 -= L21 Y^T (lower part)
-    {
-      const int r = tid & 31;
-      const int cb = tid >> 5;
-      double acc[4] = {0.0, 0.0, 0.0, 0.0};
+  const int r = tid & 31;
+  const int cb = tid >> 5;
+  // Y = L21 M1
+  double p[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll 8
-      for (int j = 0; j < 32; ++j) {
-        const double lr = Y[r * kHLd + j] * dinv[j];
+  for (int l = 0; l < 32; ++l) {
+    const double x = T[32 + r][l];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          acc[q] = fma(lr, Y[(cb + 8 * q) * kHLd + j], acc[q]);
-        }
-      }
+    for (int q = 0; q < 4; ++q) {
+      p[q] = fma(x, M1[l * kHLd + cb + 8 * q], p[q]);
+    }
+  }
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int c = cb + 8 * q;
-        T[32 + r][c] = Y[r * kHLd + c] * dinv[c];
-        if (r >= c) {
-          T[32 + r][32 + c] -= acc[q];
-        }
-      }
-    }
-    __syncthreads();
-    if (tid < 128) {
-      const bool z = DiagonalBlockLdlt<double>(&T[32][32], kTLd, w - 32, lbuf, wbuf);
-      if (tid == 0 && z) {
-        *zflag = 1;
-      }
-    }
-    __syncthreads();
+  for (int q = 0; q < 4; ++q) {
+    Y[r * kHLd + cb + 8 * q] = p[q];
   }
-  if (tid < w) {
-    A.dvec[S.first_col + c0 + tid] = T[tid][tid];
-  }
-  // L of the tile into the front
-  for (int e = tid; e < kDT * kDT; e += kDThreads) {
-    const int j = e >> 6;
-    const int i = e & 63;
-    if (i < w && j < i) {
-      if ((i >> 5) == (j >> 5)) {
-        Fs[static_cast<int64_t>(c0 + i) * F + c0 + j] = T[i][j];
-      } else {
-        Fs[static_cast<int64_t>(c0 + j) * F + c0 + i] = T[i][j];
-      }
-    }
-  }
-  if (tid == 0 && *zflag != 0) {
-    atomicOr(V.status + S.instance, kStatusZeroPivot);
-  }
-  {
-    // L^-1 = [M1 0; -M2 L21 M1  M2] of the tile (the identity beyond w),
-    // column major 64 x 64 into the workspace: the SOLVE tasks below the
-    // tile and the solve's 64-row panels multiply by it
-    double* Mo = A.inv + S.dense_inv + static_cast<int64_t>(k) * kDT * kDT;
-    if (w <= 32) {
-      // a narrow last tile: L11^-1 was not needed above
-      if (tid < 32) {
-        InvertUnitLower32(&T[0][0], M1);
-      }
-      __syncthreads();
-    }
-    if (tid < 32) {
-      InvertUnitLower32(&T[32][32], M2);
-    }
-    // P = L21 M1 into Y: P(r, c) = sum_l L21(r, l) M1(l, c), with M1
-    // column c read as a row of its transpose
-    __syncthreads();
-    {
-      const int r = tid & 31;
-      const int cb = tid >> 5;
-      double p[4] = {0.0, 0.0, 0.0, 0.0};
+  __syncthreads();
+  double m[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll 8
-      for (int l = 0; l < 32; ++l) {
-        const double x = T[32 + r][l];
+  for (int l = 0; l < 32; ++l) {
+    const double x = M2[r * kHLd + l];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          p[q] = fma(x, M1[l * kHLd + cb + 8 * q], p[q]);
-        }
-      }
-      __syncthreads();
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        Y[r * kHLd + cb + 8 * q] = p[q];
-      }
+    for (int q = 0; q < 4; ++q) {
+      m[q] = fma(x, Y[l * kHLd + cb + 8 * q], m[q]);
     }
-    __syncthreads();
-    {
-      const int r = tid & 31;
-      const int cb = tid >> 5;
-      double m[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll 8
-      for (int l = 0; l < 32; ++l) {
-        const double x = M2[r * kHLd + l];
+  }
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          m[q] = fma(x, Y[l * kHLd + cb + 8 * q], m[q]);
-        }
-      }
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int c = cb + 8 * q;
-        Mo[static_cast<int64_t>(c) * kDT + 32 + r] = -m[q];
-        Mo[static_cast<int64_t>(c) * kDT + r] = M1[r * kHLd + c];
-        Mo[static_cast<int64_t>(32 + c) * kDT + 32 + r] = M2[r * kHLd + c];
-        Mo[static_cast<int64_t>(32 + c) * kDT + r] = 0.0;
-      }
-    }
+  for (int q = 0; q < 4; ++q) {
+    const int c = cb + 8 * q;
+    Mo[static_cast<int64_t>(c) * kDT + 32 + r] = -m[q];
+    Mo[static_cast<int64_t>(c) * kDT + r] = M1[r * kHLd + c];
+    Mo[static_cast<int64_t>(32 + c) * kDT + 32 + r] = M2[r * kHLd + c];
+    Mo[static_cast<int64_t>(32 + c) * kDT + r] = 0.0;
   }
 }
 
-/// Loads diagonal tile k's lower triangle into T (the identity beyond w),
-/// subtracting sub(r, c) when given (the update folded into the task).
-__device__ __forceinline__ void LoadDiagonal(const SupernodeRec& S, const double* Fs, int k, double* sm) {
-  const int64_t F = S.F;
-  const int c0 = k * kDT;
-  const int w = min(kDT, S.ncols - c0);
-  double(*T)[kTLd] = reinterpret_cast<double(*)[kTLd]>(sm);
-  for (int e = threadIdx.x; e < kDT * kDT; e += kDThreads) {
-    const int j = e >> 6;
-    const int i = e & 63;
-    double v;
-    if (i < w && j < w) {
-      v = i >= j ? Fs[static_cast<int64_t>(c0 + j) * F + c0 + i] : 0.0;
-    } else {
-      v = i == j ? 1.0 : 0.0;
-    }
-    T[i][j] = v;
-  }
-  __syncthreads();
-}
-
-/// SOLVE(i, k): L(i, k) = A(i, k) M^T D^-1 with M = L(k, k)^-1.
+/// SOLVE(i, k): L(i, k) = A(i, k) L(k, k)^-T D(k)^-1.
 __device__ void SolveTile(const DeviceView& V, const SupernodeRec& S, int i, int k, const DenseArgs& A,
                           double* sm) {
   const int64_t F = S.F;
-  const int c0 = k * kDT;
-  const int r0 = i * kDT;
-  const int w = min(kDT, S.ncols - c0);
-  const int h = min(kDT, S.ncols - r0);
   double* Fs = V.fronts + S.front_off;
-  const double* Mo = A.inv + S.dense_inv + static_cast<int64_t>(k) * kDT * kDT;
-  double acc[4][4] = {};
-  TileProduct(Fs + static_cast<int64_t>(c0) * F + r0, F, h, Mo, kDT, w, w, nullptr, sm, acc);
-  const int tx = threadIdx.x & 15;
-  const int ty = threadIdx.x >> 4;
-  const double* d = A.dvec + S.first_col + c0;
+  double* tile = Fs + static_cast<int64_t>(k) * kDT * F + i * kDT;
+  const int h = min(kDT, S.ncols - i * kDT);
+  double* X = sm;
+  double* L = sm + kTileDoubles;
+  double* d = L + kRegion2;
+  StageTile(X, tile, F, h);
+  StageFactor(S, Fs, k, A, L, d);
+  WaitElements();
+  SubstituteRows(X, L, d + 2 * kDT);
+  StoreSolved(tile, F, h, X, d + kDT);
+}
+
+/// The entries of tile (i, j) that a thread owns in TileProduct's layout,
+/// read before the product so that their latency hides behind it, and written
+/// back less the product (lower part).
+struct OwnedTile {
+  double* base;
+  int64_t ld;
+  int r0, c0, h, w;
+  bool diagonal;
+  double old[2][4][2];
+  __device__ __forceinline__ bool In(int i, int j, int e) const {
+    const int r = r0 + 8 * i;
+    const int c = c0 + 8 * j + e;
+    return r < h && c < w && (!diagonal || r >= c);
+  }
+  __device__ __forceinline__ void Read(const SupernodeRec& S, double* Fs, int ti, int tj, int wr, int wc) {
+    const int lane = threadIdx.x & 31;
+    ld = S.F;
+    base = Fs + static_cast<int64_t>(tj) * kDT * ld + ti * kDT;
+    r0 = wr + (lane >> 2);
+    c0 = wc + 2 * (lane & 3);
+    h = min(kDT, S.ncols - ti * kDT);
+    w = min(kDT, S.ncols - tj * kDT);
+    diagonal = ti == tj;
 #pragma unroll
-  for (int b = 0; b < 4; ++b) {
-    const int c = ty + 16 * b;
-    if (c < w) {
-      const double di = Recip(d[c]);
+    for (int i = 0; i < 2; ++i) {
 #pragma unroll
-      for (int a = 0; a < 4; ++a) {
-        const int r = tx + 16 * a;
-        if (r < h) {
-          Fs[static_cast<int64_t>(c0 + c) * F + r0 + r] = acc[a][b] * di;
+      for (int j = 0; j < 4; ++j) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          old[i][j][e] = In(i, j, e) ? __ldcg(base + (c0 + 8 * j + e) * ld + r0 + 8 * i) : 0.0;
         }
       }
     }
   }
-}
-
-/// acc = L(i, k) D(k) L(j, k)^T for output tile (i, j).
-__device__ __forceinline__ void UpdateProduct(const SupernodeRec& S, const double* Fs, int i, int j, int k,
-                                              const DenseArgs& A, double* sm, double acc[4][4]) {
-  const int64_t F = S.F;
-  const int c0 = k * kDT;
-  const int w = min(kDT, S.ncols - c0);
-  const int hi = min(kDT, S.ncols - i * kDT);
-  const int hj = min(kDT, S.ncols - j * kDT);
-  TileProduct(Fs + static_cast<int64_t>(c0) * F + i * kDT, F, hi, Fs + static_cast<int64_t>(c0) * F + j * kDT, F, hj,
-              w, A.dvec + S.first_col + c0, sm, acc);
-}
+  __device__ __forceinline__ void WriteLess(const double (&acc)[2][4][2]) const {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          if (In(i, j, e)) {
+            base[(c0 + 8 * j + e) * ld + r0 + 8 * i] = old[i][j][e] - acc[i][j][e];
+          }
+        }
+      }
+    }
+  }
+};
 
 /// UPDATE(i, j, k): A(i, j) -= L(i, k) D(k) L(j, k)^T, lower part.
 __device__ void UpdateTile(const DeviceView& V, const SupernodeRec& S, int i, int j, int k, const DenseArgs& A,
                            double* sm) {
   const int64_t F = S.F;
-  const int ri = i * kDT;
-  const int rj = j * kDT;
-  const int hi = min(kDT, S.ncols - ri);
-  const int hj = min(kDT, S.ncols - rj);
   double* Fs = V.fronts + S.front_off;
-  double acc[4][4] = {};
-  UpdateProduct(S, Fs, i, j, k, A, sm, acc);
-  const int tx = threadIdx.x & 15;
-  const int ty = threadIdx.x >> 4;
-  // all sixteen reads, then the writes
-  double old[4][4];
-#pragma unroll
-  for (int b = 0; b < 4; ++b) {
-    const int c = ty + 16 * b;
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-      const int r = tx + 16 * a;
-      const bool in = r < hi && c < hj && (i != j || r >= c);
-      old[a][b] = in ? Fs[static_cast<int64_t>(rj + c) * F + ri + r] : 0.0;
-    }
+  const double* col = Fs + static_cast<int64_t>(k) * kDT * F;
+  double* X = sm;
+  double* Y = i == j ? X : sm + kTileDoubles;
+  double* d = sm + kTileDoubles + kRegion2;
+  StageTile(X, col + i * kDT, F, min(kDT, S.ncols - i * kDT));
+  if (i != j) {
+    StageTile(Y, col + j * kDT, F, min(kDT, S.ncols - j * kDT));
   }
-#pragma unroll
-  for (int b = 0; b < 4; ++b) {
-    const int c = ty + 16 * b;
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-      const int r = tx + 16 * a;
-      if (r < hi && c < hj && (i != j || r >= c)) {
-        Fs[static_cast<int64_t>(rj + c) * F + ri + r] = old[a][b] - acc[a][b];
-      }
-    }
+  if (threadIdx.x < kDT) {
+    d[threadIdx.x] = __ldcg(A.dvec + S.first_col + k * kDT + threadIdx.x);
+  }
+  const int warp = threadIdx.x >> 5;
+  const int wr = 16 * (warp & 3);
+  const int wc = 32 * (warp >> 2);
+  OwnedTile C;
+  C.Read(S, Fs, i, j, wr, wc);
+  WaitElements();
+  __syncthreads();
+  if (i != j || wc < wr + 16) {
+    double acc[2][4][2] = {};
+    TileProduct(X, Y, d, wr, wc, acc);
+    C.WriteLess(acc);
   }
 }
 
 /// FACTOR(k). For k >= 1 the task first does the two steps that feed it:
 /// SOLVE(k, k - 1) (published as soon as it is written, for the other
 /// updates of step k - 1) and UPDATE(k, k, k - 1), whose result goes
-/// straight into the shared-memory tile instead of the front.
-__device__ void FactorTask(const DeviceView& V, const SupernodeRec& S, int k, int nt, const DenseArgs& A,
-                           int32_t* cnt, double* sm) {
+/// straight into the shared-memory trapezoid instead of the front. Returns
+/// false when a wait ran out.
+__device__ bool FactorTask(const DeviceView& V, const SupernodeRec& S, int k, int nt, const DenseArgs& A,
+                           int32_t* cnt, double* sm, int* factored) {
+  const int64_t F = S.F;
   double* Fs = V.fronts + S.front_off;
+  const int c0 = k * kDT;
+  const int w = min(kDT, S.ncols - c0);
+  const int kp = (w + 7) & ~7;
+  double* X = sm;
+  double* M = sm + kTileDoubles;
+  double* d = M + kRegion2;
+  const int tid = threadIdx.x;
+  const int lane = tid & 31;
+  const int warp = tid >> 5;
+  const int wr = 16 * (warp & 3);
+  const int wc = 32 * (warp >> 2);
+  const int pm = LdltPitch(kp);
+  OwnedTile C;
+  double acc[2][4][2] = {};
   if (k == 0) {
-    LoadDiagonal(S, Fs, 0, sm);
+    C.Read(S, Fs, 0, 0, wr, wc);
   } else {
-    SolveTile(V, S, k, k - 1, A, sm);
+    // the tile to solve and the one to update wait for the earlier steps only:
+    // they are on their way while tile k - 1 is still being factored
+    double* tile = Fs + static_cast<int64_t>(k - 1) * kDT * F + c0;
+    StageTile(X, tile, F, w);
+    C.Read(S, Fs, k, k, wr, wc);
+    if (tid == 0) {
+      *factored = WaitTile(cnt + (k - 1) * nt + (k - 1), k, A.abort, A.wait_limit) ? 1 : 0;
+    }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (*factored == 0) {
+      WaitElements();
+      return false;
+    }
+    StageFactor(S, Fs, k - 1, A, M, d);
+    WaitElements();
+    SubstituteRows(X, M, d + 2 * kDT);
+    StoreSolved(tile, F, w, X, d + kDT);
+    __syncthreads();
+    if (tid == 0) {
       __threadfence();
       PublishTile(cnt + k * nt + (k - 1), k);
     }
-    double acc[4][4] = {};
-    UpdateProduct(S, Fs, k, k, k - 1, A, sm, acc);
-    const int64_t F = S.F;
-    const int c0 = k * kDT;
-    const int w = min(kDT, S.ncols - c0);
-    double(*T)[kTLd] = reinterpret_cast<double(*)[kTLd]>(sm);
-    const int tx = threadIdx.x & 15;
-    const int ty = threadIdx.x >> 4;
+    if (wc < wr + 16) {
+      TileProduct(X, X, d + kDT, wr, wc, acc);
+    }
+  }
+  __syncthreads();
+  // the updated tile (the identity on the padding pivots)
 #pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      const int c = ty + 16 * b;
+  for (int i = 0; i < 2; ++i) {
 #pragma unroll
-      for (int a = 0; a < 4; ++a) {
-        const int r = tx + 16 * a;
-        double v;
-        if (r < w && c < w) {
-          v = r >= c ? Fs[static_cast<int64_t>(c0 + c) * F + c0 + r] - acc[a][b] : 0.0;
-        } else {
-          v = r == c ? 1.0 : 0.0;
+    for (int j = 0; j < 4; ++j) {
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int r = C.r0 + 8 * i;
+        const int c = C.c0 + 8 * j + e;
+        if (r < kp && c < kp) {
+          M[c * pm + r] = C.In(i, j, e) ? C.old[i][j][e] - acc[i][j][e] : (r == c ? 1.0 : 0.0);
         }
-        T[r][c] = v;
       }
     }
-    __syncthreads();
   }
-  FactorLoaded(V, S, k, nt, A, sm);
+  // rows of L of the tile, row major, for the inverse (the identity beyond w)
+  double(*T)[kTLd] = reinterpret_cast<double(*)[kTLd]>(X);
+  for (int e = tid; e < kDT * kDT; e += kDThreads) {
+    T[e >> 6][e & 63] = 0.0;
+  }
+  __syncthreads();
+  const bool zero = BlockLdlt<kDThreads>(
+      M, pm, kp, kp,
+      [&](int r, int p0, const double(&l)[8]) {
+        if (r < w) {
+          // within a 32 x 32 diagonal block transposed into its upper triangle
+          const bool upper = (r ^ p0) < 32;
+          double* dst = upper ? Fs + (c0 + r) * F + c0 + p0 : Fs + (c0 + p0) * F + c0 + r;
+          const int64_t step = upper ? 1 : F;
+#pragma unroll
+          for (int t = 0; t < 8; ++t) {
+            dst[t * step] = l[t];
+            T[r][p0 + t] = l[t];
+          }
+        }
+      },
+      [&](int p0, const double* diag, int lane_) {
+        const int i = lane_ >> 2;
+        if (p0 + i < w) {
+          for (int t = lane_ & 3; t < i; t += 4) {
+            Fs[(c0 + p0 + i) * F + c0 + p0 + t] = diag[8 * i + t];
+            T[p0 + i][p0 + t] = diag[8 * i + t];
+          }
+          if ((lane_ & 3) == 0) {
+            A.dvec[S.first_col + c0 + p0 + i] = diag[72 + i];
+          }
+        }
+      });
+  if (zero && lane == 0) {
+    atomicOr(V.status + S.instance, kStatusZeroPivot);
+  }
+  __syncthreads();
+  if (tid == 0) {
+    __threadfence();
+    PublishTile(cnt + k * nt + k, k + 1);
+  }
+  InvertTile(T, M, A.inv + S.dense_inv + static_cast<int64_t>(k) * kDT * kDT);
+  return true;
 }
 
-__global__ void __launch_bounds__(kDThreads, 1) KDenseRoot(DeviceView V, DenseArgs A) {
+__global__ void __launch_bounds__(kDThreads, 2) KDenseRoot(DeviceView V, DenseArgs A) {
   extern __shared__ double dense_sm[];
   __shared__ int task;
   __shared__ int go;
+  __shared__ int factored;  // FACTOR's own wait
   const int tid = threadIdx.x;
   for (;;) {
     __syncthreads();
@@ -517,9 +565,9 @@ __global__ void __launch_bounds__(kDThreads, 1) KDenseRoot(DeviceView V, DenseAr
       }
       bool ok;
       if (i == k) {
-        // FACTOR(k) with SOLVE(k, k - 1) and UPDATE(k, k, k - 1) folded in
-        ok = k == 0 || (WaitTile(cnt + (k - 1) * nt + (k - 1), k, A.abort, A.wait_limit) &&
-                        WaitTile(cnt + k * nt + (k - 1), k - 1, A.abort, A.wait_limit) &&
+        // FACTOR(k) with SOLVE(k, k - 1) and UPDATE(k, k, k - 1) folded in; it
+        // waits for tile (k - 1, k - 1) itself
+        ok = k == 0 || (WaitTile(cnt + k * nt + (k - 1), k - 1, A.abort, A.wait_limit) &&
                         WaitTile(cnt + k * nt + k, k - 1, A.abort, A.wait_limit));
       } else if (j == k) {
         ok = WaitTile(cnt + k * nt + k, k + 1, A.abort, A.wait_limit) &&
@@ -543,8 +591,17 @@ __global__ void __launch_bounds__(kDThreads, 1) KDenseRoot(DeviceView V, DenseAr
       continue;
     }
     if (i == k) {
-      FactorTask(V, S, k, nt, A, cnt, dense_sm);
-    } else if (j == k) {
+      // (publishes its tile itself, before the inverse)
+      if (!FactorTask(V, S, k, nt, A, cnt, dense_sm, &factored) && tid == 0) {
+        atomicOr(V.status + S.instance, kStatusWaitTimeout);
+        atomicExch(A.abort, 1);
+      }
+      if (tid == 0 && A.trace != nullptr) {
+        A.trace[3 * t + 2] = GlobalTimer();
+      }
+      continue;
+    }
+    if (j == k) {
       SolveTile(V, S, i, k, A, dense_sm);
     } else {
       UpdateTile(V, S, i, j, k, A, dense_sm);

@@ -25,7 +25,7 @@ struct DenseArgs {
 };
 
 /// Launches the persistent tiled factorization over args.count tasks on
-/// `stream` (one block per SM, never more blocks than tasks).
+/// `stream` (as many blocks as are resident, never more than tasks).
 /// Returns the launches made (0 or 1).
 int LaunchDenseRoots(const DeviceView& V, const DenseArgs& args, cudaStream_t stream);
 
