@@ -17,7 +17,7 @@
 //                  substitution, every warp on eight rows of its own
 //                  (i >= k + 2);
 //   UPDATE(i,j,k)  A(i, j) -= L(i, k) D(k) L(j, k)^T, j <= i (lower part;
-//                  not (k + 1, k + 1, k)).
+//                  not (k + 1, k + 1, k)); a tile's early steps in groups.
 //
 // The products run on the FP64 tensor cores. Bound by the chain of the FACTOR
 // tasks where the root is small, by the updates where it is large.
@@ -61,14 +61,15 @@ constexpr int kTLd = kDT + 1;  // pitch of the row-major tile of the inverse
 constexpr int kHLd = 33;
 constexpr int kTileDoubles = kDT * kDLd;
 // Shared memory: a staged tile, then a region for a second tile or FACTOR's
-// trapezoid, then D, 1 / D and the inverses of eight 8 x 8 diagonal blocks.
+// trapezoid, then D, 1 / D and the inverses of eight 8 x 8 diagonal blocks,
+// then the second pair of tiles of a grouped update.
 // The inverse of a factored tile reuses both (its rows of L in the first, three
 // 32 x 33 blocks in the second).
 constexpr int kRegion2 = 64 * LdltPitch(64) + 8 * LdltPanelPitch(64) + 2 * kLdltDiag;
 static_assert(kRegion2 >= kTileDoubles && kRegion2 >= 3 * 32 * kHLd && kTileDoubles >= kDT * kTLd);
 constexpr int kDiagInv = kWarps * 64;
 constexpr size_t kDenseSmem =
-    static_cast<size_t>(kTileDoubles + kRegion2 + 2 * kDT + kDiagInv) * sizeof(double);
+    static_cast<size_t>(kTileDoubles + kRegion2 + 2 * kDT + kDiagInv + 2 * kTileDoubles) * sizeof(double);
 
 __device__ __forceinline__ bool WaitTile(const int32_t* word, int32_t expected, const int32_t* abort,
                                          uint32_t limit) {
@@ -111,13 +112,18 @@ __device__ __forceinline__ void StageTile(double* dst, const double* src, int64_
 
 /// acc += X S Y^T for 64 x 64 tiles staged column major, S = diag(s): a warp
 /// owns 16 x 32 entries, C(wr + 8 i + lane / 4, wc + 8 j + 2 (lane % 4) + e) in
-/// acc[i][j][e].
+/// acc[i][j][e]. between(l) runs once per four columns l: copies issued there
+/// overlap the products (issued at once before them they hold the warps for a
+/// third of the product's time).
+template <typename Between>
 __device__ __forceinline__ void TileProduct(const double* X, const double* Y, const double* s, int wr, int wc,
-                                            double (&acc)[2][4][2]) {
+                                            double (&acc)[2][4][2], Between&& between) {
   const int q = threadIdx.x & 3;
   const int g = (threadIdx.x & 31) >> 2;
 #pragma unroll 4
-  for (int l = q; l < kDT; l += 4) {
+  for (int l0 = 0; l0 < kDT; l0 += 4) {
+    const int l = l0 + q;
+    between(l0);
     const double d = s[l];
     const double a0 = X[l * kDLd + wr + g] * d;
     const double a1 = X[l * kDLd + wr + 8 + g] * d;
@@ -156,12 +162,56 @@ __device__ __forceinline__ void StageFactor(const SupernodeRec& S, const double*
   }
 }
 
+/// The A fragments (columns 4 h + lane % 4, h = 0, 1) of an 8 x 8 block held
+/// as a C fragment (columns 2 (lane % 4) + {0, 1}): an exchange among the four
+/// lanes of a row.
+__device__ __forceinline__ void BlockAsA(const double (&c)[2], double (&a)[2]) {
+  const int lane = threadIdx.x & 31;
+  const int from = (lane & ~3) + ((lane & 3) >> 1);
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const double even = __shfl_sync(0xffffffffu, c[0], from + 2 * h);
+    const double odd = __shfl_sync(0xffffffffu, c[1], from + 2 * h);
+    a[h] = (lane & 1) != 0 ? odd : even;
+  }
+}
+
+/// Column blocks P.. of SubstituteRows (a template per block: every register
+/// index is a constant): W_P = C_P L_PP^-T, then the later blocks less
+/// W_P L_pP^T.
+template <int P>
+__device__ __forceinline__ void SubstituteFrom(double (&C)[8][2], const double* L, const double* minv) {
+  if constexpr (P < 8) {
+    const int q = threadIdx.x & 3;
+    const int g = (threadIdx.x & 31) >> 2;
+    double a[2];
+    BlockAsA(C[P], a);
+    // B(k, n) = L_PP^-1(n, k)
+    double w[2] = {0.0, 0.0};
+    Dmma884(w, a[0], minv[64 * P + 8 * q + g]);
+    Dmma884(w, a[1], minv[64 * P + 8 * (q + 4) + g]);
+    C[P][0] = w[0];
+    C[P][1] = w[1];
+    if constexpr (P < 7) {
+      BlockAsA(w, a);
+      const double* L0 = L + (8 * P + q) * kDLd + g;
+#pragma unroll
+      for (int p = P + 1; p < 8; ++p) {
+        Dmma884(C[p], -a[0], L0[8 * p]);
+        Dmma884(C[p], -a[1], L0[4 * kDLd + 8 * p]);
+      }
+    }
+    SubstituteFrom<P + 1>(C, L, minv);
+  }
+}
+
 /// W = A L^-T in place for the 64 x 64 tile A staged at X (column major) and
 /// the staged unit lower triangle L, eight rows per warp with no exchange
-/// between warps: per 8-column block p, A_p - sum_{q < p} W_q L_pq^T, then times
-/// L_pp^-T with the inverses of the 8 x 8 diagonal blocks (warp p forms the
-/// p-th in minv). Starts and ends with a block barrier.
-__device__ __forceinline__ void SubstituteRows(double* X, const double* L, double* minv) {
+/// between warps; the rows stay in registers as C fragments (the inverses of
+/// the 8 x 8 diagonal blocks, warp p the p-th, go to minv). L(i, k) = W D^-1 also
+/// goes to dst (rows below h). Starts and ends with a block barrier.
+__device__ __forceinline__ void SubstituteRows(double* X, const double* L, double* minv, const double* dinv,
+                                               double* dst, int64_t ld, int h) {
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const int q = lane & 3;
@@ -188,42 +238,27 @@ __device__ __forceinline__ void SubstituteRows(double* X, const double* L, doubl
       minv[64 * warp + 8 * lane + i] = m[i];
     }
   }
-  __syncthreads();
-  double* W = X + 8 * warp;  // the warp's rows
-#pragma unroll 1
+  const int r = 8 * warp + g;
+  double C[8][2];
+#pragma unroll
   for (int p = 0; p < 8; ++p) {
-    double c0[2] = {0.0, 0.0};
-    double c1[2] = {0.0, 0.0};
-    const double* Lp = L + 8 * p + g;
-    for (int l = q; l < 8 * p; l += 8) {
-      Dmma884(c0, W[l * kDLd + g], Lp[l * kDLd]);
-      Dmma884(c1, W[(l + 4) * kDLd + g], Lp[(l + 4) * kDLd]);
-    }
-    double* C = W + (8 * p + 2 * q) * kDLd + g;
-    C[0] -= c0[0] + c1[0];
-    C[kDLd] -= c0[1] + c1[1];
-    __syncwarp();
-    // times L_pp^-T: B(k, n) = L_pp^-1(n, k)
-    const double* Mi = minv + 64 * p;
-    double w[2] = {0.0, 0.0};
-    Dmma884(w, W[(8 * p + q) * kDLd + g], Mi[8 * q + g]);
-    Dmma884(w, W[(8 * p + 4 + q) * kDLd + g], Mi[8 * (q + 4) + g]);
-    __syncwarp();
-    C[0] = w[0];
-    C[kDLd] = w[1];
-    __syncwarp();
+    C[p][0] = X[(8 * p + 2 * q) * kDLd + r];
+    C[p][1] = X[(8 * p + 2 * q + 1) * kDLd + r];
   }
   __syncthreads();
-}
-
-/// L(i, k) = W D^-1 into the front.
-__device__ __forceinline__ void StoreSolved(double* dst, int64_t ld, int h, const double* W, const double* dinv) {
-  const int r = threadIdx.x & (kDT - 1);
-  if (r < h) {
-    for (int c = threadIdx.x >> 6; c < kDT; c += kDThreads / kDT) {
-      dst[c * ld + r] = W[c * kDLd + r] * dinv[c];
+  SubstituteFrom<0>(C, L, minv);
+#pragma unroll
+  for (int p = 0; p < 8; ++p) {
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int c = 8 * p + 2 * q + e;
+      X[c * kDLd + r] = C[p][e];
+      if (r < h) {
+        dst[c * ld + r] = C[p][e] * dinv[c];
+      }
     }
   }
+  __syncthreads();
 }
 
 /// Columns c of M = L^-1 for the unit lower 32 x 32 triangle at T
@@ -335,8 +370,7 @@ __device__ void SolveTile(const DeviceView& V, const SupernodeRec& S, int i, int
   StageTile(X, tile, F, h);
   StageFactor(S, Fs, k, A, L, d);
   WaitElements();
-  SubstituteRows(X, L, d + 2 * kDT);
-  StoreSolved(tile, F, h, X, d + kDT);
+  SubstituteRows(X, L, d + 2 * kDT, d + kDT, tile, F, h);
 }
 
 /// The entries of tile (i, j) that a thread owns in TileProduct's layout,
@@ -389,32 +423,64 @@ struct OwnedTile {
   }
 };
 
-/// UPDATE(i, j, k): A(i, j) -= L(i, k) D(k) L(j, k)^T, lower part.
-__device__ void UpdateTile(const DeviceView& V, const SupernodeRec& S, int i, int j, int k, const DenseArgs& A,
-                           double* sm) {
+/// UPDATE(i, j, [k, k + len)): A(i, j) -= sum of L(i, l) D(l) L(j, l)^T over the
+/// steps l, lower part; the next step's tiles are staged while the current
+/// ones are multiplied.
+__device__ void UpdateTile(const DeviceView& V, const SupernodeRec& S, int i, int j, int k, int len,
+                           const DenseArgs& A, double* sm) {
   const int64_t F = S.F;
   double* Fs = V.fronts + S.front_off;
-  const double* col = Fs + static_cast<int64_t>(k) * kDT * F;
-  double* X = sm;
-  double* Y = i == j ? X : sm + kTileDoubles;
-  double* d = sm + kTileDoubles + kRegion2;
-  StageTile(X, col + i * kDT, F, min(kDT, S.ncols - i * kDT));
-  if (i != j) {
-    StageTile(Y, col + j * kDT, F, min(kDT, S.ncols - j * kDT));
-  }
-  if (threadIdx.x < kDT) {
-    d[threadIdx.x] = __ldcg(A.dvec + S.first_col + k * kDT + threadIdx.x);
+  // two pairs of staged tiles and two copies of D
+  // (offsets, not an array of pointers: those would be generic addresses)
+  constexpr int kSecond = kTileDoubles + kRegion2 + 2 * kDT + kDiagInv;
+  double* const d = sm + kTileDoubles + kRegion2;
+  const int hi = min(kDT, S.ncols - i * kDT);
+  // four columns from c0 of step l's tiles (a thread stages one row of one)
+  const int r = threadIdx.x & (kDT - 1);
+  auto stage = [&](int l, int c0) {
+    const int c = c0 + static_cast<int>(threadIdx.x >> 6);
+    const double* col = Fs + (static_cast<int64_t>(k + l) * kDT + c) * F + r;
+    double* x = sm + (l & 1) * kSecond + c * kDLd + r;
+    if (r < hi) {
+      LoadElement(x, col + i * kDT);
+    } else {
+      *x = 0.0;
+    }
+    if (i != j) {
+      LoadElement(x + kTileDoubles, col + j * kDT);  // (j < i: a full tile)
+    }
+    if (c0 == 0 && threadIdx.x < kDT) {
+      LoadElement(d + (l & 1) * kDT + threadIdx.x, A.dvec + S.first_col + (k + l) * kDT + threadIdx.x);
+    }
+  };
+  for (int c0 = 0; c0 < kDT; c0 += 4) {
+    stage(0, c0);
   }
   const int warp = threadIdx.x >> 5;
   const int wr = 16 * (warp & 3);
   const int wc = 32 * (warp >> 2);
   OwnedTile C;
   C.Read(S, Fs, i, j, wr, wc);
-  WaitElements();
-  __syncthreads();
-  if (i != j || wc < wr + 16) {
-    double acc[2][4][2] = {};
-    TileProduct(X, Y, d, wr, wc, acc);
+  const bool mine = i != j || wc < wr + 16;
+  double acc[2][4][2] = {};
+  for (int l = 0; l < len; ++l) {
+    WaitElements();
+    __syncthreads();
+    const bool more = l + 1 < len;
+    if (mine) {
+      const double* X = sm + (l & 1) * kSecond;
+      TileProduct(X, X + (i != j ? kTileDoubles : 0), d + (l & 1) * kDT, wr, wc, acc, [&](int c0) {
+        if (more) {
+          stage(l + 1, c0);
+        }
+      });
+    } else if (more) {
+      for (int c0 = 0; c0 < kDT; c0 += 4) {
+        stage(l + 1, c0);
+      }
+    }
+  }
+  if (mine) {
     C.WriteLess(acc);
   }
 }
@@ -437,19 +503,38 @@ __device__ bool FactorTask(const DeviceView& V, const SupernodeRec& S, int k, in
   const int tid = threadIdx.x;
   const int lane = tid & 31;
   const int warp = tid >> 5;
-  const int wr = 16 * (warp & 3);
-  const int wc = 32 * (warp >> 2);
   const int pm = LdltPitch(kp);
-  OwnedTile C;
-  double acc[2][4][2] = {};
-  if (k == 0) {
-    C.Read(S, Fs, 0, 0, wr, wc);
-  } else {
+  // the lower triangle's 36 blocks of 8 x 8, five or four per warp: warps v and
+  // v + 4 share the block rows v (v + 1 blocks) and 7 - v (8 - v blocks)
+  const int v = warp & 3;
+  const int b0 = warp < 4 ? 0 : 5;
+  const int nb = warp < 4 ? 5 : 4;
+  auto block = [&](int x, int* br, int* bc) {
+    const int e = b0 + x;  // 0..8: row 7 - v first
+    *br = e < 8 - v ? 7 - v : v;
+    *bc = e < 8 - v ? e : e - (8 - v);
+  };
+  const int q = lane & 3;
+  const int g = lane >> 2;
+  double old[5][2];
+  double acc[5][2] = {};
+#pragma unroll
+  for (int x = 0; x < 5; ++x) {
+    int br;
+    int bc;
+    block(x, &br, &bc);
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int r = 8 * br + g;
+      const int c = 8 * bc + 2 * q + e;
+      old[x][e] = x < nb && r < w && r >= c ? __ldcg(Fs + (c0 + c) * F + c0 + r) : (r == c ? 1.0 : 0.0);
+    }
+  }
+  if (k > 0) {
     // the tile to solve and the one to update wait for the earlier steps only:
     // they are on their way while tile k - 1 is still being factored
     double* tile = Fs + static_cast<int64_t>(k - 1) * kDT * F + c0;
     StageTile(X, tile, F, w);
-    C.Read(S, Fs, k, k, wr, wc);
     if (tid == 0) {
       *factored = WaitTile(cnt + (k - 1) * nt + (k - 1), k, A.abort, A.wait_limit) ? 1 : 0;
     }
@@ -460,30 +545,40 @@ __device__ bool FactorTask(const DeviceView& V, const SupernodeRec& S, int k, in
     }
     StageFactor(S, Fs, k - 1, A, M, d);
     WaitElements();
-    SubstituteRows(X, M, d + 2 * kDT);
-    StoreSolved(tile, F, w, X, d + kDT);
-    __syncthreads();
+    SubstituteRows(X, M, d + 2 * kDT, d + kDT, tile, F, w);
     if (tid == 0) {
       __threadfence();
       PublishTile(cnt + k * nt + (k - 1), k);
     }
-    if (wc < wr + 16) {
-      TileProduct(X, X, d + kDT, wr, wc, acc);
+    int br[5];
+    int bc[5];
+#pragma unroll
+    for (int x = 0; x < 5; ++x) {
+      block(x, &br[x], &bc[x]);
+    }
+#pragma unroll 4
+    for (int l = q; l < kDT; l += 4) {
+      const double* col = X + l * kDLd + g;
+      const double inv = d[kDT + l];
+#pragma unroll
+      for (int x = 0; x < 5; ++x) {
+        if (x < nb) {
+          Dmma884(acc[x], col[8 * br[x]] * inv, col[8 * bc[x]]);
+        }
+      }
     }
   }
   __syncthreads();
   // the updated tile (the identity on the padding pivots)
 #pragma unroll
-  for (int i = 0; i < 2; ++i) {
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
+  for (int x = 0; x < 5; ++x) {
+    int br;
+    int bc;
+    block(x, &br, &bc);
+    if (x < nb && 8 * br < kp) {
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        const int r = C.r0 + 8 * i;
-        const int c = C.c0 + 8 * j + e;
-        if (r < kp && c < kp) {
-          M[c * pm + r] = C.In(i, j, e) ? C.old[i][j][e] - acc[i][j][e] : (r == c ? 1.0 : 0.0);
-        }
+        M[(8 * bc + 2 * q + e) * pm + 8 * br + g] = old[x][e] - acc[x][e];
       }
     }
   }
@@ -532,7 +627,7 @@ __device__ bool FactorTask(const DeviceView& V, const SupernodeRec& S, int k, in
   return true;
 }
 
-__global__ void __launch_bounds__(kDThreads, 2) KDenseRoot(DeviceView V, DenseArgs A) {
+__global__ void __launch_bounds__(kDThreads, 1) KDenseRoot(DeviceView V, DenseArgs A) {
   extern __shared__ double dense_sm[];
   __shared__ int task;
   __shared__ int go;
@@ -552,7 +647,8 @@ __global__ void __launch_bounds__(kDThreads, 2) KDenseRoot(DeviceView V, DenseAr
     const int s = q[0];
     const int i = q[1];
     const int j = q[2];
-    const int k = q[3];
+    const int k = q[3] & 0xffff;
+    const int len = (q[3] >> 16) + 1;
     const SupernodeRec S = V.sn[s];
     if (V.active[S.instance] == 0) {
       continue;
@@ -573,8 +669,10 @@ __global__ void __launch_bounds__(kDThreads, 2) KDenseRoot(DeviceView V, DenseAr
         ok = WaitTile(cnt + k * nt + k, k + 1, A.abort, A.wait_limit) &&
              WaitTile(cnt + i * nt + k, k, A.abort, A.wait_limit);
       } else {
-        ok = WaitTile(cnt + i * nt + k, k + 1, A.abort, A.wait_limit) &&
-             (i == j || WaitTile(cnt + j * nt + k, k + 1, A.abort, A.wait_limit)) &&
+        // (tile (i, l) is solved after (i, l - 1): the last step's are enough)
+        const int l = k + len - 1;
+        ok = WaitTile(cnt + i * nt + l, l + 1, A.abort, A.wait_limit) &&
+             (i == j || WaitTile(cnt + j * nt + l, l + 1, A.abort, A.wait_limit)) &&
              WaitTile(cnt + i * nt + j, k, A.abort, A.wait_limit);
       }
       if (!ok) {
@@ -604,12 +702,12 @@ __global__ void __launch_bounds__(kDThreads, 2) KDenseRoot(DeviceView V, DenseAr
     if (j == k) {
       SolveTile(V, S, i, k, A, dense_sm);
     } else {
-      UpdateTile(V, S, i, j, k, A, dense_sm);
+      UpdateTile(V, S, i, j, k, len, A, dense_sm);
     }
     __syncthreads();
     if (tid == 0) {
       __threadfence();
-      PublishTile(cnt + i * nt + j, k + 1);
+      PublishTile(cnt + i * nt + j, k + len);
       if (A.trace != nullptr) {
         A.trace[3 * t + 2] = GlobalTimer();
       }

@@ -28,7 +28,7 @@ __device__ __forceinline__ float Recip(float d) { return 1.0f / d; }
 /// c += A B for an 8 x 8 block by one warp on the FP64 tensor cores: lane l
 /// holds A(l / 4, l % 4), B(l % 4, l / 4) and C(l / 4, 2 (l % 4) + {0, 1}).
 __device__ __forceinline__ void Dmma884(double (&c)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
                : "+d"(c[0]), "+d"(c[1])
                : "d"(a), "d"(b));
 }
@@ -98,11 +98,13 @@ __host__ __device__ constexpr size_t LdltSmemDoubles(int kp, int R) {
   return static_cast<size_t>(kp) * LdltPitch(R) + 8 * static_cast<size_t>(LdltPanelPitch(R)) + 2 * kLdltDiag;
 }
 
-/// Copies one element of a front into the trapezoid (asynchronously where no
-/// conversion is needed).
+/// Copies one element of a front into shared memory (asynchronously where no
+/// conversion is needed; the destination is read after WaitElements and a
+/// barrier, which order the accesses around them, so that the copies
+/// themselves need not keep the compiler from moving other accesses).
 __device__ __forceinline__ void LoadElement(double* dst, const double* src) {
   const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src));
 }
 __device__ __forceinline__ void LoadElement(double* dst, const float* src) { *dst = static_cast<double>(*src); }
 __device__ __forceinline__ void WaitElements() {

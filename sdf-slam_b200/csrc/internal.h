@@ -224,19 +224,23 @@ constexpr int kZeroCols = 8;
 constexpr int kTcMinRowsDefault = 256;
 /// Tile edge of the tiled dense-root factorization.
 constexpr int kDenseTileCols = 64;
+/// Steps of a grouped UPDATE of the tiled factorization at most.
+constexpr int kDenseUpdateGroup = 4;
 /// One task of the tiled factorization of a dense root: FACTOR (i == j ==
-/// k), SOLVE (j == k < i) or UPDATE (k < j <= i), with its bottom level.
+/// k), SOLVE (j == k < i) or UPDATE (k < j <= i, the steps [k, k + len)), with
+/// its bottom level.
 struct DenseTileTask {
   double prio;
   int32_t sn;
   int32_t i;
   int32_t j;
   int32_t k;
+  int32_t len;
 };
 
 /// Appends the tasks of an n-column dense root's tiled LDL^T (kDenseTileCols
-/// tiles) with their bottom levels: the longest path of task weights
-/// (FACTOR 8, SOLVE 2, UPDATE 2) from the task to the end of the graph.
+/// tiles) with their bottom levels: the longest path of task weights from the
+/// task to the end of the graph.
 /// Sorted by it descending, every task follows the tasks it waits for.
 void AppendDenseTileTasks(int32_t sn, int n, std::vector<DenseTileTask>* out);
 /// The order blocks take the tasks in: bottom level descending (ties by k,
@@ -350,8 +354,8 @@ struct Symbolic {
   int64_t tc_pack_rows{0};
   // Dense pose roots (no rows below, more than small_pivots pivots) are
   // factored by one persistent launch per level over 64 x 64 tiles instead
-  // of panels: (sn, i, j, k) task quads (FACTOR i == j == k, SOLVE j == k <
-  // i, UPDATE k < j <= i) in descending bottom level, dense_range per level,
+  // of panels: (sn, i, j, k + 65536 (len - 1)) task quads (FACTOR i == j == k,
+  // SOLVE j == k < i, UPDATE k < j <= i) in descending bottom level, dense_range per level,
   // the tile counters (nt x nt per front) and the diagonal-tile inverses
   // (64 x 64 doubles per tile) they use.
   // (sn, first column) pairs of kZeroCols columns: the fronts' lower

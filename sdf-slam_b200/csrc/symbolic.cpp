@@ -951,7 +951,7 @@ void Finalize(Symbolic& S, std::vector<int> height, int panel_width, int tile) {
       S.dense_tasks.push_back(t.sn);
       S.dense_tasks.push_back(t.i);
       S.dense_tasks.push_back(t.j);
-      S.dense_tasks.push_back(t.k);
+      S.dense_tasks.push_back(t.k | ((t.len - 1) << 16));
     }
     S.dense_range[static_cast<size_t>(l)].count = static_cast<int64_t>(level_tasks.size());
   }
@@ -960,87 +960,61 @@ void Finalize(Symbolic& S, std::vector<int> height, int panel_width, int tile) {
 }  // namespace
 
 /// Appends the tasks of an n-column dense root's tiled LDL^T with their
-/// bottom levels: the longest path of task weights (about their relative
-/// durations) from the task to the end of the graph, so that sorting by it
-/// descending lists each task after the tasks it waits for. Tasks: FACTOR(k)
-/// (with SOLVE(k, k - 1) and UPDATE(k, k, k - 1) folded in for k >= 1),
-/// SOLVE(i, k) for i >= k + 2, UPDATE(i, j, k) for k < j <= i except
-/// (k + 1, k + 1, k). Successors:
-///   FACTOR(k)     -> FACTOR(k + 1), SOLVE(i, k), UPDATE(i, k, k - 1) (it
+/// bottom levels: the longest path of task weights (about their durations in
+/// us) from the task to the end of the graph, so that sorting by it descending
+/// lists each task after the tasks it waits for. Tasks: FACTOR(k) (with
+/// SOLVE(k, k - 1) and UPDATE(k, k, k - 1) folded in for k >= 1), SOLVE(i, k) for
+/// i >= k + 2, UPDATE(i, j, [k, k + len)) for k < j <= i except (j, j, j - 1).
+/// A tile's last two updates are tasks of their own (the chain may wait for
+/// them); the earlier ones go in groups of kDenseUpdateGroup, which read and
+/// write the tile once and stage one step's operands while the previous
+/// step's are multiplied. Successors:
+///   FACTOR(k)     -> FACTOR(k + 1), SOLVE(i, k), UPDATE(i, k, ..k - 1) (it
 ///                    produces L(k, k - 1));
-///   SOLVE(i, k)   -> UPDATE(i, j, k), UPDATE(i', i, k);
-///   UPDATE(i,j,k) -> the next step's task on tile (i, j): UPDATE(i, j, k + 1)
-///                    or, folded into them, FACTOR(j) (i == j == k + 2) and
-///                    FACTOR(j + 1) (i == j + 1 == k + 2); SOLVE(i, j) when
-///                    j == k + 1 and i >= j + 2.
-/// A topological order is tau = 4k (FACTOR), 4k + 1 (SOLVE), 4k + 2 (UPDATE,
-/// j >= k + 2), 4k + 4.5 (UPDATE, j == k + 1); the bottom levels are
-/// computed in decreasing tau.
+///   SOLVE(i, k)   -> the groups of tiles (i, j) and (i', i) that hold k;
+///   UPDATE        -> the tile's next group or, behind the last, FACTOR(j)
+///                    (i == j), FACTOR(j + 1) (i == j + 1) or SOLVE(i, j).
+/// A topological order is tau = 4k (FACTOR), 4k + 1 (SOLVE), and with k the
+/// group's last step 4k + 2 (UPDATE, j >= k + 2) or 4k + 4.5 (UPDATE,
+/// j == k + 1); the bottom levels are computed in decreasing tau, so that a
+/// tile's latest level is the one of the group that the task at hand feeds.
 void AppendDenseTileTasks(int32_t sn, int n, std::vector<DenseTileTask>* out) {
   const int nt = (n + kDenseTileCols - 1) / kDenseTileCols;
-  constexpr double kWFactor = 6.0;     // FACTOR(0) alone
-  constexpr double kWFolded = 14.0;    // FACTOR(k >= 1) with its SOLVE and UPDATE
-  constexpr double kWSolve = 4.0;
-  constexpr double kWUpdate = 4.0;
+  constexpr double kWFactor = 9.0;   // FACTOR(0) alone
+  constexpr double kWFolded = 14.0;  // FACTOR(k >= 1) with its SOLVE and UPDATE
+  constexpr double kWSolve = 4.7;
+  constexpr double kWUpdate = 3.0;   // the tile read and written
+  constexpr double kWStep = 2.3;     // each step
   struct Item {
     double tau;
-    int32_t i, j, k;
+    int32_t i, j, k, len;
   };
   std::vector<Item> items;
   for (int k = 0; k < nt; ++k) {
-    items.push_back({4.0 * k, k, k, k});
+    items.push_back({4.0 * k, k, k, k, 1});
     for (int i = k + 2; i < nt; ++i) {
-      items.push_back({4.0 * k + 1.0, i, k, k});
+      items.push_back({4.0 * k + 1.0, i, k, k, 1});
     }
-    for (int j = k + 1; j < nt; ++j) {
-      for (int i = j; i < nt; ++i) {
-        if (i == k + 1 && j == k + 1) {
-          continue;
-        }
-        items.push_back({j == k + 1 ? 4.0 * k + 4.5 : 4.0 * k + 2.0, i, j, k});
+  }
+  for (int j = 1; j < nt; ++j) {
+    for (int i = j; i < nt; ++i) {
+      const int steps = i == j ? j - 1 : j;
+      for (int k = 0; k < steps;) {
+        const int len = std::max(1, std::min(kDenseUpdateGroup, steps - 2 - k));
+        const int last = k + len - 1;
+        items.push_back({last + 1 == j ? 4.0 * last + 4.5 : 4.0 * last + 2.0, i, j, k, len});
+        k += len;
       }
     }
   }
   std::sort(items.begin(), items.end(), [](const Item& a, const Item& b) { return a.tau > b.tau; });
-  const size_t nn = static_cast<size_t>(nt) * nt;
-  // bottom levels: FACTOR per k, SOLVE per (i, k), UPDATE per (i, j) of the
-  // step being computed and of the step after it (tau orders steps so that
-  // both are all that is read)
+  // bottom levels: FACTOR per k, SOLVE per (i, k), per tile the group computed
+  // last (0: none yet)
   std::vector<double> bf(static_cast<size_t>(nt), 0.0);
+  const size_t nn = static_cast<size_t>(nt) * nt;
   std::vector<double> bs(nn, 0.0);
-  std::vector<std::vector<double>> bu(static_cast<size_t>(nt) + 1);
-  auto ub = [&](int i, int j, int k) -> double {
-    if (k >= nt || bu[static_cast<size_t>(k)].empty()) {
-      return 0.0;
-    }
-    return bu[static_cast<size_t>(k)][static_cast<size_t>(i) * nt + j];
-  };
-  auto uset = [&](int i, int j, int k, double v) {
-    std::vector<double>& b = bu[static_cast<size_t>(k)];
-    if (b.empty()) {
-      b.assign(nn, 0.0);
-    }
-    b[static_cast<size_t>(i) * nt + j] = v;
-  };
-  auto next_on_tile = [&](int i, int j, int k) -> double {
-    // the task that next reads or writes tile (i, j) after UPDATE(i, j, k)
-    if (k + 1 < j) {
-      if (i == j && j == k + 2) {
-        return bf[static_cast<size_t>(j)];
-      }
-      if (i == j + 1 && j == k + 1) {
-        return bf[static_cast<size_t>(i)];
-      }
-      return ub(i, j, k + 1);
-    }
-    // j == k + 1: the tile is complete
-    if (i == j + 1) {
-      return bf[static_cast<size_t>(i)];
-    }
-    return bs[static_cast<size_t>(i) * nt + j];
-  };
-  std::vector<DenseTileTask> local;
-  local.reserve(items.size());
+  std::vector<double> bu(nn, 0.0);
+  auto at = [nt](int i, int j) { return static_cast<size_t>(i) * nt + j; };
   for (const Item& it : items) {
     const int i = it.i;
     const int j = it.j;
@@ -1049,36 +1023,32 @@ void AppendDenseTileTasks(int32_t sn, int n, std::vector<DenseTileTask>* out) {
     if (i == k && j == k) {
       double m = k + 1 < nt ? bf[static_cast<size_t>(k) + 1] : 0.0;
       for (int r = k + 2; r < nt; ++r) {
-        m = std::max(m, bs[static_cast<size_t>(r) * nt + k]);
+        m = std::max(m, bs[at(r, k)]);
       }
-      if (k >= 1) {
-        for (int r = k + 1; r < nt; ++r) {
-          m = std::max(m, ub(r, k, k - 1));
-        }
+      for (int r = k + 1; k >= 1 && r < nt; ++r) {
+        m = std::max(m, bu[at(r, k)]);
       }
       b = (k == 0 ? kWFactor : kWFolded) + m;
       bf[static_cast<size_t>(k)] = b;
     } else if (j == k) {
       double m = 0.0;
       for (int c = k + 1; c <= i; ++c) {
-        m = std::max(m, ub(i, c, k));
+        m = std::max(m, bu[at(i, c)]);
       }
       for (int r = i; r < nt; ++r) {
-        m = std::max(m, ub(r, i, k));
+        m = std::max(m, bu[at(r, i)]);
       }
       b = kWSolve + m;
-      bs[static_cast<size_t>(i) * nt + k] = b;
+      bs[at(i, k)] = b;
     } else {
-      b = kWUpdate + next_on_tile(i, j, k);
-      uset(i, j, k, b);
+      double& u = bu[at(i, j)];
+      const double next = u > 0.0 ? u : i == j ? bf[static_cast<size_t>(j)]
+                                  : i == j + 1 ? bf[static_cast<size_t>(i)] : bs[at(i, j)];
+      b = kWUpdate + kWStep * it.len + next;
+      u = b;
     }
-    local.push_back({b, sn, i, j, k});
-    // steps two behind the one being computed are no longer read
-    if (k + 3 <= nt && !bu[static_cast<size_t>(k) + 2].empty() && i == k && j == k) {
-      std::vector<double>().swap(bu[static_cast<size_t>(k) + 2]);
-    }
+    out->push_back({b, sn, i, j, k, it.len});
   }
-  out->insert(out->end(), local.begin(), local.end());
 }
 
 void OrderDenseTileTasks(std::vector<DenseTileTask>* tasks) {
