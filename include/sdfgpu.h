@@ -299,9 +299,9 @@ int sdfgpu_linearization_get(sdfgpu_problem* problem, double* residuals, int32_t
                              int32_t* n_outer, int32_t* n_inner, double* n_values, double* rhs,
                              double* step);
 
-/* Timing breakdown of the last solve on this handle, measured with CUDA
- * events on the handle's stream, in seconds of GPU time per phase summed over
- * its iterations: [0] residuals + Jacobian + cell sort, [1] J^T J + J^T r,
+/* Timing breakdown of the last solve on this handle, measured with the
+ * device's timer as each phase's first kernel starts, in seconds of GPU time per
+ * phase summed over its iterations: [0] residuals + Jacobian + cell sort, [1] J^T J + J^T r,
  * [2] factorization, [3] triangular solves, [4] step + cost; [5] iterations;
  * [6] device time from the first iteration's start to the last one's end;
  * [7] kernels launched by the iterations; [8] useful FP64 flops of one

@@ -737,7 +737,8 @@ __global__ void __launch_bounds__(256) KPoseFrames(DeviceView V) {
 /// first of kZeroCols columns). The upper triangles are never read before
 /// the factorization writes them, so they are left as they are (half the
 /// bytes of clearing the whole buffer).
-__global__ void KZeroFronts(DeviceView V, const int32_t* tasks) {
+__global__ void KZeroFronts(DeviceView V, const int32_t* tasks, uint64_t* stamp) {
+  StampPhase(stamp);
   const int32_t* t = tasks + 2 * static_cast<int64_t>(blockIdx.x);
   const SupernodeRec S = V.sn[t[0]];
   const int c = t[1] + static_cast<int>(threadIdx.x >> 5);
@@ -857,7 +858,8 @@ __global__ void KBackup(DeviceView V, int dir, const int32_t* revert_mask) {
 /// replaces the accepted angles and their cos / sin by the platform libm's
 /// (KCommitPoses), so that the next linearization rotates with the
 /// reference's bits.
-__global__ void KApplyStep(DeviceView V) {
+__global__ void KApplyStep(DeviceView V, uint64_t* stamp) {
+  StampPhase(stamp);
   const int col = blockIdx.x * blockDim.x + threadIdx.x;
   if (col >= V.n) {
     return;
@@ -897,19 +899,51 @@ __global__ void KApplyStep(DeviceView V) {
 /// The accepted angles of the moved frames and their cos and sin, as the
 /// host computed them with the platform's libm (WrapAngle, pose.hpp:9):
 /// theta_out holds (theta, cos, sin, flag) per frame, flag 1 to commit.
-__global__ void KCommitPoses(DeviceView V) {
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void CommitPose(const DeviceView& V, int f) {
   if (f >= V.total_frames || V.theta_out[4 * f + 3] == 0.0) {
     return;
   }
   V.poses[3 * static_cast<int64_t>(f) + 2] = V.theta_out[4 * f];
   V.pose_cs[f] = make_double2(V.theta_out[4 * f + 1], V.theta_out[4 * f + 2]);
 }
+__global__ void KCommitPoses(DeviceView V) { CommitPose(V, blockIdx.x * blockDim.x + threadIdx.x); }
+
+/// Start of an iteration: its parameters from pinned host memory (read in
+/// place: three copies of a few bytes cost about 12 us of copy-engine gaps per
+/// iteration on B200, this kernel 4), cleared status words, and with *commit
+/// the last accepted step's angles (as KCommitPoses).
+__global__ void KBeginIteration(DeviceView V, const int32_t* active, const double* lam, const int32_t* marquardt,
+                                const int32_t* commit, uint64_t* stamp) {
+  StampPhase(stamp);
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < V.num_inst) {
+    V.active[t] = active[t];
+    V.lam[t] = lam[t];
+    V.marquardt[t] = marquardt[t];
+    V.status[t] = 0;
+  }
+  if (*commit != 0) {
+    CommitPose(V, t);
+  }
+}
+
+/// Clears a few words (a kernel between kernels starts at once; a memset of
+/// this size goes through the copy engine, with gaps of about 2 us).
+__global__ void KClearWords(uint32_t* words, int64_t count, uint64_t* stamp) {
+  StampPhase(stamp);
+  for (int64_t q = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; q < count;
+       q += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    words[q] = 0u;
+  }
+}
 
 /// Per-row cost terms of Problem::Cost (problem.cpp:132-156): point rows with
 /// the exact (non-smooth) evaluation and the Huber loss, Eikonal rows,
-/// odometry rows. Terms are laid out points, then Eikonal, then odometry.
-__global__ void KCostTerms(DeviceView V, double* terms) {
+/// odometry rows. Terms are laid out points, then Eikonal, then odometry; with
+/// `step` the per-column terms of the step norm and of the trust-region
+/// prediction follow (lm_solver.cpp:378, 389-391): delta^2 of every column,
+/// then delta * (lambda delta + rhs).
+__global__ void KCostTerms(DeviceView V, double* terms, int step) {
   const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (t < V.total_points) {
     const int f = V.pt_frame[t];
@@ -988,19 +1022,14 @@ __global__ void KCostTerms(DeviceView V, double* terms) {
     const double e1 = sw * (((-s) * dtx + c * dty) - m[1]);
     const double e2 = sw * WrapAngle(pj[2] - pi[2] - m[2]);
     terms[t] = (e0 * e0 + e1 * e1) + e2 * e2;
-  }
-}
-
-/// Per-column terms for the step norm and the trust-region prediction
-/// (lm_solver.cpp:378, 389-391): delta^2 and delta * (lambda delta + rhs).
-__global__ void KStepTerms(DeviceView V, double* sq, double* pred) {
-  const int col = blockIdx.x * blockDim.x + threadIdx.x;
-  if (col >= V.n) {
     return;
   }
-  const double d = V.step[col];
-  sq[col] = d * d;
-  pred[col] = d * (V.lam[V.col_inst[col]] * d + V.rhs[col]);
+  const int64_t col = o - V.total_odom;
+  if (step != 0 && col < V.n) {
+    const double d = V.step[col];
+    terms[t] = d * d;
+    terms[t + V.n] = d * (V.lam[V.col_inst[col]] * d + V.rhs[col]);
+  }
 }
 
 /// Deterministic segmented sum, first level: block (seg, part) sums the
@@ -1036,9 +1065,16 @@ __global__ void __launch_bounds__(256) KSegmentPartial(const double* x, const in
 }
 
 /// Second level: one warp per segment adds its kSegParts partials with a
-/// fixed butterfly.
-__global__ void KSegmentFinal(const double* partial, int num_segments, double* out) {
-  const int seg = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+/// fixed butterfly; the sums and the instances' status words go straight to
+/// pinned host memory.
+__global__ void KSegmentFinal(DeviceView V, const double* partial, int num_segments, double* out,
+                              int32_t* status_out, uint64_t* stamp) {
+  StampPhase(stamp);
+  const int thread = blockIdx.x * blockDim.x + threadIdx.x;
+  for (int i = thread; i < V.num_inst; i += gridDim.x * blockDim.x) {
+    status_out[i] = V.status[i];
+  }
+  const int seg = thread >> 5;
   const int lane = threadIdx.x & 31;
   if (seg >= num_segments) {
     return;

@@ -87,12 +87,6 @@ __device__ __forceinline__ bool WaitTile(const int32_t* word, int32_t expected, 
   return false;
 }
 
-__device__ __forceinline__ uint64_t GlobalTimer() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
 __device__ __forceinline__ void PublishTile(int32_t* word, int32_t value) {
   asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(word), "r"(value) : "memory");
 }

@@ -112,9 +112,10 @@ struct DeviceView {
   // decides the step holds correctly rounded device values until then
   double2* pose_cs;
   double2* pose_cs_backup;
-  // ApplyStep hand-off: the unwrapped angle theta + delta of each frame the
-  // step moved (theta_upd 1), and the host's wrapped angle, cos, sin and a
-  // commit flag per frame
+  // ApplyStep hand-off, in pinned host memory that the kernels write and read
+  // in place: the unwrapped angle theta + delta of each frame the step moved
+  // (theta_upd 1), and the host's wrapped angle, cos, sin and a commit flag per
+  // frame
   double* theta_pre;
   int32_t* theta_upd;
   const double* theta_out;  // 4 per frame
@@ -163,6 +164,21 @@ struct DeviceView {
   const int32_t* fmp_col;
   const int64_t* fmp_off;
 };
+
+/// The device's global timer, ns.
+__device__ __forceinline__ uint64_t GlobalTimer() {
+  uint64_t t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+/// Start of an iteration phase, written to pinned host memory by the phase's
+/// first kernel (an event recorded between two kernels of a graph keeps the
+/// device idle for about 5 us on B200).
+__device__ __forceinline__ void StampPhase(uint64_t* stamp) {
+  if (stamp != nullptr && blockIdx.x == 0 && threadIdx.x == 0) {
+    *stamp = GlobalTimer();
+  }
+}
 
 /// True when supernode S is factored in FP32 (a mixed solve's grid supernode).
 __device__ __forceinline__ bool Fp32Front(const DeviceView& V, const SupernodeRec& S) {

@@ -21,15 +21,18 @@ __global__ void KCellStart(const int32_t* keys, int64_t n, int64_t num_cells, in
 __global__ void KCellPass(DeviceView V, const int64_t* cells, int64_t count);
 __global__ void KPoseFrames(DeviceView V);
 __global__ void KFinalizeNormal(DeviceView V);
-__global__ void KZeroFronts(DeviceView V, const int32_t* tasks);
+__global__ void KZeroFronts(DeviceView V, const int32_t* tasks, uint64_t* stamp);
+__global__ void KClearWords(uint32_t* words, int64_t count, uint64_t* stamp);
 __global__ void KPosePairs(DeviceView V);
 __global__ void KBackup(DeviceView V, int dir, const int32_t* revert_mask);
-__global__ void KApplyStep(DeviceView V);
+__global__ void KApplyStep(DeviceView V, uint64_t* stamp);
 __global__ void KCommitPoses(DeviceView V);
-__global__ void KCostTerms(DeviceView V, double* terms);
-__global__ void KStepTerms(DeviceView V, double* sq, double* pred);
+__global__ void KBeginIteration(DeviceView V, const int32_t* active, const double* lam, const int32_t* marquardt,
+                                const int32_t* commit, uint64_t* stamp);
+__global__ void KCostTerms(DeviceView V, double* terms, int step);
 __global__ void KSegmentPartial(const double* x, const int64_t* seg_begin, const int64_t* seg_end, double* partial);
-__global__ void KSegmentFinal(const double* partial, int num_segments, double* out);
+__global__ void KSegmentFinal(DeviceView V, const double* partial, int num_segments, double* out,
+                              int32_t* status_out, uint64_t* stamp);
 __global__ void KConvertFronts(DeviceView V, const int32_t* tasks);
 __global__ void KNormalMatVecMap(DeviceView V, const double* x, double* y);
 __global__ void KNormalMatVecPose(DeviceView V, const double* x, double* y);
@@ -99,6 +102,7 @@ void Engine::Init(std::vector<SymPiece>* pieces) {
   for (auto& e : span_) {
     CudaCheck(cudaEventCreate(&e), "cudaEventCreate");
   }
+  CudaCheck(cudaEventCreateWithFlags(&ready_, cudaEventDisableTiming), "cudaEventCreate");
   const char* ng = std::getenv("SDFGPU_NO_GRAPH");
   use_graph_ = !(ng != nullptr && ng[0] == '1');
   BuildLayout();
@@ -107,6 +111,8 @@ void Engine::Init(std::vector<SymPiece>* pieces) {
   h_lam_.Alloc(host_.size());
   h_seg_.Alloc(5 * host_.size());
   h_status_.Alloc(host_.size());
+  h_stamps_.Alloc(6);
+  h_commit_.Alloc(1);
   mixed_.assign(host_.size(), 0);  // plain FP64 until a solve asks otherwise
   refine_tol_.assign(host_.size(), kDefaultRefineTol);
   AnalyzeAndUpload(pieces, 0);
@@ -157,6 +163,7 @@ void Engine::Replace(HostProblem next, SymPiece* piece, int64_t keep_rows) {
   keep_rows = std::max<int64_t>(0, std::min<int64_t>({keep_rows, host_[0].num_points(), next.num_points()}));
   // no background analysis may still read the current problem
   DropSpeculations(nullptr);
+  FlushCommit();
   // nothing enqueued may still read the current problem's buffers
   CudaCheck(cudaStreamSynchronize(stream_), "replace sync");
   DropGraph();
@@ -172,11 +179,9 @@ void Engine::Replace(HostProblem next, SymPiece* piece, int64_t keep_rows) {
 }
 
 void Engine::DropGraph() {
-  for (auto& g : graph_exec_) {
-    if (g != nullptr) {
-      cudaGraphExecDestroy(g);
-      g = nullptr;
-    }
+  if (graph_exec_ != nullptr) {
+    cudaGraphExecDestroy(graph_exec_);
+    graph_exec_ = nullptr;
   }
 }
 
@@ -194,6 +199,9 @@ Engine::~Engine() {
     if (e != nullptr) {
       cudaEventDestroy(e);
     }
+  }
+  if (ready_ != nullptr) {
+    cudaEventDestroy(ready_);
   }
   for (auto& e : span_) {
     if (e != nullptr) {
@@ -445,9 +453,6 @@ void Engine::UploadProblem(int64_t keep_rows) {
     const size_t F = static_cast<size_t>(total_frames_);
     pose_cs_.Alloc(F);
     pose_cs_backup_.Alloc(F);
-    theta_pre_.Alloc(F);
-    theta_upd_.Alloc(F);
-    theta_out_.Alloc(4 * F);
     h_theta_pre_.Alloc(F);
     h_theta_upd_.Alloc(F);
     h_theta_out_.Alloc(4 * F);
@@ -492,11 +497,8 @@ void Engine::UploadProblem(int64_t keep_rows) {
   status_.Alloc(I);
   active_.Alloc(I);
   revert_.Alloc(I);
-  terms_.Alloc(static_cast<size_t>(total_points_ + total_eik_ + total_odom_));
-  sq_terms_.Alloc(static_cast<size_t>(n_));
-  pred_terms_.Alloc(static_cast<size_t>(n_));
-  seg_out_.Alloc(5 * I);
-  seg_partial_.Alloc(32 * 3 * I);
+  terms_.Alloc(static_cast<size_t>(total_points_ + total_eik_ + total_odom_) + 2 * static_cast<size_t>(n_));
+  seg_partial_.Alloc(32 * 5 * I);
   std::vector<int64_t> sb;
   std::vector<int64_t> se;
   for (size_t i = 0; i < I; ++i) {
@@ -508,16 +510,15 @@ void Engine::UploadProblem(int64_t keep_rows) {
     sb.push_back(total_points_ + total_eik_ + L.odom_off);
     se.push_back(total_points_ + total_eik_ + L.odom_off + L.num_odom);
   }
+  for (int part = 0; part < 2; ++part) {
+    const int64_t base = total_points_ + total_eik_ + total_odom_ + part * static_cast<int64_t>(n_);
+    for (size_t i = 0; i < I; ++i) {
+      sb.push_back(base + layout_[i].col_off);
+      se.push_back(base + layout_[i].col_off + host_[i].num_params());
+    }
+  }
   seg_begin_.Upload(sb, s);
   seg_end_.Upload(se, s);
-  std::vector<int64_t> ssb;
-  std::vector<int64_t> sse;
-  for (size_t i = 0; i < I; ++i) {
-    ssb.push_back(layout_[i].col_off);
-    sse.push_back(layout_[i].col_off + host_[i].num_params());
-  }
-  step_seg_begin_.Upload(ssb, s);
-  step_seg_end_.Upload(sse, s);
   std::vector<int32_t> ones(I, 1);
   active_.Upload(ones, s);
   std::vector<int32_t> zeros(I, 0);
@@ -674,9 +675,9 @@ void Engine::RefreshView() {
   V.poses_backup = poses_backup_.get();
   V.pose_cs = pose_cs_.get();
   V.pose_cs_backup = pose_cs_backup_.get();
-  V.theta_pre = theta_pre_.get();
-  V.theta_upd = theta_upd_.get();
-  V.theta_out = theta_out_.get();
+  V.theta_pre = h_theta_pre_.get();
+  V.theta_upd = h_theta_upd_.get();
+  V.theta_out = h_theta_out_.get();
   V.pt_rec = pt_rec_.get();
   V.pt_poff = pt_poff_.get();
   V.pt_cell = pt_cell_.get();
@@ -841,7 +842,8 @@ int64_t Engine::ZeroTaskCount() const {
 void Engine::LaunchNormal() {
   const int64_t zero_count = ZeroTaskCount();
   if (zero_count > 0) {
-    KZeroFronts<<<static_cast<unsigned>(zero_count), 32 * kZeroCols, 0, stream_>>>(V_, zero_tasks_.get());
+    KZeroFronts<<<static_cast<unsigned>(zero_count), 32 * kZeroCols, 0, stream_>>>(V_, zero_tasks_.get(),
+                                                                                  Stamp(1));
     CudaCheck(cudaGetLastError(), "front zeroing");
     ++times_.launches;
   }
@@ -877,13 +879,18 @@ void Engine::LaunchNormal() {
   times_.launches += (total_cells_ > 0 ? 4 : 0) + 1 + (num_pairs_ > 0 ? 1 : 0) + (n_ > 0 ? 1 : 0);
 }
 
-void Engine::SegmentSum(const double* x, const int64_t* seg_begin, const int64_t* seg_end, int segments,
-                        double* out) {
-  KSegmentPartial<<<static_cast<unsigned>(segments * 32), 256, 0, stream_>>>(x, seg_begin, seg_end,
-                                                                            seg_partial_.get());
-  KSegmentFinal<<<Blocks(static_cast<int64_t>(segments) * 32, 128), 128, 0, stream_>>>(seg_partial_.get(), segments,
-                                                                                      out);
-  times_.launches += 2;
+void Engine::LaunchTerms(bool step) {
+  const int64_t terms = total_points_ + total_eik_ + total_odom_ + (step ? n_ : 0);
+  if (terms > 0) {
+    KCostTerms<<<Blocks(terms, 128), 128, 0, stream_>>>(V_, terms_.get(), step ? 1 : 0);
+  }
+  const int segments = (step ? 5 : 3) * static_cast<int>(host_.size());
+  KSegmentPartial<<<static_cast<unsigned>(segments * 32), 256, 0, stream_>>>(terms_.get(), seg_begin_.get(),
+                                                                            seg_end_.get(), seg_partial_.get());
+  KSegmentFinal<<<Blocks(static_cast<int64_t>(segments) * 32, 128), 128, 0, stream_>>>(
+      V_, seg_partial_.get(), segments, h_seg_.get(), h_status_.get(), Stamp(5));
+  CudaCheck(cudaGetLastError(), "cost kernels");
+  times_.launches += (terms > 0 ? 1 : 0) + 2;
 }
 
 FactorPlan Engine::Plan() {
@@ -926,6 +933,11 @@ FactorPlan Engine::Plan() {
 }
 
 void Engine::LaunchFactor() {
+  // the dense roots' counters (and the phase's time stamp)
+  const int64_t words = sym_.dense_cnt_words > 0 ? static_cast<int64_t>(DenseSyncWords(sym_)) : 0;
+  KClearWords<<<static_cast<unsigned>(std::clamp<int64_t>((words + 255) / 256, 1, 148)), 256, 0, stream_>>>(
+      reinterpret_cast<uint32_t*>(dense_sync_.get()), words, Stamp(2));
+  ++times_.launches;
   const int64_t conv_count = ZeroTaskCount();
   if (any_mixed_ && conv_count > 0) {
     // work copies of the assembled fronts (FP32 for mixed grid supernodes),
@@ -938,7 +950,9 @@ void Engine::LaunchFactor() {
 }
 
 void Engine::LaunchSolve() {
-  times_.launches += LaunchSolveLevels(sym_, V_, Plan(), stream_);
+  FactorPlan P = Plan();
+  P.solve_stamp = Stamp(3);
+  times_.launches += LaunchSolveLevels(sym_, V_, P, stream_);
   if (!any_mixed_ || n_ == 0) {
     return;
   }
@@ -974,20 +988,13 @@ void Engine::LaunchSolve() {
 }
 
 void Engine::LaunchCost(std::vector<double>& cost) {
-  const int64_t terms = total_points_ + total_eik_ + total_odom_;
+  FlushCommit();
   ClearStatus();
-  if (terms > 0) {
-    KCostTerms<<<Blocks(terms, 128), 128, 0, stream_>>>(V_, terms_.get());
-  }
+  LaunchTerms(false);
   const size_t I = host_.size();
-  SegmentSum(terms_.get(), seg_begin_.get(), seg_end_.get(), static_cast<int>(3 * I), seg_out_.get());
-  std::vector<double> out(3 * I);
-  CudaCheck(cudaMemcpyAsync(out.data(), seg_out_.get(), out.size() * sizeof(double), cudaMemcpyDeviceToHost, stream_),
-            "cost");
-  std::vector<int32_t> st(I);
-  CudaCheck(cudaMemcpyAsync(st.data(), status_.get(), I * sizeof(int32_t), cudaMemcpyDeviceToHost, stream_),
-            "status");
   CudaCheck(cudaStreamSynchronize(stream_), "cost sync");
+  const double* out = h_seg_.get();
+  const int32_t* st = h_status_.get();
   cost.resize(I);
   for (size_t i = 0; i < I; ++i) {
     cost[i] = (out[3 * i] + out[3 * i + 1]) + out[3 * i + 2];
@@ -1002,28 +1009,13 @@ void Engine::LaunchStepAndCost(bool backup) {
   if (backup) {
     KBackup<<<Blocks(big, 256), 256, 0, stream_>>>(V_, 0, revert_.get());
   }
-  if (n_ > 0) {
-    LaunchApplyStep();
-    KStepTerms<<<Blocks(n_, 256), 256, 0, stream_>>>(V_, sq_terms_.get(), pred_terms_.get());
-  }
-  const size_t I = host_.size();
-  SegmentSum(sq_terms_.get(), step_seg_begin_.get(), step_seg_end_.get(), static_cast<int>(I), seg_out_.get() + 3 * I);
-  SegmentSum(pred_terms_.get(), step_seg_begin_.get(), step_seg_end_.get(), static_cast<int>(I),
-             seg_out_.get() + 4 * I);
-  const int64_t terms = total_points_ + total_eik_ + total_odom_;
-  if (terms > 0) {
-    KCostTerms<<<Blocks(terms, 128), 128, 0, stream_>>>(V_, terms_.get());
-  }
-  SegmentSum(terms_.get(), seg_begin_.get(), seg_end_.get(), static_cast<int>(3 * I), seg_out_.get());
-  times_.launches += (backup ? 1 : 0) + (n_ > 0 ? 1 : 0) + (terms > 0 ? 1 : 0);
-  CudaCheck(cudaMemcpyAsync(h_seg_.get(), seg_out_.get(), 5 * I * sizeof(double), cudaMemcpyDeviceToHost, stream_),
-            "step terms");
-  CudaCheck(cudaMemcpyAsync(h_status_.get(), status_.get(), I * sizeof(int32_t), cudaMemcpyDeviceToHost, stream_),
-            "status");
-  CudaCheck(cudaGetLastError(), "step kernels");
+  LaunchApplyStep();
+  LaunchTerms(true);
+  times_.launches += backup ? 1 : 0;
 }
 
 void Engine::Reanalyze(const std::vector<int>& which) {
+  FlushCommit();
   const auto t0 = std::chrono::steady_clock::now();
   // a background analysis of these instances is superseded by this one
   DropSpeculations(&which);
@@ -1102,6 +1094,7 @@ void Engine::UploadSchedule() {
 }
 
 double Engine::Autotune(std::vector<std::pair<Schedule, double>>* trials) {
+  FlushCommit();
   // Candidate schedules: the pivot count below which a front is factored by
   // one kernel, that kernel's rows per block, and the rows per panel task
   // (0: wider fronts by whole outer blocks of 128 pivots, KPanelBlock).
@@ -1323,6 +1316,7 @@ void Engine::StepSpeculations() {
   near_.clear();
   if (!start.empty()) {
     // the accepted states (a revert of other instances may still be queued)
+    FlushCommit();
     std::vector<double> poses(3 * static_cast<size_t>(total_frames_));
     CudaCheck(cudaMemcpyAsync(poses.data(), poses_.get(), poses.size() * sizeof(double), cudaMemcpyDeviceToHost,
                               stream_),
@@ -1337,6 +1331,7 @@ void Engine::StepSpeculations() {
 /// Rows + normal equations; re-runs the symbolic analysis (once) when a point
 /// left its pose's analysed cell set. Returns the per-instance status OR.
 int Engine::AssembleWithPattern() {
+  FlushCommit();
   for (int attempt = 0; attempt < 2; ++attempt) {
     ClearStatus();
     CudaCheck(cudaEventRecord(ev_[0], stream_), "event");
@@ -1365,6 +1360,7 @@ int Engine::AssembleWithPattern() {
 }
 
 void Engine::GetState(int i, double* map_values, double* poses) {
+  FlushCommit();
   const InstanceLayout& L = layout_[static_cast<size_t>(i)];
   if (map_values != nullptr) {
     CudaCheck(cudaMemcpyAsync(map_values, map_.get() + L.node_off,
@@ -1380,6 +1376,7 @@ void Engine::GetState(int i, double* map_values, double* poses) {
 }
 
 void Engine::SetState(int i, const double* map_values, const double* poses) {
+  FlushCommit();
   const InstanceLayout& L = layout_[static_cast<size_t>(i)];
   if (map_values != nullptr) {
     CudaCheck(cudaMemcpyAsync(map_.get() + L.node_off, map_values,
@@ -1416,23 +1413,16 @@ void Engine::LaunchApplyStep() {
   if (n_ <= 0) {
     return;
   }
-  const size_t F = static_cast<size_t>(total_frames_);
-  CudaCheck(cudaMemsetAsync(theta_upd_.get(), 0, F * sizeof(int32_t), stream_), "angle flags");
-  KApplyStep<<<Blocks(n_, 256), 256, 0, stream_>>>(V_);
-  // the moved frames' angles for the host's exact wrap (CommitAngles)
-  CudaCheck(cudaMemcpyAsync(h_theta_pre_.get(), theta_pre_.get(), F * sizeof(double), cudaMemcpyDeviceToHost,
-                            stream_),
-            "angles");
-  CudaCheck(cudaMemcpyAsync(h_theta_upd_.get(), theta_upd_.get(), F * sizeof(int32_t), cudaMemcpyDeviceToHost,
-                            stream_),
-            "angle flags");
+  // (the moved frames' angles go to the pinned h_theta_pre_ / h_theta_upd_,
+  // whose flags the caller cleared, for the host's exact wrap in CommitAngles)
+  KApplyStep<<<Blocks(n_, 256), 256, 0, stream_>>>(V_, Stamp(4));
   CudaCheck(cudaGetLastError(), "apply step");
   times_.launches += 1;
 }
 
 void Engine::CommitAngles(const std::vector<int32_t>* revert) {
   // the stream has drained: h_theta_pre_ / h_theta_upd_ hold the last step's
-  // angles, and the previous commit's upload has read h_theta_out_
+  // angles, and the previous commit has read h_theta_out_
   const int F = total_frames_;
   if (F <= 0 || n_ <= 0) {
     return;
@@ -1464,12 +1454,18 @@ void Engine::CommitAngles(const std::vector<int32_t>* revert) {
       }
     }
   });
-  CudaCheck(cudaMemcpyAsync(theta_out_.get(), out, 4 * static_cast<size_t>(F) * sizeof(double), cudaMemcpyHostToDevice,
-                            stream_),
-            "wrapped angles");
-  KCommitPoses<<<Blocks(F, 128), 128, 0, stream_>>>(V_);
+  // by the next iteration's first kernel, or by FlushCommit before anything
+  // else reads the poses
+  commit_pending_ = true;
+}
+
+void Engine::FlushCommit() {
+  if (!commit_pending_) {
+    return;
+  }
+  commit_pending_ = false;
+  KCommitPoses<<<Blocks(total_frames_, 128), 128, 0, stream_>>>(V_);
   CudaCheck(cudaGetLastError(), "commit angles");
-  ++times_.launches;
 }
 
 double Engine::Cost(int i) {
@@ -1479,6 +1475,7 @@ double Engine::Cost(int i) {
 }
 
 void Engine::ApplyStep(int i, const double* step) {
+  FlushCommit();
   const InstanceLayout& L = layout_[static_cast<size_t>(i)];
   std::vector<int32_t> active(host_.size(), 0);
   active[static_cast<size_t>(i)] = 1;
@@ -1487,6 +1484,7 @@ void Engine::ApplyStep(int i, const double* step) {
   CudaCheck(cudaMemcpyAsync(step_.get() + L.col_off, step, sizeof(double) * host_[static_cast<size_t>(i)].num_params(),
                             cudaMemcpyHostToDevice, stream_),
             "step");
+  std::fill_n(h_theta_upd_.get(), total_frames_, 0);  // SetActive drained the stream
   LaunchApplyStep();
   CudaCheck(cudaStreamSynchronize(stream_), "apply step sync");
   CommitAngles(nullptr);
@@ -1769,14 +1767,9 @@ bool Engine::SolveDone() const {
 void Engine::EnqueuePhase(int phase) {
   switch (phase) {
     case 0: {
-      const size_t I = host_.size();
-      CudaCheck(cudaMemcpyAsync(active_.get(), h_active_.get(), I * sizeof(int32_t), cudaMemcpyHostToDevice, stream_),
-                "active");
-      CudaCheck(cudaMemcpyAsync(lam_.get(), h_lam_.get(), I * sizeof(double), cudaMemcpyHostToDevice, stream_),
-                "lambda");
-      CudaCheck(cudaMemcpyAsync(marq_.get(), h_marq_.get(), I * sizeof(int32_t), cudaMemcpyHostToDevice, stream_),
-                "marquardt");
-      ClearStatus();
+      KBeginIteration<<<Blocks(std::max<int64_t>(static_cast<int64_t>(host_.size()), total_frames_), 128), 128, 0,
+                        stream_>>>(V_, h_active_.get(), h_lam_.get(), h_marq_.get(), h_commit_.get(), Stamp(0));
+      ++times_.launches;
       LaunchRows();
       break;
     }
@@ -1828,49 +1821,55 @@ void Engine::LaunchIteration() {
 }
 
 void Engine::EnqueueIteration() {
-  if (use_graph_ && (graph_exec_[0] == nullptr || graph_backup_ != need_backup_)) {
+  // the stream has drained: nothing still writes the moved frames' flags
+  std::fill_n(h_theta_upd_.get(), total_frames_, 0);
+  std::fill_n(h_stamps_.get(), 6, uint64_t{0});
+  h_commit_[0] = commit_pending_ ? 1 : 0;
+  commit_pending_ = false;
+  auto phases = [this] {
+    stamping_ = true;
+    for (int phase = 0; phase < 5; ++phase) {
+      EnqueuePhase(phase);
+    }
+    stamping_ = false;
+  };
+  if (!use_graph_) {
+    phases();
+    CudaCheck(cudaEventRecord(ready_, stream_), "event");
+    return;
+  }
+  if (graph_exec_ == nullptr || graph_backup_ != need_backup_) {
     const auto t0 = std::chrono::steady_clock::now();
     DropGraph();
     const int64_t before = times_.launches;
-    for (int phase = 0; phase < 5; ++phase) {
-      cudaGraph_t graph = nullptr;
-      CudaCheck(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal), "begin capture");
-      try {
-        EnqueuePhase(phase);
-      } catch (...) {
-        cudaStreamEndCapture(stream_, &graph);
-        if (graph != nullptr) {
-          cudaGraphDestroy(graph);
-        }
-        DropGraph();
-        throw;
+    cudaGraph_t graph = nullptr;
+    CudaCheck(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal), "begin capture");
+    try {
+      phases();
+    } catch (...) {
+      stamping_ = false;
+      cudaStreamEndCapture(stream_, &graph);
+      if (graph != nullptr) {
+        cudaGraphDestroy(graph);
       }
-      CudaCheck(cudaStreamEndCapture(stream_, &graph), "end capture");
-      const cudaError_t e = cudaGraphInstantiate(&graph_exec_[phase], graph, 0);
-      cudaGraphDestroy(graph);
-      CudaCheck(e, "graph instantiate");
+      throw;
     }
+    CudaCheck(cudaStreamEndCapture(stream_, &graph), "end capture");
+    const cudaError_t e = cudaGraphInstantiate(&graph_exec_, graph, 0);
+    cudaGraphDestroy(graph);
+    CudaCheck(e, "graph instantiate");
     graph_launches_ = times_.launches - before;
     times_.launches = before;
     graph_backup_ = need_backup_;
     times_.capture_host += std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
   }
-  for (int phase = 0; phase < 5; ++phase) {
-    CudaCheck(cudaEventRecord(ev_[phase], stream_), "event");
-    if (use_graph_) {
-      CudaCheck(cudaGraphLaunch(graph_exec_[phase], stream_), "graph launch");
-    } else {
-      EnqueuePhase(phase);
-    }
-  }
-  CudaCheck(cudaEventRecord(ev_[5], stream_), "event");
-  if (use_graph_) {
-    times_.launches += graph_launches_;
-  }
+  CudaCheck(cudaGraphLaunch(graph_exec_, stream_), "graph launch");
+  CudaCheck(cudaEventRecord(ready_, stream_), "event");
+  times_.launches += graph_launches_;
 }
 
 bool Engine::IterationReady() const {
-  const cudaError_t e = cudaEventQuery(ev_[5]);
+  const cudaError_t e = cudaEventQuery(ready_);
   if (e == cudaErrorNotReady) {
     return false;
   }
@@ -1932,11 +1931,13 @@ void Engine::FinishIteration() {
       }
     }
   }
-  float ms = 0.0f;
   double* acc[5] = {&times_.assemble, &times_.normal, &times_.factor, &times_.solve, &times_.update};
+  uint64_t start = h_stamps_[0];
   for (int q = 0; q < 5; ++q) {
-    CudaCheck(cudaEventElapsedTime(&ms, ev_[q], ev_[q + 1]), "phase timing");
-    *acc[q] += ms * 1e-3;
+    // (a phase without work leaves no stamp)
+    const uint64_t end = h_stamps_[q + 1] != 0 ? h_stamps_[q + 1] : start;
+    *acc[q] += static_cast<double>(end - start) * 1e-9;
+    start = end;
   }
   timer_.Accumulate();
   ++times_.iterations;

@@ -176,7 +176,7 @@ struct FactorPlan {
   bool fp32_fronts{false};
   /// Tiled dense roots: task quads (Symbolic::dense_tasks), the sync words
   /// (a claim counter per level, the abort flag, then the tile counters;
-  /// zeroed at the start of every factorization) and the inverse workspace.
+  /// zeroed by the caller before every factorization) and the inverse workspace.
   const int32_t* dense_tasks{nullptr};
   int32_t* dense_sync{nullptr};
   double* dense_inv{nullptr};
@@ -187,6 +187,8 @@ struct FactorPlan {
   /// default of about a second).
   int solve_withhold{-1};
   uint32_t solve_wait_polls{0};
+  /// Where the solve writes its start time (null: nowhere).
+  uint64_t* solve_stamp{nullptr};
   /// Per-kernel device time of the launches (null: not timed).
   KernelTimer* timer{nullptr};
 };
@@ -393,6 +395,10 @@ class Engine {
   /// frames (the platform libm's WrapAngle, cos and sin), uploaded and
   /// committed, except for the instances `revert` marks.
   void CommitAngles(const std::vector<int32_t>* revert);
+  /// Applies committed angles that no iteration has taken over yet.
+  void FlushCommit();
+  /// Host slot of an iteration phase's time stamp (null outside an iteration).
+  uint64_t* Stamp(int phase) const { return stamping_ ? h_stamps_.get() + phase : nullptr; }
   /// (cos, sin) of frames [frame_off, frame_off + frames) from host poses.
   void UploadPoseTrig(const double* poses, int frame_off, int frames);
   void LaunchCost(std::vector<double>& cost);
@@ -431,7 +437,9 @@ class Engine {
   void EnqueueIteration();
   int AssembleWithPattern();
   [[nodiscard]] FactorPlan Plan();
-  void SegmentSum(const double* x, const int64_t* seg_begin, const int64_t* seg_end, int segments, double* out);
+  /// Cost terms (and, with `step`, the step's) of the current state and their
+  /// sums, with the status words, into h_seg_ and h_status_.
+  void LaunchTerms(bool step);
 
   std::vector<HostProblem> host_;
   std::vector<InstanceLayout> layout_;
@@ -446,8 +454,9 @@ class Engine {
   double tc_trial_ms_[2]{0.0, 0.0};
   Symbolic sym_;
   cudaStream_t stream_{nullptr};
-  cudaEvent_t ev_[6]{};
+  cudaEvent_t ev_[3]{};
   cudaEvent_t span_[2]{};
+  cudaEvent_t ready_{nullptr};  // the iteration enqueued last has finished
   bool span_started_{false};
   int device_{0};
   int64_t device_bytes_{0};
@@ -481,8 +490,6 @@ class Engine {
   // state and per-iteration buffers
   DevBuf<double> map_, poses_, map_backup_, poses_backup_;
   DevBuf<double2> pose_cs_, pose_cs_backup_;
-  DevBuf<double> theta_pre_, theta_out_;
-  DevBuf<int32_t> theta_upd_;
   std::vector<int32_t> frame_inst_host_;  // global frame -> instance
   HostBuf<double> h_theta_pre_, h_theta_out_;
   HostBuf<int32_t> h_theta_upd_;
@@ -492,8 +499,8 @@ class Engine {
   DevBuf<int64_t> pass_cells_;
   DevBuf<double> rhs_, step_, xs_, lam_, dvec_;
   DevBuf<int32_t> marq_, status_, active_, revert_;
-  DevBuf<double> terms_, sq_terms_, pred_terms_, seg_out_, seg_partial_;
-  DevBuf<int64_t> seg_begin_, seg_end_, step_seg_begin_, step_seg_end_;
+  DevBuf<double> terms_, seg_partial_;
+  DevBuf<int64_t> seg_begin_, seg_end_;  // cost parts x3 per instance, then |delta|^2, then prediction
   // symbolic buffers
   DevBuf<int32_t> perm_, pinv_, sn_rows_, sn_rel_, child_list_, level_sn_;
   DevBuf<SupernodeRec> sn_;
@@ -543,12 +550,15 @@ class Engine {
   int32_t* cell_rows_ptr_{nullptr};
   HostBuf<double> h_seg_;      // 5 per instance: cost parts x3, |delta|^2, prediction
   HostBuf<int32_t> h_status_;
-  HostBuf<int32_t> h_active_;  // per-iteration parameters read by the graph's copies
+  HostBuf<int32_t> h_active_;  // per-iteration parameters read by the iteration's first kernel
   HostBuf<int32_t> h_marq_;
+  HostBuf<int32_t> h_commit_;  // whether the next iteration commits h_theta_out_
+  HostBuf<uint64_t> h_stamps_;  // phase starts and the end of the last iteration, device ns
+  bool commit_pending_{false};
+  bool stamping_{false};
   HostBuf<double> h_lam_;
-  // CUDA graphs of one LM iteration, one per phase (fixed per symbolic
-  // analysis); the phase events are recorded between the graph launches
-  cudaGraphExec_t graph_exec_[5]{};
+  // CUDA graph of one LM iteration (fixed per symbolic analysis)
+  cudaGraphExec_t graph_exec_{nullptr};
   bool graph_backup_{false};
   bool use_graph_{true};
   int64_t graph_launches_{0};

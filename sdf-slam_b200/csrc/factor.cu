@@ -2296,6 +2296,8 @@ __global__ void __launch_bounds__(256, 1) KSolveTree(DeviceView V, SolveArgs A) 
 
 namespace sdfgpu {
 
+__global__ void KClearWords(uint32_t* words, int64_t count, uint64_t* stamp);  // assembly.cu
+
 static_assert(kInvBlock == kInvBlockDoubles, "inverted block size");
 
 /// Dynamic shared memory a block may use on B200.
@@ -2372,9 +2374,6 @@ int LaunchFactorLevels(const Symbolic& S, const DeviceView& V, const FactorPlan&
     }
     return w;
   };
-  if (P.dense_sync != nullptr && S.dense_cnt_words > 0) {
-    CudaCheck(cudaMemsetAsync(P.dense_sync, 0, DenseSyncWords(S) * sizeof(int32_t), stream), "dense sync reset");
-  }
   for (int l = 0; l < S.num_levels; ++l) {
     if (l == S.pose_level && P.pose.count > 0) {
       // every grid front is factored: their pose rows' products into the pose
@@ -2585,8 +2584,9 @@ int LaunchSolveLevels(const Symbolic& S, const DeviceView& V, const FactorPlan& 
     // one resident block per SM (the kernel's register bound); blocks that
     // find no task left return at once
     const int blocks = std::min(P.num_solve_tasks, sms);
-    CudaCheck(cudaMemsetAsync(P.solve_sync, 0, SolveSyncWords(num_sn, P.num_inv) * sizeof(uint32_t), stream),
-              "solve flags");
+    const auto words = static_cast<int64_t>(SolveSyncWords(num_sn, P.num_inv));
+    KClearWords<<<static_cast<unsigned>(std::min<int64_t>(148, (words + 255) / 256)), 256, 0, stream>>>(
+        P.solve_sync, words, P.solve_stamp);
     const TimedLaunch tl(P.timer, KernelTimer::kSolveTree, stream, [&] {
       // every entry of L read twice (forward, backward), FP32 in the grid
       // fronts of a mixed solve, and the inverted diagonal blocks
@@ -2615,7 +2615,7 @@ int LaunchSolveLevels(const Symbolic& S, const DeviceView& V, const FactorPlan& 
     A.wait_limit = P.solve_wait_polls > 0 ? P.solve_wait_polls : kWaitLimit;
     KSolveTree<<<static_cast<unsigned>(blocks), 256, tree_smem, stream>>>(V, A);
     CudaCheck(cudaGetLastError(), "solve kernel");
-    return 1;
+    return 2;
   }
   for (int l = 0; l < S.num_levels; ++l) {
     const int b = S.level_begin[static_cast<size_t>(l)];

@@ -139,6 +139,7 @@ void LdltEngine::Factorize(const double* values) {
     KScatterValues<<<static_cast<unsigned>((nnz_ + 255) / 256), 256, 0, s>>>(values_.get(), value_off_.get(), nnz_,
                                                                               fronts_.get());
   }
+  CudaCheck(cudaMemsetAsync(dense_sync_.get(), 0, DenseSyncWords(sym_) * sizeof(int32_t), s), "dense sync reset");
   LaunchFactorLevels(sym_, V_, plan_, s);
   int32_t st = 0;
   CudaCheck(cudaMemcpyAsync(&st, status_.get(), sizeof(int32_t), cudaMemcpyDeviceToHost, s), "status");
