@@ -577,7 +577,7 @@ void Engine::UploadSymbolic() {
     max_front_ = std::max(max_front_, r.F);
   }
   ConfigureSolveKernels(max_front_);
-  solve_sync_.Alloc(SolveSyncWords(static_cast<int>(sym_.sn.size()), static_cast<int>(sym_.inv_tasks.size() / 2)));
+  solve_sync_.Alloc(SolveSyncWords(sym_));
   UploadSolveTasks(s);
   inv_tasks_.Upload(sym_.inv_tasks, s);
   inv_.Alloc(std::max<size_t>(1, sym_.inv_tasks.size() / 2) * kInvBlockDoubles);

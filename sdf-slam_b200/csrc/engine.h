@@ -203,10 +203,14 @@ inline size_t DenseSyncWords(const Symbolic& S) {
 /// transpose).
 constexpr int kInvBlockDoubles = 2 * 32 * 32;
 
-/// Words of the one-launch solve's counter and flags for num_sn supernodes
-/// and num_inv diagonal blocks.
-inline size_t SolveSyncWords(int num_sn, int num_inv) {
-  return 2 + 4 * static_cast<size_t>(num_sn) + 2 * static_cast<size_t>(num_inv);
+/// Words of the one-launch solve's counter and flags (an even number), and
+/// with them the hand-over words of the tiled dense roots: two 64-bit words per
+/// column of their tiles, behind the flags.
+inline size_t SolveFlagWords(const Symbolic& S) {
+  return (2 + 4 * S.sn.size() + S.inv_tasks.size() + 1) & ~size_t{1};
+}
+inline size_t SolveSyncWords(const Symbolic& S) {
+  return SolveFlagWords(S) + 4 * static_cast<size_t>(S.dense_inv_doubles / kDenseTileCols);
 }
 
 /// Level-scheduled multifrontal LDL^T of the assembled fronts.

@@ -1772,7 +1772,9 @@ __device__ __forceinline__ bool WaitCount(const uint32_t* word, uint32_t expecte
     if (v >= expected) {
       return true;
     }
-    __nanosleep(100);
+    if (it > 64) {
+      __nanosleep(100);
+    }
   }
   return false;
 }
@@ -1794,6 +1796,8 @@ struct SolveArgs {
   const double* inv;
   const double* dense_inv;  // tile inverses of the tiled dense roots (64-row panels)
   uint32_t* sync;         // counter, then fdone, bdone, ydone, zdone per sn, then two flags per diagonal block
+  uint64_t* handover;     // y, then x, of the tiled dense roots' columns (0: not there yet)
+  int64_t handover_cols;
   int num_sn;
   int num_inv;
   int withhold;
@@ -1816,72 +1820,50 @@ __device__ __forceinline__ bool BlockWait(const DeviceView& V, const SupernodeRe
   return ok != 0;
 }
 
-/// Forward panel q of a tiled dense root (64-row panels, FP64): v_q -=
-/// L(q, p) y_p for every earlier panel p as its flag arrives (four threads
-/// per row, sixteen columns each, summed in a fixed order), then y_q = M_q
-/// v_q with M_q the tile inverse the factorization stored, D^-1 y_q into xs.
-__device__ __forceinline__ void RootForwardPanel64(const DeviceView& V, const SupernodeRec& S, const SolveArgs& A,
-                                                   int q, uint32_t* pflag, double* buf) {
-  constexpr int kW = kDenseTileCols;
-  const int k = S.ncols;
-  const int64_t F64 = S.F;
-  const double* Fs = V.fronts + S.front_off;
-  const int p0 = q * kW;
-  const int w = min(kW, k - p0);
-  const int tid = threadIdx.x;
-  double* vq = buf;           // kW
-  double* yp = buf + kW;      // kW
-  double* part = buf + 2 * kW;  // 4 x kW
-  const int i = tid & (kW - 1);
-  const int g = tid >> 6;  // four groups of sixteen columns
-  if (tid < kW) {
-    vq[tid] = tid < w ? A.ys[S.first_col + p0 + tid] : 0.0;
-  }
-  for (int p = 0; p < q; ++p) {
-    double l[16];
-#pragma unroll
-    for (int c = 0; c < 16; ++c) {
-      l[c] = i < w ? Fs[static_cast<int64_t>(p * kW + 16 * g + c) * F64 + p0 + i] : 0.0;
+/// Hand-over of a solved entry between the blocks of a tiled dense root: the
+/// value itself is the flag (its bits, changed so that zero means "not there
+/// yet": the pattern that would read as such is a NaN no operation produces),
+/// so that a panel waits one trip through L2 per predecessor instead of one for
+/// a flag and one for the data behind it.
+constexpr uint64_t kHandoverKey = 0x7ff4deadbeef0001ull;
+__device__ __forceinline__ void HandOver(uint64_t* slot, double v) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(slot),
+               "l"(static_cast<uint64_t>(__double_as_longlong(v)) ^ kHandoverKey)
+               : "memory");
+}
+/// Bounded wait for a handed-over entry; a wait that runs out marks the
+/// instance, reads as zero and leaves no limit for the thread's further waits.
+__device__ __forceinline__ double TakeOver(const DeviceView& V, const SupernodeRec& S, const uint64_t* slot,
+                                           uint32_t& limit) {
+  for (uint32_t it = 0; it < limit; ++it) {
+    uint64_t v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(slot) : "memory");
+    if (v != 0) {
+      return __longlong_as_double(static_cast<long long>(v ^ kHandoverKey));
     }
-    BlockWait(V, S, pflag + S.panel_base + p, 1u, A.wait_limit);
-    if (tid < kW) {
-      yp[tid] = __ldcg(A.ys + S.first_col + p * kW + tid);
-    }
-    __syncthreads();
-    double acc = 0.0;
-#pragma unroll
-    for (int c = 0; c < 16; ++c) {
-      acc = fma(l[c], yp[16 * g + c], acc);
-    }
-    part[g * kW + i] = acc;
-    __syncthreads();
-    if (tid < kW) {
-      vq[i] -= (part[i] + part[kW + i]) + (part[2 * kW + i] + part[3 * kW + i]);
+    if (it > 64) {
+      __nanosleep(50);
     }
   }
-  __syncthreads();
-  // y = M v: thread (row i, group g) sums sixteen columns of M
-  const double* M = A.dense_inv + S.dense_inv + static_cast<int64_t>(q) * kW * kW;
-  double acc = 0.0;
-#pragma unroll
-  for (int c = 0; c < 16; ++c) {
-    const int j = 16 * g + c;
-    acc = fma(M[static_cast<int64_t>(j) * kW + i], vq[j], acc);
-  }
-  part[g * kW + i] = acc;
-  __syncthreads();
-  if (tid < w) {
-    const double y = (part[i] + part[kW + i]) + (part[2 * kW + i] + part[3 * kW + i]);
-    A.ys[S.first_col + p0 + tid] = y;
-    V.xs[S.first_col + p0 + tid] = (1.0 / A.dvec[S.first_col + p0 + tid]) * y;
-  }
+  atomicOr(V.status + S.instance, kStatusWaitTimeout);
+  limit = 1;
+  return 0.0;
 }
 
-/// Backward panel q of a tiled dense root: z_q = (D^-1 y)_q minus
-/// L(p, q)^T x_p for every later panel p as its flag arrives, then x_q =
-/// M_q^T z_q into xs and the step.
-__device__ __forceinline__ void RootBackwardPanel64(const DeviceView& V, const SupernodeRec& S, const SolveArgs& A,
-                                                    int q, uint32_t* bflag, double* buf) {
+/// Panel q of a tiled dense root's solve (64-row panels, FP64), one block: the
+/// panels that come before it (forward: p < q, backward: p > q) hand their
+/// solutions over one by one; thread (row i of the panel, sixteen columns
+/// g of theirs) keeps its sum and its part of the tile inverse in registers and
+/// loads the next panel's L while it waits for the current one's solution, so
+/// that what follows the last hand-over is one sum over the four groups, one
+/// product with the inverse and one more sum. Forward: y_q = M_q (v_q - sum L(q, p) y_p), D^-1 y_q into xs. Backward:
+/// x_q = M_q^T (D^-1 y_q - sum L(p, q)^T x_p) into xs and the step. Bound by the
+/// chain of hand-overs. Measured on B200, the whole solve launch with a flag per
+/// panel and the sums through shared memory -> this: 910-pose office (43 panels
+/// each way) 1033 -> 887 us, 331-pose room 434 -> 380 us.
+template <bool kForward>
+__device__ __forceinline__ void RootPanel64(const DeviceView& V, const SupernodeRec& S, const SolveArgs& A, int q,
+                                            double* buf) {
   constexpr int kW = kDenseTileCols;
   const int k = S.ncols;
   const int64_t F64 = S.F;
@@ -1890,54 +1872,86 @@ __device__ __forceinline__ void RootBackwardPanel64(const DeviceView& V, const S
   const int p0 = q * kW;
   const int w = min(kW, k - p0);
   const int tid = threadIdx.x;
-  double* zq = buf;
-  double* xp = buf + kW;
-  double* part = buf + 2 * kW;
-  // thread (row i of z, group g of sixteen rows of panel p)
-  const int i = tid >> 2;
-  const int g = tid & 3;
-  if (tid < kW) {
-    zq[tid] = tid < w ? __ldcg(V.xs + S.first_col + p0 + tid) : 0.0;
-  }
-  for (int p = np - 1; p > q; --p) {
+  double* yp = buf;             // two panels' solutions, alternating
+  double* part = buf + 2 * kW;  // 4 x kW
+  double* vq = buf + 6 * kW;
+  // forward: rows along the lanes (L(q, p) column major); backward: four
+  // threads of sixteen consecutive entries per column of L(p, q)
+  const int i = kForward ? tid & (kW - 1) : tid >> 2;
+  const int g = kForward ? tid >> 6 : tid & 3;
+  const int64_t base = S.dense_inv / kW;
+  uint64_t* slots = A.handover + (kForward ? 0 : A.handover_cols) + base;
+  auto load = [&](int p, double (&l)[16]) {
     const int wp = min(kW, k - p * kW);
-    double l[16];
 #pragma unroll
     for (int c = 0; c < 16; ++c) {
       const int r = 16 * g + c;
-      l[c] = (i < w && r < wp) ? Fs[static_cast<int64_t>(p0 + i) * F64 + p * kW + r] : 0.0;
+      if (kForward) {
+        l[c] = i < w ? Fs[static_cast<int64_t>(p * kW + r) * F64 + p0 + i] : 0.0;
+      } else {
+        l[c] = i < w && r < wp ? Fs[static_cast<int64_t>(p0 + i) * F64 + p * kW + r] : 0.0;
+      }
     }
-    BlockWait(V, S, bflag + S.panel_base + p, 1u, A.wait_limit);
-    if (tid < kW) {
-      xp[tid] = tid < wp ? __ldcg(V.xs + S.first_col + p * kW + tid) : 0.0;
-    }
-    __syncthreads();
-    double acc = 0.0;
-#pragma unroll
-    for (int c = 0; c < 16; ++c) {
-      acc = fma(l[c], xp[16 * g + c], acc);
-    }
-    part[g * kW + i] = acc;
-    __syncthreads();
-    if (tid < kW) {
-      zq[tid] -= (part[tid] + part[kW + tid]) + (part[2 * kW + tid] + part[3 * kW + tid]);
-    }
-  }
-  __syncthreads();
-  // x = M^T z: thread (row i, group g) sums sixteen entries of column i of M
+  };
+  const int steps = kForward ? q : np - 1 - q;
+  double l[16];
+  double m[16];
+  // this panel's part of the inverse, row i of M (forward) or of M^T
   const double* M = A.dense_inv + S.dense_inv + static_cast<int64_t>(q) * kW * kW;
-  double acc = 0.0;
 #pragma unroll
   for (int c = 0; c < 16; ++c) {
     const int j = 16 * g + c;
-    acc = fma(M[static_cast<int64_t>(i) * kW + j], zq[j], acc);
+    m[c] = kForward ? M[j * kW + i] : M[i * kW + j];
+  }
+  if (steps > 0) {
+    load(kForward ? 0 : np - 1, l);
+  }
+  double own = 0.0;
+  if (tid < w) {
+    own = kForward ? __ldcg(A.ys + S.first_col + p0 + tid) : __ldcg(V.xs + S.first_col + p0 + tid);
+  }
+  uint32_t limit = A.wait_limit;
+  double acc = 0.0;
+#pragma unroll 1
+  for (int s = 0; s < steps; ++s) {
+    const int p = kForward ? s : np - 1 - s;
+    double* y = yp + (s & 1) * kW;
+    if (tid < kW) {
+      const int wp = min(kW, k - p * kW);
+      y[tid] = tid < wp ? TakeOver(V, S, slots + p * kW + tid, limit) : 0.0;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int c = 0; c < 16; ++c) {
+      acc = fma(l[c], y[16 * g + c], acc);
+    }
+    if (s + 1 < steps) {
+      load(kForward ? p + 1 : p - 1, l);
+    }
+  }
+  part[g * kW + i] = acc;
+  __syncthreads();
+  if (tid < kW) {
+    vq[tid] = own - ((part[tid] + part[kW + tid]) + (part[2 * kW + tid] + part[3 * kW + tid]));
+  }
+  __syncthreads();
+  acc = 0.0;
+#pragma unroll
+  for (int c = 0; c < 16; ++c) {
+    acc = fma(m[c], vq[16 * g + c], acc);
   }
   part[g * kW + i] = acc;
   __syncthreads();
   if (tid < w) {
     const double x = (part[tid] + part[kW + tid]) + (part[2 * kW + tid] + part[3 * kW + tid]);
-    V.xs[S.first_col + p0 + tid] = x;
-    V.step[V.perm[S.first_col + p0 + tid]] = x;
+    HandOver(slots + p0 + tid, x);
+    const int64_t col = S.first_col + p0 + tid;
+    if (kForward) {
+      V.xs[col] = (1.0 / A.dvec[col]) * x;
+    } else {
+      V.xs[col] = x;
+      V.step[V.perm[col]] = x;
+    }
   }
 }
 
@@ -2209,7 +2223,7 @@ __global__ void __launch_bounds__(256, 1) KSolveTree(DeviceView V, SolveArgs A) 
           break;
         case kTaskRootForward:
           if (S.dense_cnt >= 0) {
-            RootForwardPanel64(V, S, A, part, pflag, buf);
+            RootPanel64<true>(V, S, A, part, buf);
           } else if (f32) {
             RootForwardPanel<float>(V, S, A, part, pflag, buf);
           } else {
@@ -2218,7 +2232,7 @@ __global__ void __launch_bounds__(256, 1) KSolveTree(DeviceView V, SolveArgs A) 
           break;
         case kTaskRootBackward:
           if (S.dense_cnt >= 0) {
-            RootBackwardPanel64(V, S, A, part, bflag, buf);
+            RootPanel64<false>(V, S, A, part, buf);
           } else if (f32) {
             RootBackwardPanel<float>(V, S, A, part, bflag, buf);
           } else {
@@ -2584,7 +2598,7 @@ int LaunchSolveLevels(const Symbolic& S, const DeviceView& V, const FactorPlan& 
     // one resident block per SM (the kernel's register bound); blocks that
     // find no task left return at once
     const int blocks = std::min(P.num_solve_tasks, sms);
-    const auto words = static_cast<int64_t>(SolveSyncWords(num_sn, P.num_inv));
+    const auto words = static_cast<int64_t>(SolveSyncWords(S));
     KClearWords<<<static_cast<unsigned>(std::min<int64_t>(148, (words + 255) / 256)), 256, 0, stream>>>(
         P.solve_sync, words, P.solve_stamp);
     const TimedLaunch tl(P.timer, KernelTimer::kSolveTree, stream, [&] {
@@ -2611,6 +2625,8 @@ int LaunchSolveLevels(const Symbolic& S, const DeviceView& V, const FactorPlan& 
     A.sync = P.solve_sync;
     A.num_sn = num_sn;
     A.num_inv = P.num_inv;
+    A.handover = reinterpret_cast<uint64_t*>(P.solve_sync + SolveFlagWords(S));
+    A.handover_cols = S.dense_inv_doubles / kDenseTileCols;
     A.withhold = P.solve_withhold;
     A.wait_limit = P.solve_wait_polls > 0 ? P.solve_wait_polls : kWaitLimit;
     KSolveTree<<<static_cast<unsigned>(blocks), 256, tree_smem, stream>>>(V, A);

@@ -92,7 +92,7 @@ LdltEngine::LdltEngine(int n, const int32_t* outer, const int32_t* inner, const 
   plan_.level_sn = level_sn_.get();
   plan_.dvec = dvec_.get();
   plan_.max_front = max_front;
-  solve_sync_.Alloc(SolveSyncWords(static_cast<int>(sym_.sn.size()), static_cast<int>(sym_.inv_tasks.size() / 2)));
+  solve_sync_.Alloc(SolveSyncWords(sym_));
   plan_.solve_sync = solve_sync_.get();
   solve_tasks_.Upload(sym_.solve_tasks, s);
   solve_parts_.Upload(sym_.solve_parts, s);
