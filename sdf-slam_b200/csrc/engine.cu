@@ -576,11 +576,7 @@ void Engine::UploadSymbolic() {
   for (const SupernodeRec& r : sym_.sn) {
     max_front_ = std::max(max_front_, r.F);
   }
-  ConfigureSolveKernels(max_front_);
-  solve_sync_.Alloc(SolveSyncWords(sym_));
   UploadSolveTasks(s);
-  inv_tasks_.Upload(sym_.inv_tasks, s);
-  inv_.Alloc(std::max<size_t>(1, sym_.inv_tasks.size() / 2) * kInvBlockDoubles);
   std::vector<InstDev> inst(host_.size());
   for (size_t i = 0; i < host_.size(); ++i) {
     const InstanceLayout& L = layout_[i];
@@ -912,6 +908,8 @@ FactorPlan Engine::Plan() {
   P.zpart = zpart_.get();
   P.inv_tasks = inv_tasks_.get();
   P.num_inv = static_cast<int>(sym_.inv_tasks.size() / 2);
+  P.front_inv_tasks = front_inv_tasks_.get();
+  P.num_front_inv = static_cast<int>(sym_.front_inv_tasks.size() / 2);
   P.inv = inv_.get();
   P.fp32_fronts = any_mixed_;
   P.dense_tasks = dense_tasks_.get();
@@ -1070,6 +1068,11 @@ void Engine::UploadSolveTasks(cudaStream_t s) {
   dense_tasks_.Upload(sym_.dense_tasks, s);
   dense_sync_.Alloc(DenseSyncWords(sym_));
   dense_inv_.Alloc(static_cast<size_t>(std::max<int64_t>(1, sym_.dense_inv_doubles)));
+  ConfigureSolveKernels(max_front_, sym_.solve_panel_front);
+  solve_sync_.Alloc(SolveSyncWords(sym_));
+  inv_tasks_.Upload(sym_.inv_tasks, s);
+  front_inv_tasks_.Upload(sym_.front_inv_tasks, s);
+  inv_.Alloc(static_cast<size_t>(std::max<int64_t>(1, sym_.inv_doubles)));
   solve_tasks_.Upload(sym_.solve_tasks, s);
   solve_parts_.Upload(sym_.solve_parts, s);
   zpart_off_.Upload(sym_.zpart_off, s);

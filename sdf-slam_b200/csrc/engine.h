@@ -159,10 +159,13 @@ struct FactorPlan {
   const int64_t* zpart_off{nullptr};
   double* ys{nullptr};
   double* zpart{nullptr};
-  /// (sn, panel) pairs of the diagonal blocks and their inverses
-  /// (kInvBlockDoubles each), written after every factorization.
+  /// What the solve multiplies by, written after every factorization: (sn,
+  /// panel) pairs of the diagonal blocks of fronts solved by panels and (sn,
+  /// block) pairs of the other fronts' pivot block inverses.
   const int32_t* inv_tasks{nullptr};
   int num_inv{0};
+  const int32_t* front_inv_tasks{nullptr};
+  int num_front_inv{0};
   double* inv{nullptr};
   /// Tensor-core Schur complements of the mixed solve's wide FP32 fronts:
   /// the packed operands' tensor map (null: every Schur update on the SIMT
@@ -199,10 +202,6 @@ inline size_t DenseSyncWords(const Symbolic& S) {
   return static_cast<size_t>(S.num_levels) + 1 + static_cast<size_t>(S.dense_cnt_words);
 }
 
-/// Doubles per inverted 32 x 32 diagonal block (the inverse and its
-/// transpose).
-constexpr int kInvBlockDoubles = 2 * 32 * 32;
-
 /// Words of the one-launch solve's counter and flags (an even number), and
 /// with them the hand-over words of the tiled dense roots: two 64-bit words per
 /// column of their tiles, behind the flags.
@@ -219,7 +218,7 @@ int LaunchFactorLevels(const Symbolic& S, const DeviceView& V, const FactorPlan&
 /// Forward sweep, diagonal, backward sweep: V.step = A^-1 V.rhs (natural order).
 int LaunchSolveLevels(const Symbolic& S, const DeviceView& V, const FactorPlan& P, cudaStream_t stream);
 /// Raises the dynamic shared memory limit of the solve kernels.
-void ConfigureSolveKernels(int max_front);
+void ConfigureSolveKernels(int max_front, int solve_panel_front);
 
 /// Pinned host buffer.
 template <typename T>
@@ -524,7 +523,7 @@ class Engine {
   DevBuf<int32_t> solve_tasks_, solve_parts_;
   DevBuf<int64_t> zpart_off_;
   DevBuf<double> ys_, zpart_;
-  DevBuf<int32_t> inv_tasks_;     // diagonal blocks of L and their inverses
+  DevBuf<int32_t> inv_tasks_, front_inv_tasks_;  // diagonal blocks of L and their inverses
   DevBuf<double> inv_;
   // mixed precision: assembled FP64 normal matrix, FP32 work fronts and the
   // refinement vectors (the conversion runs over zero_tasks_)

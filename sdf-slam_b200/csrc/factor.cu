@@ -1365,6 +1365,215 @@ __global__ void __launch_bounds__(128) KInvertDiagonal(DeviceView V, const int32
   }
 }
 
+/// L(r, c), r > c, of a front's pivot block: the transposed triangle of
+/// single-kernel fronts and of every 32-column diagonal block, column major
+/// below the diagonal blocks of the others.
+template <typename T>
+__device__ __forceinline__ double PivotEntry(const T* Fs, int64_t F, bool upper, int r, int c) {
+  return static_cast<double>(upper || r / kPanel == c / kPanel ? Fs[r * F + c] : Fs[c * F + r]);
+}
+
+/// Shared memory of KInvertFronts: a tile of L, its inverse, a temporary and
+/// the finished rows of a strip.
+constexpr int kInvPitch = kFrontInvCols + 1;
+struct InvertSmem {
+  double L[kFrontInvCols][kInvPitch];
+  double M[kFrontInvCols][kInvPitch];
+  double T[kFrontInvCols * kFrontInvStrip];
+  double X[kSolvePivots * kFrontInvStrip];
+};
+
+/// One doubling step of a unit lower triangle's inverse, one block: for every
+/// pair of finished H x H inverses M11, M22 on the diagonal, the block between
+/// them M21 = -M22 (L21 M11). Lanes along the columns (L and M22 are
+/// broadcasts), rows eight apart per thread.
+template <int H>
+__device__ __forceinline__ void DoubleInverse(InvertSmem& sm) {
+  constexpr int kRows = H / 8;
+  const int j = threadIdx.x & (H - 1);
+  const int i0 = (threadIdx.x / H) & 7;
+  const int u = threadIdx.x / (8 * H);
+  const int base = 2 * H * u;
+  double acc[kRows] = {};
+#pragma unroll 8
+  for (int t = 0; t < H; ++t) {
+    const double m = sm.M[base + t][base + j];
+#pragma unroll
+    for (int q = 0; q < kRows; ++q) {
+      acc[q] = fma(sm.L[base + H + i0 + 8 * q][base + t], m, acc[q]);
+    }
+  }
+  double* T = sm.T + u * H * H;
+#pragma unroll
+  for (int q = 0; q < kRows; ++q) {
+    T[(i0 + 8 * q) * H + j] = acc[q];
+    acc[q] = 0.0;
+  }
+  __syncthreads();
+#pragma unroll 8
+  for (int t = 0; t < H; ++t) {
+    const double x = T[t * H + j];
+#pragma unroll
+    for (int q = 0; q < kRows; ++q) {
+      acc[q] = fma(-sm.M[base + H + i0 + 8 * q][base + H + t], x, acc[q]);
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < kRows; ++q) {
+    sm.M[base + H + i0 + 8 * q][base + j] = acc[q];
+  }
+  __syncthreads();
+}
+
+/// sm.M = the inverse of the unit lower triangle sm.L (zeros on and above the
+/// diagonal and past `rows`), one block, between barriers: the 8 x 8 diagonal
+/// blocks by substitution, a thread per column, then three doublings.
+__device__ __forceinline__ void InvertTriangle(InvertSmem& sm, int rows) {
+  const int tid = threadIdx.x;
+  for (int e = tid; e < kFrontInvCols * kFrontInvCols; e += blockDim.x) {
+    const int i = e / kFrontInvCols;
+    const int j = e & (kFrontInvCols - 1);
+    if (i / 8 != j / 8) {
+      sm.M[i][j] = 0.0;
+    }
+  }
+  if (tid < kFrontInvCols) {
+    const int b = tid & ~7;
+    const int c = tid & 7;
+    double x[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      x[q] = q == c ? 1.0 : 0.0;
+#pragma unroll
+      for (int t = 0; t < q; ++t) {
+        x[q] = fma(-sm.L[b + q][b + t], x[t], x[q]);
+      }
+      sm.M[b + q][b + c] = x[q];
+    }
+  }
+  __syncthreads();
+  DoubleInverse<8>(sm);
+  if (rows > 16) {
+    DoubleInverse<16>(sm);
+  }
+  if (rows > 32) {
+    DoubleInverse<32>(sm);
+  }
+}
+
+/// sm.L = the tile L(64 I.., 64 l..) of a front's pivot block (its strictly
+/// lower triangle for l == I). Columns along the lanes: the contiguous way of
+/// the transposed storage, which all but a few fronts have.
+template <typename T>
+__device__ __forceinline__ void LoadPivotTile(const T* Fs, const SupernodeRec& S, int I, int l, InvertSmem& sm) {
+  const int rows = min(kFrontInvCols, S.ncols - I * kFrontInvCols);
+  const bool upper = S.upper_l11 != 0;
+#pragma unroll
+  for (int e0 = 0; e0 < kFrontInvCols * kFrontInvCols; e0 += 256) {
+    const int i = (e0 + static_cast<int>(threadIdx.x)) / kFrontInvCols;
+    const int j = threadIdx.x & (kFrontInvCols - 1);
+    sm.L[i][j] = i < rows && (l < I || j < i)
+                     ? PivotEntry(Fs, static_cast<int64_t>(S.F), upper, I * kFrontInvCols + i, l * kFrontInvCols + j)
+                     : 0.0;
+  }
+}
+
+/// L11^-1 of one front (row major into out): all of it (at most 64 pivots), or
+/// the kFrontInvStrip columns from c0, row tile by row tile: X_I =
+/// L_II^-1 (E_I - sum L(I, l) X_l).
+template <typename T>
+__device__ __forceinline__ void InvertFrontColumns(const DeviceView& V, const SupernodeRec& S, int c0, double* out,
+                                                   InvertSmem& sm) {
+  constexpr int kW = kFrontInvCols;
+  constexpr int kS = kFrontInvStrip;
+  const int k = S.ncols;
+  const T* Fs = WorkFront<T>(V, S);
+  const int tid = threadIdx.x;
+  if (k <= kW) {
+    LoadPivotTile(Fs, S, 0, 0, sm);
+    __syncthreads();
+    InvertTriangle(sm, k);
+    for (int e = tid; e < kW * kW; e += blockDim.x) {
+      const int i = e / kW;
+      const int j = e & (kW - 1);
+      if (i < k && j <= i) {
+        out[i * k + j] = sm.M[i][j];
+      }
+    }
+    return;
+  }
+  // thread: a row of the tile, four columns of the strip
+  const int r = tid & (kW - 1);
+  const int cg = 4 * (tid / kW);
+  const int J = c0 / kW;
+  for (int I = J; I * kW < k; ++I) {
+    double w[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      w[q] = I * kW + r == c0 + cg + q ? 1.0 : 0.0;
+    }
+    for (int l = J; l < I; ++l) {
+      __syncthreads();
+      LoadPivotTile(Fs, S, I, l, sm);
+      __syncthreads();
+      const double* X = sm.X + (l - J) * kW * kS + cg;
+#pragma unroll 8
+      for (int t = 0; t < kW; ++t) {
+        const double a = sm.L[r][t];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          w[q] = fma(-a, X[t * kS + q], w[q]);
+        }
+      }
+    }
+    __syncthreads();
+    LoadPivotTile(Fs, S, I, I, sm);
+    __syncthreads();
+    InvertTriangle(sm, min(kW, k - I * kW));
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      sm.T[r * kS + cg + q] = w[q];
+      w[q] = 0.0;
+    }
+    __syncthreads();
+#pragma unroll 8
+    for (int t = 0; t < kW; ++t) {
+      const double a = sm.M[r][t];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        w[q] = fma(a, sm.T[t * kS + cg + q], w[q]);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      sm.X[((I - J) * kW + r) * kS + cg + q] = w[q];
+      if (I * kW + r < k && c0 + cg + q < k) {
+        out[static_cast<int64_t>(I * kW + r) * k + c0 + cg + q] = w[q];
+      }
+    }
+  }
+}
+
+/// Inverses of the pivot blocks of the fronts of at most kSolvePivots pivots,
+/// a block per front of at most 64 pivots and per strip of columns of the
+/// others. tasks: (sn, first column) pairs. Bound by the latency of one tile's
+/// steps (two blocks share an SM). Measured on B200 against substitution of
+/// whole 64-row tiles: 64 fronts of at most 50 pivots 12 against 16 us, 1437
+/// fronts, one of 200 pivots, 105 against 143 us.
+__global__ void __launch_bounds__(256, 2) KInvertFronts(DeviceView V, const int32_t* tasks, double* inv) {
+  extern __shared__ __align__(16) double invert_sm[];
+  InvertSmem& sm = *reinterpret_cast<InvertSmem*>(invert_sm);
+  const SupernodeRec S = V.sn[tasks[2 * blockIdx.x]];
+  if (V.active[S.instance] == 0) {
+    return;
+  }
+  if (Fp32Front(V, S)) {
+    InvertFrontColumns<float>(V, S, tasks[2 * blockIdx.x + 1], inv + S.inv_off, sm);
+  } else {
+    InvertFrontColumns<double>(V, S, tasks[2 * blockIdx.x + 1], inv + S.inv_off, sm);
+  }
+}
+
 /// Issues an asynchronous copy of one kPanel x kPanel block of doubles
 /// (16-byte chunks, L2 only) into shared memory and commits it as a group.
 __device__ __forceinline__ void CopyBlockAsync(double* dst, const double* src) {
@@ -1875,8 +2084,10 @@ __device__ __forceinline__ void RootPanel64(const DeviceView& V, const Supernode
   double* yp = buf;             // two panels' solutions, alternating
   double* part = buf + 2 * kW;  // 4 x kW
   double* vq = buf + 6 * kW;
-  // forward: rows along the lanes (L(q, p) column major); backward: four
-  // threads of sixteen consecutive entries per column of L(p, q)
+  // forward: rows along the lanes (L(q, p) column major), sixteen columns per
+  // group; backward: the four lanes of a column of L(p, q) take its entries in
+  // turn (whole sectors; sixteen consecutive ones each cost a line per lane and
+  // bound the sweep: 2.5 us a panel)
   const int i = kForward ? tid & (kW - 1) : tid >> 2;
   const int g = kForward ? tid >> 6 : tid & 3;
   const int64_t base = S.dense_inv / kW;
@@ -1885,7 +2096,7 @@ __device__ __forceinline__ void RootPanel64(const DeviceView& V, const Supernode
     const int wp = min(kW, k - p * kW);
 #pragma unroll
     for (int c = 0; c < 16; ++c) {
-      const int r = 16 * g + c;
+      const int r = kForward ? 16 * g + c : 4 * c + g;
       if (kForward) {
         l[c] = i < w ? Fs[static_cast<int64_t>(p * kW + r) * F64 + p0 + i] : 0.0;
       } else {
@@ -1900,15 +2111,34 @@ __device__ __forceinline__ void RootPanel64(const DeviceView& V, const Supernode
   const double* M = A.dense_inv + S.dense_inv + static_cast<int64_t>(q) * kW * kW;
 #pragma unroll
   for (int c = 0; c < 16; ++c) {
-    const int j = 16 * g + c;
+    const int j = kForward ? 16 * g + c : 4 * c + g;
     m[c] = kForward ? M[j * kW + i] : M[i * kW + j];
   }
   if (steps > 0) {
     load(kForward ? 0 : np - 1, l);
   }
   double own = 0.0;
+  if (kForward) {
+    // the panel's right-hand side and its part of the children's updates
+    if (tid < kW) {
+      vq[tid] = tid < w ? V.rhs[V.perm[S.first_col + p0 + tid]] : 0.0;
+    }
+    __syncthreads();
+    for (int ci = 0; ci < S.child_count; ++ci) {
+      const SupernodeRec C = V.sn[V.child_list[S.child_begin + ci]];
+      const int32_t* rel = V.sn_rel + C.rows_off;
+      const double* u = V.upd + C.upd_off;
+      for (int r = tid; r < C.nrows; r += blockDim.x) {
+        const int at = rel[r] - p0;
+        if (at >= 0 && at < w) {
+          vq[at] += __ldcg(u + r);
+        }
+      }
+      __syncthreads();
+    }
+  }
   if (tid < w) {
-    own = kForward ? __ldcg(A.ys + S.first_col + p0 + tid) : __ldcg(V.xs + S.first_col + p0 + tid);
+    own = kForward ? vq[tid] : __ldcg(V.xs + S.first_col + p0 + tid);
   }
   uint32_t limit = A.wait_limit;
   double acc = 0.0;
@@ -1923,7 +2153,7 @@ __device__ __forceinline__ void RootPanel64(const DeviceView& V, const Supernode
     __syncthreads();
 #pragma unroll
     for (int c = 0; c < 16; ++c) {
-      acc = fma(l[c], y[16 * g + c], acc);
+      acc = fma(l[c], y[kForward ? 16 * g + c : 4 * c + g], acc);
     }
     if (s + 1 < steps) {
       load(kForward ? p + 1 : p - 1, l);
@@ -1938,7 +2168,7 @@ __device__ __forceinline__ void RootPanel64(const DeviceView& V, const Supernode
   acc = 0.0;
 #pragma unroll
   for (int c = 0; c < 16; ++c) {
-    acc = fma(m[c], vq[16 * g + c], acc);
+    acc = fma(m[c], vq[kForward ? 16 * g + c : 4 * c + g], acc);
   }
   part[g * kW + i] = acc;
   __syncthreads();
@@ -2120,22 +2350,407 @@ __device__ __forceinline__ void RootBackwardPanel(const DeviceView& V, const Sup
   }
 }
 
+/// One chunk's place in shared memory: the values of L21 it owns (column
+/// major, an odd pitch so that lanes along the columns hit different banks),
+/// the gathered vector (pivots, then the chunk's rows), y or z, partial sums.
+constexpr int kSolveVec = kSolvePivots + kSolveMaxRows;
+constexpr int kSolveDoubles = kSolveSlab + kSolveVec + 2 * kSolvePivots;
+/// Child rows whose positions a thread reads before the wait.
+constexpr int kSolveRel = 4;
+
+/// Starts the copy of the front's values L21(r0:r0 + nr, :) into shared memory.
+template <typename T>
+__device__ __forceinline__ void StageRows(const T* Fs, const SupernodeRec& S, int r0, int nr, int pitch, T* slab) {
+  const int lane = threadIdx.x & 31;
+  for (int j = threadIdx.x >> 5; j < S.ncols; j += blockDim.x >> 5) {
+    const T* src = Fs + static_cast<int64_t>(j) * S.F + S.ncols + r0;
+    T* dst = slab + j * pitch;
+    for (int r = lane; r < nr; r += 32) {
+      LoadElement(dst + r, src + r);
+    }
+  }
+}
+
+/// Positions of a child's rows [base, base + 256 kSolveRel) in the chunk's
+/// gathered vector (-1: not in the chunk).
+__device__ __forceinline__ void ChildSlots(const DeviceView& V, const SupernodeRec& C, int base, int k, int r0, int nr,
+                                           int (&slot)[kSolveRel]) {
+  const int32_t* rel = V.sn_rel + C.rows_off;
+#pragma unroll
+  for (int q = 0; q < kSolveRel; ++q) {
+    const int r = base + 256 * q + static_cast<int>(threadIdx.x);
+    const int at = r < C.nrows ? rel[r] : -1;
+    slot[q] = at < k ? at : at - r0 < k + nr && at - r0 >= k ? at - r0 : -1;
+  }
+}
+
+/// Forward solve of a front's row chunk `part` (at most kSolvePivots pivots):
+/// the right-hand side with the children's updates of the pivots and of the
+/// chunk's rows, y = L11^-1 v (every chunk forms all of it, the first one
+/// stores D^-1 y), u = v_m - L21 y. What does not depend on the children (the
+/// chunk's L, the inverse, positions, right-hand side) is read before the wait
+/// for them: behind it come one read of their updates and two products.
+template <typename T, typename Wait>
+__device__ __forceinline__ void FrontForward(const DeviceView& V, const SupernodeRec& S, const SolveArgs& A, int part,
+                                             double* buf, Wait wait) {
+  const int k = S.ncols;
+  const int rows = SolveRows(k);
+  const int r0 = part * rows;
+  const int nr = min(rows, S.nrows - r0);
+  const int pitch = nr | 1;
+  const int tid = threadIdx.x;
+  T* slab = reinterpret_cast<T*>(buf);
+  double* v = buf + kSolveSlab;
+  double* y = v + kSolveVec;
+  double* sums = y + kSolvePivots;
+  const double* M = A.inv + S.inv_off;
+  StageRows<T>(WorkFront<T>(V, S), S, r0, nr, pitch, slab);
+  // four lanes per row of the inverse, entries in turn
+  const int mi = tid >> 2;
+  const int mg = tid & 3;
+  double m[16];
+#pragma unroll
+  for (int c = 0; c < 16; ++c) {
+    m[c] = 4 * c + mg <= mi && mi < k ? M[mi * k + 4 * c + mg] : 0.0;
+  }
+  for (int j = tid; j < k + nr; j += blockDim.x) {
+    v[j] = j < k ? V.rhs[V.perm[S.first_col + j]] : 0.0;
+  }
+  const double d = part == 0 && tid < k ? A.dvec[S.first_col + tid] : 1.0;
+  int slot0[kSolveRel];
+  int slot1[kSolveRel];
+  SupernodeRec C0{};
+  SupernodeRec C1{};
+  auto child_pair = [&](int ci) {
+    C0.nrows = 0;
+    C1.nrows = 0;
+    if (ci < S.child_count) {
+      C0 = V.sn[V.child_list[S.child_begin + ci]];
+    }
+    if (ci + 1 < S.child_count) {
+      C1 = V.sn[V.child_list[S.child_begin + ci + 1]];
+    }
+  };
+  child_pair(0);
+  ChildSlots(V, C0, 0, k, r0, nr, slot0);
+  ChildSlots(V, C1, 0, k, r0, nr, slot1);
+  if (!wait()) {
+    WaitElements();
+    return;
+  }
+  // children in order, each one's rows in distinct places
+  for (int ci = 0; ci < S.child_count; ci += 2) {
+    for (int base = 0; base < max(C0.nrows, C1.nrows); base += 256 * kSolveRel) {
+      if (ci > 0 || base > 0) {
+        ChildSlots(V, C0, base, k, r0, nr, slot0);
+        ChildSlots(V, C1, base, k, r0, nr, slot1);
+      }
+      double u0[kSolveRel];
+      double u1[kSolveRel];
+#pragma unroll
+      for (int q = 0; q < kSolveRel; ++q) {
+        const int r = base + 256 * q + tid;
+        u0[q] = slot0[q] >= 0 ? __ldcg(V.upd + C0.upd_off + r) : 0.0;
+        u1[q] = slot1[q] >= 0 ? __ldcg(V.upd + C1.upd_off + r) : 0.0;
+      }
+#pragma unroll
+      for (int q = 0; q < kSolveRel; ++q) {
+        if (slot0[q] >= 0) {
+          v[slot0[q]] += u0[q];
+        }
+      }
+      __syncthreads();
+#pragma unroll
+      for (int q = 0; q < kSolveRel; ++q) {
+        if (slot1[q] >= 0) {
+          v[slot1[q]] += u1[q];
+        }
+      }
+      __syncthreads();
+    }
+    if (ci + 2 < S.child_count) {
+      child_pair(ci + 2);
+    }
+  }
+  for (int i0 = 0; i0 < k; i0 += 64) {
+    double acc = 0.0;
+    const int i = i0 + mi;
+    for (int j0 = 0; j0 <= i0; j0 += 64) {
+      if (i0 > 0) {
+#pragma unroll
+        for (int c = 0; c < 16; ++c) {
+          const int j = j0 + 4 * c + mg;
+          m[c] = j <= i && i < k ? M[i * k + j] : 0.0;
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < 16; ++c) {
+        const int j = j0 + 4 * c + mg;
+        acc = fma(m[c], j < k ? v[j] : 0.0, acc);
+      }
+    }
+    acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+    acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+    if (mg == 0 && i < k) {
+      y[i] = acc;
+    }
+  }
+  WaitElements();
+  __syncthreads();
+  if (part == 0 && tid < k) {
+    V.xs[S.first_col + tid] = (1.0 / d) * y[tid];
+  }
+  // threads per row: as many groups of columns as rows leave room for
+  double* out = V.upd + S.upd_off + r0;
+  const int rb = nr > 128 ? 256 : nr > 64 ? 128 : nr > 32 ? 64 : 32;
+  const int groups = 256 / rb;
+  const int g = tid / rb;
+  const int cols = (k + groups - 1) / groups;
+  const int j0 = min(k, g * cols);
+  const int j1 = min(k, j0 + cols);
+  if (nr <= 0) {
+    return;
+  }
+  for (int r = tid & (rb - 1); r < (groups > 1 ? rb : nr); r += rb) {
+    const T* lr = slab + min(r, nr - 1);
+    double a0 = 0.0;
+    double a1 = 0.0;
+    double a2 = 0.0;
+    double a3 = 0.0;
+    int j = j0;
+    for (; j + 4 <= j1; j += 4) {
+      a0 = fma(static_cast<double>(lr[j * pitch]), y[j], a0);
+      a1 = fma(static_cast<double>(lr[(j + 1) * pitch]), y[j + 1], a1);
+      a2 = fma(static_cast<double>(lr[(j + 2) * pitch]), y[j + 2], a2);
+      a3 = fma(static_cast<double>(lr[(j + 3) * pitch]), y[j + 3], a3);
+    }
+    for (; j < j1; ++j) {
+      a0 = fma(static_cast<double>(lr[j * pitch]), y[j], a0);
+    }
+    const double acc = (a0 + a1) + (a2 + a3);
+    if (groups == 1) {
+      out[r] = v[k + r] - acc;
+    } else {
+      sums[tid] = acc;
+    }
+  }
+  if (groups > 1) {
+    __syncthreads();
+    if (tid < nr) {
+      double acc = sums[tid];
+      for (int q = 1; q < groups; ++q) {
+        acc += sums[q * rb + tid];
+      }
+      out[tid] = v[k + tid] - acc;
+    }
+  }
+}
+
+/// Backward solve of a front's row chunk `part`: the chunk's L21^T x_R, and in
+/// the block whose chunk is the front's last to arrive (in any order; the
+/// chunks' products are summed in theirs) z = D^-1 y - L21^T x_R and x =
+/// L11^-T z into xs and the step. True in that block: the front is done.
+template <typename T, typename Wait>
+__device__ __forceinline__ bool FrontBackward(const DeviceView& V, const SupernodeRec& S, const SolveArgs& A, int part,
+                                              int parts, uint32_t* arrived, double* zpart, double* buf, Wait wait) {
+  __shared__ int last;
+  const int k = S.ncols;
+  const int rows = SolveRows(k);
+  const int r0 = part * rows;
+  const int nr = min(rows, S.nrows - r0);
+  const int pitch = nr | 1;
+  const int tid = threadIdx.x;
+  T* slab = reinterpret_cast<T*>(buf);
+  double* xr = buf + kSolveSlab;
+  double* z = xr + kSolveVec;
+  double* sums = z + kSolvePivots;
+  const double* M = A.inv + S.inv_off;
+  StageRows<T>(WorkFront<T>(V, S), S, r0, nr, pitch, slab);
+  // columns of the inverse along the lanes, sixteen rows per group
+  const int mi = tid & 63;
+  const int mg = tid >> 6;
+  double m[16];
+#pragma unroll
+  for (int c = 0; c < 16; ++c) {
+    const int j = 16 * mg + c;
+    m[c] = j >= mi && j < k ? M[j * k + mi] : 0.0;
+  }
+  int at[kSolveMaxRows / 256];
+#pragma unroll
+  for (int q = 0; q < kSolveMaxRows / 256; ++q) {
+    const int r = tid + 256 * q;
+    at[q] = r < nr ? V.sn_rows[S.rows_off + r0 + r] : -1;
+  }
+  const int where = tid < k ? V.perm[S.first_col + tid] : 0;
+  const bool go = wait();
+  double own = 0.0;
+  if (go) {
+    own = tid < k ? __ldcg(V.xs + S.first_col + tid) : 0.0;
+#pragma unroll
+    for (int q = 0; q < kSolveMaxRows / 256; ++q) {
+      if (at[q] >= 0) {
+        xr[tid + 256 * q] = __ldcg(V.xs + at[q]);
+      }
+    }
+  }
+  WaitElements();
+  __syncthreads();
+  double sum = 0.0;
+  if (go) {
+    const int kb = k > 128 ? 256 : k > 64 ? 128 : k > 32 ? 64 : k > 16 ? 32 : 16;
+    const int groups = 256 / kb;
+    const int j = tid & (kb - 1);
+    const T* lc = slab + min(j, k - 1) * pitch;
+    double a0 = 0.0;
+    double a1 = 0.0;
+    double a2 = 0.0;
+    double a3 = 0.0;
+    int r = tid / kb;
+    for (; r + 3 * groups < nr; r += 4 * groups) {
+      a0 = fma(static_cast<double>(lc[r]), xr[r], a0);
+      a1 = fma(static_cast<double>(lc[r + groups]), xr[r + groups], a1);
+      a2 = fma(static_cast<double>(lc[r + 2 * groups]), xr[r + 2 * groups], a2);
+      a3 = fma(static_cast<double>(lc[r + 3 * groups]), xr[r + 3 * groups], a3);
+    }
+    for (; r < nr; r += groups) {
+      a0 = fma(static_cast<double>(lc[r]), xr[r], a0);
+    }
+    sums[tid] = (a0 + a1) + (a2 + a3);
+    __syncthreads();
+    if (tid < k) {
+      sum = sums[tid];
+      for (int q = 1; q < groups; ++q) {
+        sum += sums[q * kb + tid];
+      }
+      if (parts > 1) {
+        zpart[static_cast<int64_t>(part) * k + tid] = sum;
+      }
+    }
+  }
+  if (parts > 1) {
+    __syncthreads();
+    if (tid == 0) {
+      uint32_t before;
+      asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(before) : "l"(arrived) : "memory");
+      last = before == static_cast<uint32_t>(parts - 1) ? 1 : 0;
+    }
+    __syncthreads();
+    if (last == 0) {
+      return false;
+    }
+    if (tid < k) {
+      sum = 0.0;
+      for (int p = 0; p < parts; ++p) {
+        sum += __ldcg(zpart + static_cast<int64_t>(p) * k + tid);
+      }
+    }
+  }
+  if (!go) {
+    return true;
+  }
+  if (tid < k) {
+    z[tid] = own - sum;
+  }
+  __syncthreads();
+  for (int i0 = 0; i0 < k; i0 += 64) {
+    double acc = 0.0;
+    const int i = i0 + mi;
+    for (int j0 = i0; j0 < k; j0 += 64) {
+      if (i0 + j0 > 0) {
+#pragma unroll
+        for (int c = 0; c < 16; ++c) {
+          const int j = j0 + 16 * mg + c;
+          m[c] = j >= i && j < k ? M[j * k + i] : 0.0;
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < 16; ++c) {
+        const int j = j0 + 16 * mg + c;
+        acc = fma(m[c], j < k ? z[j] : 0.0, acc);
+      }
+    }
+    sums[tid] = acc;
+    __syncthreads();
+    if (tid >= i0 && tid < min(k, i0 + 64)) {
+      const int q = tid - i0;
+      const double x = (sums[q] + sums[64 + q]) + (sums[128 + q] + sums[192 + q]);
+      V.xs[S.first_col + tid] = x;
+      V.step[where] = x;
+    }
+    __syncthreads();
+  }
+  return true;
+}
+
+/// A task of a front solved by 32-column panels.
+__device__ __forceinline__ void PanelFrontTask(const DeviceView& V, const SupernodeRec& S, const SolveArgs& A, int type,
+                                               int s, int part, bool f32, double* buf) {
+  switch (type) {
+    case kTaskForward: {
+      double* ys = A.zoff[s] >= 0 ? A.ys : nullptr;
+      if (f32) {
+        ForwardTreeBody<float>(V, S, A.dvec, A.inv, buf, ys);
+      } else {
+        ForwardTreeBody<double>(V, S, A.dvec, A.inv, buf, ys);
+      }
+      break;
+    }
+    case kTaskForwardRows:
+      if (f32) {
+        ForwardRowsTask<float>(V, S, A.ys, part, buf);
+      } else {
+        ForwardRowsTask<double>(V, S, A.ys, part, buf);
+      }
+      break;
+    case kTaskRootGather:
+      RootGather(V, S, A.ys, buf);
+      break;
+    case kTaskBackwardRows:
+      if (f32) {
+        BackwardRowsTask<float>(V, S, part, A.zpart + A.zoff[s], buf);
+      } else {
+        BackwardRowsTask<double>(V, S, part, A.zpart + A.zoff[s], buf);
+      }
+      break;
+    default: {
+      const int parts = A.zoff[s] >= 0 ? A.parts[2 * s] - 1 : 0;
+      const double* zp = parts > 0 ? A.zpart + A.zoff[s] : nullptr;
+      if (f32) {
+        BackwardTreeBody<float>(V, S, A.inv, buf, zp, parts);
+      } else {
+        BackwardTreeBody<double>(V, S, A.inv, buf, zp, parts);
+      }
+      break;
+    }
+  }
+}
+
 /// Whole solve (forward sweep, diagonal, backward sweep) in one launch, with
-/// the inverted diagonal blocks of KInvertDiagonal. Blocks take the tasks of
-/// A.tasks in order from a counter (see Symbolic::solve_tasks): every task
-/// waits only on tasks taken before it by running blocks, so the launch
-/// completes whatever the number of resident blocks, and no level boundary
-/// holds fast fronts behind slow ones. A front's forward parts done counter
-/// (fdone) is what its parent waits for, its backward parts done (bdone)
-/// what its children wait for; ydone says a wide front's y (or a split
-/// root's right-hand side) is out, zdone counts a wide front's backward row
-/// chunks; a split root's panels publish one flag each per direction. A wait
+/// the inverses of KInvertFronts and KInvertDiagonal. Blocks take the tasks of
+/// A.tasks in order from a counter (see Symbolic::solve_tasks), the next one
+/// while they work on the current: every task waits only on tasks before it,
+/// and the lowest unfinished one is always being worked on (a block holds the
+/// next task only behind a lower one), so the launch completes whatever the
+/// number of resident blocks, and no level boundary holds fast fronts behind
+/// slow ones. A front's forward parts done counter (fdone) is what its parent
+/// waits for, its backward parts done (bdone) what its children wait for;
+/// zdone counts the backward row chunks. A tiled dense root's panels hand
+/// their values over one by one. With fronts solved by 32-column panels
+/// (kPanels): ydone says a wide front's y (or a split root's right-hand side)
+/// is out, a split root's panels publish one flag each per direction. A wait
 /// that runs out of its limit marks the instance kStatusWaitTimeout and lets
 /// the task's dependents go. withhold: a supernode whose forward parts are
 /// never published (-1: none), the test hook that makes a wait run out.
-__global__ void __launch_bounds__(256, 1) KSolveTree(DeviceView V, SolveArgs A) {
-  extern __shared__ double buf[];
-  __shared__ int task;
+/// Bound by the chain of levels (a front's reads wait for its children's, then
+/// its parent's publication) and, in large trees, by the L2 and shared-memory
+/// traffic of L. Measured on B200, against pivot blocks of 32-column panels
+/// with every read behind the wait and one block per SM: 10-frame room 82 -> 57
+/// us, 76-frame floor plan 188 -> 120, 910-pose office 887 -> 424, 32 instances
+/// 892 -> 406; its four FP32 rounds in the mixed office 3396 -> 1260.
+template <bool kPanels>
+__global__ void __launch_bounds__(256, kPanels ? 1 : 2) KSolveTree(DeviceView V, SolveArgs A) {
+  extern __shared__ __align__(16) double buf[];
+  __shared__ int4 next[2];
   __shared__ int go;
   uint32_t* fdone = A.sync + 2;
   uint32_t* bdone = fdone + A.num_sn;
@@ -2146,34 +2761,54 @@ __global__ void __launch_bounds__(256, 1) KSolveTree(DeviceView V, SolveArgs A) 
   if (V.refine_left != nullptr && *V.refine_left == 0) {
     return;  // a refinement round after every instance's step became final
   }
-  for (;;) {
-    if (threadIdx.x == 0) {
-      task = static_cast<int>(atomicAdd(A.sync, 1u));
-    }
-    __syncthreads();
-    const int t = task;
-    if (t >= A.num_tasks) {
+  const int4* tasks = reinterpret_cast<const int4*>(A.tasks);
+  auto take = [&] {
+    const int t = static_cast<int>(atomicAdd(A.sync, 1u));
+    return t < A.num_tasks ? tasks[t] : make_int4(-1, 0, 0, 0);
+  };
+  if (threadIdx.x == 0) {
+    next[0] = take();
+  }
+  __syncthreads();
+  for (int turn = 0;; turn ^= 1) {
+    const int type = next[turn].x;
+    if (type < 0) {
       return;
     }
-    const int type = A.tasks[4 * t];
-    const int s = A.tasks[4 * t + 1];
-    const int part = A.tasks[4 * t + 2];
+    const int s = next[turn].y;
+    const int part = next[turn].z;
+    int4 ahead{};
+    if (threadIdx.x == 0) {
+      ahead = take();
+    }
     const SupernodeRec S = V.sn[s];
     // refinement rounds skip the instances whose step is final
     const bool active = V.active[S.instance] != 0 && (V.refine_done == nullptr || V.refine_done[S.instance] == 0);
-    if (threadIdx.x == 0) {
-      bool ready = true;
-      if (active) {
+    // what the task waits for, polled by one thread; the whole block learns
+    // whether it came
+    auto wait = [&] {
+      if (threadIdx.x == 0) {
+        bool ready = true;
         switch (type) {
           case kTaskForward:
           case kTaskRootGather:
+          case kTaskFrontForward:
             for (int ci = 0; ci < S.child_count && ready; ++ci) {
               const int c = V.child_list[S.child_begin + ci];
               ready = WaitCount(fdone + c, static_cast<uint32_t>(A.parts[2 * c]), A.wait_limit);
             }
             break;
-          case kTaskForwardRows:
           case kTaskRootForward:
+            if (S.dense_cnt >= 0) {
+              for (int ci = 0; ci < S.child_count && ready; ++ci) {
+                const int c = V.child_list[S.child_begin + ci];
+                ready = WaitCount(fdone + c, static_cast<uint32_t>(A.parts[2 * c]), A.wait_limit);
+              }
+            } else {
+              ready = WaitCount(ydone + s, 1u, A.wait_limit);
+            }
+            break;
+          case kTaskForwardRows:
             ready = WaitCount(ydone + s, 1u, A.wait_limit);
             break;
           case kTaskRootBackward:
@@ -2182,8 +2817,8 @@ __global__ void __launch_bounds__(256, 1) KSolveTree(DeviceView V, SolveArgs A) 
           case kTaskBackwardRows:
             ready = WaitCount(bdone + S.parent, static_cast<uint32_t>(A.parts[2 * S.parent + 1]), A.wait_limit);
             break;
-          default:  // kTaskBackward
-            if (A.zoff[s] >= 0) {
+          default:  // kTaskBackward, kTaskFrontBackward
+            if (type == kTaskBackward && A.zoff[s] >= 0) {
               ready = WaitCount(zdone + s, static_cast<uint32_t>(A.parts[2 * s] - 1), A.wait_limit);
             } else if (S.parent >= 0) {
               ready = WaitCount(bdone + S.parent, static_cast<uint32_t>(A.parts[2 * S.parent + 1]), A.wait_limit);
@@ -2195,72 +2830,65 @@ __global__ void __launch_bounds__(256, 1) KSolveTree(DeviceView V, SolveArgs A) 
         if (!ready) {
           atomicOr(V.status + S.instance, kStatusWaitTimeout);
         }
+        go = ready ? 1 : 0;
       }
-      go = active && ready ? 1 : 0;
-    }
-    __syncthreads();
+      __syncthreads();
+      return go != 0;
+    };
+    bool done = true;  // whether the front's backward part is complete
     const bool f32 = Fp32Front(V, S);
-    if (go != 0) {
-      switch (type) {
-        case kTaskForward: {
-          double* ys = A.zoff[s] >= 0 ? A.ys : nullptr;
-          if (f32) {
-            ForwardTreeBody<float>(V, S, A.dvec, A.inv, buf, ys);
-          } else {
-            ForwardTreeBody<double>(V, S, A.dvec, A.inv, buf, ys);
-          }
-          break;
+    if (active) {
+      if (type == kTaskFrontForward) {
+        if (f32) {
+          FrontForward<float>(V, S, A, part, buf, wait);
+        } else {
+          FrontForward<double>(V, S, A, part, buf, wait);
         }
-        case kTaskForwardRows:
-          if (f32) {
-            ForwardRowsTask<float>(V, S, A.ys, part, buf);
-          } else {
-            ForwardRowsTask<double>(V, S, A.ys, part, buf);
-          }
-          break;
-        case kTaskRootGather:
-          RootGather(V, S, A.ys, buf);
-          break;
-        case kTaskRootForward:
-          if (S.dense_cnt >= 0) {
-            RootPanel64<true>(V, S, A, part, buf);
-          } else if (f32) {
-            RootForwardPanel<float>(V, S, A, part, pflag, buf);
-          } else {
-            RootForwardPanel<double>(V, S, A, part, pflag, buf);
-          }
-          break;
-        case kTaskRootBackward:
-          if (S.dense_cnt >= 0) {
-            RootPanel64<false>(V, S, A, part, buf);
-          } else if (f32) {
-            RootBackwardPanel<float>(V, S, A, part, bflag, buf);
-          } else {
-            RootBackwardPanel<double>(V, S, A, part, bflag, buf);
-          }
-          break;
-        case kTaskBackwardRows:
-          if (f32) {
-            BackwardRowsTask<float>(V, S, part, A.zpart + A.zoff[s], buf);
-          } else {
-            BackwardRowsTask<double>(V, S, part, A.zpart + A.zoff[s], buf);
-          }
-          break;
-        default: {
-          const int parts = A.zoff[s] >= 0 ? A.parts[2 * s] - 1 : 0;
-          const double* zp = parts > 0 ? A.zpart + A.zoff[s] : nullptr;
-          if (f32) {
-            BackwardTreeBody<float>(V, S, A.inv, buf, zp, parts);
-          } else {
-            BackwardTreeBody<double>(V, S, A.inv, buf, zp, parts);
-          }
-          break;
+      } else if (type == kTaskFrontBackward) {
+        const int parts = A.parts[2 * s];
+        double* zp = A.zpart + A.zoff[s];
+        if (f32) {
+          done = FrontBackward<float>(V, S, A, part, parts, zdone + s, zp, buf, wait);
+        } else {
+          done = FrontBackward<double>(V, S, A, part, parts, zdone + s, zp, buf, wait);
+        }
+      } else if (wait()) {
+        switch (type) {
+          case kTaskRootForward:
+            if (S.dense_cnt >= 0) {
+              RootPanel64<true>(V, S, A, part, buf);
+            } else if (kPanels) {
+              if (f32) {
+                RootForwardPanel<float>(V, S, A, part, pflag, buf);
+              } else {
+                RootForwardPanel<double>(V, S, A, part, pflag, buf);
+              }
+            }
+            break;
+          case kTaskRootBackward:
+            if (S.dense_cnt >= 0) {
+              RootPanel64<false>(V, S, A, part, buf);
+            } else if (kPanels) {
+              if (f32) {
+                RootBackwardPanel<float>(V, S, A, part, bflag, buf);
+              } else {
+                RootBackwardPanel<double>(V, S, A, part, bflag, buf);
+              }
+            }
+            break;
+          default:
+            if (kPanels) {
+              PanelFrontTask(V, S, A, type, s, part, f32, buf);
+            }
+            break;
         }
       }
+    }
+    if (threadIdx.x == 0) {
+      next[turn ^ 1] = ahead;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-      __threadfence();
       switch (type) {
         case kTaskForward:
           if (A.zoff[s] >= 0) {
@@ -2270,6 +2898,7 @@ __global__ void __launch_bounds__(256, 1) KSolveTree(DeviceView V, SolveArgs A) 
             Publish(fdone + s);
           }
           break;
+        case kTaskFrontForward:
         case kTaskForwardRows:
           if (s != A.withhold) {
             Publish(fdone + s);
@@ -2279,20 +2908,26 @@ __global__ void __launch_bounds__(256, 1) KSolveTree(DeviceView V, SolveArgs A) 
           Publish(ydone + s);
           break;
         case kTaskRootForward:
-          Publish(pflag + S.panel_base + part);
+          if (S.dense_cnt < 0) {
+            Publish(pflag + S.panel_base + part);
+          }
           if (s != A.withhold) {
             Publish(fdone + s);
           }
           break;
         case kTaskRootBackward:
-          Publish(bflag + S.panel_base + part);
+          if (S.dense_cnt < 0) {
+            Publish(bflag + S.panel_base + part);
+          }
           Publish(bdone + s);
           break;
         case kTaskBackwardRows:
           Publish(zdone + s);
           break;
         default:
-          Publish(bdone + s);
+          if (done) {
+            Publish(bdone + s);
+          }
           break;
       }
     }
@@ -2319,7 +2954,14 @@ constexpr int kMaxSmem = 227 * 1024;
 
 int64_t FrontTaskSmem(int k, int rows) { return static_cast<int64_t>(FactorFrontSmem(k, rows)); }
 
-void ConfigureSolveKernels(int max_front) {
+/// Shared memory of the one-launch solve: a chunk's, or that of the largest
+/// front solved by panels.
+size_t SolveSmem(int solve_panel_front) {
+  const size_t chunk = kSolveDoubles * sizeof(double);
+  return solve_panel_front > 0 ? std::max(chunk, SolveTreeSmem(solve_panel_front)) : chunk;
+}
+
+void ConfigureSolveKernels(int max_front, int solve_panel_front) {
   // The attribute belongs to the kernel, not to an engine: it only grows, so
   // an engine with smaller fronts never lowers another engine's limit.
   static std::mutex mu;
@@ -2345,10 +2987,13 @@ void ConfigureSolveKernels(int max_front) {
     CudaCheck(cudaFuncSetAttribute(KBackward, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "smem attr");
     configured = smem;
   }
-  static int tree_configured = 48 * 1024;
-  const int tree = static_cast<int>(SolveTreeSmem(max_front));
+  static int tree_configured = 0;
+  const int tree = static_cast<int>(SolveSmem(solve_panel_front));
   if (tree <= kMaxSmem && tree > tree_configured) {
-    CudaCheck(cudaFuncSetAttribute(KSolveTree, cudaFuncAttributeMaxDynamicSharedMemorySize, tree), "smem attr");
+    CudaCheck(cudaFuncSetAttribute(KSolveTree<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   static_cast<int>(SolveSmem(0))),
+              "smem attr");
+    CudaCheck(cudaFuncSetAttribute(KSolveTree<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, tree), "smem attr");
     tree_configured = tree;
   }
 }
@@ -2365,6 +3010,9 @@ int LaunchFactorLevels(const Symbolic& S, const DeviceView& V, const FactorPlan&
       CudaCheck(cudaFuncSetAttribute(KPanelBlock, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      static_cast<int>(PanelBlockSmem())),
                 "block smem attr");
+      CudaCheck(cudaFuncSetAttribute(KInvertFronts, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     static_cast<int>(sizeof(InvertSmem))),
+                "inverse smem attr");
       CudaCheck(cudaFuncSetAttribute(KSchur, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      static_cast<int>(kSchurSmem)),
                 "schur smem attr");
@@ -2566,13 +3214,19 @@ int LaunchFactorLevels(const Symbolic& S, const DeviceView& V, const FactorPlan&
       }
     }
   }
-  if (P.inv != nullptr && P.num_inv > 0) {
-    // inverted diagonal blocks for the one-launch solve
+  if (P.inv != nullptr && P.num_inv + P.num_front_inv > 0) {
+    // what the one-launch solve multiplies by
     const TimedLaunch tl(P.timer, KernelTimer::kInvertDiagonal, stream,
-                         [&] { return static_cast<double>(P.num_inv) * (8.0 + 16.0) * 1024.0; });
-    KInvertDiagonal<<<static_cast<unsigned>((P.num_inv + 3) / 4), 128, 0, stream>>>(V, P.inv_tasks, P.num_inv,
-                                                                                   P.inv);
-    ++launches;
+                         [&] { return 1.5 * 8.0 * static_cast<double>(S.inv_doubles); });
+    if (P.num_front_inv > 0) {
+      KInvertFronts<<<static_cast<unsigned>(P.num_front_inv), 256, sizeof(InvertSmem), stream>>>(V, P.front_inv_tasks, P.inv);
+      ++launches;
+    }
+    if (P.num_inv > 0) {
+      KInvertDiagonal<<<static_cast<unsigned>((P.num_inv + 3) / 4), 128, 0, stream>>>(V, P.inv_tasks, P.num_inv,
+                                                                                     P.inv);
+      ++launches;
+    }
   }
   CudaCheck(cudaGetLastError(), "factor kernels");
   return launches;
@@ -2582,7 +3236,7 @@ int LaunchSolveLevels(const Symbolic& S, const DeviceView& V, const FactorPlan& 
   int launches = 0;
   const size_t smem = static_cast<size_t>(P.max_front) * sizeof(double);
   const int num_sn = static_cast<int>(S.sn.size());
-  const size_t tree_smem = SolveTreeSmem(P.max_front);
+  const size_t tree_smem = SolveSmem(S.solve_panel_front);
   if (P.solve_sync != nullptr && P.inv != nullptr && P.solve_tasks != nullptr &&
       tree_smem <= static_cast<size_t>(kMaxSmem)) {
     if (num_sn == 0) {
@@ -2595,16 +3249,16 @@ int LaunchSolveLevels(const Symbolic& S, const DeviceView& V, const FactorPlan& 
       CudaCheck(cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev), "SM count");
       return count;
     }();
-    // one resident block per SM (the kernel's register bound); blocks that
-    // find no task left return at once
-    const int blocks = std::min(P.num_solve_tasks, sms);
+    // the resident blocks: two per SM by shared memory and registers, one with
+    // fronts solved by panels; blocks that find no task left return at once
+    const int blocks = std::min(P.num_solve_tasks, S.solve_panels ? sms : 2 * sms);
     const auto words = static_cast<int64_t>(SolveSyncWords(S));
     KClearWords<<<static_cast<unsigned>(std::min<int64_t>(148, (words + 255) / 256)), 256, 0, stream>>>(
         P.solve_sync, words, P.solve_stamp);
     const TimedLaunch tl(P.timer, KernelTimer::kSolveTree, stream, [&] {
       // every entry of L read twice (forward, backward), FP32 in the grid
       // fronts of a mixed solve, and the inverted diagonal blocks
-      double b = static_cast<double>(P.num_inv) * 2.0 * 8.0 * 1024.0;
+      double b = 2.0 * 8.0 * static_cast<double>(S.inv_doubles);
       for (const SupernodeRec& r : S.sn) {
         const double k = r.ncols;
         const double elem = (P.tc_map != nullptr && r.pose_root == 0) ? 4.0 : 8.0;
@@ -2629,7 +3283,11 @@ int LaunchSolveLevels(const Symbolic& S, const DeviceView& V, const FactorPlan& 
     A.handover_cols = S.dense_inv_doubles / kDenseTileCols;
     A.withhold = P.solve_withhold;
     A.wait_limit = P.solve_wait_polls > 0 ? P.solve_wait_polls : kWaitLimit;
-    KSolveTree<<<static_cast<unsigned>(blocks), 256, tree_smem, stream>>>(V, A);
+    if (S.solve_panels) {
+      KSolveTree<true><<<static_cast<unsigned>(blocks), 256, tree_smem, stream>>>(V, A);
+    } else {
+      KSolveTree<false><<<static_cast<unsigned>(blocks), 256, tree_smem, stream>>>(V, A);
+    }
     CudaCheck(cudaGetLastError(), "solve kernel");
     return 2;
   }

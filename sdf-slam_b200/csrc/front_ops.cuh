@@ -107,6 +107,10 @@ __device__ __forceinline__ void LoadElement(double* dst, const double* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src));
 }
 __device__ __forceinline__ void LoadElement(double* dst, const float* src) { *dst = static_cast<double>(*src); }
+__device__ __forceinline__ void LoadElement(float* dst, const float* src) {
+  const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src));
+}
 __device__ __forceinline__ void WaitElements() {
   asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
 }

@@ -186,10 +186,11 @@ struct SupernodeRec {
   int32_t instance;
   int32_t pose_root;  // 1: the dense pose block of its instance
   int32_t upper_l11;  // 1: L of the pivot block is stored transposed in its upper triangle
-  int32_t panel_base; // first of its ceil(ncols / 32) inverted diagonal blocks
+  int32_t panel_base; // a front solved by 32-column panels: first of its inverted diagonal blocks
   int64_t tc_pack;    // first packed operand row of its tensor-core Schur update (within its level), or -1
   int64_t dense_cnt;  // a tiled dense root: first of its tile counters, else -1
   int64_t dense_inv;  // a tiled dense root: first double of its diagonal-tile inverses
+  int64_t inv_off;    // a front of at most kSolvePivots pivots: first double of L11^-1 (row major), else -1
 };
 
 /// Task types of the one-launch solve.
@@ -201,6 +202,8 @@ enum SolveTask : int32_t {
   kTaskRootBackward = 4, // one 32-row panel of a panel-split root, backward
   kTaskBackwardRows = 5, // L21^T x_R over one chunk of rows of a wide front
   kTaskBackward = 6,     // z = x_k - L21^T x_R, pivot block back-substitution
+  kTaskFrontForward = 7,   // y = L11^-1 v and u = v_m - L21 y for one chunk of rows
+  kTaskFrontBackward = 8,  // L21^T x_R over one chunk of rows, the last one x = L11^-T z
 };
 /// Fronts with more than small_pivots pivots factor their pivot block in
 /// outer blocks of kOuterPanels 32-column panels, one of two ways (the
@@ -251,6 +254,26 @@ constexpr int kBlockRows = 64;
 constexpr int kSolveWideRows = 512;
 constexpr int kSolveRowChunk = 256;
 constexpr int kSolveRootSplit = 256;
+/// Doubles per inverted 32-column diagonal block (the unit triangle's inverse
+/// and its transpose). Columns a task inverts of a pivot block: all of it, or
+/// a strip of it past kFrontInvCols.
+constexpr int kInvBlockDoubles = 2 * 32 * 32;
+constexpr int kFrontInvCols = 64;
+constexpr int kFrontInvStrip = 16;
+/// Fronts with at most kSolvePivots pivots solve by the inverse of their
+/// pivot block, each chunk of rows by its own task: a chunk forms y = L11^-1 v
+/// again rather than wait for another task's, which costs k^2 / 2 reads from L2
+/// beside the chunk's own k rows. Past that many pivots the repeated product
+/// outweighs the chunk (43 rows at 256 pivots) and the front solves by 32-column
+/// panels. kSolveSlab: the values of L a task holds in shared memory, so that
+/// two blocks fit one SM; SolveRows: the rows of a chunk.
+constexpr int kSolvePivots = 256;
+constexpr int kSolveSlab = 11264;
+constexpr int kSolveMaxRows = 1024;
+constexpr int SolveRows(int k) {
+  const int rows = kSolveSlab / (k > 0 ? k : 1) - 1;
+  return rows < kSolveMaxRows ? rows : kSolveMaxRows;
+}
 
 /// One task of the pose Schur complement (KPoseSchur): the part of the pose
 /// root's 64 x 64 tile (I, J), I >= J, that the fronts [q0, q1) of its
@@ -334,19 +357,24 @@ struct Symbolic {
   // buffer is reused level after level (tc_pack_rows rows of the widest).
   // Task list of the one-launch solve, in the order blocks take them: the
   // forward tasks of every supernode in level order, then the backward
-  // tasks in reverse. (type, sn, part, 0) quads, SolveTask types. A front
-  // with at least kSolveWideRows rows below its pivots splits its forward
-  // update u = v_m - L21 y and its backward product L21^T x_R into chunks of
-  // kSolveRowChunk rows; a front without rows below and with more than
-  // small_pivots pivots (a dense pose root) solves its pivot block by
-  // 32-row panels, one task per panel, each waiting for the panels before
-  // it. solve_parts: per supernode, the forward and backward tasks whose
-  // completion its dependents wait for; zpart_off: per supernode the first
-  // double of its backward partial products (-1 when not split).
+  // tasks in reverse. (type, sn, part, 0) quads, SolveTask types. A front of
+  // at most kSolvePivots pivots takes one task per chunk of SolveRows rows
+  // each way; a tiled dense root one per 64-row panel. Other fronts solve by
+  // 32-column panels (solve_panels: there are some): with at least
+  // kSolveWideRows rows below the pivots the forward update u = v_m - L21 y
+  // and the backward product L21^T x_R split into chunks of kSolveRowChunk
+  // rows, and without rows below the pivot block splits into one task per
+  // panel, each waiting for the panels before it. solve_parts: per supernode,
+  // the forward and backward tasks whose completion its dependents wait for;
+  // zpart_off: per supernode the first double of its backward partial products
+  // (-1 when not split); solve_panel_front: rows of the largest front solved
+  // by 32-column panels.
   std::vector<int32_t> solve_tasks;
   std::vector<int32_t> solve_parts;
   std::vector<int64_t> zpart_off;
   int64_t zpart_doubles{0};
+  bool solve_panels{false};
+  int solve_panel_front{0};
   std::vector<int32_t> pack_tasks;
   std::vector<TaskRange> pack_range;
   std::vector<int32_t> tc_tasks;
@@ -398,9 +426,12 @@ struct Symbolic {
   // block take the tensor-core Schur update (0: none does)
   int tc_min_rows{kTcMinRowsDefault};
   std::vector<int> height;                   // per supernode: height in the assembly tree
-  // (sn, panel) of every 32-column diagonal block, in panel_base order: the
-  // inverted unit triangles the solve multiplies by
+  // what the solve multiplies by: (sn, panel) of every 32-column diagonal
+  // block of the fronts solved by panels, in panel_base order, and (sn, first
+  // column) of the other fronts' inverses; the doubles of both
   std::vector<int32_t> inv_tasks;
+  std::vector<int32_t> front_inv_tasks;
+  int64_t inv_doubles{0};
   std::vector<int32_t> small_tasks;
   std::vector<TaskRange> small_range;        // per level
   std::vector<int64_t> small_smem;           // per level: shared memory of its largest task

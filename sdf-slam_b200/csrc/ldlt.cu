@@ -69,7 +69,7 @@ LdltEngine::LdltEngine(int n, const int32_t* outer, const int32_t* inner, const 
   for (const SupernodeRec& r : sym_.sn) {
     max_front = std::max(max_front, r.F);
   }
-  ConfigureSolveKernels(max_front);
+  ConfigureSolveKernels(max_front, sym_.solve_panel_front);
   V_.num_inst = 1;
   V_.n = n;
   V_.perm = perm_.get();
@@ -112,9 +112,12 @@ LdltEngine::LdltEngine(int n, const int32_t* outer, const int32_t* inner, const 
   plan_.ys = ys_.get();
   plan_.zpart = zpart_.get();
   inv_tasks_.Upload(sym_.inv_tasks, s);
-  inv_.Alloc(std::max<size_t>(1, sym_.inv_tasks.size() / 2) * kInvBlockDoubles);
+  front_inv_tasks_.Upload(sym_.front_inv_tasks, s);
+  inv_.Alloc(static_cast<size_t>(std::max<int64_t>(1, sym_.inv_doubles)));
   plan_.inv_tasks = inv_tasks_.get();
   plan_.num_inv = static_cast<int>(sym_.inv_tasks.size() / 2);
+  plan_.front_inv_tasks = front_inv_tasks_.get();
+  plan_.num_front_inv = static_cast<int>(sym_.front_inv_tasks.size() / 2);
   plan_.inv = inv_.get();
   CudaCheck(cudaStreamSynchronize(s), "ldlt analyze");
 }

@@ -551,13 +551,37 @@ void Finalize(Symbolic& S, std::vector<int> height, int panel_width, int tile) {
   for (SupernodeRec& r : S.sn) {
     r.upper_l11 = r.ncols <= S.small_pivots ? 1 : 0;
   }
+  // inverses the solve multiplies by: 32-column blocks first, then the pivot
+  // blocks of the other fronts
+  auto by_panels = [&tiled](const SupernodeRec& r) { return !tiled(r) && r.ncols > kSolvePivots; };
   S.inv_tasks.clear();
+  S.front_inv_tasks.clear();
+  S.solve_panels = false;
+  S.solve_panel_front = 0;
   for (int s = 0; s < Sn; ++s) {
     SupernodeRec& r = S.sn[static_cast<size_t>(s)];
     r.panel_base = static_cast<int32_t>(S.inv_tasks.size() / 2);
-    for (int p = 0; p * B < r.ncols; ++p) {
-      S.inv_tasks.push_back(s);
-      S.inv_tasks.push_back(p);
+    if (by_panels(r)) {
+      S.solve_panels = true;
+      S.solve_panel_front = std::max(S.solve_panel_front, r.F);
+      for (int p = 0; p * B < r.ncols; ++p) {
+        S.inv_tasks.push_back(s);
+        S.inv_tasks.push_back(p);
+      }
+    }
+  }
+  S.inv_doubles = static_cast<int64_t>(S.inv_tasks.size() / 2) * kInvBlockDoubles;
+  for (int s = 0; s < Sn; ++s) {
+    SupernodeRec& r = S.sn[static_cast<size_t>(s)];
+    r.inv_off = -1;
+    if (!by_panels(r) && !tiled(r)) {
+      r.inv_off = S.inv_doubles;
+      S.inv_doubles += static_cast<int64_t>(r.ncols) * r.ncols;
+      const int step = r.ncols <= kFrontInvCols ? kFrontInvCols : kFrontInvStrip;
+      for (int c = 0; c < r.ncols; c += step) {
+        S.front_inv_tasks.push_back(s);
+        S.front_inv_tasks.push_back(c);
+      }
     }
   }
   // blocks that keep every SM of a B200 (148) busy
@@ -815,10 +839,27 @@ void Finalize(Symbolic& S, std::vector<int> height, int panel_width, int tile) {
   for (int q = 0; q < Sn; ++q) {
     const int s = S.level_sn[static_cast<size_t>(q)];
     const SupernodeRec& r = S.sn[static_cast<size_t>(s)];
-    if (root_split(r)) {
-      // a tiled dense root solves by 64-row panels with its tile inverses
-      const int pw = tiled(r) ? kDenseTileCols : B;
-      const int np = (r.ncols + pw - 1) / pw;
+    if (tiled(r)) {
+      // by 64-row panels with the factorization's tile inverses
+      const int np = (r.ncols + kDenseTileCols - 1) / kDenseTileCols;
+      for (int p = 0; p < np; ++p) {
+        push_task(kTaskRootForward, s, p);
+      }
+      S.solve_parts[2 * static_cast<size_t>(s)] = np;
+      S.solve_parts[2 * static_cast<size_t>(s) + 1] = np;
+    } else if (!by_panels(r)) {
+      const int rows = SolveRows(r.ncols);
+      const int chunks = std::max(1, (r.nrows + rows - 1) / rows);
+      for (int p = 0; p < chunks; ++p) {
+        push_task(kTaskFrontForward, s, p);
+      }
+      S.solve_parts[2 * static_cast<size_t>(s)] = chunks;
+      if (chunks > 1) {
+        S.zpart_off[static_cast<size_t>(s)] = S.zpart_doubles;
+        S.zpart_doubles += static_cast<int64_t>(chunks) * r.ncols;
+      }
+    } else if (root_split(r)) {
+      const int np = (r.ncols + B - 1) / B;
       push_task(kTaskRootGather, s, 0);
       for (int p = 0; p < np; ++p) {
         push_task(kTaskRootForward, s, p);
@@ -841,10 +882,14 @@ void Finalize(Symbolic& S, std::vector<int> height, int panel_width, int tile) {
   for (int q = Sn - 1; q >= 0; --q) {
     const int s = S.level_sn[static_cast<size_t>(q)];
     const SupernodeRec& r = S.sn[static_cast<size_t>(s)];
-    if (root_split(r)) {
+    if (tiled(r) || (by_panels(r) && root_split(r))) {
       const int pw = tiled(r) ? kDenseTileCols : B;
       for (int p = (r.ncols + pw - 1) / pw - 1; p >= 0; --p) {
         push_task(kTaskRootBackward, s, p);
+      }
+    } else if (!by_panels(r)) {
+      for (int p = 0; p < S.solve_parts[2 * static_cast<size_t>(s)]; ++p) {
+        push_task(kTaskFrontBackward, s, p);
       }
     } else if (r.nrows >= kSolveWideRows) {
       const int chunks = (r.nrows + kSolveRowChunk - 1) / kSolveRowChunk;
