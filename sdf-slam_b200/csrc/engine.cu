@@ -830,8 +830,12 @@ void Engine::LaunchRows() {
 }
 
 int64_t Engine::ZeroTaskCount() const {
-  // the leaf fronts' trailing columns only for an in-place tensor-core
-  // Schur complement
+  // without FP32 fronts the pivot columns (KChildSchur writes the others);
+  // the leaf fronts' trailing columns only for an in-place tensor-core Schur
+  // complement
+  if (!any_mixed_) {
+    return sym_.zero_pivots;
+  }
   return V_.tc_schur != 0 ? static_cast<int64_t>(sym_.zero_tasks.size() / 2) : sym_.zero_main;
 }
 
@@ -912,11 +916,14 @@ FactorPlan Engine::Plan() {
   P.num_front_inv = static_cast<int>(sym_.front_inv_tasks.size() / 2);
   P.inv = inv_.get();
   P.fp32_fronts = any_mixed_;
+  P.fp64_trees = std::any_of(mixed_.begin(), mixed_.end(), [](int32_t v) { return v == 0; });
   P.dense_tasks = dense_tasks_.get();
   P.dense_sync = dense_sync_.get();
   P.dense_inv = dense_inv_.get();
   P.pose = PoseSchurArgs{pose_tasks_.get(), static_cast<int64_t>(sym_.pose_tasks.size()), pose_fronts_.get(),
                          pose_mask_.get(), pose_start_.get(), dvec_.get(), pose_parts_.get(), pose_counters_.get()};
+  P.child_tasks = child_tasks_.get();
+  P.child_entries = child_entries_.get();
   P.solve_withhold = solve_withhold_;
   P.solve_wait_polls = solve_wait_polls_;
   // only the iteration's own factor and solve phases are timed
@@ -1056,6 +1063,8 @@ void Engine::SetSolveFault(int withhold, uint32_t wait_polls) {
 
 void Engine::UploadSolveTasks(cudaStream_t s) {
   zero_tasks_.Upload(sym_.zero_tasks, s);
+  child_tasks_.Upload(sym_.child_tasks, s);
+  child_entries_.Upload(sym_.child_entries, s);
   if (!sym_.pose_tasks.empty()) {
     pose_tasks_.Upload(sym_.pose_tasks, s);
     pose_fronts_.Upload(sym_.pose_fronts, s);

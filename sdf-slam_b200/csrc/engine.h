@@ -174,15 +174,21 @@ struct FactorPlan {
   const int32_t* pack_tasks{nullptr};
   const int32_t* tc_tasks{nullptr};
   TcArgs tc{};
-  /// Whether any front may be factored in FP32 (a mixed instance): their
-  /// Schur tiles take KUpdate, the FP64 ones KSchur.
+  /// Whether any front may be factored in FP32 (a mixed instance: its Schur
+  /// tiles take KSchurF32 and the tensor cores), and whether any instance is
+  /// not mixed (its Schur tiles take KChildSchur).
   bool fp32_fronts{false};
+  bool fp64_trees{true};
   /// Tiled dense roots: task quads (Symbolic::dense_tasks), the sync words
   /// (a claim counter per level, the abort flag, then the tile counters;
   /// zeroed by the caller before every factorization) and the inverse workspace.
   const int32_t* dense_tasks{nullptr};
   int32_t* dense_sync{nullptr};
   double* dense_inv{nullptr};
+  /// Tiles of the parents' fronts and their children's rows (Symbolic::
+  /// child_tasks): the grid Schur complements where no front is FP32.
+  const ChildTask* child_tasks{nullptr};
+  const ChildEntry* child_entries{nullptr};
   /// Pose Schur complement (count 0: no pose rows below any front).
   PoseSchurArgs pose{};
   /// Test hook of the one-launch solve: a supernode whose forward flag is
@@ -513,6 +519,8 @@ class Engine {
   DevBuf<int32_t> ea_tasks_, ea_child_, panel_tasks_, update_tasks_, small_tasks_;
   DevBuf<double> fronts_, upd_;
   DevBuf<int32_t> dense_tasks_, dense_sync_;  // tiled dense roots
+  DevBuf<ChildTask> child_tasks_;
+  DevBuf<ChildEntry> child_entries_;
   DevBuf<PoseTask> pose_tasks_;               // pose Schur complement
   DevBuf<int32_t> pose_fronts_, pose_start_, pose_counters_;
   DevBuf<uint64_t> pose_mask_;

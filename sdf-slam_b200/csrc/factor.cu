@@ -630,45 +630,6 @@ __global__ void __launch_bounds__(kFrontThreads, 2) KFactorFront(DeviceView V, c
   }
 }
 
-/// Adds one 64 x 64 tile of a front's Schur complement (cur - acc over the
-/// front's trailing rows r and columns c, r >= c; rows and columns counted
-/// from the front's first row, k pivots) into the parent front at the rows
-/// rel[r - k], rel[c - k]. All sixteen parent reads first, then the writes.
-template <typename TP, typename T>
-__device__ __forceinline__ void ScatterSchur(TP* Fp, int64_t PF, const int32_t* rel, int k, int F, int r0, int cc0,
-                                             const T (&cur)[4][4], const T (&acc)[4][4]) {
-  const int tx = threadIdx.x % 16;
-  const int ty = threadIdx.x / 16;
-  int64_t pos[4][4];
-#pragma unroll
-  for (int b = 0; b < 4; ++b) {
-    const int c = cc0 + ty + 16 * b;
-    const int64_t pc = c < F ? static_cast<int64_t>(rel[c - k]) * PF : -1;
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-      const int r = r0 + tx + 16 * a;
-      pos[a][b] = (pc >= 0 && r < F && r >= c) ? pc + rel[r - k] : -1;
-    }
-  }
-  TP old[4][4];
-#pragma unroll
-  for (int b = 0; b < 4; ++b) {
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-      old[a][b] = pos[a][b] >= 0 ? Fp[pos[a][b]] : TP(0);
-    }
-  }
-#pragma unroll
-  for (int b = 0; b < 4; ++b) {
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-      if (pos[a][b] >= 0) {
-        Fp[pos[a][b]] = old[a][b] + static_cast<TP>(static_cast<T>(cur[a][b] - acc[a][b]));
-      }
-    }
-  }
-}
-
 template <typename T>
 __device__ __forceinline__ void UpdateBody(const DeviceView& V, const SupernodeRec& S, int panel, int ti, int tj,
                                            const double* dvec, T (*As)[kTile], T (*Bs)[kTile]) {
@@ -684,7 +645,7 @@ __device__ __forceinline__ void UpdateBody(const DeviceView& V, const SupernodeR
     r0 = ke + ti * kTile;
     cc0 = ke + tj * kTile;
     clim = S.ncols;
-  } else if (panel <= -2) {
+  } else {
     // outer blocks of kOuterPanels panels (UpdateCodeInner / Outer): a
     // panel's update within its outer block, or the finished block's
     // rank-(kOuterPanels * kPanel) update of the pivot columns past it
@@ -701,12 +662,6 @@ __device__ __forceinline__ void UpdateBody(const DeviceView& V, const SupernodeR
     }
     r0 = ke + ti * kTile;
     cc0 = ke + tj * kTile;
-  } else {
-    kb = 0;
-    ke = S.ncols;
-    r0 = S.ncols + ti * kTile;
-    cc0 = S.ncols + tj * kTile;
-    clim = F;
   }
   T* Fs = WorkFront<T>(V, S);
   const double* d = dvec + S.first_col;
@@ -722,9 +677,7 @@ __device__ __forceinline__ void UpdateBody(const DeviceView& V, const SupernodeR
     }
   }
   // the tile's current values, loaded now so that their latency hides
-  // behind the K loop (no other block touches this tile); a leaf's trailing
-  // block holds no child contribution and is taken as zero, not loaded
-  const bool fresh = panel == -1 && S.child_count == 0;
+  // behind the K loop (no other block touches this tile)
   T cur[4][4];
 #pragma unroll
   for (int b = 0; b < 4; ++b) {
@@ -732,7 +685,7 @@ __device__ __forceinline__ void UpdateBody(const DeviceView& V, const SupernodeR
 #pragma unroll
     for (int a = 0; a < 4; ++a) {
       const int r = r0 + tx + 16 * a;
-      cur[a][b] = (!fresh && c < clim && r < F && r >= c) ? Fs[static_cast<int64_t>(c) * F + r] : T(0);
+      cur[a][b] = (c < clim && r < F && r >= c) ? Fs[static_cast<int64_t>(c) * F + r] : T(0);
     }
   }
   // K chunks of kPanel columns: the next chunk is loaded into registers
@@ -795,18 +748,6 @@ __device__ __forceinline__ void UpdateBody(const DeviceView& V, const SupernodeR
     }
     __syncthreads();
   }
-  if (panel == -1 && S.parent >= 0) {
-    // the Schur complement goes straight into the parent's front (what the
-    // extend-add did with the update matrix), T-rounded as it was stored
-    const SupernodeRec P = V.sn[S.parent];
-    const int32_t* rel = V.sn_rel + S.rows_off;
-    if (Fp32Front(V, P)) {
-      ScatterSchur<float, T>(WorkFront<float>(V, P), P.F, rel, S.ncols, F, r0, cc0, cur, acc);
-    } else {
-      ScatterSchur<double, T>(WorkFront<double>(V, P), P.F, rel, S.ncols, F, r0, cc0, cur, acc);
-    }
-    return;
-  }
 #pragma unroll
   for (int b = 0; b < 4; ++b) {
     const int c = cc0 + ty + 16 * b;
@@ -824,17 +765,13 @@ __device__ __forceinline__ void UpdateBody(const DeviceView& V, const SupernodeR
 }
 
 /// Tiled rank-k update C -= L_I D L_J^T (lower part only). panel <= -2: the
-/// outer-block updates (UpdateCodeInner / Outer). panel >= 0:
-/// update of the remaining pivot columns by one panel; panel == -1: Schur
-/// complement of the trailing m x m block by all k pivots.
+/// outer-block updates (UpdateCodeInner / Outer). panel >= 0: update of the
+/// remaining pivot columns by one panel.
 __global__ void __launch_bounds__(256, 2) KUpdate(DeviceView V, const int32_t* tasks, const double* dvec) {
   const int32_t* t = tasks + 4 * static_cast<int64_t>(blockIdx.x);
   const SupernodeRec S = V.sn[t[0]];
   if (V.active[S.instance] == 0) {
     return;
-  }
-  if (t[1] == -1) {
-    return;  // Schur tiles: KSchur, KSchurF32; wide FP32 fronts: the tensor cores
   }
   __shared__ double as_buf[kPanel * kTile];
   __shared__ double bs_buf[kPanel * kTile];
@@ -848,74 +785,23 @@ __global__ void __launch_bounds__(256, 2) KUpdate(DeviceView V, const int32_t* t
 }
 
 /// Schur complement tiles added into the parent front (the task list of the
-/// Schur update, panel -1), FP64 fronts and the FP32 fronts of a mixed solve
-/// that the tensor cores do not take, built for occupancy: the K chunks are
-/// copied global -> shared with cp.async (element-sized copies: a front's
-/// columns start at any element offset), two chunks in flight, so no
-/// staging registers; each thread then scales the A entries it copied by d
-/// (the same product the register path forms); the tile's current values
-/// are read after the K loop. Three blocks per SM (64 KB of shared memory
-/// each; an FP32 tile uses half) against two for KUpdate.
+/// Schur update, panel -1): the FP32 fronts of a mixed solve that the tensor
+/// cores do not take (FP64 fronts: KChildSchur), built for occupancy: the K
+/// chunks are copied global -> shared with cp.async (element-sized copies: a
+/// front's columns start at any element offset), two chunks in flight, so no
+/// staging registers; each thread then scales the A entries it copied by d;
+/// the tile's current values are read after the K loop.
 constexpr int kSchurK = 32;
 constexpr int kSchurBlocksPerSm = 3;
 constexpr int kSchurPerThread = kSchurK * 64 / 256;  // entries of a chunk each thread copies
-constexpr size_t kSchurSmem = 2 * 2 * static_cast<size_t>(kSchurK) * 64 * sizeof(double);
+constexpr size_t kSchurSmem = 2 * 2 * static_cast<size_t>(kSchurK) * 64 * sizeof(float);
 
-__device__ __forceinline__ void CpAsync(double* dst, const double* src) {
-  const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
-}
 __device__ __forceinline__ void CpAsync(float* dst, const float* src) {
   const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
 }
 
-/// The end of a KSchur tile: C - acc added into the parent front (or written
-/// in place for a front with no parent), one column group of four entries at
-/// a time, all parent reads of a group before its writes. kLoadC false: C is
-/// known to be zero and is not read.
-template <bool kLoadC>
-__device__ __forceinline__ void SchurEpilogue(const DeviceView& V, const SupernodeRec& S, const double* Fs, int r0,
-                                              int c0, const double (&acc)[4][4]) {
-  const int k = S.ncols;
-  const int F = S.F;
-  const int fc = S.fcols;
-  const int tx = threadIdx.x & 15;
-  const int ty = threadIdx.x >> 4;
-  const bool scatter = S.parent >= 0;
-  const SupernodeRec P = scatter ? V.sn[S.parent] : S;
-  const int32_t* rel = V.sn_rel + S.rows_off;
-  double* Fp = scatter ? V.fronts + P.front_off : V.fronts + S.front_off;
-  const int64_t PF = P.F;
-#pragma unroll
-  for (int b = 0; b < 4; ++b) {
-    const int c = c0 + ty + 16 * b;
-    double cur[4];
-    int64_t pos[4];
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-      const int r = r0 + tx + 16 * a;
-      const bool in = c < fc && r < F && r >= c;
-      cur[a] = (kLoadC && in) ? Fs[static_cast<int64_t>(c) * F + r] : 0.0;
-      pos[a] = !in ? -1
-                   : (scatter ? static_cast<int64_t>(rel[c - k]) * PF + rel[r - k] : static_cast<int64_t>(c) * F + r);
-    }
-    double old[4];
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-      old[a] = (scatter && pos[a] >= 0) ? Fp[pos[a]] : 0.0;
-    }
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-      if (pos[a] >= 0) {
-        Fp[pos[a]] = scatter ? old[a] + (cur[a] - acc[a][b]) : cur[a] - acc[a][b];
-      }
-    }
-  }
-}
-
-/// The end of a KSchur tile of an FP32 front (the SIMT Schur complement of
-/// a mixed solve): the tile's values (zero for a leaf, not loaded) minus
+/// The end of a KSchurF32 tile: the tile's values (zero for a leaf, not loaded) minus
 /// acc, added into the parent front Fp (FP32, or the FP64 pose root), or
 /// written in place for a front with no parent (Fp is then the front
 /// itself); one column group of four entries at a time, all parent reads of
@@ -955,14 +841,12 @@ __device__ __forceinline__ void SchurEpilogueF32(TP* Fp, int64_t PF, const int32
   }
 }
 
-/// One 64 x 64 Schur complement tile of a front held in T (double: the
-/// plain path and the pose root; float: a mixed solve's grid fronts that
-/// the tensor cores do not take): K chunks staged by cp.async, two in
-/// flight, A scaled by d in shared memory, acc accumulated in T in
-/// ascending pivot order.
-template <typename T>
+/// One 64 x 64 Schur complement tile of an FP32 front of a mixed solve that
+/// the tensor cores do not take: K chunks staged by cp.async, two in flight,
+/// A scaled by d in shared memory, acc accumulated in ascending pivot order.
 __device__ __forceinline__ void SchurTile(const DeviceView& V, const SupernodeRec& S, const int32_t* t,
-                                          const double* dvec, T* sm) {
+                                          const double* dvec, float* sm) {
+  using T = float;
   auto As = reinterpret_cast<T(*)[kSchurK][64]>(sm);
   auto Bs = reinterpret_cast<T(*)[kSchurK][64]>(sm + 2 * kSchurK * 64);
   const int k = S.ncols;
@@ -1050,46 +934,21 @@ __device__ __forceinline__ void SchurTile(const DeviceView& V, const SupernodeRe
       issue((ch + 2) * kSchurK, buf);
     }
   }
-  if constexpr (sizeof(T) == sizeof(double)) {
-    // C - acc, added into the parent (or written in place for a front with
-    // no parent); a leaf's C is zero (no child adds into it) and is not
-    // loaded
-    if (S.child_count == 0) {
-      SchurEpilogue<false>(V, S, Fs, r0, c0, acc);
-    } else {
-      SchurEpilogue<true>(V, S, Fs, r0, c0, acc);
-    }
+  // a leaf's C is zero (no child adds into it) and is not loaded
+  const float* C = S.child_count > 0 ? Fs : nullptr;
+  if (S.parent < 0) {
+    SchurEpilogueF32<float>(Fs, F, nullptr, C, k, F, fc, r0, c0, acc);
   } else {
-    // a leaf's C is zero (no child adds into it) and is not loaded
-    const float* C = S.child_count > 0 ? Fs : nullptr;
-    if (S.parent < 0) {
-      SchurEpilogueF32<float>(Fs, F, nullptr, C, k, F, fc, r0, c0, acc);
+    const SupernodeRec P = V.sn[S.parent];
+    const int32_t* rel = V.sn_rel + S.rows_off;
+    if (Fp32Front(V, P)) {
+      SchurEpilogueF32<float>(WorkFront<float>(V, P), P.F, rel, C, k, F, fc, r0, c0, acc);
     } else {
-      const SupernodeRec P = V.sn[S.parent];
-      const int32_t* rel = V.sn_rel + S.rows_off;
-      if (Fp32Front(V, P)) {
-        SchurEpilogueF32<float>(WorkFront<float>(V, P), P.F, rel, C, k, F, fc, r0, c0, acc);
-      } else {
-        SchurEpilogueF32<double>(WorkFront<double>(V, P), P.F, rel, C, k, F, fc, r0, c0, acc);
-      }
+      SchurEpilogueF32<double>(WorkFront<double>(V, P), P.F, rel, C, k, F, fc, r0, c0, acc);
     }
   }
 }
 
-__global__ void __launch_bounds__(256, kSchurBlocksPerSm)
-    KSchur(DeviceView V, const int32_t* tasks, const double* dvec) {
-  const int32_t* t = tasks + 4 * static_cast<int64_t>(blockIdx.x);
-  const SupernodeRec S = V.sn[t[0]];
-  if (V.active[S.instance] == 0 || Fp32Front(V, S)) {
-    return;  // FP32 fronts of a mixed solve: KSchurF32 or the tensor cores
-  }
-  extern __shared__ __align__(16) double schur_sm[];
-  SchurTile<double>(V, S, t, dvec, schur_sm);
-}
-
-/// The same tiles for the FP32 fronts of a mixed solve that the tensor
-/// cores do not take (a kernel of its own, so that neither variant's
-/// registers limit the other's).
 __global__ void __launch_bounds__(256, kSchurBlocksPerSm)
     KSchurF32(DeviceView V, const int32_t* tasks, const double* dvec) {
   const int32_t* t = tasks + 4 * static_cast<int64_t>(blockIdx.x);
@@ -1097,8 +956,8 @@ __global__ void __launch_bounds__(256, kSchurBlocksPerSm)
   if (V.active[S.instance] == 0 || !Fp32Front(V, S) || (S.tc_pack >= 0 && V.tc_schur != 0)) {
     return;
   }
-  extern __shared__ __align__(16) double schur_sm[];
-  SchurTile<float>(V, S, t, dvec, reinterpret_cast<float*>(schur_sm));
+  extern __shared__ __align__(16) float schur_sm[];
+  SchurTile(V, S, t, dvec, schur_sm);
 }
 
 template <typename T>
@@ -3013,9 +2872,6 @@ int LaunchFactorLevels(const Symbolic& S, const DeviceView& V, const FactorPlan&
       CudaCheck(cudaFuncSetAttribute(KInvertFronts, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      static_cast<int>(sizeof(InvertSmem))),
                 "inverse smem attr");
-      CudaCheck(cudaFuncSetAttribute(KSchur, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(kSchurSmem)),
-                "schur smem attr");
       if (dev >= 0 && dev < 64) {
         configured[dev] = true;
       }
@@ -3037,6 +2893,23 @@ int LaunchFactorLevels(const Symbolic& S, const DeviceView& V, const FactorPlan&
     return w;
   };
   for (int l = 0; l < S.num_levels; ++l) {
+    const TaskRange pull = P.fp64_trees ? S.child_range[static_cast<size_t>(l)] : TaskRange{};
+    if (pull.count > 0) {
+      const TimedLaunch tl(P.timer, KernelTimer::kUpdateSchur, stream, [&] {
+        return level_sum(l, [&S](const SupernodeRec& r) {
+          double w = 0.0;
+          for (int ci = 0; ci < r.child_count; ++ci) {
+            const SupernodeRec& c = S.sn[static_cast<size_t>(S.child_list[static_cast<size_t>(r.child_begin + ci)])];
+            const double m = c.nrows;
+            const double p = c.F - c.fcols;
+            w += static_cast<double>(c.ncols) * (m * (m + 1.0) - p * (p + 1.0));
+          }
+          return w;
+        });
+      });
+      LaunchChildSchur(V, P.child_tasks + pull.begin, pull.count, P.child_entries, P.dvec, stream);
+      ++launches;
+    }
     if (l == S.pose_level && P.pose.count > 0) {
       // every grid front is factored: their pose rows' products into the pose
       // roots, the last level
@@ -3186,6 +3059,10 @@ int LaunchFactorLevels(const Symbolic& S, const DeviceView& V, const FactorPlan&
       launches += LaunchSchurTc(*P.tc_map, P.tc, P.pack_tasks + 3 * pk.begin, pk.count, P.tc_tasks + 3 * tr.begin,
                                 tr.count, stream, P.timer, pack_bytes, tc_flops);
     }
+    if (!P.fp32_fronts) {
+      continue;
+    }
+    // a mixed solve's Schur complements, pushed by the children
     for (int q = S.schur_base[static_cast<size_t>(l)]; q < S.schur_base[static_cast<size_t>(l) + 1]; ++q) {
       const TaskRange sr = S.schur_range[static_cast<size_t>(q)];
       if (sr.count == 0) {
@@ -3203,15 +3080,9 @@ int LaunchFactorLevels(const Symbolic& S, const DeviceView& V, const FactorPlan&
                                        : static_cast<double>(r.ncols) * (m * (m + 1.0) - p * (p + 1.0));
         }) : 0.0;
       });
-      KSchur<<<static_cast<unsigned>(sr.count), 256, kSchurSmem, stream>>>(V, P.update_tasks + 4 * sr.begin,
-                                                                            P.dvec);
+      KSchurF32<<<static_cast<unsigned>(sr.count), 256, kSchurSmem, stream>>>(V, P.update_tasks + 4 * sr.begin,
+                                                                             P.dvec);
       ++launches;
-      if (P.fp32_fronts) {
-        // the FP32 fronts of a mixed solve that the tensor cores do not take
-        KSchurF32<<<static_cast<unsigned>(sr.count), 256, kSchurSmem / 2, stream>>>(
-            V, P.update_tasks + 4 * sr.begin, P.dvec);
-        ++launches;
-      }
     }
   }
   if (P.inv != nullptr && P.num_inv + P.num_front_inv > 0) {

@@ -294,6 +294,33 @@ struct PoseTask {
   int32_t counter;  // arrival counter of the parts (parts > 1)
   int64_t cost;     // relative work, the order tasks are launched in
 };
+/// One task of the grid Schur complements (KChildSchur): the 64 x 64 tile (I,
+/// J), I >= J, of a front's stored columns, and the children (entries) with
+/// rows in both of its blocks.
+struct ChildTask {
+  int64_t front;  // the front's first double
+  int32_t F;
+  int32_t k;
+  int32_t fcols;
+  int32_t instance;
+  int32_t I;
+  int32_t J;
+  int32_t begin;  // entries [begin, begin + count), in child order
+  int32_t count;
+};
+/// A child's rows in a tile: its rows from row-list position ra on fall into
+/// block I at the places `rows`, those from ca on into block J at `cols`.
+struct ChildEntry {
+  int64_t front;
+  uint64_t rows;
+  uint64_t cols;
+  int32_t F;
+  int32_t k;
+  int32_t first;  // first pivot column
+  int32_t leaf;   // 1: no update matrix of its own
+  int32_t ra;
+  int32_t ca;
+};
 /// Pose variables from which an instance's pose Schur complement is summed
 /// straight into its pose root; below, its fronts carry their pose columns up
 /// the tree, which costs no extra launch and fewer serial steps. Measured on
@@ -393,6 +420,7 @@ struct Symbolic {
   // as zero without loading them), cleared only for the tensor-core Schur
   // complement of a mixed solve, which accumulates into them in place.
   std::vector<int32_t> zero_tasks;
+  int64_t zero_pivots{0};                    // clearing tasks of pivot columns (the first ones)
   int64_t zero_main{0};
   // Pose Schur complement: the pose rows of a grid front update pose columns
   // only of the pose root, so their products are summed straight into the
@@ -405,6 +433,9 @@ struct Symbolic {
   std::vector<int32_t> pose_fronts;
   std::vector<uint64_t> pose_mask;
   std::vector<int32_t> pose_start;
+  std::vector<ChildTask> child_tasks;        // grid Schur complements pulled by their parents
+  std::vector<ChildEntry> child_entries;
+  std::vector<TaskRange> child_range;        // per level of the parents
   std::vector<PoseTask> pose_tasks;
   int64_t pose_slots{0};
   int32_t pose_counters{0};

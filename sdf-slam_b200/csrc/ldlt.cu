@@ -91,6 +91,10 @@ LdltEngine::LdltEngine(int n, const int32_t* outer, const int32_t* inner, const 
   plan_.update_tasks = update_tasks_.get();
   plan_.level_sn = level_sn_.get();
   plan_.dvec = dvec_.get();
+  child_tasks_.Upload(sym_.child_tasks, s);
+  child_entries_.Upload(sym_.child_entries, s);
+  plan_.child_tasks = child_tasks_.get();
+  plan_.child_entries = child_entries_.get();
   plan_.max_front = max_front;
   solve_sync_.Alloc(SolveSyncWords(sym_));
   plan_.solve_sync = solve_sync_.get();

@@ -41,6 +41,8 @@ class LdltEngine {
   DevBuf<double> dense_inv_;
   DevBuf<int64_t> zpart_off_;
   DevBuf<double> ys_, zpart_;
+  DevBuf<ChildTask> child_tasks_;
+  DevBuf<ChildEntry> child_entries_;
   DevBuf<int32_t> inv_tasks_, front_inv_tasks_;
   DevBuf<double> inv_;
 };

@@ -41,6 +41,7 @@ constexpr int kLd = kT + 4;    // doubles per staged pivot: the four pivots a wa
 constexpr int kStages = 3;
 constexpr int kScan = kThreads;  // fronts looked at per scan
 constexpr int kBlocksPerSm = 3;
+constexpr int kChildScan = 16;  // children looked at per scan
 
 /// One front of the current scan that has rows in both blocks.
 struct Match {
@@ -49,6 +50,8 @@ struct Match {
   int32_t F;
   int32_t k;
   int32_t first;           // first pivot column (D)
+  int32_t leaf;            // a child: without an update matrix
+  int32_t update;          // a child: front column of the first of its columns of block J
   uint32_t groups;         // 8-row groups with a row present: block I, then block J
 };
 
@@ -93,6 +96,133 @@ __device__ __forceinline__ uint32_t Groups(uint64_t m) {
   return g;
 }
 
+/// acc += sum over the matches of A D B^T, A and B the match's rows of the
+/// tile's two blocks at their positions: stages of kK pivots by asynchronous
+/// copies, kStages in flight, one match's stages behind another's. wr, wc: the
+/// warp's first row and column of the tile; matches > 0, sm.match behind a
+/// barrier. started(): called once the first stages are on their way.
+template <typename T, typename Started>
+__device__ __forceinline__ void MultiplyMatches(Smem<T>& sm, int matches, const T* fronts, const double* dvec,
+                                                bool diagonal, int wr, int wc, double (&acc)[2][4][2], Started started) {
+  const int tid = threadIdx.x;
+  const int lane = tid & 31;
+  // staging: the first four warps copy block I's rows, the others block J's;
+  // a thread copies row pos of half a stage's pivots
+  const bool side = tid >= kThreads / 2;
+  const int pos = tid & (kT - 1);
+  const int l0 = ((tid >> 6) & 1) * (kK / 2);
+  const uint64_t below = (uint64_t{1} << pos) - 1;
+  T* const dst = side ? &sm.b[0][l0][pos] : &sm.a[0][l0][pos];
+  // producer position: match pm, `left` of its pivots still to stage; the
+  // thread's sources advance by one stage (or to the next match) per issue
+  int pm = -1;
+  int left = 0;
+  const T* src = nullptr;
+  const double* src_d = nullptr;
+  int64_t F = 0;
+  int size = 0;
+  auto issue = [&](int stage) {
+    if (left <= 0 && pm < matches) {
+      if (++pm < matches) {
+        const Match& m = sm.match[pm];
+        const uint64_t mask = side ? m.mb : m.ma;
+        left = m.k;
+        F = m.F;
+        src = fronts + (side ? m.base_b : m.base_a) + l0 * F + __popcll(mask & below);
+        // absent rows are staged as zeros
+        size = ((mask >> pos) & 1) != 0 ? static_cast<int>(sizeof(T)) : 0;
+        src_d = dvec + m.first + tid;
+      }
+    }
+    if (left > 0) {
+      if (!(side && diagonal)) {
+        T* to = dst + stage * (kK * kLd);
+        if (left >= kK) {
+#pragma unroll
+          for (int l = 0; l < kK / 2; ++l) {
+            CopyZfill(to + l * kLd, src + l * F, size);
+          }
+        } else {
+          // pivots past the last are staged as zeros
+#pragma unroll
+          for (int l = 0; l < kK / 2; ++l) {
+            CopyZfill(to + l * kLd, src + l * F, l0 + l < left ? size : 0);
+          }
+        }
+        src += kK * F;
+      }
+      if (tid < kK) {
+        CopyZfill(&sm.d[stage][tid], src_d, tid < left ? 8 : 0);
+        src_d += kK;
+      }
+      left -= kK;
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int s = 0; s < kStages - 1; ++s) {
+    issue(s);
+  }
+  started();
+  int stage = 0;
+  int ahead = kStages - 1;
+  for (int cm = 0; cm < matches; ++cm) {
+    const int k = sm.match[cm].k;
+    const uint32_t ga = (sm.match[cm].groups >> (wr / 8)) & 3u;
+    const uint32_t gb = (sm.match[cm].groups >> (8 + wc / 8)) & 15u;
+    // on the diagonal tile only the lower part is used
+    const bool work = ga != 0 && gb != 0 && !(diagonal && wc >= wr + 16);
+    for (int ck = 0; ck < k; ck += kK) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
+      __syncthreads();
+      issue(ahead);
+      ahead = ahead + 1 == kStages ? 0 : ahead + 1;
+      if (work) {
+        const T* as = &sm.a[stage][lane & 3][wr + (lane >> 2)];
+        const T* bs = (diagonal ? &sm.a[stage][lane & 3][0] : &sm.b[stage][lane & 3][0]) + wc + (lane >> 2);
+        double a0[kK / 4];
+        double a1[kK / 4];
+#pragma unroll
+        for (int ks = 0; ks < kK / 4; ++ks) {
+          const double d = sm.d[stage][4 * ks + (lane & 3)];
+          a0[ks] = static_cast<double>(as[4 * ks * kLd]) * d;
+          a1[ks] = static_cast<double>(as[4 * ks * kLd + 8]) * d;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          if ((gb >> j) & 1u) {
+            double bv[kK / 4];
+#pragma unroll
+            for (int ks = 0; ks < kK / 4; ++ks) {
+              bv[ks] = static_cast<double>(bs[4 * ks * kLd + 8 * j]);
+            }
+            if (ga == 3u) {
+#pragma unroll
+              for (int ks = 0; ks < kK / 4; ++ks) {
+                Dmma884(acc[0][j], a0[ks], bv[ks]);
+                Dmma884(acc[1][j], a1[ks], bv[ks]);
+              }
+            } else if (ga == 1u) {
+#pragma unroll
+              for (int ks = 0; ks < kK / 4; ++ks) {
+                Dmma884(acc[0][j], a0[ks], bv[ks]);
+              }
+            } else {
+#pragma unroll
+              for (int ks = 0; ks < kK / 4; ++ks) {
+                Dmma884(acc[1][j], a1[ks], bv[ks]);
+              }
+            }
+          }
+        }
+      }
+      stage = stage + 1 == kStages ? 0 : stage + 1;
+    }
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+}
+
 /// Bound by the FP64 tensor cores and the barriers between stages, three
 /// blocks per SM. A warp owns 16 x 32 entries of the tile. Measured on B200
 /// (910-pose office, 1,672 tasks): 1.31 ms, tensor cores busy 42 %; the same
@@ -133,13 +263,6 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm) KPoseSchur(DeviceView 
   const int32_t* start_i = A.start + t.mask + static_cast<int64_t>(t.I) * t.len;
   const int32_t* start_j = A.start + t.mask + static_cast<int64_t>(t.J) * t.len;
   const bool diagonal = t.I == t.J;
-  // staging: the first four warps copy block I's rows, the others block J's;
-  // a thread copies row pos of half a stage's pivots
-  const bool side = tid >= kThreads / 2;
-  const int pos = tid & (kT - 1);
-  const int l0 = ((tid >> 6) & 1) * (kK / 2);
-  const uint64_t below = (uint64_t{1} << pos) - 1;
-  T* const dst = side ? &sm.b[0][l0][pos] : &sm.a[0][l0][pos];
   for (int q0 = t.q0; q0 < t.q1; q0 += kScan) {
     // the fronts of this scan with rows in both blocks, in list order
     const int q = q0 + tid;
@@ -178,113 +301,7 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm) KPoseSchur(DeviceView 
     if (matches == 0) {
       continue;
     }
-    // producer position: match pm, `left` of its pivots still to stage; the
-    // thread's sources advance by one stage (or to the next match) per issue
-    int pm = -1;
-    int left = 0;
-    const T* src = nullptr;
-    const double* src_d = nullptr;
-    int64_t F = 0;
-    int size = 0;
-    auto issue = [&](int stage) {
-      if (left <= 0 && pm < matches) {
-        if (++pm < matches) {
-          const Match& m = sm.match[pm];
-          const uint64_t mask = side ? m.mb : m.ma;
-          left = m.k;
-          F = m.F;
-          src = fronts + (side ? m.base_b : m.base_a) + l0 * F + __popcll(mask & below);
-          // absent rows are staged as zeros
-          size = ((mask >> pos) & 1) != 0 ? static_cast<int>(sizeof(T)) : 0;
-          src_d = A.dvec + m.first + tid;
-        }
-      }
-      if (left > 0) {
-        if (!(side && diagonal)) {
-          T* to = dst + stage * (kK * kLd);
-          if (left >= kK) {
-#pragma unroll
-            for (int l = 0; l < kK / 2; ++l) {
-              CopyZfill(to + l * kLd, src + l * F, size);
-            }
-          } else {
-            // pivots past the last are staged as zeros
-#pragma unroll
-            for (int l = 0; l < kK / 2; ++l) {
-              CopyZfill(to + l * kLd, src + l * F, l0 + l < left ? size : 0);
-            }
-          }
-          src += kK * F;
-        }
-        if (tid < kK) {
-          CopyZfill(&sm.d[stage][tid], src_d, tid < left ? 8 : 0);
-          src_d += kK;
-        }
-        left -= kK;
-      }
-      asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-#pragma unroll
-    for (int s = 0; s < kStages - 1; ++s) {
-      issue(s);
-    }
-    int stage = 0;
-    int ahead = kStages - 1;
-    for (int cm = 0; cm < matches; ++cm) {
-      const int k = sm.match[cm].k;
-      const uint32_t ga = (sm.match[cm].groups >> (wr / 8)) & 3u;
-      const uint32_t gb = (sm.match[cm].groups >> (8 + wc / 8)) & 15u;
-      // on the diagonal tile only the lower part is used
-      const bool work = ga != 0 && gb != 0 && !(diagonal && wc >= wr + 16);
-      for (int ck = 0; ck < k; ck += kK) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
-        __syncthreads();
-        issue(ahead);
-        ahead = ahead + 1 == kStages ? 0 : ahead + 1;
-        if (work) {
-          const T* as = &sm.a[stage][lane & 3][wr + (lane >> 2)];
-          const T* bs = (diagonal ? &sm.a[stage][lane & 3][0] : &sm.b[stage][lane & 3][0]) + wc + (lane >> 2);
-          double a0[kK / 4];
-          double a1[kK / 4];
-#pragma unroll
-          for (int ks = 0; ks < kK / 4; ++ks) {
-            const double d = sm.d[stage][4 * ks + (lane & 3)];
-            a0[ks] = static_cast<double>(as[4 * ks * kLd]) * d;
-            a1[ks] = static_cast<double>(as[4 * ks * kLd + 8]) * d;
-          }
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            if ((gb >> j) & 1u) {
-              double bv[kK / 4];
-#pragma unroll
-              for (int ks = 0; ks < kK / 4; ++ks) {
-                bv[ks] = static_cast<double>(bs[4 * ks * kLd + 8 * j]);
-              }
-              if (ga == 3u) {
-#pragma unroll
-                for (int ks = 0; ks < kK / 4; ++ks) {
-                  Dmma884(acc[0][j], a0[ks], bv[ks]);
-                  Dmma884(acc[1][j], a1[ks], bv[ks]);
-                }
-              } else if (ga == 1u) {
-#pragma unroll
-                for (int ks = 0; ks < kK / 4; ++ks) {
-                  Dmma884(acc[0][j], a0[ks], bv[ks]);
-                }
-              } else {
-#pragma unroll
-                for (int ks = 0; ks < kK / 4; ++ks) {
-                  Dmma884(acc[1][j], a1[ks], bv[ks]);
-                }
-              }
-            }
-          }
-        }
-        stage = stage + 1 == kStages ? 0 : stage + 1;
-      }
-    }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();
+    MultiplyMatches<T>(sm, matches, fronts, A.dvec, diagonal, wr, wc, acc, [] {});
   }
   if (t.parts > 1) {
     // the part's sums into its slot, thread by thread; the last part to
@@ -347,17 +364,124 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm) KPoseSchur(DeviceView 
   }
 }
 
-template <typename T>
-void Configure() {
+/// Schur complements of a level's children, pulled into their parents' fronts:
+/// a block owns one 64 x 64 tile (I, J) of a parent's stored columns and takes
+/// its children with rows in both blocks, in order: the tile becomes its
+/// assembled values (pivot columns; the others hold nothing yet) plus the
+/// children's update matrices minus L D L^T of their rows. One launch per
+/// level, one read and one write per entry and no clearing of the trailing
+/// columns; pushed by the children, two that share a parent needed a launch
+/// each (three times the reads, and half the launches nearly empty). Bound by
+/// the chain from the task to the store (task, entries, values, products) and,
+/// at the wide levels, by staging. Two blocks per SM, which keep their registers.
+/// Measured on B200, the factorization with a pushing launch per sibling -> this:
+/// 10-frame room 158 -> 120 us, 76-frame floor plan 430 -> 351, 331-pose room 1095
+/// -> 1015, 32 instances 2070 -> 1842.
+__global__ void __launch_bounds__(kThreads, 2) KChildSchur(DeviceView V, const ChildTask* tasks,
+                                                                      const ChildEntry* entries, const double* dvec) {
+  extern __shared__ __align__(16) unsigned char pose_smem[];
+  Smem<double>& sm = *reinterpret_cast<Smem<double>*>(pose_smem);
+  const ChildTask t = tasks[blockIdx.x];
+  if (V.active[t.instance] == 0 || (V.fronts32 != nullptr && V.inst[t.instance].mixed != 0)) {
+    return;
+  }
+  const int tid = threadIdx.x;
+  const int lane = tid & 31;
+  const int warp = tid >> 5;
+  const int wr = 16 * ((warp + 2 * (warp >> 2)) & 3);
+  const int wc = 32 * (warp >> 2);
+  const bool diagonal = t.I == t.J;
+  double* out = V.fronts + t.front;
+  const int r0 = wr + (lane >> 2);
+  const int c0 = wc + 2 * (lane & 3);
+  // minus the result
+  double acc[2][4][2];
+#pragma unroll
+  for (int e = 0; e < 16; ++e) {
+    const int r = t.I * kT + r0 + 8 * (e >> 3);
+    const int c = t.J * kT + c0 + 8 * ((e >> 1) & 3) + (e & 1);
+    acc[e >> 3][(e >> 1) & 3][e & 1] = c < t.k && r < t.F && c <= r ? -out[static_cast<int64_t>(c) * t.F + r] : 0.0;
+  }
+  for (int q0 = 0; q0 < t.count; q0 += kChildScan) {
+    const int n = min(kChildScan, t.count - q0);
+    if (q0 > 0) {
+      __syncthreads();
+    }
+    if (tid < n) {
+      const ChildEntry E = entries[t.begin + q0 + tid];
+      Match& m = sm.match[tid];
+      m.base_a = E.front + E.k + E.ra;
+      m.base_b = E.front + E.k + E.ca;
+      m.ma = E.rows;
+      m.mb = E.cols;
+      m.F = E.F;
+      m.k = E.k;
+      m.first = E.first;
+      m.leaf = E.leaf;
+      m.update = E.k + E.ca;
+      m.groups = Groups(E.rows) | (Groups(E.cols) << 8);
+    }
+    __syncthreads();
+    MultiplyMatches<double>(sm, n, V.fronts, dvec, diagonal, wr, wc, acc, [&] {
+      // the children's own update matrices, while the first stages arrive
+      for (int q = 0; q < n; ++q) {
+        const Match& m = sm.match[q];
+        if (m.leaf != 0) {
+          continue;
+        }
+        // rows r0 and r0 + 8, four pairs of neighbouring columns
+        const uint64_t ma = m.ma >> r0;
+        const uint64_t mb = m.mb >> c0;
+        const int64_t F = m.F;
+        const int row = __popcll(m.ma & ((uint64_t{1} << r0) - 1));
+        const int row8 = row + __popc(static_cast<uint32_t>(ma) & 0xffu);
+        int col = __popcll(m.mb & ((uint64_t{1} << c0) - 1));
+        const double* C = V.fronts + m.base_a + m.update * F;
+        double v[16];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+#pragma unroll
+          for (int b = 0; b < 2; ++b) {
+            const int c = c0 + 8 * j + b;
+            const bool in_c = ((mb >> (8 * j + b)) & 1) != 0 && t.J * kT + c < t.fcols;
+            const double* Cc = C + col * F;
+            const int below = t.J * kT + c - t.I * kT;
+            v[2 * j + b] = in_c && (ma & 1) != 0 && below <= r0 ? Cc[row] : 0.0;
+            v[8 + 2 * j + b] = in_c && ((ma >> 8) & 1) != 0 && below <= r0 + 8 ? Cc[row8] : 0.0;
+            if (b == 0) {
+              col += static_cast<int>((mb >> (8 * j)) & 1);
+            } else {
+              col += __popc(static_cast<uint32_t>(mb >> (8 * j + 1)) & 0x7fu);
+            }
+          }
+        }
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+          acc[e >> 3][(e >> 1) & 3][e & 1] -= v[e];
+        }
+      }
+    });
+  }
+#pragma unroll
+  for (int e = 0; e < 16; ++e) {
+    const int r = t.I * kT + r0 + 8 * (e >> 3);
+    const int c = t.J * kT + c0 + 8 * ((e >> 1) & 3) + (e & 1);
+    if (r < t.F && c <= r && c < t.fcols) {
+      out[static_cast<int64_t>(c) * t.F + r] = -acc[e >> 3][(e >> 1) & 3][e & 1];
+    }
+  }
+}
+
+template <auto kKernel>
+void Configure(size_t smem) {
   static std::mutex mu;
   static bool configured[64] = {};
   int dev = 0;
   CudaCheck(cudaGetDevice(&dev), "device");
   const std::lock_guard<std::mutex> lock(mu);
   if (dev < 0 || dev >= 64 || !configured[dev]) {
-    CudaCheck(cudaFuncSetAttribute(KPoseSchur<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   static_cast<int>(sizeof(Smem<T>))),
-              "pose schur smem attr");
+    CudaCheck(cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
+              "schur smem attr");
     if (dev >= 0 && dev < 64) {
       configured[dev] = true;
     }
@@ -371,14 +495,21 @@ int LaunchPoseSchur(const DeviceView& V, const PoseSchurArgs& args, bool fp32, c
     return 0;
   }
   const auto grid = static_cast<unsigned>(args.count);
-  Configure<double>();
+  Configure<KPoseSchur<double>>(sizeof(Smem<double>));
   KPoseSchur<double><<<grid, kThreads, sizeof(Smem<double>), stream>>>(V, args);
   if (fp32) {
-    Configure<float>();
+    Configure<KPoseSchur<float>>(sizeof(Smem<float>));
     KPoseSchur<float><<<grid, kThreads, sizeof(Smem<float>), stream>>>(V, args);
   }
   CudaCheck(cudaGetLastError(), "pose schur launch");
   return fp32 ? 2 : 1;
+}
+
+void LaunchChildSchur(const DeviceView& V, const ChildTask* tasks, int64_t count, const ChildEntry* entries,
+                      const double* dvec, cudaStream_t stream) {
+  Configure<KChildSchur>(sizeof(Smem<double>));
+  KChildSchur<<<static_cast<unsigned>(count), kThreads, sizeof(Smem<double>), stream>>>(V, tasks, entries, dvec);
+  CudaCheck(cudaGetLastError(), "child schur launch");
 }
 
 }  // namespace sdfgpu

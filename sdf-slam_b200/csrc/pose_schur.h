@@ -1,4 +1,5 @@
-// Pose Schur complement of the grid fronts (pose_schur.cu).
+// Schur complements on the FP64 tensor cores (pose_schur.cu): of the grid fronts
+// into their pose root, and of a level's children into their parents.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -28,5 +29,10 @@ inline size_t PoseSchurDoubles(int64_t slots) {
 /// roots; fp32: the view may hold FP32 fronts (a mixed solve). Returns the
 /// number of kernels launched.
 int LaunchPoseSchur(const DeviceView& V, const PoseSchurArgs& args, bool fp32, cudaStream_t stream);
+
+/// Adds the children's Schur complements into the fronts of `count` > 0 tile
+/// tasks (one level, FP64 fronts).
+void LaunchChildSchur(const DeviceView& V, const ChildTask* tasks, int64_t count, const ChildEntry* entries,
+                      const double* dvec, cudaStream_t stream);
 
 }  // namespace sdfgpu

@@ -25,6 +25,7 @@
 #include <atomic>
 #include <cmath>
 #include <functional>
+#include <mutex>
 #include <numeric>
 
 #include "host_pool.h"
@@ -327,6 +328,99 @@ void ComputeRel(Symbolic& S) {
   }
 }
 
+/// Tiles of the fronts with children and the children's rows in them (see
+/// KChildSchur). A tile of pivot columns that no child reaches has no task;
+/// every tile with trailing columns has one: nothing else writes those.
+void ChildTasks(Symbolic& S) {
+  constexpr int T = kPoseTile;
+  const auto fronts = static_cast<int64_t>(S.level_sn.size());
+  // contiguous parts of the level order, each into its own lists
+  struct Part {
+    int64_t begin{0};
+    std::vector<ChildTask> tasks;
+    std::vector<ChildEntry> entries;
+  };
+  std::mutex mu;
+  std::vector<Part> parts;
+  std::vector<int32_t> count(static_cast<size_t>(fronts) + 1, 0);  // tasks of each front in level order
+  ParallelRanges(PoolThreads(), fronts, 64, [&](int64_t q0, int64_t q1) {
+    Part part;
+    part.begin = q0;
+    std::vector<int32_t> starts;
+    std::vector<uint64_t> places;
+    for (int64_t q = q0; q < q1; ++q) {
+      const SupernodeRec& r = S.sn[static_cast<size_t>(S.level_sn[static_cast<size_t>(q)])];
+      if (r.child_count == 0) {
+        continue;
+      }
+      const size_t before = part.tasks.size();
+      // first row of each child in each block (rows ascend), their places in it
+      const int nb = (r.F + T - 1) / T;
+      starts.assign(static_cast<size_t>(r.child_count) * (static_cast<size_t>(nb) + 1), 0);
+      places.assign(static_cast<size_t>(r.child_count) * static_cast<size_t>(nb), 0);
+      for (int ci = 0; ci < r.child_count; ++ci) {
+        const SupernodeRec& c = S.sn[static_cast<size_t>(S.child_list[static_cast<size_t>(r.child_begin + ci)])];
+        const int32_t* rel = S.sn_rel.data() + c.rows_off;
+        int32_t* st = starts.data() + static_cast<size_t>(ci) * (static_cast<size_t>(nb) + 1);
+        uint64_t* at = places.data() + static_cast<size_t>(ci) * static_cast<size_t>(nb);
+        int b = 0;
+        for (int i = 0; i < c.nrows; ++i) {
+          for (; b * T <= rel[i]; ++b) {
+            st[b] = i;
+          }
+          at[rel[i] / T] |= uint64_t{1} << (rel[i] % T);
+        }
+        for (; b <= nb; ++b) {
+          st[b] = c.nrows;
+        }
+      }
+      for (int J = 0; J * T < r.fcols; ++J) {
+        for (int I = J; I < nb; ++I) {
+          ChildTask t{r.front_off, r.F, r.ncols, r.fcols, r.instance, I, J,
+                      static_cast<int32_t>(part.entries.size()), 0};
+          for (int ci = 0; ci < r.child_count; ++ci) {
+            const SupernodeRec& c = S.sn[static_cast<size_t>(S.child_list[static_cast<size_t>(r.child_begin + ci)])];
+            const int32_t* st = starts.data() + static_cast<size_t>(ci) * (static_cast<size_t>(nb) + 1);
+            if (st[I] < st[I + 1] && st[J] < std::min(st[J + 1], c.fcols - c.ncols)) {
+              const uint64_t* at = places.data() + static_cast<size_t>(ci) * static_cast<size_t>(nb);
+              part.entries.push_back(ChildEntry{c.front_off, at[I], at[J], c.F, c.ncols, c.first_col,
+                                                c.child_count == 0 ? 1 : 0, st[I], st[J]});
+            }
+          }
+          t.count = static_cast<int32_t>(part.entries.size()) - t.begin;
+          if (t.count > 0 || std::min((J + 1) * T, r.fcols) > r.ncols) {
+            part.tasks.push_back(t);
+          }
+        }
+      }
+      count[static_cast<size_t>(q)] = static_cast<int32_t>(part.tasks.size() - before);
+    }
+    const std::lock_guard<std::mutex> lock(mu);
+    parts.push_back(std::move(part));
+  });
+  std::sort(parts.begin(), parts.end(), [](const Part& x, const Part& y) { return x.begin < y.begin; });
+  S.child_tasks.clear();
+  S.child_entries.clear();
+  for (Part& part : parts) {
+    const auto shift = static_cast<int32_t>(S.child_entries.size());
+    for (ChildTask& t : part.tasks) {
+      t.begin += shift;
+    }
+    S.child_tasks.insert(S.child_tasks.end(), part.tasks.begin(), part.tasks.end());
+    S.child_entries.insert(S.child_entries.end(), part.entries.begin(), part.entries.end());
+  }
+  S.child_range.assign(static_cast<size_t>(S.num_levels), {});
+  int64_t at = 0;
+  for (int l = 0; l < S.num_levels; ++l) {
+    TaskRange& range = S.child_range[static_cast<size_t>(l)];
+    range.begin = at;
+    for (int q = S.level_begin[static_cast<size_t>(l)]; q < S.level_begin[static_cast<size_t>(l) + 1]; ++q) {
+      at += count[static_cast<size_t>(q)];
+    }
+    range.count = at - range.begin;
+  }
+}
+
 /// Tasks of the pose Schur complement (see Symbolic::pose_fronts). A tile's
 /// fronts are split so that an instance alone fills the GPU about four
 /// times over (two blocks per SM); the split depends on the instance only, so that its sums are
@@ -382,33 +476,59 @@ void PoseTasks(Symbolic& S) {
     auto pair_cost = [](int k, int na, int nb) {
       return static_cast<int64_t>((k + 15) / 16) * (((na + 15) / 16) * ((nb + 7) / 8) + 8);
     };
-    std::vector<std::vector<std::pair<int16_t, int8_t>>> present(len);
-    std::vector<int64_t> cost(static_cast<size_t>(nb) * nb, 0);
+    ParallelRanges(PoolThreads(), static_cast<int64_t>(len), 64, [&](int64_t q0, int64_t q1) {
+      for (auto q = static_cast<size_t>(q0); q < static_cast<size_t>(q1); ++q) {
+        const SupernodeRec& r = S.sn[static_cast<size_t>(in.fronts[q])];
+        const int32_t* rows = S.sn_rows.data() + r.rows_off;
+        int last = -1;
+        for (int x = r.fcols - r.ncols; x < r.nrows; ++x) {
+          const int pos = rows[x] - root.first_col;
+          const int b = pos / kT;
+          const size_t e = static_cast<size_t>(b) * len + q;
+          if (b != last) {
+            in.start[e] = x;
+            last = b;
+          }
+          in.mask[e] |= uint64_t{1} << (pos % kT);
+        }
+      }
+    });
+    // every tile's cost, over the fronts with rows in both of its blocks
+    std::vector<int32_t> pivots(len);
     for (size_t q = 0; q < len; ++q) {
-      const SupernodeRec& r = S.sn[static_cast<size_t>(in.fronts[q])];
-      const int32_t* rows = S.sn_rows.data() + r.rows_off;
-      int last = -1;
-      for (int x = r.fcols - r.ncols; x < r.nrows; ++x) {
-        const int pos = rows[x] - root.first_col;
-        const int b = pos / kT;
-        const size_t e = static_cast<size_t>(b) * len + q;
-        if (b != last) {
-          in.start[e] = x;
-          last = b;
-          present[q].emplace_back(static_cast<int16_t>(b), 0);
-        }
-        in.mask[e] |= uint64_t{1} << (pos % kT);
-      }
-      for (auto& p : present[q]) {
-        p.second = static_cast<int8_t>(__builtin_popcountll(in.mask[static_cast<size_t>(p.first) * len + q]));
-      }
-      for (size_t a = 0; a < present[q].size(); ++a) {
-        for (size_t b = 0; b <= a; ++b) {
-          cost[static_cast<size_t>(present[q][a].first) * nb + present[q][b].first] +=
-              pair_cost(r.ncols, present[q][a].second, present[q][b].second);
-        }
-      }
+      pivots[q] = S.sn[static_cast<size_t>(in.fronts[q])].ncols;
     }
+    const size_t words = (len + 63) / 64;
+    std::vector<uint64_t> has(words * static_cast<size_t>(nb), 0);  // fronts with rows in a block
+    std::vector<uint8_t> rows_in(len * static_cast<size_t>(nb), 0);
+    PoolRun(nb, [&](int b) {
+      for (size_t q = 0; q < len; ++q) {
+        const size_t e = static_cast<size_t>(b) * len + q;
+        if (in.mask[e] != 0) {
+          has[static_cast<size_t>(b) * words + q / 64] |= uint64_t{1} << (q % 64);
+          rows_in[e] = static_cast<uint8_t>(__builtin_popcountll(in.mask[e]));
+        }
+      }
+    });
+    auto each_pair = [&](int I, int J, auto&& f) {
+      const uint8_t* a = rows_in.data() + static_cast<size_t>(I) * len;
+      const uint8_t* b = rows_in.data() + static_cast<size_t>(J) * len;
+      for (size_t w = 0; w < words; ++w) {
+        uint64_t both = has[static_cast<size_t>(I) * words + w] & has[static_cast<size_t>(J) * words + w];
+        for (; both != 0; both &= both - 1) {
+          const size_t q = 64 * w + static_cast<size_t>(__builtin_ctzll(both));
+          f(q, pair_cost(pivots[q], a[q], b[q]));
+        }
+      }
+    };
+    std::vector<int64_t> cost(static_cast<size_t>(nb) * nb, 0);
+    PoolRun(nb, [&](int I) {
+      for (int J = 0; J <= I; ++J) {
+        int64_t c = 0;
+        each_pair(I, J, [&](size_t, int64_t x) { c += x; });
+        cost[static_cast<size_t>(I) * nb + J] = c;
+      }
+    });
     int64_t total = 0;
     for (const int64_t c : cost) {
       total += c;
@@ -416,14 +536,11 @@ void PoseTasks(Symbolic& S) {
     constexpr int64_t kTargetTasks = 8 * 148;
     constexpr int64_t kMinCost = 8 * 40;  // 128 pivots of full tiles
     const int64_t target = std::max(total / kTargetTasks, kMinCost);
-    // open task per tile; a part closes once its share of the cost is reached
-    std::vector<PoseTask> open(static_cast<size_t>(nb) * nb);
-    std::vector<int64_t> sum(static_cast<size_t>(nb) * nb, 0);
+    std::vector<PoseTask> whole;
     for (int I = 0; I < nb; ++I) {
       for (int J = 0; J <= I; ++J) {
         const size_t t = static_cast<size_t>(I) * nb + J;
-        PoseTask& o = open[t];
-        o = PoseTask{};
+        PoseTask o{};
         o.len = static_cast<int32_t>(len);
         o.root = in.root;
         o.I = I;
@@ -434,48 +551,55 @@ void PoseTasks(Symbolic& S) {
           o.counter = in.counters++;
           in.slots += o.parts;
         }
-      }
-    }
-    for (size_t q = 0; q < len; ++q) {
-      const int k = S.sn[static_cast<size_t>(in.fronts[q])].ncols;
-      for (size_t a = 0; a < present[q].size(); ++a) {
-        for (size_t b = 0; b <= a; ++b) {
-          const size_t t = static_cast<size_t>(present[q][a].first) * nb + present[q][b].first;
-          sum[t] += pair_cost(k, present[q][a].second, present[q][b].second);
-          PoseTask& o = open[t];
-          if (o.part + 1 < o.parts && sum[t] * o.parts >= cost[t] * (o.part + 1)) {
-            o.q1 = static_cast<int32_t>(q) + 1;
-            o.cost = cost[t] / o.parts;
-            in.tasks.push_back(o);
-            o.q0 = o.q1;
-            ++o.part;
-          }
+        if (cost[t] > 0) {
+          o.cost = cost[t] / o.parts;
+          whole.push_back(o);
         }
       }
     }
-    for (int I = 0; I < nb; ++I) {
-      for (int J = 0; J <= I; ++J) {
-        const size_t t = static_cast<size_t>(I) * nb + J;
-        if (cost[t] == 0) {
-          continue;
+    // a part closes once its share of the cost is reached; a front that
+    // crosses several shares at once leaves empty parts
+    std::vector<size_t> first(whole.size() + 1, 0);
+    for (size_t t = 0; t < whole.size(); ++t) {
+      first[t + 1] = first[t] + static_cast<size_t>(whole[t].parts);
+    }
+    in.tasks.resize(first.back());
+    ParallelRanges(PoolThreads(), static_cast<int64_t>(whole.size()), 32, [&](int64_t t0, int64_t t1) {
+      for (auto t = static_cast<size_t>(t0); t < static_cast<size_t>(t1); ++t) {
+        PoseTask o = whole[t];
+        PoseTask* out = in.tasks.data() + first[t];
+        const int64_t all = cost[static_cast<size_t>(o.I) * nb + o.J];
+        if (o.parts > 1) {
+          int64_t sum = 0;
+          each_pair(o.I, o.J, [&](size_t q, int64_t x) {
+            sum += x;
+            if (o.part + 1 < o.parts && sum * o.parts >= all * (o.part + 1)) {
+              o.q1 = static_cast<int32_t>(q) + 1;
+              *out++ = o;
+              o.q0 = o.q1;
+              ++o.part;
+            }
+          });
         }
-        // a front that crossed several shares at once leaves empty parts
-        PoseTask& o = open[t];
         for (; o.part < o.parts; ++o.part) {
           o.q1 = static_cast<int32_t>(len);
-          o.cost = cost[t] / o.parts;
-          in.tasks.push_back(o);
+          *out++ = o;
           o.q0 = o.q1;
         }
       }
-    }
+    });
   });
   for (Inst& in : inst) {
     const auto list = static_cast<int64_t>(S.pose_fronts.size());
     const auto mask = static_cast<int64_t>(S.pose_mask.size());
     S.pose_fronts.insert(S.pose_fronts.end(), in.fronts.begin(), in.fronts.end());
-    S.pose_mask.insert(S.pose_mask.end(), in.mask.begin(), in.mask.end());
-    S.pose_start.insert(S.pose_start.end(), in.start.begin(), in.start.end());
+    if (inst.size() == 1) {
+      S.pose_mask = std::move(in.mask);
+      S.pose_start = std::move(in.start);
+    } else {
+      S.pose_mask.insert(S.pose_mask.end(), in.mask.begin(), in.mask.end());
+      S.pose_start.insert(S.pose_start.end(), in.start.begin(), in.start.end());
+    }
     for (PoseTask& t : in.tasks) {
       t.list = list;
       t.mask = mask;
@@ -949,21 +1073,22 @@ void Finalize(Symbolic& S, std::vector<int> height, int panel_width, int tile) {
   }
   // front clearing tasks
   S.zero_tasks.clear();
-  for (int pass = 0; pass < 2; ++pass) {
+  // (pivot columns, trailing columns of fronts with children, of leaves)
+  for (int pass = 0; pass < 3; ++pass) {
     for (int s = 0; s < Sn; ++s) {
       const SupernodeRec& r = S.sn[static_cast<size_t>(s)];
-      const int split = r.child_count == 0 ? r.ncols : r.fcols;
       for (int c = 0; c < r.fcols; c += kZeroCols) {
-        if ((c < split) == (pass == 0)) {
+        if ((c < r.ncols ? 0 : r.child_count > 0 ? 1 : 2) == pass) {
           S.zero_tasks.push_back(s);
           S.zero_tasks.push_back(c);
         }
       }
     }
-    if (pass == 0) {
-      S.zero_main = static_cast<int64_t>(S.zero_tasks.size() / 2);
+    if (pass < 2) {
+      (pass == 0 ? S.zero_pivots : S.zero_main) = static_cast<int64_t>(S.zero_tasks.size() / 2);
     }
   }
+  ChildTasks(S);
   PoseTasks(S);
   // tiled dense roots: counters, inverse workspace and task lists per level
   S.dense_tasks.clear();
