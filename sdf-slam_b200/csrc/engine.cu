@@ -40,7 +40,8 @@ __global__ void KRefineResidual(DeviceView V, const double* y, double* r);
 __global__ void KAddCorrection(DeviceView V, const double* corr);
 __global__ void KRefineReset(DeviceView V);
 __global__ void KRefineCheck(DeviceView V);
-void LaunchCellSort(const int32_t* pt_cell, int64_t n, int64_t num_cells, int32_t* keys_a, int32_t* vals_a,
+size_t CellSortWords(int64_t n);
+int LaunchCellSort(const int32_t* pt_cell, int64_t n, int64_t num_cells, int32_t* keys_a, int32_t* vals_a,
                     int32_t* keys_b, int32_t* vals_b, int32_t* hist, cudaStream_t stream, bool* result_in_a);
 
 void ThrowCuda(cudaError_t e, const char* what) {
@@ -487,7 +488,7 @@ void Engine::UploadProblem(int64_t keep_rows) {
   sort_vals_a_.Alloc(static_cast<size_t>(total_points_));
   sort_keys_b_.Alloc(static_cast<size_t>(total_points_));
   sort_vals_b_.Alloc(static_cast<size_t>(total_points_));
-  sort_hist_.Alloc(256 * static_cast<size_t>((total_points_ + 2047) / 2048 + 1));
+  sort_hist_.Alloc(CellSortWords(total_points_));
   rhs_.Alloc(static_cast<size_t>(n_));
   step_.Alloc(static_cast<size_t>(n_));
   xs_.Alloc(static_cast<size_t>(n_));
@@ -811,9 +812,11 @@ void Engine::LaunchRows() {
     KOdomRows<<<Blocks(total_odom_, 128), 128, 0, stream_>>>(V_);
   }
   bool in_a = true;
+  int sort_launches = 0;
   if (total_points_ > 0) {
-    LaunchCellSort(pt_cell_.get(), total_points_, total_cells_, sort_keys_a_.get(), sort_vals_a_.get(),
-                   sort_keys_b_.get(), sort_vals_b_.get(), sort_hist_.get(), stream_, &in_a);
+    sort_launches =
+        LaunchCellSort(pt_cell_.get(), total_points_, total_cells_, sort_keys_a_.get(), sort_vals_a_.get(),
+                       sort_keys_b_.get(), sort_vals_b_.get(), sort_hist_.get(), stream_, &in_a);
   }
   const int32_t* keys = in_a ? sort_keys_a_.get() : sort_keys_b_.get();
   cell_rows_ptr_ = in_a ? sort_vals_a_.get() : sort_vals_b_.get();
@@ -821,11 +824,7 @@ void Engine::LaunchRows() {
   KCellStart<<<Blocks(total_cells_ + 1, 256), 256, 0, stream_>>>(keys, total_points_, total_cells_,
                                                                    cell_start_.get());
   CudaCheck(cudaGetLastError(), "row kernels");
-  int bits = 1;
-  while ((int64_t{1} << bits) <= total_cells_) {
-    ++bits;
-  }
-  times_.launches += (total_points_ > 0 ? 1 + 1 + 3 * ((bits + 7) / 8) : 0) + (total_eik_ > 0 ? 1 : 0) +
+  times_.launches += (total_points_ > 0 ? 1 : 0) + sort_launches + (total_eik_ > 0 ? 1 : 0) +
                      (total_odom_ > 0 ? 1 : 0) + 1;
 }
 
