@@ -362,52 +362,101 @@ __device__ __forceinline__ double WarpSum(double v) {
   return v;
 }
 
-/// Front offset of the J^T J entry between the cell corners a and b of a cell
-/// whose corner columns are col[], or -1 when one corner is constant.
-__device__ __forceinline__ int64_t PairOffset(const DeviceView& V, const int* col, int a, int b) {
-  if (col[a] < 0 || col[b] < 0) {
+/// Front offset of the J^T J entry between the cell corners a and b of a cell,
+/// their columns ca and cb, or -1 when one corner is constant.
+__device__ __forceinline__ int64_t PairOffset(const DeviceView& V, int ca, int cb, int a, int b) {
+  if (ca < 0 || cb < 0) {
     return -1;
   }
   const int dw = (b & 1) - (a & 1);
   const int dh = (b >> 1) - (a >> 1);
-  const int64_t off = V.mm_off[static_cast<int64_t>(col[a]) * 9 + (dh + 1) * 3 + (dw + 1)];
+  const int64_t off = V.mm_off[static_cast<int64_t>(ca) * 9 + (dh + 1) * 3 + (dw + 1)];
   if (off >= 0) {
     return off;
   }
-  return V.mm_off[static_cast<int64_t>(col[b]) * 9 + (1 - dh) * 3 + (1 - dw)];
+  return V.mm_off[static_cast<int64_t>(cb) * 9 + (1 - dh) * 3 + (1 - dw)];
 }
 
-__device__ __forceinline__ int FindInstanceByCell(const DeviceView& V, int64_t cell) {
-  int lo = 0;
-  int hi = V.num_inst - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (V.inst[mid].cell_off <= cell) {
-      lo = mid;
-    } else {
-      hi = mid - 1;
+/// One step of a reduction that halves the values a lane holds: lanes a
+/// distance kD apart exchange halves of their kN values.
+template <int kN, int kD>
+__device__ __forceinline__ void HalveStep(double* v, int lane) {
+  const bool upper = (lane & kD) != 0;
+#pragma unroll
+  for (int q = 0; q < kN / 2; ++q) {
+    const double send = upper ? v[q] : v[q + kN / 2];
+    const double keep = upper ? v[q + kN / 2] : v[q];
+    v[q] = keep + __shfl_xor_sync(0xffffffffu, send, kD);
+  }
+}
+
+/// Sum over the warp of sixteen values per lane, in a fixed order: value q in
+/// lanes 2 q and 2 q + 1 (16 exchanges; a butterfly per value takes 80).
+__device__ __forceinline__ double WarpSum16(double (&v)[16], int lane) {
+  HalveStep<16, 16>(v, lane);
+  HalveStep<8, 8>(v, lane);
+  HalveStep<4, 4>(v, lane);
+  HalveStep<2, 2>(v, lane);
+  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
+
+/// Polls of a wait for a neighbouring cell (about a second).
+constexpr uint32_t kCellWaitLimit = 1u << 21;
+
+/// Waits until the cells that share a node with this one and come before it
+/// (a lower colour) are done, one lane per neighbour; a wait that runs out
+/// marks the instance.
+__device__ __forceinline__ void WaitForNeighbours(const DeviceView& V, int i, const uint32_t* done, int64_t cell,
+                                                  int cx, int cy, int cw, int ch, int lane) {
+  if (lane < 8) {
+    const int at = lane < 4 ? lane : lane + 1;
+    const int x = cx + at % 3 - 1;
+    const int y = cy + at / 3 - 1;
+    const int own = (cx & 1) | ((cy & 1) << 1);
+    const int colour = (x & 1) | ((y & 1) << 1);
+    if (x >= 0 && x < cw && y >= 0 && y < ch && colour < own) {
+      const uint32_t* word = done + cell + static_cast<int64_t>(y - cy) * cw + (x - cx);
+      uint32_t it = 0;
+      for (; it < kCellWaitLimit; ++it) {
+        uint32_t v;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(word) : "memory");
+        if (v != 0) {
+          break;
+        }
+        if (it > 64) {
+          __nanosleep(100);
+        }
+      }
+      if (it == kCellWaitLimit) {
+        atomicOr(V.status + i, kStatusWaitTimeout);
+      }
     }
   }
-  return lo;
+  __syncwarp();
 }
 
 }  // namespace
 
-/// One cell of a colour class (cx % 2, cy % 2) = (pass & 1, pass >> 1): cells
-/// of one class share no node, so each adds its contributions to J^T J and
-/// J^T r with plain read-modify-writes. One warp per cell: the 4x4 map block
-/// and the corner gradients are lane-strided sums over the cell's point rows
-/// reduced by a fixed butterfly; the map-pose blocks are segmented sums over
-/// runs of rows of one frame (rows of a cell are sorted, so frames are
-/// contiguous); the cell's Eikonal row (spec at its lower-left node) follows.
-/// Passes run in a fixed order, so every entry is a deterministic sum.
-__device__ __forceinline__ void CellPassOne(const DeviceView& V, int64_t cell, int lane) {
-  const int i = FindInstanceByCell(V, cell);
+/// One cell, one warp: the 4x4 map block and the corner gradients are
+/// lane-strided sums over the cell's point rows reduced in a fixed order; the
+/// map-pose blocks are segmented sums over runs of rows of one frame (rows of a
+/// cell are sorted, so frames are contiguous); the cell's Eikonal row (spec at
+/// its lower-left node) is added to them. Cells that share a node add in the
+/// order of their colours (cx % 2, cy % 2) = (colour & 1, colour >> 1), with plain
+/// read-modify-writes, so every entry is a deterministic sum. kWait: the
+/// launch holds all colours, and a cell waits for its neighbours of lower
+/// colours before its first write; everything before that runs ahead of the
+/// wait.
+template <bool kWait>
+__device__ __forceinline__ void CellPassOne(const DeviceView& V, int64_t entry, uint32_t* done, int lane) {
+  const int i = static_cast<int>(entry >> kCellBits);
+  const int64_t cell = entry & ((int64_t{1} << kCellBits) - 1);
   const InstDev& I = V.inst[i];
   if (V.active[i] == 0) {
-    return;
+    return;  // as every cell it shares a node with
   }
   const int cw = I.nx - 1;
+  const int ch = I.ny - 1;
   const int local = static_cast<int>(cell - I.cell_off);
   const int cx = local % cw;
   const int cy = local / cw;
@@ -421,23 +470,45 @@ __device__ __forceinline__ void CellPassOne(const DeviceView& V, int64_t cell, i
   const int re = V.cell_start[cell + 1];
   const int eik = V.eik_index[n0];
   if (rb == re && eik < 0) {
+    if (kWait && lane == 0) {
+      __stcg(done + cell, 1u);
+    }
     return;
   }
+  // what lanes 2 q and 2 q + 1 add in the end: pair q of corners (a, b), a <= b,
+  // or the gradient of corner q - 10; the Eikonal row's part of it (nodes (cx,
+  // cy), (cx + 1, cy), (cx, cy + 1) = corners 0, 1, 2)
+  const int q = lane >> 1;
+  const int ca = q < 10 ? (q < 4 ? 0 : q < 7 ? 1 : q < 9 ? 2 : 3) : q - 10;
+  const int cb = q < 4 ? q : q < 7 ? q - 3 : q < 9 ? q - 5 : 3;
+  const int col_a = ca == 0 ? col[0] : ca == 1 ? col[1] : ca == 2 ? col[2] : col[3];
+  const int col_b = cb == 0 ? col[0] : cb == 1 ? col[1] : cb == 2 ? col[2] : col[3];
+  const bool eik_part = eik >= 0 && ca < 3 && (q < 10 ? cb < 3 : q < 13);
+  double* target = nullptr;
+  double eik_add = 0.0;
+  if ((lane & 1) == 0 && q < 14 && (rb < re || eik_part)) {
+    if (q < 10) {
+      const int64_t off = PairOffset(V, col_a, col_b, ca, cb);
+      target = off >= 0 ? V.asm_fronts + off : nullptr;
+    } else {
+      target = col_a >= 0 ? V.rhs + col_a : nullptr;
+    }
+    if (eik_part) {
+      const double* r = V.eik_rec + static_cast<int64_t>(eik) * kEikRec;
+      eik_add = r[ca] * r[q < 10 ? cb : 3];
+    }
+  }
+  bool waited = false;
   // One pass over the cell's rows in chunks of 32 (lane l takes rows
   // rb + l + 32 t): the 4x4 map block and corner gradients accumulate per
   // lane and are reduced by a fixed butterfly at the end; the map-pose
   // blocks are segmented sums over runs of one frame inside each chunk. A
   // chunk's records, frames and front offsets are loaded while the previous
   // chunk is scanned and written (the row indices one chunk further ahead).
-  double mm[10];
-  double g[4];
+  double sums[16];  // pairs, gradients, two unused
 #pragma unroll
-  for (int q = 0; q < 10; ++q) {
-    mm[q] = 0.0;
-  }
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    g[q] = 0.0;
+  for (int e = 0; e < 16; ++e) {
+    sums[e] = 0.0;
   }
   bool overflow = false;
   struct ChunkRow {
@@ -481,15 +552,15 @@ __device__ __forceinline__ void CellPassOne(const DeviceView& V, int64_t cell, i
     const double jp[3] = {cur.p01.x, cur.p01.y, cur.p2r.x};
     const double r = cur.p2r.y;
     if (in) {
-      int q = 0;
+      int e = 0;
 #pragma unroll
       for (int aa = 0; aa < 4; ++aa) {
 #pragma unroll
         for (int bb = aa; bb < 4; ++bb) {
-          mm[q] = mm[q] + J[aa] * J[bb];
-          ++q;
+          sums[e] = sums[e] + J[aa] * J[bb];
+          ++e;
         }
-        g[aa] = g[aa] + J[aa] * r;
+        sums[10 + aa] = sums[10 + aa] + J[aa] * r;
       }
     }
     double v[12];
@@ -505,10 +576,10 @@ __device__ __forceinline__ void CellPassOne(const DeviceView& V, int64_t cell, i
     for (int d = 1; d < 32; d <<= 1) {
       const int fu = __shfl_up_sync(0xffffffffu, f, d);
 #pragma unroll
-      for (int q = 0; q < 12; ++q) {
-        const double vu = __shfl_up_sync(0xffffffffu, v[q], d);
+      for (int e = 0; e < 12; ++e) {
+        const double vu = __shfl_up_sync(0xffffffffu, v[e], d);
         if (lane >= d && fu == f) {
-          v[q] = vu + v[q];
+          v[e] = vu + v[e];
         }
       }
     }
@@ -516,6 +587,10 @@ __device__ __forceinline__ void CellPassOne(const DeviceView& V, int64_t cell, i
     const int p = base + lane;
     const bool tail = in && (lane == 31 || p + 1 >= re || fn != f);
     const int fl = f - I.frame_off;
+    if (kWait && !waited) {
+      WaitForNeighbours(V, i, done, cell, cx, cy, cw, ch, lane);
+      waited = true;
+    }
     if (tail && fl >= 1) {
       // the (up to 12) entries are distinct: all loads first, then the
       // stores, so their latencies overlap
@@ -524,9 +599,9 @@ __device__ __forceinline__ void CellPassOne(const DeviceView& V, int64_t cell, i
 #pragma unroll
       for (int aa = 0; aa < 4; ++aa) {
         if (col[aa] >= 0 && offs[aa] >= 0) {
-          old[3 * aa] = V.asm_fronts[offs[aa]];
-          old[3 * aa + 1] = V.asm_fronts[offs[aa] + 1];
-          old[3 * aa + 2] = V.asm_fronts[offs[aa] + 2];
+          old[3 * aa] = __ldcg(V.asm_fronts + offs[aa]);
+          old[3 * aa + 1] = __ldcg(V.asm_fronts + offs[aa] + 1);
+          old[3 * aa + 2] = __ldcg(V.asm_fronts + offs[aa] + 2);
         } else {
           old[3 * aa] = old[3 * aa + 1] = old[3 * aa + 2] = 0.0;
         }
@@ -550,70 +625,67 @@ __device__ __forceinline__ void CellPassOne(const DeviceView& V, int64_t cell, i
     k = k_next;
     k_next = k_after;
   }
-#pragma unroll
-  for (int q = 0; q < 10; ++q) {
-    mm[q] = WarpSum(mm[q]);
+  if (kWait && !waited) {
+    WaitForNeighbours(V, i, done, cell, cx, cy, cw, ch, lane);
   }
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    g[q] = WarpSum(g[q]);
-  }
-  if (rb < re) {
-    // lanes 0..9 write the pairs, 10..13 the gradients
-    int q = 0;
-#pragma unroll
-    for (int aa = 0; aa < 4; ++aa) {
-#pragma unroll
-      for (int bb = aa; bb < 4; ++bb) {
-        if (lane == q) {
-          const int64_t off = PairOffset(V, col, aa, bb);
-          if (off >= 0) {
-            V.asm_fronts[off] += mm[q];
-          }
-        }
-        ++q;
-      }
-    }
-#pragma unroll
-    for (int aa = 0; aa < 4; ++aa) {
-      if (lane == 10 + aa && col[aa] >= 0) {
-        V.rhs[col[aa]] += g[aa];
-      }
-    }
-  }
-  __syncwarp();
-  // the cell's Eikonal row: nodes (cx,cy), (cx+1,cy), (cx,cy+1) = corners
-  // 0, 1, 2; lanes 0..5 add the six pairs, lanes 6..8 the three gradient
-  // entries (distinct entries, one per lane)
-  if (eik >= 0 && lane < 9) {
-    const double* r = V.eik_rec + static_cast<int64_t>(eik) * kEikRec;
-    if (lane < 6) {
-      const int a = lane < 3 ? 0 : (lane < 5 ? 1 : 2);
-      const int b = lane < 3 ? lane : (lane < 5 ? lane - 2 : 2);
-      const int64_t off = PairOffset(V, col, a, b);
-      if (off >= 0) {
-        V.asm_fronts[off] += r[a] * r[b];
-      }
-    } else {
-      const int a = lane - 6;
-      V.rhs[col[a]] += r[a] * r[3];
-    }
+  const double sum = WarpSum16(sums, lane);
+  if (target != nullptr) {
+    *target = __ldcg(target) + (sum + eik_add);
   }
   if (overflow) {
     atomicOr(V.status + i, kStatusPatternOverflow);
   }
-}
-
-/// Warps walk the pass's cell list with a grid stride (the launch holds as
-/// many blocks as are resident, so no cell waits for a second wave behind a
-/// busy one).
-__global__ void __launch_bounds__(256, 2) KCellPass(DeviceView V, const int64_t* cells, int64_t count) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
-  for (int64_t w = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; w < count; w += warps) {
-    CellPassOne(V, cells[w], lane);
+  if (kWait) {
+    // every lane's writes before the flag
+    __syncwarp();
+    if (lane == 0) {
+      asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(done + cell), "r"(1u) : "memory");
+    }
   }
 }
+
+/// Cells of one colour, with a grid stride (the launch holds as many blocks as
+/// are resident, so no cell waits for a second wave behind a busy one), or with
+/// kWait all cells, colour by colour, in one launch: warps take a cell at a time
+/// from a counter, in order, the next one while they work on the current, so
+/// the cells a cell waits for are done or being worked on. cells: (instance,
+/// cell), kCellBits bits of cell. Bound by the chain of reads behind a cell's
+/// rows and, in large problems, by the segmented sums. Measured on B200 against
+/// four launches with a butterfly per sum and the offsets read behind the sums:
+/// 1,600 cells 48 -> 20 us, 9,900 cells 100 -> 90 (four launches), 39,600 cells
+/// 324 -> 294, 32 instances 608 -> 496.
+template <bool kWait>
+__global__ void __launch_bounds__(256, 2) KCellPass(DeviceView V, const int64_t* cells, int64_t count,
+                                                    uint32_t* ticket, uint32_t* done) {
+  const int lane = threadIdx.x & 31;
+  if (!kWait) {
+    const int64_t warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
+    for (int64_t w = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; w < count; w += warps) {
+      CellPassOne<false>(V, cells[w], nullptr, lane);
+    }
+    return;
+  }
+  uint32_t taken = 0;
+  if (lane == 0) {
+    taken = atomicAdd(ticket, 1u);
+  }
+  for (;;) {
+    const int64_t w = __shfl_sync(0xffffffffu, taken, 0);
+    if (w >= count) {
+      return;
+    }
+    uint32_t ahead = 0;
+    if (lane == 0) {
+      ahead = atomicAdd(ticket, 1u);
+    }
+    CellPassOne<true>(V, cells[w], done, lane);
+    taken = ahead;
+  }
+}
+template __global__ void KCellPass<false>(DeviceView V, const int64_t* cells, int64_t count, uint32_t* ticket,
+                                          uint32_t* done);
+template __global__ void KCellPass<true>(DeviceView V, const int64_t* cells, int64_t count, uint32_t* ticket,
+                                         uint32_t* done);
 
 /// Same-frame pose blocks and the pose columns of J^T r: one block of 256
 /// threads per frame, thread-strided over the frame's point rows, a fixed
@@ -734,11 +806,24 @@ __global__ void __launch_bounds__(256) KPoseFrames(DeviceView V) {
 /// max(diag, 1e-12) under Marquardt scaling).
 /// Zeroes the lower triangle of the assembly fronts before the row kernels
 /// add into them: one warp per column c, rows c..F-1 (coalesced); task (sn,
-/// first of kZeroCols columns). The upper triangles are never read before
+/// first of kZeroCols columns). Also J^T r and the cell pass's counter and
+/// flags. The upper triangles are never read before
 /// the factorization writes them, so they are left as they are (half the
 /// bytes of clearing the whole buffer).
-__global__ void KZeroFronts(DeviceView V, const int32_t* tasks, uint64_t* stamp) {
+__global__ void KZeroFronts(DeviceView V, const int32_t* tasks, int64_t count, uint32_t* words, int64_t num_words,
+                            uint64_t* stamp) {
   StampPhase(stamp);
+  const int64_t threads = static_cast<int64_t>(gridDim.x) * blockDim.x;
+  const int64_t me = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  for (int64_t e = me; e < V.n; e += threads) {
+    V.rhs[e] = 0.0;
+  }
+  for (int64_t e = me; e < num_words; e += threads) {
+    words[e] = 0;
+  }
+  if (blockIdx.x >= count) {
+    return;
+  }
   const int32_t* t = tasks + 2 * static_cast<int64_t>(blockIdx.x);
   const SupernodeRec S = V.sn[t[0]];
   const int c = t[1] + static_cast<int>(threadIdx.x >> 5);

@@ -8,6 +8,9 @@
 
 namespace sdfgpu {
 
+/// Bits of the cell in an entry of the cell pass's list (instance above).
+constexpr int kCellBits = 40;
+
 /// Per-instance constants (device copy of InstanceLayout plus schedule data).
 struct InstDev {
   int32_t nx, ny;
