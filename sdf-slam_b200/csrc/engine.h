@@ -209,13 +209,15 @@ inline size_t DenseSyncWords(const Symbolic& S) {
 }
 
 /// Words of the one-launch solve's counter and flags (an even number), and
-/// with them the hand-over words of the tiled dense roots: two 64-bit words per
-/// column of their tiles, behind the flags.
+/// with them the values handed over between its blocks, 64-bit each behind the
+/// flags: y and x of every column and, with solve_handover, the update vectors
+/// and the row chunks' backward products.
 inline size_t SolveFlagWords(const Symbolic& S) {
   return (2 + 4 * S.sn.size() + S.inv_tasks.size() + 1) & ~size_t{1};
 }
 inline size_t SolveSyncWords(const Symbolic& S) {
-  return SolveFlagWords(S) + 4 * static_cast<size_t>(S.dense_inv_doubles / kDenseTileCols);
+  const int64_t values = 2 * static_cast<int64_t>(S.n) + (S.solve_handover ? S.update_doubles + S.zpart_doubles : 0);
+  return SolveFlagWords(S) + 2 * static_cast<size_t>(values);
 }
 
 /// Level-scheduled multifrontal LDL^T of the assembled fronts.

@@ -1854,7 +1854,7 @@ __device__ __forceinline__ void Publish(uint32_t* word) {
 
 /// What the one-launch solve's tasks read besides the view.
 struct SolveArgs {
-  const int32_t* tasks;   // (type, sn, part, 0) quads
+  const int32_t* tasks;   // (type, sn, part, gate) quads
   int num_tasks;
   const int32_t* parts;   // per sn: forward, backward parts
   const int64_t* zoff;    // per sn: first partial-product double, or -1
@@ -1864,8 +1864,13 @@ struct SolveArgs {
   const double* inv;
   const double* dense_inv;  // tile inverses of the tiled dense roots (64-row panels)
   uint32_t* sync;         // counter, then fdone, bdone, ydone, zdone per sn, then two flags per diagonal block
-  uint64_t* handover;     // y, then x, of the tiled dense roots' columns (0: not there yet)
-  int64_t handover_cols;
+  // values handed over between blocks (0: not there yet): y and x of every
+  // column, and where no front is solved by panels the update vectors (at
+  // SupernodeRec::upd_off) and the row chunks' backward products (at zoff)
+  uint64_t* y;
+  uint64_t* x;
+  uint64_t* u;
+  uint64_t* z;
   int num_sn;
   int num_inv;
   int withhold;
@@ -1888,19 +1893,57 @@ __device__ __forceinline__ bool BlockWait(const DeviceView& V, const SupernodeRe
   return ok != 0;
 }
 
-/// Hand-over of a solved entry between the blocks of a tiled dense root: the
-/// value itself is the flag (its bits, changed so that zero means "not there
+/// Hand-over of a value between blocks of the solve: the value itself is the
+/// flag (its bits, changed so that zero means "not there
 /// yet": the pattern that would read as such is a NaN no operation produces),
-/// so that a panel waits one trip through L2 per predecessor instead of one for
-/// a flag and one for the data behind it.
+/// so that its reader waits one trip through L2 instead of one for a flag and
+/// one for the data behind it, and its writer needs no fence.
 constexpr uint64_t kHandoverKey = 0x7ff4deadbeef0001ull;
 __device__ __forceinline__ void HandOver(uint64_t* slot, double v) {
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(slot),
                "l"(static_cast<uint64_t>(__double_as_longlong(v)) ^ kHandoverKey)
                : "memory");
 }
-/// Bounded wait for a handed-over entry; a wait that runs out marks the
+/// Bounded wait for kN handed-over entries, the first half at base0[off[q]], the
+/// others at base1[off[q]] (off < 0: zero, not waited for), their reads in
+/// flight together; a wait that runs out marks the
 /// instance, reads as zero and leaves no limit for the thread's further waits.
+template <int kN>
+__device__ __forceinline__ void TakeOver(const DeviceView& V, const SupernodeRec& S, const uint64_t* base0,
+                                         const uint64_t* base1, const int (&off)[kN], double (&out)[kN],
+                                         uint32_t& limit) {
+  uint64_t v[kN];
+  bool all = false;
+  for (uint32_t it = 0; it < limit && !all; ++it) {
+    if (it > 64) {
+      __nanosleep(50);
+    }
+    all = true;
+#pragma unroll
+    for (int q = 0; q < kN; ++q) {
+      v[q] = kHandoverKey;
+      if (off[q] >= 0) {
+        asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];"
+                     : "=l"(v[q])
+                     : "l"((q < kN / 2 ? base0 : base1) + off[q])
+                     : "memory");
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < kN; ++q) {
+      all = all && v[q] != 0;
+    }
+  }
+  if (!all) {
+    atomicOr(V.status + S.instance, kStatusWaitTimeout);
+    limit = 1;
+  }
+#pragma unroll
+  for (int q = 0; q < kN; ++q) {
+    out[q] = v[q] != 0 ? __longlong_as_double(static_cast<long long>(v[q] ^ kHandoverKey)) : 0.0;
+  }
+}
+/// The same for one entry.
 __device__ __forceinline__ double TakeOver(const DeviceView& V, const SupernodeRec& S, const uint64_t* slot,
                                            uint32_t& limit) {
   for (uint32_t it = 0; it < limit; ++it) {
@@ -1918,18 +1961,31 @@ __device__ __forceinline__ double TakeOver(const DeviceView& V, const SupernodeR
   return 0.0;
 }
 
+/// Bounded wait until a handed-over entry is there (its value is not needed),
+/// with pauses that leave L2 to the blocks whose turn it is.
+__device__ __forceinline__ void WaitGate(const uint64_t* slot, uint32_t limit) {
+  for (uint32_t it = 0; it < limit; ++it) {
+    uint64_t v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(slot) : "memory");
+    if (v != 0) {
+      return;
+    }
+    __nanosleep(100);
+  }
+}
+
 /// Panel q of a tiled dense root's solve (64-row panels, FP64), one block: the
 /// panels that come before it (forward: p < q, backward: p > q) hand their
 /// solutions over one by one; thread (row i of the panel, sixteen columns
-/// g of theirs) keeps its sum and its part of the tile inverse in registers and
-/// loads the next panel's L while it waits for the current one's solution, so
-/// that what follows the last hand-over is one sum over the four groups, one
-/// product with the inverse and one more sum. Forward: y_q = M_q (v_q - sum L(q, p) y_p), D^-1 y_q into xs. Backward:
-/// x_q = M_q^T (D^-1 y_q - sum L(p, q)^T x_p) into xs and the step. Bound by the
+/// g of theirs) keeps its sum in registers and loads the next panel's L while it
+/// waits for the current one's solution, and the tile inverse is in shared
+/// memory by then, so that what follows the last hand-over is one sum over the four groups, one
+/// product with the inverse and one more sum. Forward: y_q = M_q (v_q - sum L(q, p) y_p). Backward: x_q = M_q^T (D^-1
+/// y_q - sum L(p, q)^T x_p), also into the step. Bound by the
 /// chain of hand-overs. Measured on B200, the whole solve launch with a flag per
 /// panel and the sums through shared memory -> this: 910-pose office (43 panels
 /// each way) 1033 -> 887 us, 331-pose room 434 -> 380 us.
-template <bool kForward>
+template <bool kForward, bool kFlags>
 __device__ __forceinline__ void RootPanel64(const DeviceView& V, const SupernodeRec& S, const SolveArgs& A, int q,
                                             double* buf) {
   constexpr int kW = kDenseTileCols;
@@ -1949,8 +2005,8 @@ __device__ __forceinline__ void RootPanel64(const DeviceView& V, const Supernode
   // bound the sweep: 2.5 us a panel)
   const int i = kForward ? tid & (kW - 1) : tid >> 2;
   const int g = kForward ? tid >> 6 : tid & 3;
-  const int64_t base = S.dense_inv / kW;
-  uint64_t* slots = A.handover + (kForward ? 0 : A.handover_cols) + base;
+  uint64_t* slots = (kForward ? A.y : A.x) + S.first_col;
+  uint32_t limit = A.wait_limit;
   auto load = [&](int p, double (&l)[16]) {
     const int wp = min(kW, k - p * kW);
 #pragma unroll
@@ -1965,13 +2021,14 @@ __device__ __forceinline__ void RootPanel64(const DeviceView& V, const Supernode
   };
   const int steps = kForward ? q : np - 1 - q;
   double l[16];
-  double m[16];
-  // this panel's part of the inverse, row i of M (forward) or of M^T
-  const double* M = A.dense_inv + S.dense_inv + static_cast<int64_t>(q) * kW * kW;
-#pragma unroll
-  for (int c = 0; c < 16; ++c) {
-    const int j = kForward ? 16 * g + c : 4 * c + g;
-    m[c] = kForward ? M[j * kW + i] : M[i * kW + j];
+  // the tile inverse, on its way while the panels before this one come in
+  constexpr int kPitch = kW + 4;
+  double* M = buf + 7 * kW;
+  {
+    const double* src = A.dense_inv + S.dense_inv + static_cast<int64_t>(q) * kW * kW;
+    for (int e = tid; e < kW * kW; e += blockDim.x) {
+      LoadElement(M + (e >> 6) * kPitch + (e & (kW - 1)), src + e);
+    }
   }
   if (steps > 0) {
     load(kForward ? 0 : np - 1, l);
@@ -1987,19 +2044,19 @@ __device__ __forceinline__ void RootPanel64(const DeviceView& V, const Supernode
       const SupernodeRec C = V.sn[V.child_list[S.child_begin + ci]];
       const int32_t* rel = V.sn_rel + C.rows_off;
       const double* u = V.upd + C.upd_off;
+#pragma unroll 1
       for (int r = tid; r < C.nrows; r += blockDim.x) {
         const int at = rel[r] - p0;
         if (at >= 0 && at < w) {
-          vq[at] += __ldcg(u + r);
+          vq[at] += kFlags ? __ldcg(u + r) : TakeOver(V, S, A.u + C.upd_off + r, limit);
         }
       }
       __syncthreads();
     }
   }
   if (tid < w) {
-    own = kForward ? vq[tid] : __ldcg(V.xs + S.first_col + p0 + tid);
+    own = kForward ? vq[tid] : (1.0 / A.dvec[S.first_col + p0 + tid]) * TakeOver(V, S, A.y + S.first_col + p0 + tid, limit);
   }
-  uint32_t limit = A.wait_limit;
   double acc = 0.0;
 #pragma unroll 1
   for (int s = 0; s < steps; ++s) {
@@ -2019,6 +2076,7 @@ __device__ __forceinline__ void RootPanel64(const DeviceView& V, const Supernode
     }
   }
   part[g * kW + i] = acc;
+  WaitElements();
   __syncthreads();
   if (tid < kW) {
     vq[tid] = own - ((part[tid] + part[kW + tid]) + (part[2 * kW + tid] + part[3 * kW + tid]));
@@ -2027,21 +2085,31 @@ __device__ __forceinline__ void RootPanel64(const DeviceView& V, const Supernode
   acc = 0.0;
 #pragma unroll
   for (int c = 0; c < 16; ++c) {
-    acc = fma(m[c], vq[kForward ? 16 * g + c : 4 * c + g], acc);
+    const int j = kForward ? 16 * g + c : 4 * c + g;
+    acc = fma(M[kForward ? j * kPitch + i : i * kPitch + j], vq[j], acc);
   }
   part[g * kW + i] = acc;
   __syncthreads();
   if (tid < w) {
     const double x = (part[tid] + part[kW + tid]) + (part[2 * kW + tid] + part[3 * kW + tid]);
     HandOver(slots + p0 + tid, x);
-    const int64_t col = S.first_col + p0 + tid;
-    if (kForward) {
-      V.xs[col] = (1.0 / A.dvec[col]) * x;
-    } else {
-      V.xs[col] = x;
+    if (!kForward) {
+      const int64_t col = S.first_col + p0 + tid;
+      if (kFlags) {
+        V.xs[col] = x;
+      }
       V.step[V.perm[col]] = x;
     }
   }
+}
+
+/// RootPanel64 by values, called rather than inlined: inlined beside the front
+/// tasks that poll, it made the kernel spill (76-frame floor plan 101 against 87
+/// us a solve).
+template <bool kForward>
+__device__ __noinline__ void RootPanel64Call(const DeviceView& V, const SupernodeRec& S, const SolveArgs& A, int q,
+                                             double* buf) {
+  RootPanel64<kForward, false>(V, S, A, q, buf);
 }
 
 /// Right-hand side of a panel-split root: v = rhs plus the children's
@@ -2249,9 +2317,9 @@ __device__ __forceinline__ void ChildSlots(const DeviceView& V, const SupernodeR
 /// stores D^-1 y), u = v_m - L21 y. What does not depend on the children (the
 /// chunk's L, the inverse, positions, right-hand side) is read before the wait
 /// for them: behind it come one read of their updates and two products.
-template <typename T, typename Wait>
+template <typename T, bool kFlags, typename Wait>
 __device__ __forceinline__ void FrontForward(const DeviceView& V, const SupernodeRec& S, const SolveArgs& A, int part,
-                                             double* buf, Wait wait) {
+                                             bool withhold, double* buf, Wait wait) {
   const int k = S.ncols;
   const int rows = SolveRows(k);
   const int r0 = part * rows;
@@ -2275,7 +2343,8 @@ __device__ __forceinline__ void FrontForward(const DeviceView& V, const Supernod
   for (int j = tid; j < k + nr; j += blockDim.x) {
     v[j] = j < k ? V.rhs[V.perm[S.first_col + j]] : 0.0;
   }
-  const double d = part == 0 && tid < k ? A.dvec[S.first_col + tid] : 1.0;
+  const double dinv = kFlags && part == 0 && tid < k ? 1.0 / A.dvec[S.first_col + tid] : 1.0;
+  uint32_t limit = A.wait_limit;
   int slot0[kSolveRel];
   int slot1[kSolveRel];
   SupernodeRec C0{};
@@ -2304,25 +2373,35 @@ __device__ __forceinline__ void FrontForward(const DeviceView& V, const Supernod
         ChildSlots(V, C0, base, k, r0, nr, slot0);
         ChildSlots(V, C1, base, k, r0, nr, slot1);
       }
-      double u0[kSolveRel];
-      double u1[kSolveRel];
+      double u[2 * kSolveRel];
+      if (kFlags) {
 #pragma unroll
-      for (int q = 0; q < kSolveRel; ++q) {
-        const int r = base + 256 * q + tid;
-        u0[q] = slot0[q] >= 0 ? __ldcg(V.upd + C0.upd_off + r) : 0.0;
-        u1[q] = slot1[q] >= 0 ? __ldcg(V.upd + C1.upd_off + r) : 0.0;
+        for (int q = 0; q < kSolveRel; ++q) {
+          const int r = base + 256 * q + tid;
+          u[q] = slot0[q] >= 0 ? __ldcg(V.upd + C0.upd_off + r) : 0.0;
+          u[kSolveRel + q] = slot1[q] >= 0 ? __ldcg(V.upd + C1.upd_off + r) : 0.0;
+        }
+      } else {
+        int off[2 * kSolveRel];
+#pragma unroll
+        for (int q = 0; q < kSolveRel; ++q) {
+          const int r = base + 256 * q + tid;
+          off[q] = slot0[q] >= 0 ? r : -1;
+          off[kSolveRel + q] = slot1[q] >= 0 ? r : -1;
+        }
+        TakeOver<2 * kSolveRel>(V, S, A.u + C0.upd_off, A.u + C1.upd_off, off, u, limit);
       }
 #pragma unroll
       for (int q = 0; q < kSolveRel; ++q) {
         if (slot0[q] >= 0) {
-          v[slot0[q]] += u0[q];
+          v[slot0[q]] += u[q];
         }
       }
       __syncthreads();
 #pragma unroll
       for (int q = 0; q < kSolveRel; ++q) {
         if (slot1[q] >= 0) {
-          v[slot1[q]] += u1[q];
+          v[slot1[q]] += u[kSolveRel + q];
         }
       }
       __syncthreads();
@@ -2357,14 +2436,25 @@ __device__ __forceinline__ void FrontForward(const DeviceView& V, const Supernod
   WaitElements();
   __syncthreads();
   if (part == 0 && tid < k) {
-    V.xs[S.first_col + tid] = (1.0 / d) * y[tid];
+    if (kFlags) {
+      V.xs[S.first_col + tid] = dinv * y[tid];
+    } else if (!withhold) {
+      HandOver(A.y + S.first_col + tid, y[tid]);
+    }
   }
   // threads per row: as many groups of columns as rows leave room for
-  double* out = V.upd + S.upd_off + r0;
-  const int rb = nr > 128 ? 256 : nr > 64 ? 128 : nr > 32 ? 64 : 32;
-  const int groups = 256 / rb;
-  const int g = tid / rb;
-  const int cols = (k + groups - 1) / groups;
+  auto put = [&](int r, double u) {
+    if (kFlags) {
+      V.upd[S.upd_off + r0 + r] = u;
+    } else if (!withhold) {
+      HandOver(A.u + S.upd_off + r0 + r, u);
+    }
+  };
+  const int shift = nr > 128 ? 8 : nr > 64 ? 7 : nr > 32 ? 6 : 5;
+  const int rb = 1 << shift;
+  const int groups = 256 >> shift;
+  const int g = tid >> shift;
+  const int cols = (k + groups - 1) >> (8 - shift);
   const int j0 = min(k, g * cols);
   const int j1 = min(k, j0 + cols);
   if (nr <= 0) {
@@ -2388,7 +2478,7 @@ __device__ __forceinline__ void FrontForward(const DeviceView& V, const Supernod
     }
     const double acc = (a0 + a1) + (a2 + a3);
     if (groups == 1) {
-      out[r] = v[k + r] - acc;
+      put(r, v[k + r] - acc);
     } else {
       sums[tid] = acc;
     }
@@ -2400,18 +2490,18 @@ __device__ __forceinline__ void FrontForward(const DeviceView& V, const Supernod
       for (int q = 1; q < groups; ++q) {
         acc += sums[q * rb + tid];
       }
-      out[tid] = v[k + tid] - acc;
+      put(tid, v[k + tid] - acc);
     }
   }
 }
 
 /// Backward solve of a front's row chunk `part`: the chunk's L21^T x_R, and in
-/// the block whose chunk is the front's last to arrive (in any order; the
-/// chunks' products are summed in theirs) z = D^-1 y - L21^T x_R and x =
+/// the block of the last chunk (kFlags: of the last to arrive; the chunks'
+/// products are summed in their order) z = D^-1 y - L21^T x_R and x =
 /// L11^-T z into xs and the step. True in that block: the front is done.
-template <typename T, typename Wait>
+template <typename T, bool kFlags, typename Wait>
 __device__ __forceinline__ bool FrontBackward(const DeviceView& V, const SupernodeRec& S, const SolveArgs& A, int part,
-                                              int parts, uint32_t* arrived, double* zpart, double* buf, Wait wait) {
+                                              int parts, uint32_t* arrived, int64_t zoff, double* buf, Wait wait) {
   __shared__ int last;
   const int k = S.ncols;
   const int rows = SolveRows(k);
@@ -2424,6 +2514,7 @@ __device__ __forceinline__ bool FrontBackward(const DeviceView& V, const Superno
   double* z = xr + kSolveVec;
   double* sums = z + kSolvePivots;
   const double* M = A.inv + S.inv_off;
+  double* zpart = A.zpart + zoff;
   StageRows<T>(WorkFront<T>(V, S), S, r0, nr, pitch, slab);
   // columns of the inverse along the lanes, sixteen rows per group
   const int mi = tid & 63;
@@ -2441,9 +2532,11 @@ __device__ __forceinline__ bool FrontBackward(const DeviceView& V, const Superno
     at[q] = r < nr ? V.sn_rows[S.rows_off + r0 + r] : -1;
   }
   const int where = tid < k ? V.perm[S.first_col + tid] : 0;
+  const double dinv = !kFlags && tid < k ? 1.0 / A.dvec[S.first_col + tid] : 1.0;
+  uint32_t limit = A.wait_limit;
   const bool go = wait();
   double own = 0.0;
-  if (go) {
+  if (kFlags && go) {
     own = tid < k ? __ldcg(V.xs + S.first_col + tid) : 0.0;
 #pragma unroll
     for (int q = 0; q < kSolveMaxRows / 256; ++q) {
@@ -2451,20 +2544,33 @@ __device__ __forceinline__ bool FrontBackward(const DeviceView& V, const Superno
         xr[tid + 256 * q] = __ldcg(V.xs + at[q]);
       }
     }
+  } else if (!kFlags) {
+    if (tid < k && part == parts - 1) {
+      own = dinv * TakeOver(V, S, A.y + S.first_col + tid, limit);
+    }
+    double x[kSolveMaxRows / 256];
+    TakeOver<kSolveMaxRows / 256>(V, S, A.x, A.x, at, x, limit);
+#pragma unroll
+    for (int q = 0; q < kSolveMaxRows / 256; ++q) {
+      if (at[q] >= 0) {
+        xr[tid + 256 * q] = x[q];
+      }
+    }
   }
   WaitElements();
   __syncthreads();
   double sum = 0.0;
   if (go) {
-    const int kb = k > 128 ? 256 : k > 64 ? 128 : k > 32 ? 64 : k > 16 ? 32 : 16;
-    const int groups = 256 / kb;
+    const int shift = k > 128 ? 8 : k > 64 ? 7 : k > 32 ? 6 : k > 16 ? 5 : 4;
+    const int kb = 1 << shift;
+    const int groups = 256 >> shift;
     const int j = tid & (kb - 1);
     const T* lc = slab + min(j, k - 1) * pitch;
     double a0 = 0.0;
     double a1 = 0.0;
     double a2 = 0.0;
     double a3 = 0.0;
-    int r = tid / kb;
+    int r = tid >> shift;
     for (; r + 3 * groups < nr; r += 4 * groups) {
       a0 = fma(static_cast<double>(lc[r]), xr[r], a0);
       a1 = fma(static_cast<double>(lc[r + groups]), xr[r + groups], a1);
@@ -2481,12 +2587,39 @@ __device__ __forceinline__ bool FrontBackward(const DeviceView& V, const Superno
       for (int q = 1; q < groups; ++q) {
         sum += sums[q * kb + tid];
       }
-      if (parts > 1) {
+      if (kFlags && parts > 1) {
         zpart[static_cast<int64_t>(part) * k + tid] = sum;
+      } else if (!kFlags && part < parts - 1) {
+        HandOver(A.z + zoff + static_cast<int64_t>(part) * k + tid, sum);
       }
     }
   }
-  if (parts > 1) {
+  if (!kFlags) {
+    if (part < parts - 1) {
+      return false;
+    }
+    if (parts > 1) {
+      // the earlier chunks' products, eight at a time, summed in their order
+      const double mine = sum;
+      sum = 0.0;
+      if (tid < k) {
+        for (int p = 0; p < parts - 1; p += 8) {
+          int off[8];
+          double x[8];
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            off[q] = p + q < parts - 1 ? (p + q) * k + tid : -1;
+          }
+          TakeOver<8>(V, S, A.z + zoff, A.z + zoff, off, x, limit);
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            sum += x[q];
+          }
+        }
+      }
+      sum += mine;
+    }
+  } else if (parts > 1) {
     __syncthreads();
     if (tid == 0) {
       uint32_t before;
@@ -2533,7 +2666,11 @@ __device__ __forceinline__ bool FrontBackward(const DeviceView& V, const Superno
     if (tid >= i0 && tid < min(k, i0 + 64)) {
       const int q = tid - i0;
       const double x = (sums[q] + sums[64 + q]) + (sums[128 + q] + sums[192 + q]);
-      V.xs[S.first_col + tid] = x;
+      if (kFlags) {
+        V.xs[S.first_col + tid] = x;
+      } else {
+        HandOver(A.x + S.first_col + tid, x);
+      }
       V.step[where] = x;
     }
     __syncthreads();
@@ -2591,23 +2728,28 @@ __device__ __forceinline__ void PanelFrontTask(const DeviceView& V, const Supern
 /// and the lowest unfinished one is always being worked on (a block holds the
 /// next task only behind a lower one), so the launch completes whatever the
 /// number of resident blocks, and no level boundary holds fast fronts behind
-/// slow ones. A front's forward parts done counter (fdone) is what its parent
-/// waits for, its backward parts done (bdone) what its children wait for;
-/// zdone counts the backward row chunks. A tiled dense root's panels hand
-/// their values over one by one. With fronts solved by 32-column panels
-/// (kPanels): ydone says a wide front's y (or a split root's right-hand side)
-/// is out, a split root's panels publish one flag each per direction. A wait
-/// that runs out of its limit marks the instance kStatusWaitTimeout and lets
-/// the task's dependents go. withhold: a supernode whose forward parts are
-/// never published (-1: none), the test hook that makes a wait run out.
+/// slow ones. Without kFlags, what a task needs from others it takes over value
+/// by value, the block polling all of it from when the task before the one it
+/// waits for is done (the task's gate); a wait that runs out of its limit marks
+/// the instance kStatusWaitTimeout and reads as zero. With kFlags tasks wait for
+/// flags: a front's forward parts done counter (fdone) is what its parent waits
+/// for, its backward parts done (bdone) what its children wait for, zdone counts
+/// the backward row chunks; a wait that runs out lets the task's dependents go.
+/// kPanels adds the fronts solved by 32-column panels: ydone says a wide front's
+/// y (or a split root's right-hand side) is out, a split root's panels publish
+/// one flag each per direction. The rule: Symbolic::solve_handover.
+/// withhold: a supernode whose forward parts are never published (-1: none), the
+/// test hook that makes a wait run out.
 /// Bound by the chain of levels (a front's reads wait for its children's, then
 /// its parent's publication) and, in large trees, by the L2 and shared-memory
 /// traffic of L. Measured on B200, against pivot blocks of 32-column panels
 /// with every read behind the wait and one block per SM: 10-frame room 82 -> 57
 /// us, 76-frame floor plan 188 -> 120, 910-pose office 887 -> 424, 32 instances
-/// 892 -> 406; its four FP32 rounds in the mixed office 3396 -> 1260.
-template <bool kPanels>
-__global__ void __launch_bounds__(256, kPanels ? 1 : 2) KSolveTree(DeviceView V, SolveArgs A) {
+/// 892 -> 406, the four FP32 rounds of the mixed office 3396 -> 1260; values
+/// instead of flags then took the room to 36 and the floor plan to 83.
+template <bool kFlags, bool kPanels>
+__global__ void __launch_bounds__(256, kPanels ? 1 : 2) KSolveTree(const __grid_constant__ DeviceView V,
+                                                                   const __grid_constant__ SolveArgs A) {
   extern __shared__ __align__(16) double buf[];
   __shared__ int4 next[2];
   __shared__ int go;
@@ -2636,6 +2778,7 @@ __global__ void __launch_bounds__(256, kPanels ? 1 : 2) KSolveTree(DeviceView V,
     }
     const int s = next[turn].y;
     const int part = next[turn].z;
+    const int gate = next[turn].w;
     int4 ahead{};
     if (threadIdx.x == 0) {
       ahead = take();
@@ -2646,6 +2789,15 @@ __global__ void __launch_bounds__(256, kPanels ? 1 : 2) KSolveTree(DeviceView V,
     // what the task waits for, polled by one thread; the whole block learns
     // whether it came
     auto wait = [&] {
+      if (!kFlags) {
+        // handed-over values are waited for where they are read; the whole
+        // block polls them only once they are about to come
+        if (threadIdx.x == 0 && gate >= 0) {
+          WaitGate(A.y + gate, A.wait_limit);
+        }
+        __syncthreads();
+        return true;
+      }
       if (threadIdx.x == 0) {
         bool ready = true;
         switch (type) {
@@ -2699,23 +2851,25 @@ __global__ void __launch_bounds__(256, kPanels ? 1 : 2) KSolveTree(DeviceView V,
     if (active) {
       if (type == kTaskFrontForward) {
         if (f32) {
-          FrontForward<float>(V, S, A, part, buf, wait);
+          FrontForward<float, kFlags>(V, S, A, part, s == A.withhold, buf, wait);
         } else {
-          FrontForward<double>(V, S, A, part, buf, wait);
+          FrontForward<double, kFlags>(V, S, A, part, s == A.withhold, buf, wait);
         }
       } else if (type == kTaskFrontBackward) {
         const int parts = A.parts[2 * s];
-        double* zp = A.zpart + A.zoff[s];
+        const int64_t zoff = A.zoff[s];
         if (f32) {
-          done = FrontBackward<float>(V, S, A, part, parts, zdone + s, zp, buf, wait);
+          done = FrontBackward<float, kFlags>(V, S, A, part, parts, zdone + s, zoff, buf, wait);
         } else {
-          done = FrontBackward<double>(V, S, A, part, parts, zdone + s, zp, buf, wait);
+          done = FrontBackward<double, kFlags>(V, S, A, part, parts, zdone + s, zoff, buf, wait);
         }
       } else if (wait()) {
         switch (type) {
           case kTaskRootForward:
-            if (S.dense_cnt >= 0) {
-              RootPanel64<true>(V, S, A, part, buf);
+            if (S.dense_cnt >= 0 && kFlags) {
+              RootPanel64<true, true>(V, S, A, part, buf);
+            } else if (S.dense_cnt >= 0) {
+              RootPanel64Call<true>(V, S, A, part, buf);
             } else if (kPanels) {
               if (f32) {
                 RootForwardPanel<float>(V, S, A, part, pflag, buf);
@@ -2725,8 +2879,10 @@ __global__ void __launch_bounds__(256, kPanels ? 1 : 2) KSolveTree(DeviceView V,
             }
             break;
           case kTaskRootBackward:
-            if (S.dense_cnt >= 0) {
-              RootPanel64<false>(V, S, A, part, buf);
+            if (S.dense_cnt >= 0 && kFlags) {
+              RootPanel64<false, true>(V, S, A, part, buf);
+            } else if (S.dense_cnt >= 0) {
+              RootPanel64Call<false>(V, S, A, part, buf);
             } else if (kPanels) {
               if (f32) {
                 RootBackwardPanel<float>(V, S, A, part, bflag, buf);
@@ -2747,7 +2903,7 @@ __global__ void __launch_bounds__(256, kPanels ? 1 : 2) KSolveTree(DeviceView V,
       next[turn ^ 1] = ahead;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (kFlags && threadIdx.x == 0) {
       switch (type) {
         case kTaskForward:
           if (A.zoff[s] >= 0) {
@@ -2849,10 +3005,13 @@ void ConfigureSolveKernels(int max_front, int solve_panel_front) {
   static int tree_configured = 0;
   const int tree = static_cast<int>(SolveSmem(solve_panel_front));
   if (tree <= kMaxSmem && tree > tree_configured) {
-    CudaCheck(cudaFuncSetAttribute(KSolveTree<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    CudaCheck(cudaFuncSetAttribute(KSolveTree<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    static_cast<int>(SolveSmem(0))),
               "smem attr");
-    CudaCheck(cudaFuncSetAttribute(KSolveTree<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, tree), "smem attr");
+    CudaCheck(cudaFuncSetAttribute(KSolveTree<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   static_cast<int>(SolveSmem(0))),
+              "smem attr");
+    CudaCheck(cudaFuncSetAttribute(KSolveTree<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, tree), "smem attr");
     tree_configured = tree;
   }
 }
@@ -3150,14 +3309,18 @@ int LaunchSolveLevels(const Symbolic& S, const DeviceView& V, const FactorPlan& 
     A.sync = P.solve_sync;
     A.num_sn = num_sn;
     A.num_inv = P.num_inv;
-    A.handover = reinterpret_cast<uint64_t*>(P.solve_sync + SolveFlagWords(S));
-    A.handover_cols = S.dense_inv_doubles / kDenseTileCols;
+    A.y = reinterpret_cast<uint64_t*>(P.solve_sync + SolveFlagWords(S));
+    A.x = A.y + S.n;
+    A.u = A.x + S.n;
+    A.z = A.u + S.update_doubles;
     A.withhold = P.solve_withhold;
     A.wait_limit = P.solve_wait_polls > 0 ? P.solve_wait_polls : kWaitLimit;
-    if (S.solve_panels) {
-      KSolveTree<true><<<static_cast<unsigned>(blocks), 256, tree_smem, stream>>>(V, A);
+    if (S.solve_handover) {
+      KSolveTree<false, false><<<static_cast<unsigned>(blocks), 256, tree_smem, stream>>>(V, A);
+    } else if (S.solve_panels) {
+      KSolveTree<true, true><<<static_cast<unsigned>(blocks), 256, tree_smem, stream>>>(V, A);
     } else {
-      KSolveTree<false><<<static_cast<unsigned>(blocks), 256, tree_smem, stream>>>(V, A);
+      KSolveTree<true, false><<<static_cast<unsigned>(blocks), 256, tree_smem, stream>>>(V, A);
     }
     CudaCheck(cudaGetLastError(), "solve kernel");
     return 2;

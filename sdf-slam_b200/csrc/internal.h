@@ -260,6 +260,13 @@ constexpr int kSolveRootSplit = 256;
 constexpr int kInvBlockDoubles = 2 * 32 * 32;
 constexpr int kFrontInvCols = 64;
 constexpr int kFrontInvStrip = 16;
+/// A value handed over saves its writer a fence and its reader a trip to L2 per
+/// level, but every waiting thread polls; behind a long chain of root panels
+/// those polls slow the chain. Measured on B200, the solve launch by flags
+/// against by values: 10-frame room 57 against 36 us, 76-frame floor plan (4
+/// panels) 120 against 83, 331-pose room (16) 207 against 238, 910-pose office
+/// (43) 410 against 590.
+constexpr int kSolveHandoverPanels = 8;
 /// Fronts with at most kSolvePivots pivots solve by the inverse of their
 /// pivot block, each chunk of rows by its own task: a chunk forms y = L11^-1 v
 /// again rather than wait for another task's, which costs k^2 / 2 reads from L2
@@ -384,7 +391,9 @@ struct Symbolic {
   // buffer is reused level after level (tc_pack_rows rows of the widest).
   // Task list of the one-launch solve, in the order blocks take them: the
   // forward tasks of every supernode in level order, then the backward
-  // tasks in reverse. (type, sn, part, 0) quads, SolveTask types. A front of
+  // tasks in reverse. (type, sn, part, gate) quads, SolveTask types; gate: a
+  // handed-over value (see KSolveTree) that comes just before the ones the task
+  // waits for, or -1. A front of
   // at most kSolvePivots pivots takes one task per chunk of SolveRows rows
   // each way; a tiled dense root one per 64-row panel. Other fronts solve by
   // 32-column panels (solve_panels: there are some): with at least
@@ -400,6 +409,10 @@ struct Symbolic {
   std::vector<int32_t> solve_parts;
   std::vector<int64_t> zpart_off;
   int64_t zpart_doubles{0};
+  // Whether the solve's tasks hand their values over one by one rather than
+  // publish flags: no front solved by panels and no tiled root of more than
+  // kSolveHandoverPanels 64-row panels.
+  bool solve_handover{false};
   bool solve_panels{false};
   int solve_panel_front{0};
   std::vector<int32_t> pack_tasks;

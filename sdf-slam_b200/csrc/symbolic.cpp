@@ -25,6 +25,7 @@
 #include <atomic>
 #include <cmath>
 #include <functional>
+#include <limits>
 #include <mutex>
 #include <numeric>
 
@@ -681,10 +682,14 @@ void Finalize(Symbolic& S, std::vector<int> height, int panel_width, int tile) {
   S.inv_tasks.clear();
   S.front_inv_tasks.clear();
   S.solve_panels = false;
+  S.solve_handover = true;
   S.solve_panel_front = 0;
   for (int s = 0; s < Sn; ++s) {
     SupernodeRec& r = S.sn[static_cast<size_t>(s)];
     r.panel_base = static_cast<int32_t>(S.inv_tasks.size() / 2);
+    if (by_panels(r) || (tiled(r) && r.ncols > kSolveHandoverPanels * kDenseTileCols)) {
+      S.solve_handover = false;
+    }
     if (by_panels(r)) {
       S.solve_panels = true;
       S.solve_panel_front = std::max(S.solve_panel_front, r.F);
@@ -952,11 +957,46 @@ void Finalize(Symbolic& S, std::vector<int> height, int panel_width, int tile) {
   S.solve_parts.assign(2 * static_cast<size_t>(Sn), 1);
   S.zpart_off.assign(static_cast<size_t>(Sn), -1);
   S.zpart_doubles = 0;
-  auto push_task = [&S](int32_t type, int32_t sn, int32_t part) {
+  // gates: slots of y [0, n), x [n, 2 n) or the update vectors behind them
+  auto slot = [](int64_t index) {
+    return index <= std::numeric_limits<int32_t>::max() ? static_cast<int32_t>(index) : -1;
+  };
+  auto gate = [&](int32_t type, int32_t sn) -> int32_t {
+    const SupernodeRec& r = S.sn[static_cast<size_t>(sn)];
+    const int64_t n = S.n;
+    if (type == kTaskFrontForward || type == kTaskRootForward) {
+      // the first grandchild's update vector
+      if (r.child_count == 0) {
+        return -1;
+      }
+      const SupernodeRec& c = S.sn[static_cast<size_t>(S.child_list[static_cast<size_t>(r.child_begin)])];
+      if (c.child_count == 0) {
+        return -1;
+      }
+      const SupernodeRec& g = S.sn[static_cast<size_t>(S.child_list[static_cast<size_t>(c.child_begin)])];
+      return g.nrows > 0 ? slot(2 * n + g.upd_off) : -1;
+    }
+    if (type == kTaskRootBackward) {
+      return slot(r.first_col + r.ncols - 1);  // y of the last panel
+    }
+    if (r.parent < 0) {
+      return -1;
+    }
+    // x of the grandparent, of the root's last panel but one, y of a root
+    const SupernodeRec& p = S.sn[static_cast<size_t>(r.parent)];
+    if (p.parent >= 0) {
+      return slot(n + S.sn[static_cast<size_t>(p.parent)].first_col);
+    }
+    if (tiled(p) && p.ncols > kDenseTileCols) {
+      return slot(n + p.first_col + kDenseTileCols);
+    }
+    return slot(p.first_col);
+  };
+  auto push_task = [&](int32_t type, int32_t sn, int32_t part) {
     S.solve_tasks.push_back(type);
     S.solve_tasks.push_back(sn);
     S.solve_tasks.push_back(part);
-    S.solve_tasks.push_back(0);
+    S.solve_tasks.push_back(gate(type, sn));
   };
   auto root_split = [&S](const SupernodeRec& r) { return r.nrows == 0 && r.ncols >= kSolveRootSplit &&
                                                          r.ncols > S.small_pivots; };
