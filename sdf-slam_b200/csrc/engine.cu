@@ -14,9 +14,7 @@
 
 namespace sdfgpu {
 
-__global__ void KPointRows(DeviceView V);
-__global__ void KEikonalRows(DeviceView V);
-__global__ void KOdomRows(DeviceView V);
+__global__ void KRows(DeviceView V, int odom_blocks, int eik_blocks);
 __global__ void KCellStart(const int32_t* keys, int64_t n, int64_t num_cells, int32_t* cell_start);
 template <bool kWait>
 __global__ void KCellPass(DeviceView V, const int64_t* cells, int64_t count, uint32_t* ticket, uint32_t* done);
@@ -25,7 +23,6 @@ __global__ void KFinalizeNormal(DeviceView V);
 __global__ void KZeroFronts(DeviceView V, const int32_t* tasks, int64_t count, uint32_t* words, int64_t num_words,
                             uint64_t* stamp);
 __global__ void KClearWords(uint32_t* words, int64_t count, uint64_t* stamp);
-__global__ void KPosePairs(DeviceView V);
 __global__ void KBackup(DeviceView V, int dir, const int32_t* revert_mask);
 __global__ void KApplyStep(DeviceView V, uint64_t* stamp);
 __global__ void KCommitPoses(DeviceView V);
@@ -807,14 +804,12 @@ std::vector<int32_t> Engine::DownloadStatus() {
 }
 
 void Engine::LaunchRows() {
-  if (total_points_ > 0) {
-    KPointRows<<<Blocks(total_points_, 256), 256, 0, stream_>>>(V_);
-  }
-  if (total_eik_ > 0) {
-    KEikonalRows<<<Blocks(total_eik_, 256), 256, 0, stream_>>>(V_);
-  }
-  if (total_odom_ > 0) {
-    KOdomRows<<<Blocks(total_odom_, 128), 128, 0, stream_>>>(V_);
+  const unsigned odom_blocks = Blocks(total_odom_, 256);
+  const unsigned eik_blocks = Blocks(total_eik_, 256);
+  const unsigned blocks = odom_blocks + eik_blocks + Blocks(total_points_, 256);
+  if (blocks > 0) {
+    KRows<<<blocks, 256, 0, stream_>>>(V_, static_cast<int>(odom_blocks), static_cast<int>(eik_blocks));
+    ++times_.launches;
   }
   bool in_a = true;
   int sort_launches = 0;
@@ -829,8 +824,7 @@ void Engine::LaunchRows() {
   KCellStart<<<Blocks(total_cells_ + 1, 256), 256, 0, stream_>>>(keys, total_points_, total_cells_,
                                                                    cell_start_.get());
   CudaCheck(cudaGetLastError(), "row kernels");
-  times_.launches += (total_points_ > 0 ? 1 : 0) + sort_launches + (total_eik_ > 0 ? 1 : 0) +
-                     (total_odom_ > 0 ? 1 : 0) + 1;
+  times_.launches += sort_launches + 1;
 }
 
 int64_t Engine::ZeroTaskCount() const {
@@ -881,15 +875,14 @@ void Engine::LaunchNormal() {
       }
     }
   }
-  KPoseFrames<<<static_cast<unsigned>(total_frames_), 256, 0, stream_>>>(V_);
-  if (num_pairs_ > 0) {
-    KPosePairs<<<Blocks(static_cast<int64_t>(num_pairs_) * 9, 128), 128, 0, stream_>>>(V_);
-  }
+  // frames, then the pairs of frames (nine entries each)
+  const unsigned pose_blocks = static_cast<unsigned>(total_frames_) + Blocks(static_cast<int64_t>(num_pairs_) * 9, 256);
+  KPoseFrames<<<pose_blocks, 256, 0, stream_>>>(V_);
   if (n_ > 0) {
     KFinalizeNormal<<<Blocks(n_, 256), 256, 0, stream_>>>(V_);
   }
   CudaCheck(cudaGetLastError(), "normal kernels");
-  times_.launches += 1 + (num_pairs_ > 0 ? 1 : 0) + (n_ > 0 ? 1 : 0);
+  times_.launches += 1 + (n_ > 0 ? 1 : 0);
 }
 
 void Engine::LaunchTerms(bool step) {
