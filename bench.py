@@ -637,19 +637,11 @@ def _serve_pass(P, args, seed0, rate, check_oracle=False):
     return out
 
 
-# DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) of a
-# kernel class on a workload, from the committed one-kernel ncu captures
-# named beside each entry (L2 flushed before the captured step, as here).
-# DRAM bytes (read + written) per launch of a kernel class, averaged over its
-# launches in one iteration of the workload, from one-kernel ncu captures
-# (-k <kernel>, one iteration's launches; dram__bytes_read / _write)
-# summarised in profiles/launch_list_office.md
-KERNEL_TRAFFIC_BYTES = {
-    ("office", "KSchur"): 3054.4e6 / 20,   # the 20 Schur launches of the iteration
-    ("office", "KDenseRoot"): 33.4e6,
-    ("office", "KSolveTree"): 275.2e6,
-    ("office", "KFactorFront"): 137.0e6 / 10,
-}
+# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per launch of a
+# kernel class on a workload, averaged over its launches in one iteration, from
+# one-kernel ncu captures summarised in profiles/launch_list_office.md; a class
+# whose kernels have no capture has no entry
+KERNEL_TRAFFIC_BYTES = {}
 
 
 def kernel_profile(P, prob, opts1, flusher, iterations=3):

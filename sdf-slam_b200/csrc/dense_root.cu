@@ -621,6 +621,13 @@ __device__ bool FactorTask(const DeviceView& V, const SupernodeRec& S, int k, in
   return true;
 }
 
+/// Bound by the chain of FACTOR steps (about 14 us each behind one another) and,
+/// in the largest roots, by the updates' products and staging. One block per SM:
+/// the registers of the product and substitution fragments. Measured on B200
+/// against 32-column halves by four warps with the inverse on the chain and one
+/// step per UPDATE: a step of the chain 35 -> 14 us; 225 columns 140 -> 64 us, 990
+/// columns 550 -> 240, 2,727 columns 1650 -> 839, roots of a 32-instance batch 330 ->
+/// 145.
 __global__ void __launch_bounds__(kDThreads, 1) KDenseRoot(DeviceView V, DenseArgs A) {
   extern __shared__ double dense_sm[];
   __shared__ int task;

@@ -519,15 +519,12 @@ __global__ void __launch_bounds__(kBlockThreads, 1) KPanelBlock(DeviceView V, co
   }
 }
 
-/// Fronts with at most kSmallPivots pivots are factored by one kernel: a block
+/// Fronts with at most small_pivots pivots are factored by one kernel: a block
 /// takes the pivot block and a chunk of the rows below it as one trapezoid in
 /// shared memory and factors it right-looking by 8-column panels (BlockLdlt).
 /// Every block of a front repeats the pivot block; the one with
 /// row_begin == k writes L11 and D.
-constexpr int kSmallPivots = 128;
 constexpr int kFrontThreads = 256;
-/// Rows below the pivot block of one task at most.
-constexpr int kFrontMaxRows = 128;
 
 /// Shared memory of a trapezoid of k pivots and `rows` rows below.
 __host__ __device__ constexpr size_t FactorFrontSmem(int k, int rows) {

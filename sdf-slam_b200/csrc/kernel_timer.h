@@ -18,10 +18,10 @@ class KernelTimer {
     kFactorFront,
     kPanel,
     kUpdatePanel,   // KUpdate: outer-block and panel updates of the later pivot columns
-    kUpdateSchur,   // KSchur / KSchurF32: the fronts' Schur complements
+    kUpdateSchur,   // KChildSchur, KPoseSchur, KSchurF32: the fronts' Schur complements
     kPackSchur,
     kSchurTc,
-    kInvertDiagonal,
+    kInvertDiagonal,  // KInvertFronts, KInvertDiagonal: what the solve multiplies by
     kSolveTree,
     kDenseRoot,     // tiled LDL^T of the dense pose roots
     kClasses
