@@ -171,13 +171,16 @@ __device__ __forceinline__ void BlockAsA(const double (&c)[2], double (&a)[2]) {
 }
 
 /// Column blocks P.. of SubstituteRows (a template per block: every register
-/// index is a constant): W_P = C_P L_PP^-T, then the later blocks less
-/// W_P L_pP^T.
+/// index is a constant): W_P = (A_P + C_P) L_PP^-T, then the later blocks' sums C_p
+/// less W_P L_pP^T (summed on their own, see LdltTiles; X: the lane's entries of A).
 template <int P>
-__device__ __forceinline__ void SubstituteFrom(double (&C)[8][2], const double* L, const double* minv) {
+__device__ __forceinline__ void SubstituteFrom(double (&C)[8][2], const double* X, const double* L,
+                                               const double* minv) {
   if constexpr (P < 8) {
     const int q = threadIdx.x & 3;
     const int g = (threadIdx.x & 31) >> 2;
+    C[P][0] += X[8 * P * kDLd];
+    C[P][1] += X[(8 * P + 1) * kDLd];
     double a[2];
     BlockAsA(C[P], a);
     // B(k, n) = L_PP^-1(n, k)
@@ -195,13 +198,13 @@ __device__ __forceinline__ void SubstituteFrom(double (&C)[8][2], const double* 
         Dmma884(C[p], -a[1], L0[4 * kDLd + 8 * p]);
       }
     }
-    SubstituteFrom<P + 1>(C, L, minv);
+    SubstituteFrom<P + 1>(C, X, L, minv);
   }
 }
 
 /// W = A L^-T in place for the 64 x 64 tile A staged at X (column major) and
 /// the staged unit lower triangle L, eight rows per warp with no exchange
-/// between warps; the rows stay in registers as C fragments (the inverses of
+/// between warps; their sums stay in registers as C fragments (the inverses of
 /// the 8 x 8 diagonal blocks, warp p the p-th, go to minv). L(i, k) = W D^-1 also
 /// goes to dst (rows below h). Starts and ends with a block barrier.
 __device__ __forceinline__ void SubstituteRows(double* X, const double* L, double* minv, const double* dinv,
@@ -233,14 +236,9 @@ __device__ __forceinline__ void SubstituteRows(double* X, const double* L, doubl
     }
   }
   const int r = 8 * warp + g;
-  double C[8][2];
-#pragma unroll
-  for (int p = 0; p < 8; ++p) {
-    C[p][0] = X[(8 * p + 2 * q) * kDLd + r];
-    C[p][1] = X[(8 * p + 2 * q + 1) * kDLd + r];
-  }
+  double C[8][2] = {};
   __syncthreads();
-  SubstituteFrom<0>(C, L, minv);
+  SubstituteFrom<0>(C, X + 2 * q * kDLd + r, L, minv);
 #pragma unroll
   for (int p = 0; p < 8; ++p) {
 #pragma unroll

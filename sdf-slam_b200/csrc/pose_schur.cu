@@ -65,6 +65,13 @@ struct Smem {
   int last;
 };
 
+/// KChildSchur: what the products are subtracted from besides, sixteen entries
+/// per thread.
+struct ChildSmem {
+  Smem<double> stage;
+  double sum[16][kThreads];
+};
+
 /// Asynchronous copy of one element; size 0 writes zero and reads nothing.
 __device__ __forceinline__ void CopyZfill(double* dst, const double* src, int size) {
   const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
@@ -374,13 +381,19 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm) KPoseSchur(DeviceView 
 /// each (three times the reads, and half the launches nearly empty). Bound by
 /// the chain from the task to the store (task, entries, values, products) and,
 /// at the wide levels, by staging. Two blocks per SM, which keep their registers.
+/// The products are summed on their own (the entry and the update matrices wait in
+/// shared memory): added to the entry one by one, each is rounded to the entry's
+/// last bit, which made the step's error against its exact value 1.2 to 1.5 times
+/// that of products summed first.
 /// Measured on B200, the factorization with a pushing launch per sibling -> this:
-/// 10-frame room 158 -> 120 us, 76-frame floor plan 430 -> 351, 331-pose room 1095
-/// -> 1015, 32 instances 2070 -> 1842.
+/// 10-frame room 158 -> 105 us, 76-frame floor plan 430 -> 345, 331-pose room 1095
+/// -> 985 (of which the sums on their own, here and in LdltTiles, 117 -> 105, 358
+/// -> 345, 1007 -> 985), 32 instances 2070 -> 1842.
 __global__ void __launch_bounds__(kThreads, 2) KChildSchur(DeviceView V, const ChildTask* tasks,
                                                                       const ChildEntry* entries, const double* dvec) {
   extern __shared__ __align__(16) unsigned char pose_smem[];
-  Smem<double>& sm = *reinterpret_cast<Smem<double>*>(pose_smem);
+  ChildSmem& cs = *reinterpret_cast<ChildSmem*>(pose_smem);
+  Smem<double>& sm = cs.stage;
   const ChildTask t = tasks[blockIdx.x];
   if (V.active[t.instance] == 0 || (V.fronts32 != nullptr && V.inst[t.instance].mixed != 0)) {
     return;
@@ -394,14 +407,13 @@ __global__ void __launch_bounds__(kThreads, 2) KChildSchur(DeviceView V, const C
   double* out = V.fronts + t.front;
   const int r0 = wr + (lane >> 2);
   const int c0 = wc + 2 * (lane & 3);
-  // minus the result
-  double acc[2][4][2];
 #pragma unroll
   for (int e = 0; e < 16; ++e) {
     const int r = t.I * kT + r0 + 8 * (e >> 3);
     const int c = t.J * kT + c0 + 8 * ((e >> 1) & 3) + (e & 1);
-    acc[e >> 3][(e >> 1) & 3][e & 1] = c < t.k && r < t.F && c <= r ? -out[static_cast<int64_t>(c) * t.F + r] : 0.0;
+    cs.sum[e][tid] = c < t.k && r < t.F && c <= r ? out[static_cast<int64_t>(c) * t.F + r] : 0.0;
   }
+  double acc[2][4][2] = {};
   for (int q0 = 0; q0 < t.count; q0 += kChildScan) {
     const int n = min(kChildScan, t.count - q0);
     if (q0 > 0) {
@@ -457,7 +469,7 @@ __global__ void __launch_bounds__(kThreads, 2) KChildSchur(DeviceView V, const C
         }
 #pragma unroll
         for (int e = 0; e < 16; ++e) {
-          acc[e >> 3][(e >> 1) & 3][e & 1] -= v[e];
+          cs.sum[e][tid] += v[e];
         }
       }
     });
@@ -467,7 +479,7 @@ __global__ void __launch_bounds__(kThreads, 2) KChildSchur(DeviceView V, const C
     const int r = t.I * kT + r0 + 8 * (e >> 3);
     const int c = t.J * kT + c0 + 8 * ((e >> 1) & 3) + (e & 1);
     if (r < t.F && c <= r && c < t.fcols) {
-      out[static_cast<int64_t>(c) * t.F + r] = -acc[e >> 3][(e >> 1) & 3][e & 1];
+      out[static_cast<int64_t>(c) * t.F + r] = cs.sum[e][tid] - acc[e >> 3][(e >> 1) & 3][e & 1];
     }
   }
 }
@@ -507,8 +519,8 @@ int LaunchPoseSchur(const DeviceView& V, const PoseSchurArgs& args, bool fp32, c
 
 void LaunchChildSchur(const DeviceView& V, const ChildTask* tasks, int64_t count, const ChildEntry* entries,
                       const double* dvec, cudaStream_t stream) {
-  Configure<KChildSchur>(sizeof(Smem<double>));
-  KChildSchur<<<static_cast<unsigned>(count), kThreads, sizeof(Smem<double>), stream>>>(V, tasks, entries, dvec);
+  Configure<KChildSchur>(sizeof(ChildSmem));
+  KChildSchur<<<static_cast<unsigned>(count), kThreads, sizeof(ChildSmem), stream>>>(V, tasks, entries, dvec);
   CudaCheck(cudaGetLastError(), "child schur launch");
 }
 
