@@ -45,7 +45,7 @@ SOURCES = {
     "server.cpp": ["-x", "cu"],
     "kernel_timer.cpp": ["-x", "cu"],
 }
-HEADERS = ["internal.h", "device.cuh", "engine.h", "ldlt.h", "server.h", "host_pool.h", "incremental.h", "schur_tc.h", "kernel_timer.h", "dense_root.h", "pose_schur.h", "front_ops.cuh",
+HEADERS = ["internal.h", "device.cuh", "engine.h", "ldlt.h", "server.h", "host_pool.h", "incremental.h", "schur_tc.h", "kernel_timer.h", "dense_root.h", "pose_schur.h", "device_limit.h", "front_ops.cuh",
            "trig.cuh"]
 
 

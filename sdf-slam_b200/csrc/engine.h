@@ -225,7 +225,8 @@ inline size_t SolveSyncWords(const Symbolic& S) {
 int LaunchFactorLevels(const Symbolic& S, const DeviceView& V, const FactorPlan& P, cudaStream_t stream);
 /// Forward sweep, diagonal, backward sweep: V.step = A^-1 V.rhs (natural order).
 int LaunchSolveLevels(const Symbolic& S, const DeviceView& V, const FactorPlan& P, cudaStream_t stream);
-/// Raises the dynamic shared memory limit of the solve kernels.
+/// Raises the dynamic shared memory limits of the factor and solve kernels on the
+/// current device.
 void ConfigureSolveKernels(int max_front, int solve_panel_front);
 
 /// Pinned host buffer.

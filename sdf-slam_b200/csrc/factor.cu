@@ -20,6 +20,7 @@
 #include <cuda_runtime.h>
 
 #include "device.cuh"
+#include "device_limit.h"
 #include "front_ops.cuh"
 
 namespace sdfgpu {
@@ -2974,42 +2975,35 @@ size_t SolveSmem(int solve_panel_front) {
 }
 
 void ConfigureSolveKernels(int max_front, int solve_panel_front) {
-  // The attribute belongs to the kernel, not to an engine: it only grows, so
-  // an engine with smaller fronts never lowers another engine's limit.
-  static std::mutex mu;
-  static int configured = 48 * 1024;
-  static bool front_configured = false;
-  {
-    std::lock_guard<std::mutex> lk(mu);
-    if (!front_configured) {
-      CudaCheck(cudaFuncSetAttribute(KFactorFront, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem), "smem attr");
-      CudaCheck(cudaFuncSetAttribute(KExtendAdd, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     kEaStageDoubles * static_cast<int>(sizeof(double))),
-                "smem attr");
-      front_configured = true;
-    }
-  }
+  constexpr int kDefaultSmem = 48 * 1024;
+  static DeviceLimit front(0);
+  static DeviceLimit level(kDefaultSmem);
+  static DeviceLimit chunk(0);
+  static DeviceLimit tree(0);
   const int smem = max_front * static_cast<int>(sizeof(double));
   if (smem > kMaxSmem) {
     Fail(SDFGPU_ERR_INVALID_ARGUMENT, "front too large for the solve kernels");
   }
-  std::lock_guard<std::mutex> lk(mu);
-  if (smem > configured) {
-    CudaCheck(cudaFuncSetAttribute(KForward, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "smem attr");
-    CudaCheck(cudaFuncSetAttribute(KBackward, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "smem attr");
-    configured = smem;
-  }
-  static int tree_configured = 0;
-  const int tree = static_cast<int>(SolveSmem(solve_panel_front));
-  if (tree <= kMaxSmem && tree > tree_configured) {
-    CudaCheck(cudaFuncSetAttribute(KSolveTree<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   static_cast<int>(SolveSmem(0))),
-              "smem attr");
-    CudaCheck(cudaFuncSetAttribute(KSolveTree<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   static_cast<int>(SolveSmem(0))),
-              "smem attr");
-    CudaCheck(cudaFuncSetAttribute(KSolveTree<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, tree), "smem attr");
-    tree_configured = tree;
+  int dev = 0;
+  CudaCheck(cudaGetDevice(&dev), "device");
+  auto allow = [](auto* kernel, int bytes) {
+    CudaCheck(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes), "smem attr");
+  };
+  front.Raise(dev, kMaxSmem, [&](int bytes) {
+    allow(KFactorFront, bytes);
+    allow(KExtendAdd, kEaStageDoubles * static_cast<int>(sizeof(double)));
+  });
+  level.Raise(dev, smem, [&](int bytes) {
+    allow(KForward, bytes);
+    allow(KBackward, bytes);
+  });
+  chunk.Raise(dev, static_cast<int>(SolveSmem(0)), [&](int bytes) {
+    allow(KSolveTree<false, false>, bytes);
+    allow(KSolveTree<true, false>, bytes);
+  });
+  const int panels = static_cast<int>(SolveSmem(solve_panel_front));
+  if (panels <= kMaxSmem) {
+    tree.Raise(dev, panels, [&](int bytes) { allow(KSolveTree<true, true>, bytes); });
   }
 }
 
