@@ -1473,7 +1473,7 @@ void Engine::CommitAngles(const std::vector<int32_t>* revert) {
     }
   });
   // by the next iteration's first kernel, or by FlushCommit before anything
-  // else reads the poses
+  // else reads the poses and at the end of the solve
   commit_pending_ = true;
 }
 
@@ -1484,6 +1484,7 @@ void Engine::FlushCommit() {
   commit_pending_ = false;
   KCommitPoses<<<Blocks(total_frames_, 128), 128, 0, stream_>>>(V_);
   CudaCheck(cudaGetLastError(), "commit angles");
+  ++times_.launches;
 }
 
 double Engine::Cost(int i) {
@@ -1506,6 +1507,7 @@ void Engine::ApplyStep(int i, const double* step) {
   LaunchApplyStep();
   CudaCheck(cudaStreamSynchronize(stream_), "apply step sync");
   CommitAngles(nullptr);
+  FlushCommit();
   std::vector<int32_t> ones(host_.size(), 1);
   SetActive(ones);
   CudaCheck(cudaStreamSynchronize(stream_), "apply step sync");
@@ -2059,6 +2061,7 @@ sdfgpu_solve_result Engine::InstanceResult(int i) const {
 
 void Engine::EndSolve(sdfgpu_solve_result* results, double* cost_history, int capacity) {
   const size_t I = host_.size();
+  FlushCommit();  // the last step's angles: the solve leaves the state complete
   if (span_started_) {
     CudaCheck(cudaEventRecord(span_[1], stream_), "event");
   }
