@@ -189,6 +189,11 @@ int sdfgpu_measure_fp64_peak(double* tflops);
  * the state is not moved and the device stays usable. withhold_front = -1
  * restores normal solves. */
 int sdfgpu_debug_solve_fault(sdfgpu_problem* problem, int32_t withhold_front, uint32_t wait_polls);
+/* No counterpart in the reference: a test hook for the failure path of an
+ * iteration's launch. The enqueue that follows `after` more iterations fails with
+ * SDFGPU_ERR_CUDA as if the driver had refused it; nothing of that iteration
+ * runs, the state is the one after the iterations before it. after = -1: none. */
+int sdfgpu_debug_enqueue_fault(sdfgpu_problem* problem, int32_t after);
 /* Supernodes of the handle's current symbolic structure (0 before its first
  * device use). */
 int32_t sdfgpu_debug_supernode_count(sdfgpu_problem* problem);

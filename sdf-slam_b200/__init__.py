@@ -424,6 +424,11 @@ class Problem:
         polls, so the solve ends with TimeoutError; -1 restores it."""
         _check(lib().sdfgpu_debug_solve_fault(self._h, int(withhold_front), int(wait_polls)))
 
+    def debug_enqueue_fault(self, after: int):
+        """Test hook (sdfgpu_debug_enqueue_fault): the enqueue that follows
+        `after` more iterations fails; -1 for none."""
+        _check(lib().sdfgpu_debug_enqueue_fault(self._h, int(after)))
+
     def kernel_timing(self, classes=None):
         """Times the launches of the named kernel classes (all when None, none
         for an empty list) from the next iteration on (sdfgpu_kernel_timing);

@@ -119,6 +119,7 @@ SIGNATURES = {
     "sdfgpu_release_cached_memory": (ctypes.c_int, []),
     "sdfgpu_measure_fp64_peak": (ctypes.c_int, [c_dbl_p]),
     "sdfgpu_debug_solve_fault": (ctypes.c_int, [vp, ctypes.c_int32, ctypes.c_uint32]),
+    "sdfgpu_debug_enqueue_fault": (ctypes.c_int, [vp, ctypes.c_int32]),
     "sdfgpu_debug_supernode_count": (ctypes.c_int32, [vp]),
     "sdfgpu_kernel_timing": (ctypes.c_int, [vp, ctypes.c_uint32]),
     "sdfgpu_kernel_times": (ctypes.c_int, [vp, c_dbl_p, c_i64_p, c_dbl_p, ctypes.c_int32]),

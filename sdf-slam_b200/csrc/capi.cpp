@@ -239,6 +239,10 @@ int sdfgpu_debug_solve_fault(sdfgpu_problem* problem, int32_t withhold_front, ui
   return Guard([&] { Eng(problem).SetSolveFault(withhold_front, wait_polls); });
 }
 
+int sdfgpu_debug_enqueue_fault(sdfgpu_problem* problem, int32_t after) {
+  return Guard([&] { Eng(problem).SetEnqueueFault(after); });
+}
+
 int32_t sdfgpu_debug_supernode_count(sdfgpu_problem* problem) {
   if (problem == nullptr || !problem->engine) {
     return 0;

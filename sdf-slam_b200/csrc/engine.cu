@@ -1845,14 +1845,19 @@ void Engine::EnqueueIteration() {
   std::fill_n(h_theta_upd_.get(), total_frames_, 0);
   std::fill_n(h_stamps_.get(), 6, uint64_t{0});
   h_commit_[0] = commit_pending_ ? 1 : 0;
-  commit_pending_ = false;
   auto phases = [this] {
     stamping_ = true;
     for (int phase = 0; phase < 5; ++phase) {
       EnqueuePhase(phase);
+      if (!use_graph_) {
+        commit_pending_ = false;  // the first phase's first kernel takes them over
+      }
     }
     stamping_ = false;
   };
+  if (enqueue_fault_ >= 0 && enqueue_fault_-- == 0) {
+    Fail(SDFGPU_ERR_CUDA, "iteration launch refused (test hook)");
+  }
   if (!use_graph_) {
     phases();
     CudaCheck(cudaEventRecord(ready_, stream_), "event");
@@ -1884,6 +1889,8 @@ void Engine::EnqueueIteration() {
     times_.capture_host += std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
   }
   CudaCheck(cudaGraphLaunch(graph_exec_, stream_), "graph launch");
+  // (not before: a capture or launch that fails leaves them to FlushCommit)
+  commit_pending_ = false;
   CudaCheck(cudaEventRecord(ready_, stream_), "event");
   times_.launches += graph_launches_;
 }

@@ -361,6 +361,9 @@ class Engine {
   /// publishes supernode `withhold`'s forward flag (-1: normal) and a wait
   /// takes at most `wait_polls` polls (0: the default).
   void SetSolveFault(int withhold, uint32_t wait_polls);
+  /// Test hook: the enqueue that follows `after` more iterations fails (-1:
+  /// none).
+  void SetEnqueueFault(int after) { enqueue_fault_ = after; }
   /// Times the launches of the kernel classes in `mask` (KernelTimer) from
   /// the next iteration on, with zeroed totals; 0 stops timing.
   void SetKernelTiming(uint32_t mask);
@@ -553,6 +556,7 @@ class Engine {
   int64_t tc_map_rows_{0};
   int solve_withhold_{-1};
   uint32_t solve_wait_polls_{0};
+  int enqueue_fault_{-1};
   KernelTimer timer_;
   bool timing_phase_{false};  // EnqueuePhase is inside the factor or solve phase
   DevBuf<int64_t> fmp_ptr_, fmp_off_;
