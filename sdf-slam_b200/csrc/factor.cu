@@ -1985,7 +1985,7 @@ __device__ __forceinline__ void WaitGate(const uint64_t* slot, uint32_t limit) {
 /// each way) 1033 -> 887 us, 331-pose room 434 -> 380 us.
 template <bool kForward, bool kFlags>
 __device__ __forceinline__ void RootPanel64(const DeviceView& V, const SupernodeRec& S, const SolveArgs& A, int q,
-                                            double* buf) {
+                                            bool withhold, double* buf) {
   constexpr int kW = kDenseTileCols;
   const int k = S.ncols;
   const int64_t F64 = S.F;
@@ -2090,7 +2090,9 @@ __device__ __forceinline__ void RootPanel64(const DeviceView& V, const Supernode
   __syncthreads();
   if (tid < w) {
     const double x = (part[tid] + part[kW + tid]) + (part[2 * kW + tid] + part[3 * kW + tid]);
-    HandOver(slots + p0 + tid, x);
+    if (kFlags || !withhold) {  // (with flags the front's flag is withheld)
+      HandOver(slots + p0 + tid, x);
+    }
     if (!kForward) {
       const int64_t col = S.first_col + p0 + tid;
       if (kFlags) {
@@ -2106,8 +2108,8 @@ __device__ __forceinline__ void RootPanel64(const DeviceView& V, const Supernode
 /// us a solve).
 template <bool kForward>
 __device__ __noinline__ void RootPanel64Call(const DeviceView& V, const SupernodeRec& S, const SolveArgs& A, int q,
-                                             double* buf) {
-  RootPanel64<kForward, false>(V, S, A, q, buf);
+                                             bool withhold, double* buf) {
+  RootPanel64<kForward, false>(V, S, A, q, withhold, buf);
 }
 
 /// Right-hand side of a panel-split root: v = rhs plus the children's
@@ -2865,9 +2867,9 @@ __global__ void __launch_bounds__(256, kPanels ? 1 : 2) KSolveTree(const __grid_
         switch (type) {
           case kTaskRootForward:
             if (S.dense_cnt >= 0 && kFlags) {
-              RootPanel64<true, true>(V, S, A, part, buf);
+              RootPanel64<true, true>(V, S, A, part, false, buf);
             } else if (S.dense_cnt >= 0) {
-              RootPanel64Call<true>(V, S, A, part, buf);
+              RootPanel64Call<true>(V, S, A, part, s == A.withhold, buf);
             } else if (kPanels) {
               if (f32) {
                 RootForwardPanel<float>(V, S, A, part, pflag, buf);
@@ -2878,9 +2880,9 @@ __global__ void __launch_bounds__(256, kPanels ? 1 : 2) KSolveTree(const __grid_
             break;
           case kTaskRootBackward:
             if (S.dense_cnt >= 0 && kFlags) {
-              RootPanel64<false, true>(V, S, A, part, buf);
+              RootPanel64<false, true>(V, S, A, part, false, buf);
             } else if (S.dense_cnt >= 0) {
-              RootPanel64Call<false>(V, S, A, part, buf);
+              RootPanel64Call<false>(V, S, A, part, false, buf);
             } else if (kPanels) {
               if (f32) {
                 RootBackwardPanel<float>(V, S, A, part, bflag, buf);
