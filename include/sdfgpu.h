@@ -174,6 +174,11 @@ int sdfgpu_problem_destroy(sdfgpu_problem* problem);
  * on the current device when the host application needs the memory. */
 int sdfgpu_release_cached_memory(void);
 
+/* No counterpart in the reference. Bytes of device memory that the handles of
+ * the current device hold (whole blocks; released blocks that stay cached are
+ * not among them). */
+int sdfgpu_device_bytes_in_use(int64_t* bytes);
+
 /* No counterpart in the reference. Measures the current device's FP64
  * fused-multiply-add throughput (TFLOP/s, best of five timed launches of
  * independent FMA chains on every SM); the roofline denominator for the FP64

@@ -738,6 +738,14 @@ def release_cached_memory() -> None:
     _check(lib().sdfgpu_release_cached_memory())
 
 
+def device_bytes_in_use() -> int:
+    """Device memory that the handles of the current device hold
+    (sdfgpu_device_bytes_in_use)."""
+    n = ctypes.c_int64()
+    _check(lib().sdfgpu_device_bytes_in_use(ctypes.byref(n)))
+    return n.value
+
+
 def measure_fp64_peak() -> float:
     """The current device's measured FP64 FMA throughput in TFLOP/s
     (sdfgpu_measure_fp64_peak), the denominator of the FP64 kernels'

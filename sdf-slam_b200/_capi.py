@@ -117,6 +117,7 @@ SIGNATURES = {
                                                    ctypes.POINTER(vp)]),
     "sdfgpu_problem_destroy": (ctypes.c_int, [vp]),
     "sdfgpu_release_cached_memory": (ctypes.c_int, []),
+    "sdfgpu_device_bytes_in_use": (ctypes.c_int, [c_i64_p]),
     "sdfgpu_measure_fp64_peak": (ctypes.c_int, [c_dbl_p]),
     "sdfgpu_debug_solve_fault": (ctypes.c_int, [vp, ctypes.c_int32, ctypes.c_uint32]),
     "sdfgpu_debug_enqueue_fault": (ctypes.c_int, [vp, ctypes.c_int32]),

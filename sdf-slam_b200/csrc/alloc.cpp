@@ -44,6 +44,7 @@ struct Cache {
   // first; device -1 for pinned host blocks
   std::map<std::pair<int, size_t>, std::deque<std::pair<void*, uint64_t>>> free_blocks;
   std::map<int, size_t> cached_bytes;
+  std::map<int, size_t> used_bytes;  // of the device blocks that are handed out
   uint64_t stamp{0};
 };
 
@@ -218,6 +219,17 @@ int CurrentDevice() {
 
 }  // namespace
 
+namespace {
+
+/// Counts a device block as handed out (or, negative, as given back).
+void CountUse(int dev, int64_t bytes) {
+  Cache& c = TheCache();
+  const std::lock_guard<std::mutex> lock(c.mu);
+  c.used_bytes[dev] += static_cast<size_t>(bytes);
+}
+
+}  // namespace
+
 void* CachedDeviceAlloc(size_t bytes, size_t* got, int* device) {
   const int dev = CurrentDevice();
   const size_t cls = SizeClass(bytes);
@@ -226,6 +238,7 @@ void* CachedDeviceAlloc(size_t bytes, size_t* got, int* device) {
     *device = dev;
   }
   if (void* p = Take(dev, got)) {
+    CountUse(dev, static_cast<int64_t>(*got));
     return p;
   }
   void* p = nullptr;
@@ -250,7 +263,15 @@ void* CachedDeviceAlloc(size_t bytes, size_t* got, int* device) {
       Fail(SDFGPU_ERR_OUT_OF_MEMORY, "device allocation of " + std::to_string(bytes) + " bytes failed");
     }
   }
+  CountUse(dev, static_cast<int64_t>(cls));
   return p;
+}
+
+int64_t DeviceBytesInUse() {
+  const int dev = CurrentDevice();
+  Cache& c = TheCache();
+  const std::lock_guard<std::mutex> lock(c.mu);
+  return static_cast<int64_t>(c.used_bytes[dev]);
 }
 
 void ReleaseCachedDeviceMemory() {
@@ -264,7 +285,10 @@ void ReleaseCachedDeviceMemory() {
   CudaCheck(cudaMemPoolTrimTo(pool->pool, 0), "pool trim");
 }
 
-void CachedDeviceFree(void* p, size_t cls, int device) { Keep(device, cls, p, kMaxCachedDevice); }
+void CachedDeviceFree(void* p, size_t cls, int device) {
+  CountUse(device, -static_cast<int64_t>(cls));
+  Keep(device, cls, p, kMaxCachedDevice);
+}
 
 void* CachedHostAlloc(size_t bytes, size_t* got) {
   const size_t cls = SizeClass(bytes);

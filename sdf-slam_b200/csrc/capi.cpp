@@ -224,6 +224,13 @@ int sdfgpu_problem_destroy(sdfgpu_problem* problem) {
   return Guard([&] { delete problem; });
 }
 
+int sdfgpu_device_bytes_in_use(int64_t* bytes) {
+  return Guard([&] {
+    NeedHandle(bytes, "bytes");
+    *bytes = sdfgpu::DeviceBytesInUse();
+  });
+}
+
 int sdfgpu_release_cached_memory(void) {
   return Guard([&] { sdfgpu::ReleaseCachedDeviceMemory(); });
 }

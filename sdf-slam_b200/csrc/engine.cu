@@ -623,10 +623,6 @@ void Engine::UploadSymbolic() {
   if (any_mixed_) {
     AllocMixed();
   }
-  device_bytes_ = 0;
-  device_bytes_ += static_cast<int64_t>(fronts_.size()) * 8 + static_cast<int64_t>(pt_rec_.size()) * 8 +
-                   static_cast<int64_t>(mp_off_.size()) * 12 + static_cast<int64_t>(mm_off_.size()) * 8 +
-                   static_cast<int64_t>(total_points_) * 80;
   RefreshView();
   CudaCheck(cudaStreamSynchronize(s), "analyze upload");
 }

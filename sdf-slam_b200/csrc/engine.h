@@ -33,6 +33,8 @@ inline void CudaCheck(cudaError_t e, const char* what) {
 /// enqueued work uses it.
 void* CachedDeviceAlloc(size_t bytes, size_t* got, int* device = nullptr);
 void CachedDeviceFree(void* p, size_t bytes, int device);
+/// Bytes of the device blocks of the current device that are handed out.
+int64_t DeviceBytesInUse();
 /// Returns the current device's cached blocks and its pool's reserve to the
 /// driver.
 void ReleaseCachedDeviceMemory();
@@ -298,7 +300,6 @@ class Engine {
 
   [[nodiscard]] int count() const { return static_cast<int>(host_.size()); }
   [[nodiscard]] const HostProblem& host(int i) const { return host_[static_cast<size_t>(i)]; }
-  [[nodiscard]] int64_t DeviceBytes() const { return device_bytes_; }
 
   void GetState(int i, double* map_values, double* poses);
   void SetState(int i, const double* map_values, const double* poses);
@@ -474,7 +475,6 @@ class Engine {
   cudaEvent_t ready_{nullptr};  // the iteration enqueued last has finished
   bool span_started_{false};
   int device_{0};
-  int64_t device_bytes_{0};
   DeviceView V_{};
   IterTimes times_;
   int64_t total_cells_{0};

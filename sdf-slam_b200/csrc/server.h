@@ -30,9 +30,9 @@
 
 namespace sdfgpu {
 
-/// Device bytes an engine for `hp` will hold (state, specs, symbolic
-/// structure, fronts; the mixed-precision copies when `mixed`), from its
-/// host-side symbolic analysis `piece`.
+/// Device bytes an engine for `hp` will hold at most (state, specs, symbolic
+/// structure, task lists, inverses and workspaces, fronts; the mixed-precision
+/// copies when `mixed`), from its host-side symbolic analysis `piece`.
 int64_t EstimateDeviceBytes(const HostProblem& hp, const SymPiece& piece, bool mixed);
 
 class Server {
