@@ -278,27 +278,6 @@ __device__ __forceinline__ void InvertUnitLower32(const double* T, double* Mo) {
   }
 }
 
-/// out(r, c) = sum over l < 32 of X[r * xld + l] Y[c * yld + l] for the
-/// 32 x 32 block: thread (r = lane, c = warp + 8 q), four outputs each.
-template <typename F>
-__device__ __forceinline__ void Small32(const double* X, int xld, const double* Y, int yld, F&& sink) {
-  const int r = threadIdx.x & 31;
-  const int c0 = threadIdx.x >> 5;
-  double s[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll 8
-  for (int l = 0; l < 32; ++l) {
-    const double x = X[r * xld + l];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      s[q] = fma(x, Y[(c0 + 8 * q) * yld + l], s[q]);
-    }
-  }
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    sink(r, c0 + 8 * q, s[q]);
-  }
-}
-
 /// L^-1 = [M1 0; -M2 L21 M1  M2] of a factored tile whose L stands row major
 /// in T (the identity beyond w), column major 64 x 64 into the workspace: the
 /// triangular solve's 64-row panels multiply by it. H: three 32 x 33 blocks.
@@ -655,9 +634,6 @@ __global__ void __launch_bounds__(kDThreads, 1) KDenseRoot(DeviceView V, DenseAr
     const int nt = (S.ncols + kDT - 1) / kDT;
     int32_t* cnt = A.cnt + S.dense_cnt;
     if (tid == 0) {
-      if (A.trace != nullptr) {
-        A.trace[3 * t] = GlobalTimer();
-      }
       bool ok;
       if (i == k) {
         // FACTOR(k) with SOLVE(k, k - 1) and UPDATE(k, k, k - 1) folded in; it
@@ -679,9 +655,6 @@ __global__ void __launch_bounds__(kDThreads, 1) KDenseRoot(DeviceView V, DenseAr
         atomicExch(A.abort, 1);
       }
       go = ok ? 1 : 0;
-      if (A.trace != nullptr) {
-        A.trace[3 * t + 1] = GlobalTimer();
-      }
     }
     __syncthreads();
     if (go == 0) {
@@ -692,9 +665,6 @@ __global__ void __launch_bounds__(kDThreads, 1) KDenseRoot(DeviceView V, DenseAr
       if (!FactorTask(V, S, k, nt, A, cnt, dense_sm, &factored) && tid == 0) {
         atomicOr(V.status + S.instance, kStatusWaitTimeout);
         atomicExch(A.abort, 1);
-      }
-      if (tid == 0 && A.trace != nullptr) {
-        A.trace[3 * t + 2] = GlobalTimer();
       }
       continue;
     }
@@ -707,9 +677,6 @@ __global__ void __launch_bounds__(kDThreads, 1) KDenseRoot(DeviceView V, DenseAr
     if (tid == 0) {
       __threadfence();
       PublishTile(cnt + i * nt + j, k + len);
-      if (A.trace != nullptr) {
-        A.trace[3 * t + 2] = GlobalTimer();
-      }
     }
   }
 }
