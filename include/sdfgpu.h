@@ -194,6 +194,12 @@ int sdfgpu_measure_fp64_peak(double* tflops);
  * the state is not moved and the device stays usable. withhold_front = -1
  * restores normal solves. */
 int sdfgpu_debug_solve_fault(sdfgpu_problem* problem, int32_t withhold_front, uint32_t wait_polls);
+/* No counterpart in the reference: the same for the cell pass of the normal
+ * equations, whose cells wait for neighbours while one launch holds all of them
+ * (up to about 2,400 cells). Cell `withhold_cell` (row major over the cells of the
+ * handle's instances, one after the other) never says that it is done, and every
+ * wait gives up after `wait_polls` polls (0: the default). -1: normal. */
+int sdfgpu_debug_cell_fault(sdfgpu_problem* problem, int64_t withhold_cell, uint32_t wait_polls);
 /* No counterpart in the reference: a test hook for the failure path of an
  * iteration's launch. The enqueue that follows `after` more iterations fails with
  * SDFGPU_ERR_CUDA as if the driver had refused it; nothing of that iteration

@@ -424,6 +424,12 @@ class Problem:
         polls, so the solve ends with TimeoutError; -1 restores it."""
         _check(lib().sdfgpu_debug_solve_fault(self._h, int(withhold_front), int(wait_polls)))
 
+    def debug_cell_fault(self, withhold_cell: int, wait_polls: int = 0):
+        """Test hook (sdfgpu_debug_cell_fault): the one-launch cell pass never
+        marks `withhold_cell` done and a wait gives up after `wait_polls`
+        polls; -1 restores it."""
+        _check(lib().sdfgpu_debug_cell_fault(self._h, int(withhold_cell), int(wait_polls)))
+
     def debug_enqueue_fault(self, after: int):
         """Test hook (sdfgpu_debug_enqueue_fault): the enqueue that follows
         `after` more iterations fails; -1 for none."""

@@ -120,6 +120,7 @@ SIGNATURES = {
     "sdfgpu_device_bytes_in_use": (ctypes.c_int, [c_i64_p]),
     "sdfgpu_measure_fp64_peak": (ctypes.c_int, [c_dbl_p]),
     "sdfgpu_debug_solve_fault": (ctypes.c_int, [vp, ctypes.c_int32, ctypes.c_uint32]),
+    "sdfgpu_debug_cell_fault": (ctypes.c_int, [vp, ctypes.c_int64, ctypes.c_uint32]),
     "sdfgpu_debug_enqueue_fault": (ctypes.c_int, [vp, ctypes.c_int32]),
     "sdfgpu_debug_supernode_count": (ctypes.c_int32, [vp]),
     "sdfgpu_kernel_timing": (ctypes.c_int, [vp, ctypes.c_uint32]),

@@ -412,13 +412,10 @@ __device__ __forceinline__ double WarpSum16(double (&v)[16], int lane) {
   return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
 }
 
-/// Polls of a wait for a neighbouring cell (about a second).
-constexpr uint32_t kCellWaitLimit = 1u << 21;
-
 /// Waits until the cells that share a node with this one and come before it
 /// (a lower colour) are done, one lane per neighbour; a wait that runs out
 /// marks the instance.
-__device__ __forceinline__ void WaitForNeighbours(const DeviceView& V, int i, const uint32_t* done, int64_t cell,
+__device__ __forceinline__ void WaitForNeighbours(const DeviceView& V, int i, const CellSync& sync, int64_t cell,
                                                   int cx, int cy, int cw, int ch, int lane) {
   if (lane < 8) {
     const int at = lane < 4 ? lane : lane + 1;
@@ -427,9 +424,9 @@ __device__ __forceinline__ void WaitForNeighbours(const DeviceView& V, int i, co
     const int own = (cx & 1) | ((cy & 1) << 1);
     const int colour = (x & 1) | ((y & 1) << 1);
     if (x >= 0 && x < cw && y >= 0 && y < ch && colour < own) {
-      const uint32_t* word = done + cell + static_cast<int64_t>(y - cy) * cw + (x - cx);
+      const uint32_t* word = sync.done + cell + static_cast<int64_t>(y - cy) * cw + (x - cx);
       uint32_t it = 0;
-      for (; it < kCellWaitLimit; ++it) {
+      for (; it < sync.limit; ++it) {
         uint32_t v;
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(word) : "memory");
         if (v != 0) {
@@ -439,7 +436,7 @@ __device__ __forceinline__ void WaitForNeighbours(const DeviceView& V, int i, co
           __nanosleep(100);
         }
       }
-      if (it == kCellWaitLimit) {
+      if (it == sync.limit) {
         atomicOr(V.status + i, kStatusWaitTimeout);
       }
     }
@@ -460,7 +457,7 @@ __device__ __forceinline__ void WaitForNeighbours(const DeviceView& V, int i, co
 /// colours before its first write; everything before that runs ahead of the
 /// wait.
 template <bool kWait>
-__device__ __forceinline__ void CellPassOne(const DeviceView& V, int64_t entry, uint32_t* done, int lane) {
+__device__ __forceinline__ void CellPassOne(const DeviceView& V, int64_t entry, const CellSync& sync, int lane) {
   const int i = static_cast<int>(entry >> kCellBits);
   const int64_t cell = entry & ((int64_t{1} << kCellBits) - 1);
   const InstDev& I = V.inst[i];
@@ -482,8 +479,8 @@ __device__ __forceinline__ void CellPassOne(const DeviceView& V, int64_t entry, 
   const int re = V.cell_start[cell + 1];
   const int eik = V.eik_index[n0];
   if (rb == re && eik < 0) {
-    if (kWait && lane == 0) {
-      __stcg(done + cell, 1u);
+    if (kWait && lane == 0 && cell != sync.withhold) {
+      __stcg(sync.done + cell, 1u);
     }
     return;
   }
@@ -600,7 +597,7 @@ __device__ __forceinline__ void CellPassOne(const DeviceView& V, int64_t entry, 
     const bool tail = in && (lane == 31 || p + 1 >= re || fn != f);
     const int fl = f - I.frame_off;
     if (kWait && !waited) {
-      WaitForNeighbours(V, i, done, cell, cx, cy, cw, ch, lane);
+      WaitForNeighbours(V, i, sync, cell, cx, cy, cw, ch, lane);
       waited = true;
     }
     if (tail && fl >= 1) {
@@ -638,7 +635,7 @@ __device__ __forceinline__ void CellPassOne(const DeviceView& V, int64_t entry, 
     k_next = k_after;
   }
   if (kWait && !waited) {
-    WaitForNeighbours(V, i, done, cell, cx, cy, cw, ch, lane);
+    WaitForNeighbours(V, i, sync, cell, cx, cy, cw, ch, lane);
   }
   const double sum = WarpSum16(sums, lane);
   if (target != nullptr) {
@@ -650,8 +647,8 @@ __device__ __forceinline__ void CellPassOne(const DeviceView& V, int64_t entry, 
   if (kWait) {
     // every lane's writes before the flag
     __syncwarp();
-    if (lane == 0) {
-      asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(done + cell), "r"(1u) : "memory");
+    if (lane == 0 && cell != sync.withhold) {
+      asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(sync.done + cell), "r"(1u) : "memory");
     }
   }
 }
@@ -668,18 +665,18 @@ __device__ __forceinline__ void CellPassOne(const DeviceView& V, int64_t entry, 
 /// 324 -> 294, 32 instances 608 -> 496.
 template <bool kWait>
 __global__ void __launch_bounds__(256, 2) KCellPass(DeviceView V, const int64_t* cells, int64_t count,
-                                                    uint32_t* ticket, uint32_t* done) {
+                                                    CellSync sync) {
   const int lane = threadIdx.x & 31;
   if (!kWait) {
     const int64_t warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
     for (int64_t w = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; w < count; w += warps) {
-      CellPassOne<false>(V, cells[w], nullptr, lane);
+      CellPassOne<false>(V, cells[w], sync, lane);
     }
     return;
   }
   uint32_t taken = 0;
   if (lane == 0) {
-    taken = atomicAdd(ticket, 1u);
+    taken = atomicAdd(sync.ticket, 1u);
   }
   for (;;) {
     const int64_t w = __shfl_sync(0xffffffffu, taken, 0);
@@ -688,16 +685,14 @@ __global__ void __launch_bounds__(256, 2) KCellPass(DeviceView V, const int64_t*
     }
     uint32_t ahead = 0;
     if (lane == 0) {
-      ahead = atomicAdd(ticket, 1u);
+      ahead = atomicAdd(sync.ticket, 1u);
     }
-    CellPassOne<true>(V, cells[w], done, lane);
+    CellPassOne<true>(V, cells[w], sync, lane);
     taken = ahead;
   }
 }
-template __global__ void KCellPass<false>(DeviceView V, const int64_t* cells, int64_t count, uint32_t* ticket,
-                                          uint32_t* done);
-template __global__ void KCellPass<true>(DeviceView V, const int64_t* cells, int64_t count, uint32_t* ticket,
-                                         uint32_t* done);
+template __global__ void KCellPass<false>(DeviceView V, const int64_t* cells, int64_t count, CellSync sync);
+template __global__ void KCellPass<true>(DeviceView V, const int64_t* cells, int64_t count, CellSync sync);
 
 /// Cross-frame pose blocks of frame pairs linked by odometry / relation rows.
 __device__ __forceinline__ void PosePairEntry(const DeviceView& V, int64_t t) {

@@ -246,6 +246,10 @@ int sdfgpu_debug_solve_fault(sdfgpu_problem* problem, int32_t withhold_front, ui
   return Guard([&] { Eng(problem).SetSolveFault(withhold_front, wait_polls); });
 }
 
+int sdfgpu_debug_cell_fault(sdfgpu_problem* problem, int64_t withhold_cell, uint32_t wait_polls) {
+  return Guard([&] { Eng(problem).SetCellFault(withhold_cell, wait_polls); });
+}
+
 int sdfgpu_debug_enqueue_fault(sdfgpu_problem* problem, int32_t after) {
   return Guard([&] { Eng(problem).SetEnqueueFault(after); });
 }

@@ -11,6 +11,18 @@ namespace sdfgpu {
 /// Bits of the cell in an entry of the cell pass's list (instance above).
 constexpr int kCellBits = 40;
 
+/// Polls of a cell's wait for a neighbour (about a second).
+constexpr uint32_t kCellWaitLimit = 1u << 21;
+/// What the cells of a one-launch cell pass wait by: the counter they are taken
+/// from, a flag per cell, a cell that never sets its own (-1: none) and the polls of
+/// a wait.
+struct CellSync {
+  uint32_t* ticket;
+  uint32_t* done;
+  int64_t withhold;
+  uint32_t limit;
+};
+
 /// Per-instance constants (device copy of InstanceLayout plus schedule data).
 struct InstDev {
   int32_t nx, ny;

@@ -17,7 +17,7 @@ namespace sdfgpu {
 __global__ void KRows(DeviceView V, int odom_blocks, int eik_blocks);
 __global__ void KCellStart(const int32_t* keys, int64_t n, int64_t num_cells, int32_t* cell_start);
 template <bool kWait>
-__global__ void KCellPass(DeviceView V, const int64_t* cells, int64_t count, uint32_t* ticket, uint32_t* done);
+__global__ void KCellPass(DeviceView V, const int64_t* cells, int64_t count, CellSync sync);
 __global__ void KPoseFrames(DeviceView V);
 __global__ void KFinalizeNormal(DeviceView V);
 __global__ void KZeroFronts(DeviceView V, const int32_t* tasks, int64_t count, uint32_t* words, int64_t num_words,
@@ -856,8 +856,9 @@ void Engine::LaunchNormal() {
     // B200, one launch against four: 1,600 cells 20 against 48 us, 9,900 cells
     // 133 against 90, 39,600 cells 665 against 294.
     if (total_cells_ <= 8 * resident) {
-      KCellPass<true><<<Blocks(total_cells_ * 32, 256), 256, 0, stream_>>>(V_, pass_cells_.get(), total_cells_,
-                                                                           cell_words_.get(), cell_words_.get() + 1);
+      const CellSync sync{cell_words_.get(), cell_words_.get() + 1, cell_withhold_,
+                          cell_wait_polls_ > 0 ? cell_wait_polls_ : kCellWaitLimit};
+      KCellPass<true><<<Blocks(total_cells_ * 32, 256), 256, 0, stream_>>>(V_, pass_cells_.get(), total_cells_, sync);
       ++times_.launches;
     } else {
       for (int pass = 0; pass < 4; ++pass) {
@@ -865,7 +866,7 @@ void Engine::LaunchNormal() {
         if (count > 0) {
           const int64_t blocks = std::min<int64_t>(Blocks(count * 32, 256), resident);
           KCellPass<false><<<static_cast<unsigned>(blocks), 256, 0, stream_>>>(
-              V_, pass_cells_.get() + pass_begin_[pass], count, nullptr, nullptr);
+              V_, pass_cells_.get() + pass_begin_[pass], count, CellSync{});
           ++times_.launches;
         }
       }
@@ -1061,6 +1062,15 @@ void Engine::SetSolveFault(int withhold, uint32_t wait_polls) {
   solve_withhold_ = withhold;
   solve_wait_polls_ = wait_polls;
   DropGraph();  // the captured solve holds the previous parameters
+}
+
+void Engine::SetCellFault(int64_t withhold, uint32_t wait_polls) {
+  if (withhold < -1 || withhold >= total_cells_) {
+    Fail(SDFGPU_ERR_INVALID_ARGUMENT, "cell index out of range");
+  }
+  cell_withhold_ = withhold;
+  cell_wait_polls_ = wait_polls;
+  DropGraph();  // the captured cell pass holds the previous parameters
 }
 
 void Engine::UploadSolveTasks(cudaStream_t s) {

@@ -362,6 +362,9 @@ class Engine {
   /// publishes supernode `withhold`'s forward flag (-1: normal) and a wait
   /// takes at most `wait_polls` polls (0: the default).
   void SetSolveFault(int withhold, uint32_t wait_polls);
+  /// Test hook: the one-launch cell pass never marks cell `withhold` done (-1:
+  /// normal) and a wait takes at most `wait_polls` polls (0: the default).
+  void SetCellFault(int64_t withhold, uint32_t wait_polls);
   /// Test hook: the enqueue that follows `after` more iterations fails (-1:
   /// none).
   void SetEnqueueFault(int after) { enqueue_fault_ = after; }
@@ -556,6 +559,8 @@ class Engine {
   int64_t tc_map_rows_{0};
   int solve_withhold_{-1};
   uint32_t solve_wait_polls_{0};
+  int64_t cell_withhold_{-1};
+  uint32_t cell_wait_polls_{0};
   int enqueue_fault_{-1};
   KernelTimer timer_;
   bool timing_phase_{false};  // EnqueuePhase is inside the factor or solve phase

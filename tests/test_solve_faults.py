@@ -25,3 +25,29 @@ def test_withheld_supernode_ends_the_solve(frames, where):
     assert np.array_equal(before[0], after[0]) and np.array_equal(before[1], after[1])
     gpu.debug_solve_fault(-1, 0)
     assert P.solve(gpu, P.SolverOptions(max_iterations=2, step_tolerance=0.0)).iterations == 2
+
+
+@pytest.mark.parametrize("cell", [0, 20 * 39 + 20, 39 * 39 - 1])
+def test_withheld_cell_ends_the_solve(cell):
+    """The one-launch cell pass (39 x 39 cells): a corner and a middle cell of the
+    first colour, which neighbours wait for; the last corner, of the first colour
+    too."""
+    gpu = P.Problem.from_scene(scenes.room_scene(seed=4, grid=40, frames=10, beams=90, max_range=8), P.ProblemOptions())
+    P.solve(gpu, P.SolverOptions(max_iterations=1, step_tolerance=0.0))
+    before = gpu.state()
+    gpu.debug_cell_fault(cell, 4096)
+    with pytest.raises(TimeoutError):
+        P.solve(gpu, P.SolverOptions(max_iterations=2, step_tolerance=0.0))
+    after = gpu.state()
+    assert np.array_equal(before[0], after[0]) and np.array_equal(before[1], after[1])
+    gpu.debug_cell_fault(-1, 0)
+    assert P.solve(gpu, P.SolverOptions(max_iterations=2, step_tolerance=0.0)).iterations == 2
+
+
+def test_fault_hooks_refuse_what_is_out_of_range():
+    gpu = P.Problem.from_scene(scenes.room_scene(seed=4, grid=40, frames=10, beams=90, max_range=8), P.ProblemOptions())
+    gpu.cost()
+    for call in (lambda: gpu.debug_cell_fault(39 * 39), lambda: gpu.debug_cell_fault(-2),
+                 lambda: gpu.debug_solve_fault(gpu.debug_supernode_count()), lambda: gpu.debug_solve_fault(-2)):
+        with pytest.raises(ValueError):
+            call()
