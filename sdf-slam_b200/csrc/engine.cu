@@ -549,14 +549,26 @@ Symbolic Engine::GlobalStructure() {
   return Concatenate(pieces_, layout_, 32, 64, sched_, std::move(sym_));
 }
 
+void Engine::UploadMixedLists() {
+  ea_tasks_.Upload(sym_.ea_tasks, stream_);
+  ea_child_.Upload(sym_.ea_child, stream_);
+  update_tasks_.Upload(sym_.update_tasks, stream_);
+  pack_tasks_.Upload(sym_.pack_tasks, stream_);
+  tc_tasks_.Upload(sym_.tc_tasks, stream_);
+  zero_tasks_.Upload(sym_.zero_tasks, stream_);
+  sn_.Upload(sym_.sn, stream_);  // tc_pack
+}
+
 void Engine::UploadSymbolic() {
   DropGraph();
+  if (any_mixed_) {
+    AddMixedLists(sym_);
+  }
   // the previous structure may still be read by enqueued work
   CudaCheck(cudaStreamSynchronize(stream_), "analysis sync");
   cudaStream_t s = stream_;
   perm_.Upload(sym_.perm, s);
   pinv_.Upload(sym_.pinv, s);
-  sn_.Upload(sym_.sn, s);
   sn_rows_.Upload(sym_.sn_rows, s);
   sn_rel_.Upload(sym_.sn_rel, s);
   child_list_.Upload(sym_.child_list, s);
@@ -566,13 +578,9 @@ void Engine::UploadSymbolic() {
   mp_off_.Upload(sym_.mp_off, s);
   mp_frame_.Upload(sym_.mp_frame, s);
   allow_bits_.Upload(sym_.allow_bits, s);
-  ea_tasks_.Upload(sym_.ea_tasks, s);
-  ea_child_.Upload(sym_.ea_child, s);
   panel_tasks_.Upload(sym_.panel_tasks, s);
-  update_tasks_.Upload(sym_.update_tasks, s);
   small_tasks_.Upload(sym_.small_tasks, s);
-  pack_tasks_.Upload(sym_.pack_tasks, s);
-  tc_tasks_.Upload(sym_.tc_tasks, s);
+  UploadMixedLists();
   fronts_.AllocGrowable(static_cast<size_t>(sym_.front_doubles));
   upd_.Alloc(static_cast<size_t>(std::max<int64_t>(1, sym_.update_doubles)));
   max_front_ = 1;
@@ -745,6 +753,10 @@ void Engine::SetMode(const std::vector<int32_t>& mixed, int refine_steps, const 
   }
   inst_.Upload(inst_host_, stream_);
   if (any_mixed_) {
+    if (!sym_.mixed_lists) {
+      AddMixedLists(sym_);
+      UploadMixedLists();
+    }
     AllocMixed();
   }
   RefreshView();
@@ -1074,7 +1086,6 @@ void Engine::SetCellFault(int64_t withhold, uint32_t wait_polls) {
 }
 
 void Engine::UploadSolveTasks(cudaStream_t s) {
-  zero_tasks_.Upload(sym_.zero_tasks, s);
   child_tasks_.Upload(sym_.child_tasks, s);
   child_entries_.Upload(sym_.child_entries, s);
   if (!sym_.pose_tasks.empty()) {
@@ -1104,15 +1115,13 @@ void Engine::UploadSolveTasks(cudaStream_t s) {
 void Engine::UploadSchedule() {
   DropGraph();
   CudaCheck(cudaStreamSynchronize(stream_), "schedule sync");
-  ea_tasks_.Upload(sym_.ea_tasks, stream_);
-  ea_child_.Upload(sym_.ea_child, stream_);
+  if (any_mixed_) {
+    AddMixedLists(sym_);
+  }
   panel_tasks_.Upload(sym_.panel_tasks, stream_);
-  update_tasks_.Upload(sym_.update_tasks, stream_);
   small_tasks_.Upload(sym_.small_tasks, stream_);
-  pack_tasks_.Upload(sym_.pack_tasks, stream_);
-  tc_tasks_.Upload(sym_.tc_tasks, stream_);
   level_sn_.Upload(sym_.level_sn, stream_);
-  sn_.Upload(sym_.sn, stream_);
+  UploadMixedLists();
   UploadSolveTasks(stream_);
   CudaCheck(cudaStreamSynchronize(stream_), "schedule upload");
 }
@@ -1249,6 +1258,7 @@ void Engine::StartSpeculation(int i, const std::vector<double>& poses) {
                    poses.begin() + 3 * static_cast<int64_t>(L.frame_off + L.num_frames));
   sp->adopt_at = iters_[static_cast<size_t>(i)] + kSpeculationDelay;
   sp->has_structure = host_.size() == 1;
+  sp->mixed = any_mixed_;
   sp->sched = sched_;
   // the thread reads only this instance's problem, which stays unchanged
   // until the speculation is installed or dropped
@@ -1257,6 +1267,9 @@ void Engine::StartSpeculation(int i, const std::vector<double>& poses) {
     raw->piece = AnalyzeInstance(host_[static_cast<size_t>(raw->inst)], raw->margin, 0, &raw->poses);
     if (raw->has_structure) {
       raw->structure = ConcatenateOne(std::move(raw->piece), 32, 64, raw->sched);
+      if (raw->mixed) {
+        AddMixedLists(raw->structure);
+      }
     }
   });
   specs_.push_back(std::move(sp));

@@ -387,6 +387,8 @@ class Engine {
   Symbolic GlobalStructure();
   void UploadSymbolic();
   void UploadSchedule();
+  /// The lists of sym_ that only mixed solves read (AddMixedLists).
+  void UploadMixedLists();
   void InstallSchedule();          // sched_ into the structure, task lists and view
   double TimeMixedFactorSolve();   // fastest of three mixed factor + solve runs, ms
   /// The one-launch solve's task list and its scratch.
@@ -442,6 +444,7 @@ class Engine {
     Symbolic structure;
     Schedule sched;
     bool has_structure{false};
+    bool mixed{false};  // the structure gets the mixed solves' lists too
     std::future<void> done;
     int64_t adopt_at{0};  // iters_[inst] at which the analysis is installed
   };

@@ -370,6 +370,10 @@ struct Symbolic {
   std::vector<int32_t> level_begin;
   std::vector<int32_t> level_sn;
   std::vector<int32_t> level_panels;         // max panel count per level
+  // (what only the FP32 fronts of a mixed solve need is built when a handle first
+  // solves mixed: the extend-add, the pushed and the tensor-core Schur tasks, the
+  // clearing of update columns)
+  bool mixed_lists{false};
   std::vector<int32_t> ea_tasks;             // (sn, col_lo, col_hi, ea_child offset) quads
   std::vector<int32_t> ea_child;             // per task and child: update column range [begin, end)
   std::vector<TaskRange> ea_range;           // per level
@@ -604,6 +608,9 @@ Symbolic ConcatenateOne(SymPiece&& piece, int panel_width, int tile, const Sched
 
 /// Rebuilds the level schedule and task lists of S for another schedule.
 void Reschedule(Symbolic& S, const Schedule& sched);
+/// Builds the lists that only mixed solves read, unless they are there
+/// (Concatenate, ConcatenateOne and Reschedule leave them out).
+void AddMixedLists(Symbolic& S);
 
 /// Builds the supernodal symbolic factorization for a set of instances.
 Symbolic Analyze(const std::vector<HostProblem>& problems, const std::vector<InstanceLayout>& layout,

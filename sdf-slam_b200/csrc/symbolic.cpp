@@ -616,6 +616,30 @@ void PoseTasks(Symbolic& S) {
                    [](const PoseTask& a, const PoseTask& b) { return a.cost > b.cost; });
 }
 
+/// Blocks that keep every SM of a B200 busy, columns of an extend-add task.
+constexpr int64_t kFillBlocks = 148;
+constexpr int kEaCols = 16;
+
+/// The lists that only mixed solves read (AddMixedLists), empty.
+void ClearMixedLists(Symbolic& S) {
+  const auto levels = static_cast<size_t>(S.num_levels);
+  S.mixed_lists = false;
+  S.ea_tasks.clear();
+  S.ea_child.clear();
+  S.ea_range.assign(levels, {});
+  S.ea_stage.assign(levels, 0);
+  S.schur_range.clear();
+  S.schur_base.assign(levels + 1, 0);
+  S.pack_tasks.clear();
+  S.pack_range.assign(levels, {});
+  S.tc_tasks.clear();
+  S.tc_range.assign(levels, {});
+  S.tc_pack_rows = 0;
+  for (SupernodeRec& r : S.sn) {
+    r.tc_pack = -1;
+  }
+}
+
 /// Level lists and task lists once all supernodes exist.
 void Finalize(Symbolic& S, std::vector<int> height, int panel_width, int tile) {
   S.panel_width = panel_width;
@@ -663,7 +687,6 @@ void Finalize(Symbolic& S, std::vector<int> height, int panel_width, int tile) {
   }
   const int B = panel_width;
   const int T = tile;
-  constexpr int kEaCols = 16;
   const int kFrontRows = S.front_rows;
   // launch slots of the wide fronts: one per outer block when whole outer
   // blocks are factored at once (panel_rows 0), else one per panel
@@ -713,8 +736,6 @@ void Finalize(Symbolic& S, std::vector<int> height, int panel_width, int tile) {
       }
     }
   }
-  // blocks that keep every SM of a B200 (148) busy
-  constexpr int64_t kFillBlocks = 148;
   const int small = S.small_pivots;
   S.level_panels.assign(static_cast<size_t>(levels), 0);
   S.panel_index_base.assign(static_cast<size_t>(levels) + 1, 0);
@@ -769,84 +790,9 @@ void Finalize(Symbolic& S, std::vector<int> height, int panel_width, int tile) {
   const int slots = S.panel_index_base.back();
   S.panel_range.assign(static_cast<size_t>(slots), {});
   S.update_range.assign(static_cast<size_t>(slots), {});
-  S.ea_range.assign(static_cast<size_t>(levels), {});
-  S.ea_stage.assign(static_cast<size_t>(levels), 0);
-  // sibling slots (see the Schur tasks below)
-  std::vector<int32_t> sibling_slot(static_cast<size_t>(Sn), 0);
-  {
-    std::vector<int32_t> per_level(static_cast<size_t>(levels), 0);
-    for (int p = 0; p < Sn; ++p) {
-      const SupernodeRec& r = S.sn[static_cast<size_t>(p)];
-      for (int ci = 0; ci < r.child_count; ++ci) {
-        const int c = S.child_list[static_cast<size_t>(r.child_begin + ci)];
-        sibling_slot[static_cast<size_t>(c)] = per_level[static_cast<size_t>(height[static_cast<size_t>(c)])]++;
-      }
-      for (int ci = 0; ci < r.child_count; ++ci) {
-        const int c = S.child_list[static_cast<size_t>(r.child_begin + ci)];
-        per_level[static_cast<size_t>(height[static_cast<size_t>(c)])] = 0;
-      }
-    }
-  }
-  S.schur_range.clear();
-  S.schur_base.assign(static_cast<size_t>(levels) + 1, 0);
   for (int l = 0; l < levels; ++l) {
     const int qb = S.level_begin[static_cast<size_t>(l)];
     const int qe = S.level_begin[static_cast<size_t>(l) + 1];
-    // extend-add: parent columns in chunks, only for supernodes with children
-    S.ea_range[static_cast<size_t>(l)].begin = static_cast<int64_t>(S.ea_tasks.size() / 4);
-    // narrower column ranges on levels that would not fill the GPU
-    int ea_cols = kEaCols;
-    {
-      int64_t tasks = 0;
-      for (int q = qb; q < qe; ++q) {
-        const SupernodeRec& r = S.sn[static_cast<size_t>(S.level_sn[static_cast<size_t>(q)])];
-        if (r.child_count > 0) {
-          tasks += (r.fcols + kEaCols - 1) / kEaCols;
-        }
-      }
-      if (tasks < 2 * kFillBlocks) {
-        ea_cols = 4;
-      }
-    }
-    std::vector<int32_t> cursor;
-    int32_t stage = 0;
-    for (int q = qb; q < qe; ++q) {
-      const int s = S.level_sn[static_cast<size_t>(q)];
-      const SupernodeRec& r = S.sn[static_cast<size_t>(s)];
-      if (r.child_count == 0) {
-        continue;
-      }
-      // a task of a front up to kEaStageMaxF wide stages its columns' lower
-      // part in shared memory (narrower ranges where they would not fit)
-      const bool staged = r.F <= kEaStageMaxF;
-      const int cols = staged ? std::max(1, std::min(ea_cols, kEaStageDoubles / r.F)) : ea_cols;
-      // per child: the range of its update columns that land in [c, chi);
-      // the positions ascend, so one cursor per child walks them once
-      cursor.assign(static_cast<size_t>(r.child_count), 0);
-      for (int c = 0; c < r.fcols; c += cols) {
-        const int chi = std::min(r.fcols, c + cols);
-        if (staged) {
-          stage = std::max(stage, (chi - c) * (r.F - c));
-        }
-        S.ea_tasks.push_back(s);
-        S.ea_tasks.push_back(c);
-        S.ea_tasks.push_back(chi);
-        S.ea_tasks.push_back(static_cast<int32_t>(S.ea_child.size()));
-        for (int ci = 0; ci < r.child_count; ++ci) {
-          const SupernodeRec& ch = S.sn[static_cast<size_t>(S.child_list[static_cast<size_t>(r.child_begin + ci)])];
-          const int32_t* rel = S.sn_rel.data() + ch.rows_off;
-          int32_t& k = cursor[static_cast<size_t>(ci)];
-          S.ea_child.push_back(k);
-          while (k < ch.fcols - ch.ncols && rel[k] < chi) {
-            ++k;
-          }
-          S.ea_child.push_back(k);
-        }
-      }
-    }
-    S.ea_range[static_cast<size_t>(l)].count =
-        static_cast<int64_t>(S.ea_tasks.size() / 4) - S.ea_range[static_cast<size_t>(l)].begin;
-    S.ea_stage[static_cast<size_t>(l)] = stage;
     for (int t = 0; t < S.level_panels[static_cast<size_t>(l)]; ++t) {
       const size_t slot = static_cast<size_t>(S.panel_index_base[static_cast<size_t>(l)] + t);
       S.panel_range[slot].begin = static_cast<int64_t>(S.panel_tasks.size() / 3);
@@ -917,41 +863,7 @@ void Finalize(Symbolic& S, std::vector<int> height, int panel_width, int tile) {
       S.panel_range[slot].count = static_cast<int64_t>(S.panel_tasks.size() / 3) - S.panel_range[slot].begin;
       S.update_range[slot].count = static_cast<int64_t>(S.update_tasks.size() / 4) - S.update_range[slot].begin;
     }
-    // Schur complements, added straight into the parents' fronts: fronts of
-    // the level that share a parent go in separate launches, one per sibling
-    // slot (the front's rank among its parent's children of this level, in
-    // child-list order), so no two blocks of a launch add into one entry
-    // and each parent entry takes its children's terms in a fixed order
-    S.schur_base[static_cast<size_t>(l)] = static_cast<int32_t>(S.schur_range.size());
-    for (int slot = 0;; ++slot) {
-      TaskRange range;
-      range.begin = static_cast<int64_t>(S.update_tasks.size() / 4);
-      bool any = false;
-      for (int q = qb; q < qe; ++q) {
-        const int s = S.level_sn[static_cast<size_t>(q)];
-        if (sibling_slot[static_cast<size_t>(s)] != slot) {
-          continue;
-        }
-        any = true;
-        const SupernodeRec& r = S.sn[static_cast<size_t>(s)];
-        const int m = r.nrows;
-        for (int tj = 0; tj * T < r.fcols - r.ncols; ++tj) {
-          for (int ti = tj; ti * T < m; ++ti) {
-            S.update_tasks.push_back(s);
-            S.update_tasks.push_back(-1);
-            S.update_tasks.push_back(ti);
-            S.update_tasks.push_back(tj);
-          }
-        }
-      }
-      if (!any) {
-        break;
-      }
-      range.count = static_cast<int64_t>(S.update_tasks.size() / 4) - range.begin;
-      S.schur_range.push_back(range);
-    }
   }
-  S.schur_base[static_cast<size_t>(levels)] = static_cast<int32_t>(S.schur_range.size());
   // one-launch solve tasks
   S.solve_tasks.clear();
   S.solve_parts.assign(2 * static_cast<size_t>(Sn), 1);
@@ -1065,69 +977,16 @@ void Finalize(Symbolic& S, std::vector<int> height, int panel_width, int tile) {
       push_task(kTaskBackward, s, 0);
     }
   }
-  // tensor-core Schur tasks of the wide grid fronts (used by mixed solves)
-  S.pack_tasks.clear();
-  S.tc_tasks.clear();
-  S.pack_range.assign(static_cast<size_t>(levels), {});
-  S.tc_range.assign(static_cast<size_t>(levels), {});
-  S.tc_pack_rows = 0;
-  for (SupernodeRec& r : S.sn) {
-    r.tc_pack = -1;
-  }
-  for (int l = 0; l < levels; ++l) {
-    const int qb = S.level_begin[static_cast<size_t>(l)];
-    const int qe = S.level_begin[static_cast<size_t>(l) + 1];
-    int64_t rows = 0;
-    S.pack_range[static_cast<size_t>(l)].begin = static_cast<int64_t>(S.pack_tasks.size() / 3);
-    S.tc_range[static_cast<size_t>(l)].begin = static_cast<int64_t>(S.tc_tasks.size() / 3);
-    for (int q = qb; q < qe; ++q) {
-      const int s = S.level_sn[static_cast<size_t>(q)];
-      SupernodeRec& r = S.sn[static_cast<size_t>(s)];
-      if (r.pose_root != 0 || S.tc_min_rows <= 0 || r.nrows < S.tc_min_rows || r.ncols < 1) {
-        continue;
-      }
-      r.tc_pack = rows;
-      rows += TcPackRows(r.ncols, r.nrows);
-      const int nT = (r.nrows + kTcTile - 1) / kTcTile;
-      const int nC = (r.ncols + kTcChunk - 1) / kTcChunk;
-      for (int t = 0; t < nT; ++t) {
-        for (int c = 0; c < nC; ++c) {
-          S.pack_tasks.push_back(s);
-          S.pack_tasks.push_back(t);
-          S.pack_tasks.push_back(c);
-        }
-      }
-      for (int tj = 0; tj * kTcTile < r.fcols - r.ncols; ++tj) {
-        for (int ti = tj; ti < nT; ++ti) {
-          S.tc_tasks.push_back(s);
-          S.tc_tasks.push_back(ti);
-          S.tc_tasks.push_back(tj);
-        }
-      }
-    }
-    S.pack_range[static_cast<size_t>(l)].count =
-        static_cast<int64_t>(S.pack_tasks.size() / 3) - S.pack_range[static_cast<size_t>(l)].begin;
-    S.tc_range[static_cast<size_t>(l)].count =
-        static_cast<int64_t>(S.tc_tasks.size() / 3) - S.tc_range[static_cast<size_t>(l)].begin;
-    S.tc_pack_rows = std::max(S.tc_pack_rows, rows);
-  }
-  // front clearing tasks
+  // front clearing tasks of the pivot columns (KChildSchur writes the others)
   S.zero_tasks.clear();
-  // (pivot columns, trailing columns of fronts with children, of leaves)
-  for (int pass = 0; pass < 3; ++pass) {
-    for (int s = 0; s < Sn; ++s) {
-      const SupernodeRec& r = S.sn[static_cast<size_t>(s)];
-      for (int c = 0; c < r.fcols; c += kZeroCols) {
-        if ((c < r.ncols ? 0 : r.child_count > 0 ? 1 : 2) == pass) {
-          S.zero_tasks.push_back(s);
-          S.zero_tasks.push_back(c);
-        }
-      }
-    }
-    if (pass < 2) {
-      (pass == 0 ? S.zero_pivots : S.zero_main) = static_cast<int64_t>(S.zero_tasks.size() / 2);
+  for (int s = 0; s < Sn; ++s) {
+    for (int c = 0; c < S.sn[static_cast<size_t>(s)].ncols; c += kZeroCols) {
+      S.zero_tasks.push_back(s);
+      S.zero_tasks.push_back(c);
     }
   }
+  S.zero_pivots = S.zero_main = static_cast<int64_t>(S.zero_tasks.size() / 2);
+  ClearMixedLists(S);
   ChildTasks(S);
   PoseTasks(S);
   // tiled dense roots: counters, inverse workspace and task lists per level
@@ -1168,6 +1027,181 @@ void Finalize(Symbolic& S, std::vector<int> height, int panel_width, int tile) {
 }
 
 }  // namespace
+
+void AddMixedLists(Symbolic& S) {
+  if (S.mixed_lists) {
+    return;
+  }
+  ClearMixedLists(S);
+  S.mixed_lists = true;
+  const int Sn = static_cast<int>(S.sn.size());
+  const int levels = S.num_levels;
+  const std::vector<int>& height = S.height;
+  const int T = S.tile;
+  // sibling slots (see the Schur tasks below)
+  std::vector<int32_t> sibling_slot(static_cast<size_t>(Sn), 0);
+  {
+    std::vector<int32_t> per_level(static_cast<size_t>(levels), 0);
+    for (int p = 0; p < Sn; ++p) {
+      const SupernodeRec& r = S.sn[static_cast<size_t>(p)];
+      for (int ci = 0; ci < r.child_count; ++ci) {
+        const int c = S.child_list[static_cast<size_t>(r.child_begin + ci)];
+        sibling_slot[static_cast<size_t>(c)] = per_level[static_cast<size_t>(height[static_cast<size_t>(c)])]++;
+      }
+      for (int ci = 0; ci < r.child_count; ++ci) {
+        const int c = S.child_list[static_cast<size_t>(r.child_begin + ci)];
+        per_level[static_cast<size_t>(height[static_cast<size_t>(c)])] = 0;
+      }
+    }
+  }
+  for (int l = 0; l < levels; ++l) {
+    const int qb = S.level_begin[static_cast<size_t>(l)];
+    const int qe = S.level_begin[static_cast<size_t>(l) + 1];
+    // extend-add: parent columns in chunks, only for supernodes with children
+    S.ea_range[static_cast<size_t>(l)].begin = static_cast<int64_t>(S.ea_tasks.size() / 4);
+    // narrower column ranges on levels that would not fill the GPU
+    int ea_cols = kEaCols;
+    {
+      int64_t tasks = 0;
+      for (int q = qb; q < qe; ++q) {
+        const SupernodeRec& r = S.sn[static_cast<size_t>(S.level_sn[static_cast<size_t>(q)])];
+        if (r.child_count > 0) {
+          tasks += (r.fcols + kEaCols - 1) / kEaCols;
+        }
+      }
+      if (tasks < 2 * kFillBlocks) {
+        ea_cols = 4;
+      }
+    }
+    std::vector<int32_t> cursor;
+    int32_t stage = 0;
+    for (int q = qb; q < qe; ++q) {
+      const int s = S.level_sn[static_cast<size_t>(q)];
+      const SupernodeRec& r = S.sn[static_cast<size_t>(s)];
+      if (r.child_count == 0) {
+        continue;
+      }
+      // a task of a front up to kEaStageMaxF wide stages its columns' lower
+      // part in shared memory (narrower ranges where they would not fit)
+      const bool staged = r.F <= kEaStageMaxF;
+      const int cols = staged ? std::max(1, std::min(ea_cols, kEaStageDoubles / r.F)) : ea_cols;
+      // per child: the range of its update columns that land in [c, chi);
+      // the positions ascend, so one cursor per child walks them once
+      cursor.assign(static_cast<size_t>(r.child_count), 0);
+      for (int c = 0; c < r.fcols; c += cols) {
+        const int chi = std::min(r.fcols, c + cols);
+        if (staged) {
+          stage = std::max(stage, (chi - c) * (r.F - c));
+        }
+        S.ea_tasks.push_back(s);
+        S.ea_tasks.push_back(c);
+        S.ea_tasks.push_back(chi);
+        S.ea_tasks.push_back(static_cast<int32_t>(S.ea_child.size()));
+        for (int ci = 0; ci < r.child_count; ++ci) {
+          const SupernodeRec& ch = S.sn[static_cast<size_t>(S.child_list[static_cast<size_t>(r.child_begin + ci)])];
+          const int32_t* rel = S.sn_rel.data() + ch.rows_off;
+          int32_t& k = cursor[static_cast<size_t>(ci)];
+          S.ea_child.push_back(k);
+          while (k < ch.fcols - ch.ncols && rel[k] < chi) {
+            ++k;
+          }
+          S.ea_child.push_back(k);
+        }
+      }
+    }
+    S.ea_range[static_cast<size_t>(l)].count =
+        static_cast<int64_t>(S.ea_tasks.size() / 4) - S.ea_range[static_cast<size_t>(l)].begin;
+    S.ea_stage[static_cast<size_t>(l)] = stage;
+    // Schur complements, added straight into the parents' fronts: fronts of
+    // the level that share a parent go in separate launches, one per sibling
+    // slot (the front's rank among its parent's children of this level, in
+    // child-list order), so no two blocks of a launch add into one entry
+    // and each parent entry takes its children's terms in a fixed order
+    S.schur_base[static_cast<size_t>(l)] = static_cast<int32_t>(S.schur_range.size());
+    for (int slot = 0;; ++slot) {
+      TaskRange range;
+      range.begin = static_cast<int64_t>(S.update_tasks.size() / 4);
+      bool any = false;
+      for (int q = qb; q < qe; ++q) {
+        const int s = S.level_sn[static_cast<size_t>(q)];
+        if (sibling_slot[static_cast<size_t>(s)] != slot) {
+          continue;
+        }
+        any = true;
+        const SupernodeRec& r = S.sn[static_cast<size_t>(s)];
+        const int m = r.nrows;
+        for (int tj = 0; tj * T < r.fcols - r.ncols; ++tj) {
+          for (int ti = tj; ti * T < m; ++ti) {
+            S.update_tasks.push_back(s);
+            S.update_tasks.push_back(-1);
+            S.update_tasks.push_back(ti);
+            S.update_tasks.push_back(tj);
+          }
+        }
+      }
+      if (!any) {
+        break;
+      }
+      range.count = static_cast<int64_t>(S.update_tasks.size() / 4) - range.begin;
+      S.schur_range.push_back(range);
+    }
+  }
+  S.schur_base[static_cast<size_t>(levels)] = static_cast<int32_t>(S.schur_range.size());
+  // tensor-core Schur tasks of the wide grid fronts
+  for (int l = 0; l < levels; ++l) {
+    const int qb = S.level_begin[static_cast<size_t>(l)];
+    const int qe = S.level_begin[static_cast<size_t>(l) + 1];
+    int64_t rows = 0;
+    S.pack_range[static_cast<size_t>(l)].begin = static_cast<int64_t>(S.pack_tasks.size() / 3);
+    S.tc_range[static_cast<size_t>(l)].begin = static_cast<int64_t>(S.tc_tasks.size() / 3);
+    for (int q = qb; q < qe; ++q) {
+      const int s = S.level_sn[static_cast<size_t>(q)];
+      SupernodeRec& r = S.sn[static_cast<size_t>(s)];
+      if (r.pose_root != 0 || S.tc_min_rows <= 0 || r.nrows < S.tc_min_rows || r.ncols < 1) {
+        continue;
+      }
+      r.tc_pack = rows;
+      rows += TcPackRows(r.ncols, r.nrows);
+      const int nT = (r.nrows + kTcTile - 1) / kTcTile;
+      const int nC = (r.ncols + kTcChunk - 1) / kTcChunk;
+      for (int t = 0; t < nT; ++t) {
+        for (int c = 0; c < nC; ++c) {
+          S.pack_tasks.push_back(s);
+          S.pack_tasks.push_back(t);
+          S.pack_tasks.push_back(c);
+        }
+      }
+      for (int tj = 0; tj * kTcTile < r.fcols - r.ncols; ++tj) {
+        for (int ti = tj; ti < nT; ++ti) {
+          S.tc_tasks.push_back(s);
+          S.tc_tasks.push_back(ti);
+          S.tc_tasks.push_back(tj);
+        }
+      }
+    }
+    S.pack_range[static_cast<size_t>(l)].count =
+        static_cast<int64_t>(S.pack_tasks.size() / 3) - S.pack_range[static_cast<size_t>(l)].begin;
+    S.tc_range[static_cast<size_t>(l)].count =
+        static_cast<int64_t>(S.tc_tasks.size() / 3) - S.tc_range[static_cast<size_t>(l)].begin;
+    S.tc_pack_rows = std::max(S.tc_pack_rows, rows);
+  }
+  // clearing of the update columns: of fronts with children, then of leaves
+  for (const bool leaves : {false, true}) {
+    for (int s = 0; s < Sn; ++s) {
+      const SupernodeRec& r = S.sn[static_cast<size_t>(s)];
+      if ((r.child_count == 0) != leaves) {
+        continue;
+      }
+      for (int c = (r.ncols + kZeroCols - 1) / kZeroCols * kZeroCols; c < r.fcols; c += kZeroCols) {
+        S.zero_tasks.push_back(s);
+        S.zero_tasks.push_back(c);
+      }
+    }
+    if (!leaves) {
+      S.zero_main = static_cast<int64_t>(S.zero_tasks.size() / 2);
+    }
+  }
+}
 
 /// Appends the tasks of an n-column dense root's tiled LDL^T with their
 /// bottom levels: the longest path of task weights (about their durations in
@@ -1872,13 +1906,9 @@ void Reschedule(Symbolic& S, const Schedule& sched) {
   S.front_rows = sched.front_rows;
   S.panel_rows = sched.panel_rows;
   S.tc_min_rows = sched.tc_min_rows;
-  S.ea_tasks.clear();
-  S.ea_child.clear();
   S.panel_tasks.clear();
   S.update_tasks.clear();
   S.small_tasks.clear();
-  S.ea_range.clear();
-  S.ea_stage.clear();
   S.panel_range.clear();
   S.update_range.clear();
   S.small_range.clear();
