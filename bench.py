@@ -639,9 +639,11 @@ def _serve_pass(P, args, seed0, rate, check_oracle=False):
 
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per launch of a
 # kernel class on a workload, averaged over its launches in one iteration, from
-# one-kernel ncu captures summarised in profiles/launch_list_office.md; a class
-# whose kernels have no capture has no entry
-KERNEL_TRAFFIC_BYTES = {}
+# the ncu capture summarised in profiles/launch_list_office.md; a class whose
+# kernels have no capture has no entry
+KERNEL_TRAFFIC_BYTES = {("office", "KSchur"): 105.0e6}
+# the kernels of the classes that are not one kernel of that name (FP64 path)
+CLASS_KERNELS = {"KSchur": "KPoseSchur, KChildSchur", "KInvertDiagonal": "KInvertFronts, KInvertDiagonal"}
 
 
 def kernel_profile(P, prob, opts1, flusher, iterations=3):
@@ -776,11 +778,12 @@ def run_gpu(args, dist, world, rank, local):
         achieved = work_per_launch / (avg_ms * 1e-3) / 1e12
         peak, unit, bound = fp64_peak, "TFLOP/s", "tensor"
         src = "measured FP64 FMA throughput of this GPU (sdfgpu_measure_fp64_peak): the FP64 pipe bounds it"
+    traffic = KERNEL_TRAFFIC_BYTES.get((args.workload, dominant_kernel))
     roofline = {
         "bound": bound, "achieved": achieved, "peak": peak, "unit": unit, "frac": achieved / peak,
-        "traffic": KERNEL_TRAFFIC_BYTES.get((args.workload, dominant_kernel)),
-        "traffic_source": "one-kernel ncu capture, DRAM bytes per launch (profiles/launch_list_office.md)",
-        "kernel": dominant_kernel, "peak_source": src, "launches_timed": dom["launches"],
+        "traffic": traffic,
+        **({"traffic_source": "ncu capture, DRAM bytes per launch (profiles/launch_list_office.md)"} if traffic else {}),
+        "kernel": CLASS_KERNELS.get(dominant_kernel, dominant_kernel), "peak_source": src, "launches_timed": dom["launches"],
         "avg_launch_ms": avg_ms, "work_per_launch": work_per_launch, "work_unit": dom["work_unit"]}
     roofline_factor = {
         "bound": "tensor", "achieved": flops / per_step[2] / 1e12, "peak": fp64_peak, "unit": "TFLOP/s",
