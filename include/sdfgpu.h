@@ -186,9 +186,9 @@ int sdfgpu_device_bytes_in_use(int64_t* bytes);
 int sdfgpu_measure_fp64_peak(double* tflops);
 
 /* No counterpart in the reference: a test hook for the failure path of the
- * one-launch triangular solve, whose blocks wait on flags that other blocks
- * publish. From the next solve on, supernode `withhold_front` (an index into
- * the handle's current symbolic structure) never publishes its forward flag
+ * one-launch triangular solve, whose blocks wait on flags or values that other
+ * blocks publish. From the next solve on, supernode `withhold_front` (an index into
+ * the handle's current symbolic structure) never publishes its forward result
  * and every wait gives up after `wait_polls` polls (0: the default of about
  * a second); the wait that runs out ends the solve with SDFGPU_ERR_TIMEOUT,
  * the state is not moved and the device stays usable. withhold_front = -1
@@ -316,7 +316,8 @@ int sdfgpu_linearization_get(sdfgpu_problem* problem, double* residuals, int32_t
                              double* step);
 
 /* Timing breakdown of the last solve on this handle, measured with the
- * device's timer as each phase's first kernel starts, in seconds of GPU time per
+ * device's timer as each phase's first kernel starts (the last one's end: as its
+ * last kernel starts), in seconds of GPU time per
  * phase summed over its iterations: [0] residuals + Jacobian + cell sort, [1] J^T J + J^T r,
  * [2] factorization, [3] triangular solves, [4] step + cost; [5] iterations;
  * [6] device time from the first iteration's start to the last one's end;

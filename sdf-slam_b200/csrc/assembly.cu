@@ -845,9 +845,6 @@ __global__ void __launch_bounds__(256) KPoseFrames(DeviceView V) {
   V.rhs[c0 + 2] = acc[8];
 }
 
-/// Turns the accumulated J^T r into -J^T r and applies the damping of
-/// lm_solver.cpp:321-330 to every diagonal entry (lambda, or lambda times
-/// max(diag, 1e-12) under Marquardt scaling).
 /// Zeroes the lower triangle of the assembly fronts before the row kernels
 /// add into them: one warp per column c, rows c..F-1 (coalesced); task (sn,
 /// first of kZeroCols columns). Also J^T r and the cell pass's counter and
@@ -881,6 +878,9 @@ __global__ void KZeroFronts(DeviceView V, const int32_t* tasks, int64_t count, u
   }
 }
 
+/// Turns the accumulated J^T r into -J^T r and applies the damping of
+/// lm_solver.cpp:321-330 to every diagonal entry (lambda, or lambda times
+/// max(diag, 1e-12) under Marquardt scaling).
 __global__ void KFinalizeNormal(DeviceView V) {
   const int col = blockIdx.x * blockDim.x + threadIdx.x;
   if (col >= V.n) {

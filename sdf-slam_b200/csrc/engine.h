@@ -409,12 +409,13 @@ class Engine {
   void LaunchFactor();
   void LaunchSolve();
   void LaunchStepAndCost(bool backup);
-  /// ApplyStep of the running instances (KApplyStep, provisional angles on
-  /// the device) and the copy of the moved frames' angles to the host.
+  /// ApplyStep of the running instances (KApplyStep: provisional angles on
+  /// the device, the moved frames' unwrapped ones in pinned host memory).
   void LaunchApplyStep();
   /// With the stream drained: the exact angles of the last step's moved
-  /// frames (the platform libm's WrapAngle, cos and sin), uploaded and
-  /// committed, except for the instances `revert` marks.
+  /// frames (the platform libm's WrapAngle, cos and sin), except for the
+  /// instances `revert` marks, in pinned memory for the next iteration's first
+  /// kernel or FlushCommit to commit.
   void CommitAngles(const std::vector<int32_t>* revert);
   /// Applies committed angles that no iteration has taken over yet.
   void FlushCommit();

@@ -8,15 +8,21 @@
 // (src/solvers/parallel_ldlt.hpp:44-51,150-244; src/solvers/lm_solver.cpp:
 // 352-364) with dense frontal work: every supernode's front is assembled from
 // J^T J (written in place by the column kernels) plus its children's update
-// matrices, its pivot columns are factored in panels of kPanel columns, and
-// the Schur complement of the remaining rows is one rank-k update.
+// matrices and its pivot columns are factored, fronts of few pivots by one
+// kernel in 8-column panels (KFactorFront), wider ones in panels of kPanel
+// columns (KPanel, or KPanelBlock by outer blocks; KUpdate), dense pose roots by
+// tiles (dense_root.cu). The Schur complements of FP64 fronts are pulled by
+// their parents, their pose rows summed straight into the pose root
+// (pose_schur.cu); those of a mixed solve's FP32 fronts are pushed (KSchurF32, or
+// the tensor cores, schur_tc.cu). The solve is one launch (KSolveTree) that
+// multiplies by inverses of the pivot blocks (KInvertFronts, KInvertDiagonal).
 //
-// Storage of a front (column major, leading dimension F = k + m): the lower
-// triangle holds the assembled values, then L below each panel's diagonal
-// block. The strictly lower part of each kPanel x kPanel diagonal block of L
-// is stored transposed in the block's upper triangle, and D in `dvec`
-// (permuted order), so the lower triangle of a diagonal block is never
-// written while other blocks of the same panel still read it.
+// Storage of a front (column major, leading dimension F = k + m, SupernodeRec::
+// fcols columns): the lower triangle holds the assembled values, then L. L of a
+// single-kernel front's pivot block is stored transposed in the pivot block's
+// upper triangle, that of the others within each kPanel x kPanel diagonal block;
+// D in `dvec` (permuted order). So the lower triangle of a diagonal block is
+// never written while other blocks of the same front still read it.
 #include <cuda_runtime.h>
 
 #include "device.cuh"

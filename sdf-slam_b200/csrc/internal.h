@@ -388,11 +388,6 @@ struct Symbolic {
   // front's Schur complement into the parent front
   std::vector<TaskRange> schur_range;
   std::vector<int32_t> schur_base;           // levels + 1 entries
-  // Tensor-core Schur complements of a mixed solve's FP32 fronts with at
-  // least kTcMinRows rows below the pivot block (their SIMT Schur tasks are
-  // skipped then): per level, operand packing tasks (sn, row tile, K chunk)
-  // and output tile tasks (sn, tile i, tile j), i >= j; the packed operand
-  // buffer is reused level after level (tc_pack_rows rows of the widest).
   // Task list of the one-launch solve, in the order blocks take them: the
   // forward tasks of every supernode in level order, then the backward
   // tasks in reverse. (type, sn, part, gate) quads, SolveTask types; gate: a
@@ -419,25 +414,26 @@ struct Symbolic {
   bool solve_handover{false};
   bool solve_panels{false};
   int solve_panel_front{0};
+  // Tensor-core Schur complements of a mixed solve's FP32 fronts with at
+  // least tc_min_rows rows below the pivot block (their SIMT Schur tasks are
+  // skipped then): per level, operand packing tasks (sn, row tile, K chunk)
+  // and output tile tasks (sn, tile i, tile j), i >= j; the packed operand
+  // buffer is reused level after level (tc_pack_rows rows of the widest).
   std::vector<int32_t> pack_tasks;
   std::vector<TaskRange> pack_range;
   std::vector<int32_t> tc_tasks;
   std::vector<TaskRange> tc_range;
   int64_t tc_pack_rows{0};
-  // Dense pose roots (no rows below, more than small_pivots pivots) are
-  // factored by one persistent launch per level over 64 x 64 tiles instead
-  // of panels: (sn, i, j, k + 65536 (len - 1)) task quads (FACTOR i == j == k,
-  // SOLVE j == k < i, UPDATE k < j <= i) in descending bottom level, dense_range per level,
-  // the tile counters (nt x nt per front) and the diagonal-tile inverses
-  // (64 x 64 doubles per tile) they use.
   // (sn, first column) pairs of kZeroCols columns: the fronts' lower
-  // triangles cleared before every assembly. The first zero_main pairs are
-  // what an FP64 assembly needs; the rest are the trailing columns of the
-  // leaf fronts (no child adds into them, and their Schur update reads them
-  // as zero without loading them), cleared only for the tensor-core Schur
-  // complement of a mixed solve, which accumulates into them in place.
+  // triangles cleared before every assembly. The first zero_pivots pairs, the
+  // pivot columns, are what an FP64 assembly needs (KChildSchur writes the
+  // others); up to zero_main come the trailing columns of the fronts with
+  // children, into which a mixed solve's children add; the rest are those of the
+  // leaf fronts (no child adds into them, and their Schur update reads them as
+  // zero without loading them), cleared only for the tensor-core Schur
+  // complement, which accumulates into them in place.
   std::vector<int32_t> zero_tasks;
-  int64_t zero_pivots{0};                    // clearing tasks of pivot columns (the first ones)
+  int64_t zero_pivots{0};
   int64_t zero_main{0};
   // Pose Schur complement: the pose rows of a grid front update pose columns
   // only of the pose root, so their products are summed straight into the
@@ -457,6 +453,12 @@ struct Symbolic {
   int64_t pose_slots{0};
   int32_t pose_counters{0};
   int pose_level{-1};                        // level of the pose roots (-1: none)
+  // Dense pose roots (no rows below, more than small_pivots pivots) are
+  // factored by one persistent launch per level over 64 x 64 tiles instead
+  // of panels: (sn, i, j, k + 65536 (len - 1)) task quads (FACTOR i == j == k,
+  // SOLVE j == k < i, UPDATE k < j <= i) in descending bottom level, dense_range
+  // per level, the tile counters (nt x nt per front) and the diagonal-tile
+  // inverses (64 x 64 doubles per tile) they use.
   std::vector<int32_t> dense_tasks;
   std::vector<TaskRange> dense_range;
   int64_t dense_cnt_words{0};

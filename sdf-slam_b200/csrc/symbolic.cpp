@@ -423,10 +423,9 @@ void ChildTasks(Symbolic& S) {
 }
 
 /// Tasks of the pose Schur complement (see Symbolic::pose_fronts). A tile's
-/// fronts are split so that an instance alone fills the GPU about four
-/// times over (two blocks per SM); the split depends on the instance only, so that its sums are
-/// the same alone and in a batch. Measured on B200 (910-pose office, 946
-/// tiles; 331-pose room, 136 tiles): see KPoseSchur.
+/// fronts are split so that an instance alone makes about 8 x 148 tasks, 2.7
+/// waves of KPoseSchur's three blocks per SM; the split depends on the instance
+/// only, so that its sums are the same alone and in a batch.
 void PoseTasks(Symbolic& S) {
   S.pose_fronts.clear();
   S.pose_mask.clear();
