@@ -232,9 +232,10 @@ __device__ __forceinline__ void MultiplyMatches(Smem<T>& sm, int matches, const 
 
 /// Bound by the FP64 tensor cores and the barriers between stages, three
 /// blocks per SM. A warp owns 16 x 32 entries of the tile. Measured on B200
-/// (910-pose office, 1,672 tasks): 1.31 ms, tensor cores busy 42 %; the same
-/// products on the packed rows with a shared-memory tile took 1.63 ms (the
-/// scatter), warps mapped without the row shuffle 1.43 ms. The whole Schur
+/// (910-pose office, 1,672 tasks): 1.31 ms against 1.63 ms for the same products
+/// on the packed rows with a shared-memory tile (the scatter) and 1.43 ms for
+/// warps mapped without the row shuffle; 1.02 ms in an iteration as it is now
+/// (1,668 tasks), tensor cores busy 42 %. The whole Schur
 /// phase with its parents' updates went from 2.72 to 2.10 ms, clearing the
 /// (now 0.5 instead of 3.5 GB of) fronts from 0.29 to 0.07 ms.
 template <typename T>
